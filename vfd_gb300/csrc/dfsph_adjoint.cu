@@ -1044,12 +1044,13 @@ struct TapeBank {
 struct ShadowKey {
     vfd_desc desc{};
     uint8_t lanes[16] = {}, tiles[16] = {};
+    int8_t halo = -1;
     uint16_t blocks[16] = {};
     uint32_t n = 0, graphs = 0, analytic = 0, cellCap = 0;
     bool operator==(const ShadowKey& o) const {
         return std::memcmp(&desc, &o.desc, sizeof(desc)) == 0 && std::memcmp(lanes, o.lanes, sizeof(lanes)) == 0 &&
                std::memcmp(tiles, o.tiles, sizeof(tiles)) == 0 && std::memcmp(blocks, o.blocks, sizeof(blocks)) == 0 &&
-               n == o.n && graphs == o.graphs && analytic == o.analytic && cellCap == o.cellCap;
+               n == o.n && halo == o.halo && graphs == o.graphs && analytic == o.analytic && cellCap == o.cellCap;
     }
 };
 
@@ -1244,6 +1245,7 @@ ShadowKey shadow_key(const vfd_sim* s) {
     k.desc = s->scenes[0].desc;
     std::memcpy(k.lanes, s->lanes, sizeof(k.lanes));
     std::memcpy(k.tiles, s->tiles, sizeof(k.tiles));
+    k.halo = s->halo;
     std::memcpy(k.blocks, s->blocks, sizeof(k.blocks));
     k.n = s->n;
     k.graphs = s->graphMode && !s->graphFailed ? 1u : 0u;
@@ -1285,8 +1287,9 @@ bool ensure_shadow(vfd_sim* s, AdjointState* A) {
     t->cellCap = s->cellCap;  // the search grid the simulation grew to, so replays do not abort on it
     std::memcpy(t->lanes, s->lanes, sizeof(t->lanes));
     std::memcpy(t->tiles, s->tiles, sizeof(t->tiles));
+    t->halo = s->halo;
     std::memcpy(t->blocks, s->blocks, sizeof(t->blocks));
-    if (ensure_ready(t) != VFD_OK || t->n != s->n || t->stride != s->stride) {
+    if (ensure_ready(t) != VFD_OK || t->n != s->n || t->stride != s->stride || t->dev[0].haloOn != s->dev[0].haloOn) {
         delete t;
         cudaGetLastError();
         return false;

@@ -25,6 +25,7 @@
 #include "../../include/vfd_dfsph.h"
 #include "dfsph_common.cuh"
 
+#include "dfsph_halo.cuh"
 #include "dfsph_sim.h"
 
 namespace vfd {
@@ -276,6 +277,33 @@ int reset_buckets(vfd_sim* s, const Dev& d) {
     return VFD_OK;
 }
 
+// Buffers of the staged-tile passes, for layouts that run on them. Without room for them the
+// row kernels run, as for smaller scenes.
+int allocate_halo(vfd_sim* s, Dev& base) {
+    base.haloOn = 0u;
+    if (s->n < kHaloMinParticles || s->n > kHaloMaxParticles) return VFD_OK;
+    const size_t st = s->stride, cellTiles = s->cellCap / kHaloTileCells + 1u, kept = s->allocs.size();
+    const size_t tiles = std::min(st, cellTiles);
+    int rc = dalloc(s, &base.haloTiles, tiles);
+    if (rc == VFD_OK) rc = dalloc(s, &base.haloInfo, 2);
+    if (rc == VFD_OK) rc = dalloc(s, &base.haloScan, base.scanBlocks + 1);
+    if (rc == VFD_OK) rc = dalloc(s, &base.haloScene, base.nscenes);
+    if (rc == VFD_OK) rc = dalloc(s, &base.haloList, 8 * st);
+    if (rc == VFD_OK) rc = dalloc(s, &base.haloBase, cellTiles * kHaloCells);
+    if (rc != VFD_OK) {
+        cudaGetLastError();
+        for (; s->allocs.size() > kept; s->allocs.pop_back()) cudaFree(s->allocs.back());
+        base.haloTiles = nullptr;
+        return VFD_OK;
+    }
+    static_assert(kHaloRow * (sizeof(float) + sizeof(uint16_t)) == kRow * sizeof(uint2), "the rows share NG's bytes");
+    base.haloGrad = reinterpret_cast<float*>(base.NG);
+    base.haloRow = reinterpret_cast<uint16_t*>(base.haloGrad + st * kHaloRow);
+    CK(prepare_halo_kernels());
+    base.haloOn = s->halo != 0 ? 1u : 0u;
+    return VFD_OK;
+}
+
 int allocate(vfd_sim* s) {
     s->releaseBuffers();
     uint32_t n = 0, maxBodies = 0;
@@ -357,7 +385,7 @@ int allocate(vfd_sim* s) {
     base.analytic = s->analyticKernel ? 1u : 0u;
     base.splK = s->table.K;
     base.splL = s->table.L;
-    base.workStride = 2u + 2u * base.nscenes;
+    base.workStride = 3u + 4u * base.nscenes;
     TRY(dalloc(s, &base.WORK, 3 * (size_t)base.workStride));
     {
         int sms = 0;
@@ -368,6 +396,7 @@ int allocate(vfd_sim* s) {
     std::memcpy(base.blocks, s->blocks, sizeof(base.blocks));
     base.compactRows = uses_tiles(s->tiles) ? 1u : 0u;
     CK(prepare_tile_kernels());
+    TRY(allocate_halo(s, base));
     TRY(dalloc(s, &s->dWM, kTableRes));
     TRY(dalloc(s, &s->dGM, kTableRes));
     TRY(dalloc(s, &s->dHalton, kHaltonCount));
@@ -2022,12 +2051,19 @@ int vfd_profile_kernels(vfd_sim* s, uint32_t steps, vfd_kernel_time* out, uint32
     return VFD_OK;
 }
 
+// Whether the layout's steps run on staged tiles (where it has the buffers for them).
+static void set_halo(vfd_sim* s, int8_t on) {
+    s->halo = on;
+    for (int k = 0; k < 2; k++) s->dev[k].haloOn = on && s->dev[k].haloTiles ? 1u : 0u;
+}
+
 int vfd_set_lanes(vfd_sim* s, const uint8_t* lanes, uint32_t count) {
     TRY(check_sim(s));
     if (!lanes || count == 0 || count > 16) return fail(VFD_E_ARG, "lanes: 1..16 entries");
     for (uint32_t k = 0; k < count; k++)
         if (lanes[k] != 4 && lanes[k] != 8 && lanes[k] != 16) return fail(VFD_E_ARG, "lanes must be 4, 8 or 16");
     std::memcpy(s->lanes, lanes, count);
+    set_halo(s, 0);
     for (int k = 0; k < 2; k++) std::memcpy(s->dev[k].lanes, s->lanes, sizeof(s->lanes));
     s->releaseGraphs();
     return VFD_OK;
@@ -2048,6 +2084,7 @@ int vfd_set_tiles(vfd_sim* s, const uint8_t* tiles, uint32_t count) {
             return fail(VFD_E_ARG, "pass form must be 0 (neighbour rows), 1 (rows, gradW recomputed), 3 (2x2x2 tiles) "
                                    "or 4 (4x2x2 tiles)");
     std::memcpy(s->tiles, tiles, count);
+    set_halo(s, 0);
     for (int k = 0; k < 2; k++) {
         std::memcpy(s->dev[k].tiles, s->tiles, sizeof(s->tiles));
         s->dev[k].compactRows = uses_tiles(s->tiles) ? 1u : 0u;
@@ -2063,6 +2100,7 @@ int vfd_set_blocks(vfd_sim* s, const uint16_t* blocks, uint32_t count) {
         if (blocks[k] != 64 && blocks[k] != 128 && blocks[k] != 256)
             return fail(VFD_E_ARG, "threads per block must be 64, 128 or 256");
     std::memcpy(s->blocks, blocks, count * sizeof(uint16_t));
+    set_halo(s, 0);
     for (int k = 0; k < 2; k++) std::memcpy(s->dev[k].blocks, s->blocks, sizeof(s->blocks));
     s->releaseGraphs();
     return VFD_OK;
@@ -2140,10 +2178,14 @@ int vfd_autotune(vfd_sim* s, uint32_t steps, uint8_t* lanes_out, uint32_t count)
                                                                 // stream, 2x2x2 and 4x2x2 tiles
     const uint16_t blockCand[3] = {128, 64, 256};  // threads per block of the row kernels
     double times[kTunedCount][3][kForms][3] = {};  // [kernel][lanes][form][block]
+    double haloTime = 0.0;  // the same kernels on staged tiles, with the pass that lists them
     int rc = VFD_OK;
-    for (int ct = 0; ct < 3 * kForms * 3 && rc == VFD_OK; ct++) {
-        const int c = ct % 3, tl = (ct / 3) % kForms, bs = ct / (3 * kForms);
+    const bool canHalo = s->dev[0].haloTiles != nullptr;
+    for (int ct = 0; ct < 3 * kForms * 3 + (canHalo ? 1 : 0) && rc == VFD_OK; ct++) {
+        const bool halo = ct == 3 * kForms * 3;
+        const int c = ct % 3, tl = (ct / 3) % kForms, bs = ct / (3 * kForms) % 3;
         for (int k = 0; k < 2; k++) {
+            s->dev[k].haloOn = halo ? 1u : 0u;
             for (int t = 0; t < kTunedCount; t++) {
                 s->dev[k].lanes[t] = cand[c];
                 s->dev[k].tiles[t] = tileCand[tl];
@@ -2164,9 +2206,14 @@ int vfd_autotune(vfd_sim* s, uint32_t steps, uint8_t* lanes_out, uint32_t count)
         }
         for (const auto& rec : prof.recs) {
             float ms = 0.0f;
-            if (rc == VFD_OK && cudaEventElapsedTime(&ms, rec.a, rec.b) == cudaSuccess)
-                for (int t = 0; t < kTunedCount; t++)
-                    if (rec.name == names[t]) times[t][c][tl][bs] += ms;
+            if (rc == VFD_OK && cudaEventElapsedTime(&ms, rec.a, rec.b) == cudaSuccess) {
+                if (halo && rec.name == "k_halo_build") haloTime += ms;
+                for (int t = 0; t < kTunedCount; t++) {
+                    if (rec.name != names[t]) continue;
+                    if (halo) haloTime += ms;
+                    else times[t][c][tl][bs] += ms;
+                }
+            }
         }
         s->cs = cs0;
         e = copy_all(false);
@@ -2180,8 +2227,10 @@ int vfd_autotune(vfd_sim* s, uint32_t steps, uint8_t* lanes_out, uint32_t count)
             std::memcpy(s->dev[k].blocks, s->blocks, sizeof(s->blocks));
             s->dev[k].compactRows = uses_tiles(s->tiles) ? 1u : 0u;
         }
+        set_halo(s, s->halo);
         return rc;
     }
+    double rowTime = 0.0;
     for (int t = 0; t < kTunedCount; t++) {
         const bool tileable = t == kTPAccel || t == kTJacobi || t == kTSpmv;
         // A configuration is (lanes c, form tl, block bs). Kernels without forms ran the same
@@ -2191,7 +2240,7 @@ int vfd_autotune(vfd_sim* s, uint32_t steps, uint8_t* lanes_out, uint32_t count)
             if (tileable) return times[t][c][tl][bs];
             double sum = 0.0;
             for (int f = 0; f < kForms; f++) sum += times[t][c][f][bs];
-            return sum;
+            return sum / kForms;
         };
         int best = 1, bestTile = 0, bestBlock = 0;
         double bt = cost(1, 0, 0);
@@ -2206,6 +2255,7 @@ int vfd_autotune(vfd_sim* s, uint32_t steps, uint8_t* lanes_out, uint32_t count)
                         bestBlock = bs;
                     }
                 }
+        rowTime += bt;
         s->lanes[t] = cand[best];
         s->tiles[t] = tileable ? tileCand[bestTile] : 0;
         s->blocks[t] = tileCand[bestTile] < kTileMinLog2 ? blockCand[bestBlock] : 0;
@@ -2216,6 +2266,7 @@ int vfd_autotune(vfd_sim* s, uint32_t steps, uint8_t* lanes_out, uint32_t count)
         std::memcpy(s->dev[k].blocks, s->blocks, sizeof(s->blocks));
         s->dev[k].compactRows = uses_tiles(s->tiles) ? 1u : 0u;
     }
+    set_halo(s, canHalo && haloTime < rowTime ? 1 : 0);
     s->releaseGraphs();
     if (lanes_out) std::memcpy(lanes_out, s->lanes, std::min<uint32_t>(count, 16));
     return VFD_OK;

@@ -120,6 +120,13 @@ struct BodyDev {
     const uint32_t* cellMap;   // field 0 cell map
 };
 
+// A non-empty tile of the staged-tile passes (dfsph_halo.cu): its first cell, its particles'
+// slots [first, last), its scene, and its halo: `staged` slots from haloList[list] (more than
+// the shared memory holds: not staged).
+struct __align__(16) HaloTile {
+    uint32_t cell0, first, last, scene, staged, list, pad[2];
+};
+
 // Device pointers and sizes of one simulation; one instance per sort parity
 // (cur = state sorted by the previous step, srt = state sorted by this step).
 struct Dev {
@@ -175,9 +182,20 @@ struct Dev {
     // pass runs on tiles, so the search writes the NBRC rows.
     uint8_t tiles[16];
     uint32_t compactRows;
-    // 1: the CG product walks the neighbour rows instead of cell tiles (the adjoint's CG
-    // runs on recorded rows of a past step, whose cell tables are no longer current)
+    // 1: the passes walk the neighbour rows instead of cell tiles (the adjoint's passes run
+    // on recorded rows of a past step, whose cell tables are no longer current)
     uint32_t rowLoops;
+    // Staged-tile passes (dfsph_halo.cu); haloOn: the step's neighbour loops run on them.
+    // The rows and gradient factors take the place of NG, whose bytes they share.
+    uint32_t haloOn;
+    HaloTile* haloTiles;
+    uint32_t* haloInfo;        // [0] tiles, [1] list slots handed out
+    uint32_t* haloScan;        // tiles before each scan block
+    uint2* haloScene;          // per scene: first tile, tiles
+    uint32_t* haloList;        // slots of the tiles' halos (at most 8 a particle)
+    uint16_t* haloBase;        // [tile of cells][kHaloCells] staged place of each halo cell's first particle
+    uint16_t* haloRow;         // [slot][kHaloRow] staged places of the neighbours (halo_place order)
+    float* haloGrad;           // [slot][kHaloRow] their gradient factors, gradW = haloGrad * r
 };
 
 // ---------------------------------------------------------------- float3 math
@@ -189,7 +207,16 @@ __device__ __forceinline__ float3 operator*(float s, float3 a) { return make_flo
 __device__ __forceinline__ float3 operator*(float3 a, float s) { return make_float3(s * a.x, s * a.y, s * a.z); }
 __device__ __forceinline__ float3& operator+=(float3& a, float3 b) { a.x += b.x; a.y += b.y; a.z += b.z; return a; }
 __device__ __forceinline__ float3& operator-=(float3& a, float3 b) { a.x -= b.x; a.y -= b.y; a.z -= b.z; return a; }
-__device__ __forceinline__ float dot3(float3 a, float3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
+// The fused operations are spelled out, because the compiler's choice (which of two products it
+// fuses) differs from kernel to kernel: kernels that form the same term then agree bit for
+// bit, and a batch or a large scene, which run other kernels, follows the same trajectory as a
+// small one.
+__device__ __forceinline__ float dot3(float3 a, float3 b) {
+    return __fmaf_rn(a.z, b.z, __fmaf_rn(a.x, b.x, __fmul_rn(a.y, b.y)));
+}
+__device__ __forceinline__ float3 fma3(float s, float3 a, float3 b) {  // s a + b
+    return make_float3(__fmaf_rn(s, a.x, b.x), __fmaf_rn(s, a.y, b.y), __fmaf_rn(s, a.z, b.z));
+}
 __device__ __forceinline__ float4 f4(float3 a, float w) { return make_float4(a.x, a.y, a.z, w); }
 __device__ __forceinline__ float3 cross3(float3 a, float3 b) {
     return make_float3(a.y * b.z - b.y * a.z, a.z * b.x - b.z * a.x, a.x * b.y - b.x * a.y);
@@ -227,9 +254,7 @@ __device__ __forceinline__ float3 pair_r(const Dev& d, float4 a, float4 b) {
     if (REL) {
         const int3 A = anchor_of(a.w), B = anchor_of(b.w);
         const float L = d.radius;
-        r.x += L * (float)(A.x - B.x);
-        r.y += L * (float)(A.y - B.y);
-        r.z += L * (float)(A.z - B.z);
+        r = fma3(L, make_float3((float)(A.x - B.x), (float)(A.y - B.y), (float)(A.z - B.z)), r);
     }
     return r;
 }
@@ -562,6 +587,9 @@ template <uint32_t G>
 __device__ __forceinline__ float3 group_sum(uint32_t mask, float3 v) {
     return make_float3(group_sum<G>(mask, v.x), group_sum<G>(mask, v.y), group_sum<G>(mask, v.z));
 }
+
+// Whether the step's neighbour loops run on staged tiles.
+__host__ __device__ inline bool halo_on(const Dev& d) { return d.haloOn != 0u && d.rowLoops == 0u; }
 
 // ------------------------------------------------------------ batch work lists
 __device__ __forceinline__ const uint32_t* work_list(const Dev& d, int loop) { return d.WORK + (size_t)loop * d.workStride; }

@@ -21,11 +21,11 @@
 #include <cfloat>
 
 #include "dfsph_common.cuh"
+#include "dfsph_halo.cuh"
+#include "dfsph_passes.cuh"
 #include "dfsph_tiles.cuh"
 
 namespace vfd {
-
-enum LoopId { kLoopDiv = 0, kLoopCG = 1, kLoopPres = 2 };
 
 __device__ __forceinline__ bool aborted_p(const Dev& d) { return is_aborted(d); }
 
@@ -35,47 +35,61 @@ __device__ __forceinline__ void set_condition(const Dev& d, int loop, uint32_t v
 }
 
 // Batches: lists the scenes for which active(s) holds into loop `loop`'s work list
-// (prefix sums of their particle counts by a block-wide scan). One block of 256 threads,
-// called by all of them after the scenes' flags are final.
+// (prefix sums of their particle counts, and of their staged tiles, by a block-wide scan). One
+// block of 256 threads, called by all of them after the scenes' flags are final.
 template <class F>
 __device__ void build_work_list(const Dev& d, int loop, F active) {
-    __shared__ uint32_t scanP[256], scanA[256];
-    __shared__ uint32_t runP, runA;
+    __shared__ uint32_t scanP[256], scanA[256], scanT[256];
+    __shared__ uint32_t runP, runA, runT;
+    const bool halo = halo_on(d);
     uint32_t* w = d.WORK + (size_t)loop * d.workStride;
     uint32_t* pre = w + 2;
     uint32_t* beg = w + 2 + d.nscenes;
-    if (threadIdx.x == 0) runP = runA = 0u;
+    uint32_t* tileN = beg + d.nscenes;
+    uint32_t* tilePre = tileN + 1;
+    uint32_t* tileBeg = tilePre + d.nscenes;
+    if (threadIdx.x == 0) runP = runA = runT = 0u;
     __syncthreads();
     for (uint32_t c = 0; c < d.nscenes; c += blockDim.x) {
         const uint32_t sc = c + threadIdx.x;
         const bool a = sc < d.nscenes && active(sc);
         const uint32_t cnt = a ? d.scenes[sc].count : 0u;
+        const uint2 tiles = a && halo ? d.haloScene[sc] : make_uint2(0u, 0u);
         scanP[threadIdx.x] = cnt;
         scanA[threadIdx.x] = a ? 1u : 0u;
+        scanT[threadIdx.x] = tiles.y;
         __syncthreads();
         for (uint32_t off = 1; off < blockDim.x; off <<= 1) {
             const uint32_t tp = threadIdx.x >= off ? scanP[threadIdx.x - off] : 0u;
             const uint32_t ta = threadIdx.x >= off ? scanA[threadIdx.x - off] : 0u;
+            const uint32_t tt = threadIdx.x >= off ? scanT[threadIdx.x - off] : 0u;
             __syncthreads();
             scanP[threadIdx.x] += tp;
             scanA[threadIdx.x] += ta;
+            scanT[threadIdx.x] += tt;
             __syncthreads();
         }
         if (a) {
             const uint32_t idx = runA + scanA[threadIdx.x] - 1u;
             pre[idx] = runP + scanP[threadIdx.x] - cnt;
             beg[idx] = d.scenes[sc].begin;
+            if (halo) {
+                tilePre[idx] = runT + scanT[threadIdx.x] - tiles.y;
+                tileBeg[idx] = tiles.x;
+            }
         }
         __syncthreads();
         if (threadIdx.x == blockDim.x - 1u) {
             runP += scanP[threadIdx.x];
             runA += scanA[threadIdx.x];
+            runT += scanT[threadIdx.x];
         }
         __syncthreads();
     }
     if (threadIdx.x == 0) {
         w[0] = runP;
         w[1] = runA;
+        *tileN = runT;
     }
 }
 
@@ -114,12 +128,6 @@ __device__ __forceinline__ Nbr neighbors(const Dev& d, uint32_t p) {
 #else
     return Nbr{d.NBR + (size_t)p * kRow, d.NG + (size_t)p * kRow, w & kCountMask, w};
 #endif
-}
-
-// kappa (or kappa_v) of particle p, mirrored into X[p].w for the neighbours' gathers.
-// (Cell-relative positions keep their anchor in X.w; the neighbours then read kappa itself.)
-__device__ __forceinline__ void set_kappa(const Dev& d, uint32_t p, float k) {
-    if (!d.cellRel) reinterpret_cast<float*>(d.X)[4 * (size_t)p + 3] = k;
 }
 
 // Row entries per lane and round of a neighbour loop (other depths measured slower).
@@ -176,30 +184,6 @@ __device__ __forceinline__ void for_neighbors(const Group<G>& grp, const Nbr& nb
     }
 }
 
-// One particle's term of a CG dot product: the FP32 dot of its two vectors (no
-// contraction, x + y then z, as the FP32 oracle forms it); the sum over particles is
-// FP64-accurate (scene_accumulate). FP64 arithmetic runs at a small fraction of the
-// FP32 rate on this GPU, so the per-particle terms stay FP32, as every per-particle sum
-// of the reference does.
-__device__ __forceinline__ float dot_term(float3 a, float3 b) {
-    return __fadd_rn(__fadd_rn(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y)), __fmul_rn(a.z, b.z));
-}
-
-// W and gradW of one pair from one table position (GetW / GetGradientW keep their own
-// range tests: |r|^2 <= R^2 for W, |r| <= R for gradW).
-__device__ __forceinline__ void kernel_wg(const Dev& d, float3 r, float& w, float& gs) {
-    const float r2 = dot3(r, r);
-    const float rl = fast_sqrt(r2);
-    if (d.analytic) {
-        w = r2 <= d.radius2 ? spline_w(d, rl) : 0.0f;
-        gs = rl <= d.radius ? spline_gs(d, rl) : 0.0f;
-        return;
-    }
-    const uint32_t pos = table_pos(d, rl);
-    w = r2 <= d.radius2 ? __ldg(d.WM + pos) : 0.0f;
-    gs = rl <= d.radius ? __ldg(d.GM + pos) : 0.0f;
-}
-
 #define GROUP_PROLOGUE(G)                    \
     const Group<G> grp;                      \
     const uint32_t p = grp.p;                \
@@ -219,8 +203,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_density_factor(Dev d) {
     const float4 xi4 = d.X[p];
     const float3 xi = f3(xi4);
     const Nbr nb = neighbors(d, p);
-    float wsum = 0.0f, g2 = 0.0f, sdiv = 0.0f;
-    float3 gi = make_float3(0.f, 0.f, 0.f);
+    DensitySums s;
     const float V = S.volume;
     const bool div = DIV && S.enableDiv;
     const float3 vi = div ? f3(d.V[p]) : make_float3(0.f, 0.f, 0.f);
@@ -232,49 +215,13 @@ __global__ void __launch_bounds__(kMaxBlock) k_density_factor(Dev d) {
         const float3 vq = div ? f3(d.V[q]) : make_float3(0.f, 0.f, 0.f);
         if (!ok) return;
         __stcs(ngRow + j, make_uint2(q, __float_as_uint(gs)));
-        wsum += w;
-        const float3 gj = (-V * gs) * r;
-        g2 += dot3(gj, gj);
-        gi -= gj;
-        if (div) sdiv += dot3(vi - vq, gs * r);
+        s.add(V, w, gs, r, div, vi - vq);
     });
-    wsum = grp.sum(wsum);
-    g2 = grp.sum(g2);
-    gi = grp.sum(gi);
-    if (DIV) sdiv = grp.sum(sdiv);
-    if (grp.lane != 0) return;
-    float rhoB = 0.0f;
-    float3 gb = make_float3(0.f, 0.f, 0.f);
-    if (nb.flags & kHasBoundary) {
-        for (uint32_t b = 0; b < S.bodyCount; b++) {
-            const float4 xb = d.XB[(size_t)b * d.stride + p];
-            if (xb.w > 0.0f) {
-                const float3 r = xi - f3(xb);
-                float w, gs;
-                kernel_wg(d, r, w, gs);
-                rhoB += xb.w * w;
-                gb += (xb.w * gs) * r;
-            }
-        }
-    }
-    gi += gb;
-    d.RHO[p] = (V * d.wZero + V * wsum + rhoB) * S.rho0;
-    g2 += dot3(gi, gi);
-    const float alpha = g2 > kEps ? 1.0f / g2 : 0.0f;
-    d.GB[p] = f4(gb, 0.0f);
-    if (!div) {
-        d.ALPHA[p] = alpha;
-        return;
-    }
-    // K4 (:498-528)
-    float rhoAdv = sdiv * V;
-    if (nb.flags & kHasBoundary) rhoAdv += dot3(vi, gb);
-    rhoAdv = nb.count < 20u ? 0.0f : fmaxf(rhoAdv, 0.0f);
-    d.RHOADV[p] = rhoAdv;
-    const float alphaDt = alpha * S.dtInv;
-    d.ALPHA[p] = alphaDt;
-    d.KAPPAV[p] = rhoAdv * alphaDt;
-    set_kappa(d, p, rhoAdv * alphaDt);
+    s.w = grp.sum(s.w);
+    s.g2 = grp.sum(s.g2);
+    s.gi = grp.sum(s.gi);
+    if (DIV) s.div = grp.sum(s.div);
+    if (grp.lane == 0) density_finish(d, p, S, xi, vi, div, s, nb.flags);
 }
 
 // Sum_j (vi - vj) . gradW_ij * V + vi . GB  (K4 :498-522, K17 :253-271); valid on lane 0.
@@ -310,7 +257,7 @@ __device__ __forceinline__ float3 pressure_accel(const Dev& d, const Group<G>& g
         const float sum = ki + (REL ? kap[q] : xq.w);
         const float3 r = pair_r<REL>(d, xi, xq);
         const float gs = NS ? grad_factor(d, r) : gsStream;
-        if (ok && fabsf(sum) > kEps) a += (sum * (-V * gs)) * r;
+        add_pressure(a, sum, V, gs, r, ok);
     });
     a = grp.sum(a);
     if (fabsf(ki) > kEps && (nb.flags & kHasBoundary)) a += ki * (-f3(d.GB[p]));
@@ -351,7 +298,6 @@ __global__ void __launch_bounds__(kMaxBlock) k_pressure_accel_b(Dev d) {
 // each with ComputeDensityPressureForce (:280-315) and the FP64-accurate residual sum.
 template <bool DIV, uint32_t G, bool REL, bool NS = false>
 __device__ __forceinline__ float jacobi_item(const Dev& d, const Group<G>& grp, uint32_t p, const SceneDev& S) {
-    float res = 0.0f;
     const Nbr nb = neighbors(d, p);
     const float4 xi = d.X[p];
     const float3 ai = f3(d.AP[p]);
@@ -363,27 +309,8 @@ __device__ __forceinline__ float jacobi_item(const Dev& d, const Group<G>& grp, 
         const float t = dot3(ai - aq, gs * r);
         if (ok) f += t;
     });
-    f = grp.sum(f) * S.volume;
-    if (grp.lane == 0) {
-        if (nb.flags & kHasBoundary) f += dot3(ai, f3(d.GB[p]));
-        float r;
-        if (DIV) {
-            f *= S.dt;
-            r = nb.count < 20u ? 0.0f : fminf(-d.RHOADV[p] - f, 0.0f);
-            const float k = d.KAPPAV[p] - r * d.ALPHA[p];
-            d.KAPPAV[p] = k;
-            set_kappa(d, p, k);
-        } else {
-            f *= S.dt2;
-            r = fminf(1.0f - d.RHOADV[p] - f, 0.0f);
-            const float k = d.KAPPA[p] - r * d.ALPHA[p];
-            d.KAPPA[p] = k;
-            set_kappa(d, p, k);
-        }
-        d.RES[p] = r;
-        res = r;
-    }
-    return res;
+    f = grp.sum(f);
+    return grp.lane == 0 ? jacobi_finish<DIV>(d, p, S, ai, f, nb.flags) : 0.0f;
 }
 
 template <bool DIV, uint32_t G, bool REL, bool NS = false>
@@ -509,12 +436,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_div_finish(Dev d) {
     if (S.enableDiv) {
         const Nbr nb = neighbors(d, p);
         const float3 a = pressure_accel<true, G, REL>(d, grp, p, S, nb);
-        if (grp.lane == 0) {
-            d.AP[p] = f4(a, 0.0f);
-            const float4 v = d.V[p];
-            d.V[p] = f4(f3(v) + S.dt * a, v.w);
-            d.ALPHA[p] *= S.dt;
-        }
+        if (grp.lane == 0) div_finish_item(d, p, S, a);
     }
     if (grp.lane == 0) d.A[p] = make_float4(S.g[0], S.g[1], S.g[2], 0.0f);
 }
@@ -531,49 +453,8 @@ __global__ void __launch_bounds__(kMaxBlock) k_st_classify(Dev d) {
     if (!S.enableST) return;
     const Nbr nb = neighbors(d, p);
     const float4 xi = d.X[p];
-    if (nb.count == 0) {
-        if (grp.lane == 0) d.STN[p] = make_float4(0.f, 0.f, 0.f, 1.0f / S.h);
-        return;
-    }
-    float3 com = make_float3(0.f, 0.f, 0.f);
-    for (uint32_t j = grp.lane; j < nb.count; j += G) com += pair_r<REL>(d, d.X[nb[j]], xi);
-    com = grp.sum(com);
-    com = make_float3(com.x / S.h, com.y / S.h, com.z / S.h);
-    const float input = sqrtf(dot3(com, com)) / (float)nb.count;
-    float3 nsum = make_float3(0.f, 0.f, 0.f);
-    float curv = 0.0f;
-    if ((float)nb.count <= S.slope * input + S.constant + 0.0f) {
-        const uint32_t samples = S.stSamples;
-        const uint32_t s0 = d.PID[p] * samples / 3u * 3u;
-        const float ratio = S.nbrRadius / S.r;
-        const float lim = ratio * ratio * S.h2;
-        uint32_t count = 0;
-        for (uint32_t k = grp.lane; k < samples; k += G) {
-            const uint32_t i3 = s0 + 3u * k;
-            const float3 pt = S.h * make_float3(__ldg(d.halton + i3 % kHaltonCount),
-                                                __ldg(d.halton + (i3 + 1u) % kHaltonCount),
-                                                __ldg(d.halton + (i3 + 2u) % kHaltonCount));
-            bool covered = false;
-            for (uint32_t j = 0; j < nb.count; j++) {
-                const float3 v = pt - pair_r<REL>(d, d.X[nb[j]], xi);
-                if (dot3(v, v) <= lim) { covered = true; break; }
-            }
-            if (!covered) { nsum += pt; count++; }
-        }
-        nsum = grp.sum(nsum);
-        count = grp.sum(count);
-        if (count > 0) {
-            if (dot3(nsum, nsum) > 0.0f) nsum = normalize3(nsum);
-            curv = 1.0f / S.h * -2.0f * sqrtf(1.0f - S.nbrRadius * S.nbrRadius / (S.r * S.r)) *
-                   cosf(acosf(1.0f - 2.0f * ((float)count / (float)samples)) + S.mcFactor);
-        } else {
-            nsum = make_float3(0.f, 0.f, 0.f);
-        }
-    }
-    if (grp.lane == 0) d.STN[p] = f4(nsum, curv);
+    st_classify_item<G>(d, grp, p, S, nb.count, [&](uint32_t j) { return pair_r<REL>(d, d.X[nb[j]], xi); });
 }
-
-__device__ __forceinline__ bool nonzero3(float4 a) { return a.x != 0.0f || a.y != 0.0f || a.z != 0.0f; }
 
 // K10: ComputeSurfaceTensionNormalsAndCurvatureKernel (:960-1006).
 template <uint32_t G, bool REL>
@@ -602,11 +483,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_st_smooth(Dev d) {
     cc = grp.sum(cc);
     cf = grp.sum(cf);
     if (grp.lane != 0) return;
-    if (dot3(nc, nc) > 0.0f) nc = normalize3(nc);
-    const float sf = S.smoothing;
-    float3 ns = (1.0f - sf) * f3(ni) + sf * nc;
-    if (dot3(ns, ns) > 0.0f) ns = normalize3(ns);
-    d.STNS[p] = f4(ns, ((1.0f - sf) * ni.w + sf * cc) / (1.0f - sf + sf * cf));
+    st_smooth_finish(d, p, S, ni, nc, cc, cf);
 }
 
 // K11: ComputeSurfaceTensionBlendingKernel (:1008-1046), pass `pass` of SurfaceTensionSmoothPassCount.
@@ -631,42 +508,6 @@ __global__ void __launch_bounds__(kBlock) k_st_blend(Dev d, uint32_t pass) {
 
 // ---------------------------------------------------------------------------
 // Viscosity (Weiler 2018 implicit, block-Jacobi PCG), DFSPHImplementation.cu:577-808.
-struct Mat3 {
-    float3 r0, r1, r2;
-};
-__device__ __forceinline__ float3 mul(const Mat3& m, float3 v) {
-    return make_float3(dot3(m.r0, v), dot3(m.r1, v), dot3(m.r2, v));
-}
-__device__ __forceinline__ void add_outer(Mat3& m, float c, float3 a, float3 b) {  // m += c a b^T
-    m.r0 += (c * a.x) * b;
-    m.r1 += (c * a.y) * b;
-    m.r2 += (c * a.z) * b;
-}
-__device__ __forceinline__ Mat3 load_mat(const float4* M, size_t stride, uint32_t p) {
-    Mat3 m;
-    m.r0 = f3(M[p]);
-    m.r1 = f3(M[stride + p]);
-    m.r2 = f3(M[2 * stride + p]);
-    return m;
-}
-__device__ __forceinline__ void store_mat(float4* M, size_t stride, uint32_t p, const Mat3& m) {
-    M[p] = f4(m.r0, 0.f);
-    M[stride + p] = f4(m.r1, 0.f);
-    M[2 * stride + p] = f4(m.r2, 0.f);
-}
-__device__ __forceinline__ Mat3 inverse3(const Mat3& a) {  // cofactors / determinant
-    const float c00 = a.r1.y * a.r2.z - a.r1.z * a.r2.y;
-    const float c01 = a.r1.z * a.r2.x - a.r1.x * a.r2.z;
-    const float c02 = a.r1.x * a.r2.y - a.r1.y * a.r2.x;
-    const float det = a.r0.x * c00 + a.r0.y * c01 + a.r0.z * c02;
-    const float id = 1.0f / det;
-    Mat3 r;
-    r.r0 = make_float3(c00 * id, (a.r0.z * a.r2.y - a.r0.y * a.r2.z) * id, (a.r0.y * a.r1.z - a.r0.z * a.r1.y) * id);
-    r.r1 = make_float3(c01 * id, (a.r0.x * a.r2.z - a.r0.z * a.r2.x) * id, (a.r0.z * a.r1.x - a.r0.x * a.r1.z) * id);
-    r.r2 = make_float3(c02 * id, (a.r0.y * a.r2.x - a.r0.x * a.r2.y) * id, (a.r0.x * a.r1.y - a.r0.y * a.r1.x) * id);
-    return r;
-}
-
 // K12 ComputeViscosityPreconditionerKernel (:604-684) + K13 ComputeViscosityGradientKernel
 // (:686-756, whose boundary term dots a zero vector: b = v) + the boundary matrix BV of
 // the SpMV's boundary term (:793-839): BV p_i = sum_k c_k (p_i . d_k) gradW_k.
@@ -694,51 +535,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_visc_precond(Dev d) {
     m.r0 = grp.sum(m.r0);
     m.r1 = grp.sum(m.r1);
     m.r2 = grp.sum(m.r2);
-    if (grp.lane != 0) return;
-    Mat3 bv = {make_float3(0.f, 0.f, 0.f), make_float3(0.f, 0.f, 0.f), make_float3(0.f, 0.f, 0.f)};
-    bool hasBV = false;
-    if (S.dynBVisc != 0.0f && (nb.flags & kHasBoundary)) {
-        for (uint32_t b = 0; b < S.bodyCount; b++) {
-            const float4 xb4 = d.XB[(size_t)b * d.stride + p];
-            if (!(xb4.w > 0.0f)) continue;
-            const float3 xb = f3(xb4);
-            float3 normal = -(xi - xb);
-            const float nl = sqrtf(dot3(normal, normal));
-            if (!(nl > 0.0001f)) continue;
-            normal = make_float3(normal.x / nl, normal.y / nl, normal.z / nl);
-            float3 t1, t2;
-            orthogonal_vectors(normal, t1, t2);
-            const float td = S.tangDist;
-            const float3 pos[4] = {xb - t1 * td, xb + t1 * td, xb - t2 * td, xb + t2 * td};
-            const float vol = 0.25f * xb4.w;
-            const float3 d1 = xi - pos[0];
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const float3 dk = xi - pos[k];
-                const float3 gk = kernel_grad(d, dk);
-                const float c = 10.0f * S.dynBVisc * vol / (dot3(dk, dk) + eps2);
-                add_outer(m, c, d1, gk);  // positionDirection1 in all four terms (:674-677)
-                add_outer(bv, c, gk, dk);
-            }
-            hasBV = true;
-        }
-    }
-    const float rho = d.RHO[p];
-    const float f = S.dt / rho;
-    Mat3 a;
-    a.r0 = make_float3(1.0f - f * m.r0.x, -f * m.r0.y, -f * m.r0.z);
-    a.r1 = make_float3(-f * m.r1.x, 1.0f - f * m.r1.y, -f * m.r1.z);
-    a.r2 = make_float3(-f * m.r2.x, -f * m.r2.y, 1.0f - f * m.r2.z);
-    store_mat(d.MINV, d.stride, p, inverse3(a));
-    if (hasBV) {
-        store_mat(d.BVM, d.stride, p, bv);
-        d.NCNT[p] = nb.flags | kHasBoundaryVisc;
-    } else if (nb.flags & kHasBoundaryVisc) {
-        d.NCNT[p] = nb.flags & ~kHasBoundaryVisc;
-    }
-    const float4 v = d.V[p];
-    d.CB[p] = v;
-    d.CG[p] = f4(f3(v) + f3(d.DV[p]), S.mass / rho);
+    if (grp.lane == 0) precond_finish(d, p, S, xi, m, nb.flags);
 }
 
 // ComputeMatrixVecProdFunctionKernel (:758-842): (A x)_i with vec[q].w = m / rho_q; lane 0.
@@ -754,14 +551,10 @@ __device__ __forceinline__ float3 visc_matvec(const Dev& d, const Group<G>& grp,
     for_neighbors<G, !NS>(grp, nb, p, [&](uint32_t q, float gsStream, uint32_t, bool ok) {
         const float3 r = pair_r<REL>(d, xi, d.X[q]);
         const float4 vq = vec[q];
-        const float r2 = dot3(r, r);
         const float gs = NS ? grad_factor(d, r) : gsStream;
-        const float3 t = (__fdividef(cmu * vq.w * dot3(vi - f3(vq), r), r2 + eps2) * gs) * r;
-        if (ok) acc += t;
+        add_viscous(acc, cmu * vq.w, vi - f3(vq), eps2, gs, r, ok);
     });
-    acc = grp.sum(acc);
-    if (nb.flags & kHasBoundaryVisc) acc += mul(load_mat(d.BVM, d.stride, p), vi);
-    return vi - (S.dt / d.RHO[p]) * acc;
+    return visc_product(d, p, S, vi, grp.sum(acc), nb.flags);
 }
 
 // Initial residual r = b - A g and the norms |b|^2, |r|^2 (:627-669).
@@ -1166,13 +959,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_pres_init(Dev d) {
     const Nbr nb = neighbors(d, p);
     const float delta = velocity_divergence<G, REL>(d, grp, p, S, nb, d.X[p], f3(d.V[p]));
     if (grp.lane != 0) return;
-    const float rhoAdv = d.RHO[p] / S.rho0 + S.dt * delta;
-    d.RHOADV[p] = rhoAdv;
-    const float alpha = d.ALPHA[p] * S.dt2Inv;
-    d.ALPHA[p] = alpha;
-    const float k = -fminf(1.0f - rhoAdv, 0.0f) * alpha;
-    d.KAPPA[p] = k;
-    set_kappa(d, p, k);
+    pres_init_finish(d, p, S, delta);
 }
 
 // K20 ComputePressureAccelerationAndVelocityKernel (:434-481) + K21 ComputePositionKernel (:54-67);
@@ -1185,25 +972,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_pres_finish(Dev d) {
     const Nbr nb = neighbors(d, p);
     const float3 a = pressure_accel<false, G, REL>(d, grp, p, S, nb);
     if (grp.lane != 0) return;
-    d.AP[p] = f4(a, 0.0f);
-    const float3 v = f3(d.V[p]) + S.dt * a;
-    d.V[p] = f4(v, 0.0f);
-    const float4 x4 = d.X[p];
-    float3 x = f3(x4) + S.dt * v;
-    if (!(isfinite(x.x) && isfinite(x.y) && isfinite(x.z))) atomicOr(d.status, 0x10u);
-    if (d.cellRel) {  // back into [0, h) of a (possibly new) anchor cell
-        const float L = d.radius;
-        int3 A = anchor_of(x4.w);
-        const float fx = floorf(x.x / L), fy = floorf(x.y / L), fz = floorf(x.z / L);
-        if (isfinite(x.x) && isfinite(x.y) && isfinite(x.z)) {
-            A = make_int3(A.x + (int)fx, A.y + (int)fy, A.z + (int)fz);
-            x = make_float3(x.x - fx * L, x.y - fy * L, x.z - fz * L);
-            if (abs(A.x) > 511 || abs(A.y) > 511 || abs(A.z) > 511) atomicOr(d.status, 0x40u);
-        }
-        d.XN[p] = f4(x, anchor_pack(A));
-    } else {
-        d.XN[p] = f4(x, 0.0f);
-    }
+    pres_finish_item(d, p, S, a);
 }
 
 // End of step: frame clock and iteration counter (DFSPHImplementation.cu:148-169);
@@ -1230,123 +999,6 @@ __global__ void k_ctrl_end(Dev d) {
 // The solver-loop passes as cell-tile kernels (dfsph_tiles.cuh). Each Op states one
 // pass's pair term and epilogue; the tile loop walks the neighbours (shared-memory halo
 // and masks, or the row for kRowPath particles) and sums the terms over the group.
-
-// K5 DivergenceSolveIterationKernel's force part / K18 (:388-432, :342-386): pressure
-// acceleration a_p = -V sum_j (k_i + k_j) gradW_ij - k_i GB_i (kappa in X.w, or staged
-// with cell-relative positions).
-template <bool DIV, bool REL>
-struct PressureAccelOp {
-    static constexpr bool kField = REL;
-    static constexpr bool kReduce = false;
-    static constexpr int kSlot = 0;
-    struct Own {
-        float4 xi;
-        float ki, V;
-    };
-    using Acc = float3;
-    __device__ static bool active(const SceneDev& S) { return (DIV ? S.div.active : S.pres.active) != 0u; }
-    __device__ static float4 field(const Dev& d, uint32_t q) {
-        return make_float4((DIV ? d.KAPPAV : d.KAPPA)[q], 0.f, 0.f, 0.f);
-    }
-    __device__ static void load(const Dev& d, uint32_t p, const SceneDev& S, Own& o) {
-        o.xi = d.X[p];
-        o.ki = (DIV ? d.KAPPAV : d.KAPPA)[p];
-        o.V = S.volume;
-    }
-    __device__ static void pair(const Dev& d, const Own& o, float4 xq, float4 fq, Acc& a) {
-        const float sum = o.ki + (REL ? fq.x : xq.w);
-        const float3 r = pair_r<REL>(d, o.xi, xq);
-        const float gs = grad_factor(d, r);
-        if (fabsf(sum) > kEps) a += (sum * (-o.V * gs)) * r;
-    }
-    __device__ static float finish(const Dev& d, uint32_t p, const SceneDev&, const Own& o, Acc a, uint32_t ncnt) {
-        if (fabsf(o.ki) > kEps && (ncnt & kHasBoundary)) a += o.ki * (-f3(d.GB[p]));
-        d.AP[p] = f4(a, 0.0f);
-        return 0.0f;
-    }
-};
-
-// K6 DivergenceSolveIterationKernel (:531-553) / K19 PressureSolveIterationKernel
-// (:317-340), each with ComputeDensityPressureForce (:280-315): the density change of
-// the pressure accelerations, the clamped residual, the kappa update, and the residual
-// into the FP64-accurate sum.
-template <bool DIV, bool REL>
-struct JacobiOp {
-    static constexpr bool kField = true;
-    static constexpr bool kReduce = true;
-    static constexpr int kSlot = 0;
-    struct Own {
-        float4 xi;
-        float3 ai;
-    };
-    using Acc = float;
-    __device__ static bool active(const SceneDev& S) { return (DIV ? S.div.active : S.pres.active) != 0u; }
-    __device__ static float4 field(const Dev& d, uint32_t q) { return d.AP[q]; }
-    __device__ static void load(const Dev& d, uint32_t p, const SceneDev&, Own& o) {
-        o.xi = d.X[p];
-        o.ai = f3(d.AP[p]);
-    }
-    __device__ static void pair(const Dev& d, const Own& o, float4 xq, float4 aq, Acc& f) {
-        const float3 r = pair_r<REL>(d, o.xi, xq);
-        const float gs = grad_factor(d, r);
-        f += dot3(o.ai - f3(aq), gs * r);
-    }
-    __device__ static float finish(const Dev& d, uint32_t p, const SceneDev& S, const Own& o, Acc f, uint32_t ncnt) {
-        f *= S.volume;
-        if (ncnt & kHasBoundary) f += dot3(o.ai, f3(d.GB[p]));
-        float r;
-        if (DIV) {
-            f *= S.dt;
-            r = (ncnt & kCountMask) < 20u ? 0.0f : fminf(-d.RHOADV[p] - f, 0.0f);
-            const float k = d.KAPPAV[p] - r * d.ALPHA[p];
-            d.KAPPAV[p] = k;
-            set_kappa(d, p, k);
-        } else {
-            f *= S.dt2;
-            r = fminf(1.0f - d.RHOADV[p] - f, 0.0f);
-            const float k = d.KAPPA[p] - r * d.ALPHA[p];
-            d.KAPPA[p] = k;
-            set_kappa(d, p, k);
-        }
-        d.RES[p] = r;
-        return r;
-    }
-};
-
-// ComputeMatrixVecProdFunctionKernel (:758-842) on the CG direction p (p.w = m / rho) and
-// the p . Ap term of the step length (:695-720).
-template <bool REL>
-struct SpmvOp {
-    static constexpr bool kField = true;
-    static constexpr bool kReduce = true;
-    static constexpr int kSlot = 0;
-    struct Own {
-        float4 xi;
-        float3 vi;
-        float cmu, eps2;
-    };
-    using Acc = float3;
-    __device__ static bool active(const SceneDev& S) { return S.cgActive != 0u; }
-    __device__ static float4 field(const Dev& d, uint32_t q) { return d.CP[q]; }
-    __device__ static void load(const Dev& d, uint32_t p, const SceneDev& S, Own& o) {
-        o.xi = d.X[p];
-        o.vi = f3(d.CP[p]);
-        o.cmu = 10.0f * S.dynVisc;
-        o.eps2 = 0.01f * S.h2;
-    }
-    __device__ static void pair(const Dev& d, const Own& o, float4 xq, float4 vq, Acc& acc) {
-        const float3 r = pair_r<REL>(d, o.xi, xq);
-        const float r2 = dot3(r, r);
-        const float gs = grad_factor_r2(d, r2);
-        acc += (__fdividef(o.cmu * vq.w * dot3(o.vi - f3(vq), r), r2 + o.eps2) * gs) * r;
-    }
-    __device__ static float finish(const Dev& d, uint32_t p, const SceneDev& S, const Own& o, Acc acc, uint32_t ncnt) {
-        if (ncnt & kHasBoundaryVisc) acc += mul(load_mat(d.BVM, d.stride, p), o.vi);
-        const float3 ap = o.vi - (S.dt / d.RHO[p]) * acc;
-        d.CAP[p] = f4(ap, 0.0f);
-        return dot_term(o.vi, ap);
-    }
-};
 
 // The tile kernels, one name per pass for profilers.
 template <bool DIV, uint32_t L, uint32_t G, bool REL>
@@ -1506,7 +1158,8 @@ cudaError_t prepare_tile_kernels() {
 void launch_density(const Dev& d, cudaStream_t s) { VFD_LAUNCH_MODE(VFD_LAUNCH_LANES, "k_density_factor", kTDensity, K_DENSITY); }
 // K2 + K3 + K4 in one pass, then the divergence loop's start.
 void launch_density_div_init(const Dev& d, cudaStream_t s) {
-    VFD_LAUNCH_MODE(VFD_LAUNCH_LANES, "k_density_factor", kTDensity, K_DENSITY_DIV);
+    if (halo_on(d)) launch_halo_pass(d, kHaloDensity, s);
+    else VFD_LAUNCH_MODE(VFD_LAUNCH_LANES, "k_density_factor", kTDensity, K_DENSITY_DIV);
     VFD_LAUNCH("k_ctrl_jacobi_init", s, k_ctrl_jacobi_init<true><<<1, 256, 0, s>>>(d));
 }
 #define K_PACCEL_DB(G) k_pressure_accel_b<true, G, false>
@@ -1532,6 +1185,12 @@ inline bool no_stream(const Dev& d, int id) { return d.tiles[id] == kRowsNoStrea
 // iterating) with a fixed grid; a single scene keeps one group per particle. Tile path:
 // single scenes and batches alike (tiles of scenes that stopped iterating are skipped).
 void launch_div_iter(const Dev& d, cudaStream_t s) {
+    if (halo_on(d)) {
+        launch_halo_pass(d, kHaloPAccelD, s);
+        launch_halo_pass(d, kHaloJacobiD, s);
+        VFD_LAUNCH("k_ctrl_jacobi", s, k_ctrl_jacobi<true><<<1, 256, 0, s>>>(d));
+        return;
+    }
     if (tiled(d, kTPAccel)) VFD_TILE_DISPATCH("k_pressure_accel", kTPAccel, FN_PACC_D, OP_PACC_D);
     else if (d.nscenes > 1) VFD_LAUNCH_MODE(VFD_LAUNCH_LANES_BATCH, "k_pressure_accel", kTPAccel, K_PACCEL_DB);
     else if (no_stream(d, kTPAccel)) VFD_LAUNCH_MODE(VFD_LAUNCH_LANES, "k_pressure_accel", kTPAccel, K_PACCEL_D_NS);
@@ -1542,22 +1201,36 @@ void launch_div_iter(const Dev& d, cudaStream_t s) {
     else VFD_LAUNCH_MODE(VFD_LAUNCH_LANES, "k_jacobi_iter", kTJacobi, K_JACOBI_D);
     VFD_LAUNCH("k_ctrl_jacobi", s, k_ctrl_jacobi<true><<<1, 256, 0, s>>>(d));
 }
-void launch_div_finish(const Dev& d, cudaStream_t s) { VFD_LAUNCH_MODE(VFD_LAUNCH_LANES, "k_div_finish", kTDivFinish, K_DIV_FINISH); }
+void launch_div_finish(const Dev& d, cudaStream_t s) {
+    if (halo_on(d)) launch_halo_pass(d, kHaloDivFinish, s);
+    else VFD_LAUNCH_MODE(VFD_LAUNCH_LANES, "k_div_finish", kTDivFinish, K_DIV_FINISH);
+}
 void launch_surface_tension(const Dev& d, uint32_t maxPasses, cudaStream_t s) {
-    VFD_LAUNCH_MODE(VFD_LAUNCH_LANES, "k_st_classify", kTStClassify, K_ST_CLASSIFY);
-    VFD_LAUNCH_MODE(VFD_LAUNCH_LANES, "k_st_smooth", kTStSmooth, K_ST_SMOOTH);
+    if (halo_on(d)) {
+        launch_halo_pass(d, kHaloClassify, s);
+        launch_halo_pass(d, kHaloSmooth, s);
+    } else {
+        VFD_LAUNCH_MODE(VFD_LAUNCH_LANES, "k_st_classify", kTStClassify, K_ST_CLASSIFY);
+        VFD_LAUNCH_MODE(VFD_LAUNCH_LANES, "k_st_smooth", kTStSmooth, K_ST_SMOOTH);
+    }
     for (uint32_t pass = 0; pass < maxPasses; pass++)
         VFD_LAUNCH("k_st_blend", s, k_st_blend<<<blocks_for(d.n), kBlock, 0, s>>>(d, pass));
 }
 void launch_visc_init(const Dev& d, cudaStream_t s) {
-    VFD_LAUNCH_MODE(VFD_LAUNCH_LANES, "k_visc_precond", kTViscPrecond, K_VISC_PRECOND);
-    VFD_LAUNCH_MODE(VFD_LAUNCH_LANES, "k_visc_setup", kTViscSetup, K_VISC_SETUP);
+    if (halo_on(d)) {
+        launch_halo_pass(d, kHaloPrecond, s);
+        launch_halo_pass(d, kHaloSetup, s);
+    } else {
+        VFD_LAUNCH_MODE(VFD_LAUNCH_LANES, "k_visc_precond", kTViscPrecond, K_VISC_PRECOND);
+        VFD_LAUNCH_MODE(VFD_LAUNCH_LANES, "k_visc_setup", kTViscSetup, K_VISC_SETUP);
+    }
     VFD_LAUNCH("k_ctrl_cg0", s, k_ctrl_cg0<<<1, 256, 0, s>>>(d));
     VFD_LAUNCH("k_cg_p0", s, k_cg_p0<<<blocks_for(d.n), kBlock, 0, s>>>(d));
     VFD_LAUNCH("k_ctrl_cg1", s, k_ctrl_cg1<<<1, 256, 0, s>>>(d));
 }
 void launch_cg_iter(const Dev& d, cudaStream_t s) {
-    if (tiled(d, kTSpmv)) VFD_TILE_DISPATCH("k_cg_spmv", kTSpmv, FN_SPMV, OP_SPMV);
+    if (halo_on(d)) launch_halo_pass(d, kHaloSpmv, s);
+    else if (tiled(d, kTSpmv)) VFD_TILE_DISPATCH("k_cg_spmv", kTSpmv, FN_SPMV, OP_SPMV);
     else if (d.nscenes > 1) VFD_LAUNCH_MODE(VFD_LAUNCH_LANES_BATCH, "k_cg_spmv", kTSpmv, K_SPMV_B);
     else if (no_stream(d, kTSpmv)) VFD_LAUNCH_MODE(VFD_LAUNCH_LANES, "k_cg_spmv", kTSpmv, K_SPMV_NS);
     else VFD_LAUNCH_MODE(VFD_LAUNCH_LANES, "k_cg_spmv", kTSpmv, K_SPMV);
@@ -1584,10 +1257,17 @@ void launch_visc_finish_dt(const Dev& d, cudaStream_t s) {
     VFD_LAUNCH("k_velocity", s, k_velocity<<<blocks_for(d.n), kBlock, 0, s>>>(d));
 }
 void launch_pres_init(const Dev& d, cudaStream_t s) {
-    VFD_LAUNCH_MODE(VFD_LAUNCH_LANES, "k_pres_init", kTPresInit, K_PRES_INIT);
+    if (halo_on(d)) launch_halo_pass(d, kHaloPresInit, s);
+    else VFD_LAUNCH_MODE(VFD_LAUNCH_LANES, "k_pres_init", kTPresInit, K_PRES_INIT);
     VFD_LAUNCH("k_ctrl_jacobi_init", s, k_ctrl_jacobi_init<false><<<1, 256, 0, s>>>(d));
 }
 void launch_pres_iter(const Dev& d, cudaStream_t s) {
+    if (halo_on(d)) {
+        launch_halo_pass(d, kHaloPAccelP, s);
+        launch_halo_pass(d, kHaloJacobiP, s);
+        VFD_LAUNCH("k_ctrl_jacobi", s, k_ctrl_jacobi<false><<<1, 256, 0, s>>>(d));
+        return;
+    }
     if (tiled(d, kTPAccel)) VFD_TILE_DISPATCH("k_pressure_accel", kTPAccel, FN_PACC_P, OP_PACC_P);
     else if (d.nscenes > 1) VFD_LAUNCH_MODE(VFD_LAUNCH_LANES_BATCH, "k_pressure_accel", kTPAccel, K_PACCEL_PB);
     else if (no_stream(d, kTPAccel)) VFD_LAUNCH_MODE(VFD_LAUNCH_LANES, "k_pressure_accel", kTPAccel, K_PACCEL_P_NS);
@@ -1599,7 +1279,8 @@ void launch_pres_iter(const Dev& d, cudaStream_t s) {
     VFD_LAUNCH("k_ctrl_jacobi", s, k_ctrl_jacobi<false><<<1, 256, 0, s>>>(d));
 }
 void launch_pres_finish(const Dev& d, cudaStream_t s) {
-    VFD_LAUNCH_MODE(VFD_LAUNCH_LANES, "k_pres_finish", kTPresFinish, K_PRES_FINISH);
+    if (halo_on(d)) launch_halo_pass(d, kHaloPresFinish, s);
+    else VFD_LAUNCH_MODE(VFD_LAUNCH_LANES, "k_pres_finish", kTPresFinish, K_PRES_FINISH);
     VFD_LAUNCH("k_ctrl_end", s, k_ctrl_end<<<1, 256, 0, s>>>(d));
 }
 

@@ -11,6 +11,7 @@
 //   * neighbour lists are rows of kRow slots per particle (row-major), capped at 70
 //     in the reference's z, y, x cell order; one pass, no count/scan/query split.
 #include "dfsph_common.cuh"
+#include "dfsph_halo.cuh"
 
 namespace vfd {
 
@@ -142,6 +143,7 @@ __global__ void k_grid(Dev d) {
         }
         S.cellCount = (!ok) ? 0u : ((cells > 0xFFFFFFFFu / 512u) ? 0xFFFFFFFFu : cells * 512u);
         S.flags = 0u;
+        if (halo_on(d)) d.haloScene[s] = make_uint2(0xFFFFFFFFu, 0u);
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -152,6 +154,7 @@ __global__ void k_grid(Dev d) {
         }
         total = (uint32_t)min(acc, (uint64_t)0xFFFFFFFFu);
         d.status[2] = total;
+        if (halo_on(d)) d.haloInfo[0] = d.haloInfo[1] = 0u;
         if (acc > d.cellCap) {
             atomicOr(d.status, 0x20u);
             atomicExch(d.status + 1, 1u);
@@ -192,7 +195,12 @@ __global__ void __launch_bounds__(kBlock) k_keys(Dev d) {
 }
 
 // N3: exclusive scan of the cell counts (thrust::exclusive_scan, ParticleSearch.cu:111-115),
-// three phases over the device-known number of cells.
+// three phases over the device-known number of cells. With staged tiles the same phases count
+// and list the non-empty tiles in cell order (a thread owns four consecutive cells, so a
+// tile is a run of kTileLanes lanes).
+constexpr uint32_t kTileLanes = kHaloTileCells / 4u;
+static_assert(kTileLanes <= 32u && kScanItems % kHaloTileCells == 0u, "a tile lies in one warp's cells");
+
 __global__ void __launch_bounds__(256) k_scan_reduce(Dev d) {
     VFD_COUNT_LAUNCH(d);
     if (aborted(d)) return;
@@ -200,18 +208,30 @@ __global__ void __launch_bounds__(256) k_scan_reduce(Dev d) {
     const uint32_t base = blockIdx.x * kScanItems;
     if (base >= total) return;
     uint32_t s = 0;
-    for (uint32_t k = threadIdx.x; k < kScanItems; k += 256u) {
-        const uint32_t c = base + k;
+#pragma unroll
+    for (uint32_t k = 0; k < 4u; k++) {
+        const uint32_t c = base + threadIdx.x * 4u + k;
         if (c < total) s += d.CELL_COUNT[c];
     }
+    const uint32_t filled = __ballot_sync(0xffffffffu, s > 0u);
     s = __reduce_add_sync(0xffffffffu, s);
-    __shared__ uint32_t ws[8];
-    if ((threadIdx.x & 31u) == 0) ws[threadIdx.x >> 5] = s;
+    __shared__ uint32_t ws[8], wt[8];
+    if ((threadIdx.x & 31u) == 0) {
+        uint32_t tiles = 0;
+#pragma unroll
+        for (uint32_t k = 0; k < 32u; k += kTileLanes) tiles += (filled >> k & ((1u << kTileLanes) - 1u)) ? 1u : 0u;
+        ws[threadIdx.x >> 5] = s;
+        wt[threadIdx.x >> 5] = tiles;
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
-        uint32_t t = 0;
-        for (int w = 0; w < 8; w++) t += ws[w];
+        uint32_t t = 0, n = 0;
+        for (int w = 0; w < 8; w++) {
+            t += ws[w];
+            n += wt[w];
+        }
         d.SCAN[blockIdx.x] = t;
+        if (halo_on(d)) d.haloScan[blockIdx.x] = n;
     }
 }
 
@@ -248,7 +268,7 @@ __global__ void __launch_bounds__(1024) k_scan_top(Dev d) {
     if (aborted(d)) return;
     const uint32_t total = d.status[2];
     const uint32_t nb = (total + kScanItems - 1) / kScanItems;
-    uint32_t carry = 0;
+    uint32_t carry = 0, tiles = 0;
     for (uint32_t base = 0; base < nb; base += 1024u) {
         const uint32_t k = base + threadIdx.x;
         const uint32_t v = k < nb ? d.SCAN[k] : 0u;
@@ -256,7 +276,14 @@ __global__ void __launch_bounds__(1024) k_scan_top(Dev d) {
         const uint32_t ex = block_exclusive_scan_1024(v, tot);
         if (k < nb) d.SCAN[k] = carry + ex;
         carry += tot;
+        if (halo_on(d)) {
+            const uint32_t n = k < nb ? d.haloScan[k] : 0u;
+            const uint32_t before = block_exclusive_scan_1024(n, tot);
+            if (k < nb) d.haloScan[k] = tiles + before;
+            tiles += tot;
+        }
     }
+    if (halo_on(d) && threadIdx.x == 0) d.haloInfo[0] = tiles;
 }
 
 __global__ void __launch_bounds__(256) k_scan_down(Dev d) {
@@ -291,6 +318,34 @@ __global__ void __launch_bounds__(256) k_scan_down(Dev d) {
         const uint32_t c = base + threadIdx.x * 4u + k;
         if (c < total) d.CELL_START[c] = run;
         run += v[k];
+    }
+    if (!halo_on(d)) return;
+    // the tile of this thread's lanes, listed by its first lane after the tiles before it
+    const uint32_t mask = ((1u << kTileLanes) - 1u) << (lane & ~(kTileLanes - 1u));
+    const uint32_t filled = __ballot_sync(0xffffffffu, s > 0u);
+    uint32_t inTile = s, before = 0, mine = 0;
+#pragma unroll
+    for (uint32_t o = kTileLanes / 2u; o > 0u; o >>= 1) inTile += __shfl_xor_sync(0xffffffffu, inTile, o);
+#pragma unroll
+    for (uint32_t k = 0; k < 32u; k += kTileLanes) {
+        const uint32_t full = (filled >> k & ((1u << kTileLanes) - 1u)) ? 1u : 0u;
+        mine += full;
+        if (k < (lane & ~(kTileLanes - 1u))) before += full;
+    }
+    __shared__ uint32_t wt[8];
+    if (lane == 0) wt[warp] = mine;
+    __syncthreads();
+    for (uint32_t w = 0; w < warp; w++) before += wt[w];
+    if (lane % kTileLanes == 0u && (filled & mask)) {
+        const uint32_t at = d.haloScan[blockIdx.x] + before, first = run - s;
+        HaloTile T = {};
+        T.cell0 = base + threadIdx.x * 4u;
+        T.first = first;
+        T.last = first + inTile;
+        T.scene = scene_of(d, first);
+        d.haloTiles[at] = T;
+        atomicMin(&d.haloScene[T.scene].x, at);
+        atomicAdd(&d.haloScene[T.scene].y, 1u);
     }
 }
 
@@ -385,6 +440,12 @@ __global__ void __launch_bounds__(kBlock) k_neighbors(Dev d) {
         const bool want = d.NBRC != nullptr && d.compactRows != 0u;
         const bool compact = want && !__any_sync(0xffffffffu, lane < 9u && runEnd - runBeg > kRunMax);
         const uint32_t rowFlag = (want && !compact) ? kRowPath : 0u;
+        // staged place of candidate i of cell j: i + (the cell's first place - the candidates before it)
+        uint32_t place = 0u;
+        const bool halo = halo_on(d);
+        if (halo && lane < 27u)
+            place = d.haloBase[(size_t)(c / kHaloTileCells) * kHaloCells +
+                               halo_cell(c, lane % 3u, lane / 3u % 3u, lane / 9u)] - excl;
         uint32_t mx = 0u;
         for (uint32_t k0 = 0; k0 < cnt; k0 += 32u) {
             const uint32_t kk = min(32u, cnt - k0);
@@ -407,6 +468,7 @@ __global__ void __launch_bounds__(kBlock) k_neighbors(Dev d) {
                 // stencil position of this candidate: its x-run and place in the run
                 const uint32_t run = j / 3u;
                 const uint32_t entry = (run << 6) | (i - __shfl_sync(0xffffffffu, excl, 3u * run));
+                const uint32_t staged = __shfl_sync(0xffffffffu, place, j) + i;
                 const float4 xq = valid ? d.X[q] : make_float4(0.f, 0.f, 0.f, 0.f);
                 for (uint32_t k = 0; k < kk; k++) {
                     const float3 e = pair_r<REL>(d, xq, sx[w][k]);
@@ -418,6 +480,7 @@ __global__ void __launch_bounds__(kBlock) k_neighbors(Dev d) {
                     if (hit && at < kMaxNeighbors) {
                         d.NBR[(size_t)(start + k0 + k) * kRow + at] = q;
                         if (compact) d.NBRC[(size_t)(start + k0 + k) * kRow + at] = (uint16_t)entry;
+                        if (halo) d.haloRow[halo_row_at(start + k0 + k, at)] = (uint16_t)staged;
                     }
                     if (lane == k) count = min(kMaxNeighbors, ck + __popc(bits));
                 }
@@ -449,6 +512,7 @@ void launch_search(const Dev& d, cudaStream_t s, bool profiled) {
     SEARCH_LAUNCH("k_scan_reduce", k_scan_reduce<<<d.scanBlocks, 256, 0, s>>>(d));
     SEARCH_LAUNCH("k_scan_top", k_scan_top<<<1, 1024, 0, s>>>(d));
     SEARCH_LAUNCH("k_scan_down", k_scan_down<<<d.scanBlocks, 256, 0, s>>>(d));
+    if (halo_on(d)) launch_halo_build(d, s);
     SEARCH_LAUNCH("k_slots", k_slots<<<nb, kBlock, 0, s>>>(d));
     SEARCH_LAUNCH("k_rank_gather", k_rank_gather<<<nb, kBlock, 0, s>>>(d));
     // a warp per cell, a fixed grid striding over the cells the device counted

@@ -185,6 +185,9 @@ struct vfd_sim {
     uint8_t tiles[16] = {};
     // threads per block of each TunedKernel's neighbour-row kernels (vfd_autotune; 0 = 128)
     uint16_t blocks[16] = {};
+    // staged-tile passes (dfsph_halo.cu): -1 = by the number of particles, 0 = not (the caller
+    // chose lanes, tiles or blocks of the row kernels), 1 = the autotuner measured them faster
+    int8_t halo = -1;
 
     // layout
     bool allocated = false, uploaded = false;

@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(kBlock) k_boundary(Dev d) {
             const float volume = s.phi1;
             if (volume > 0.0f && volume != FLT_MAX) {
                 vb = volume;
-                const float nl = sqrtf(dot3(normal, normal));
+                const float nl = sqrtf(dot3_yx(normal, normal));
                 if (nl > 1.0e-9f) {
                     normal = make_float3(normal.x / nl, normal.y / nl, normal.z / nl);
                     const float pd = fmaxf(dist + 0.5f * S.r, S.diam);
@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(kBlock) k_boundary(Dev d) {
                 }
             }
         } else if (dist <= 0.0f) {
-            const float nl = sqrtf(dot3(normal, normal));
+            const float nl = sqrtf(dot3_yx(normal, normal));
             if (nl > 1.0e-5f) {
                 normal = make_float3(normal.x / nl, normal.y / nl, normal.z / nl);
                 const float delta = fminf(S.diam - dist, 0.1f * S.r);

@@ -214,8 +214,15 @@ __device__ __forceinline__ float3& operator-=(float3& a, float3 b) { a.x -= b.x;
 __device__ __forceinline__ float dot3(float3 a, float3 b) {
     return __fmaf_rn(a.z, b.z, __fmaf_rn(a.x, b.x, __fmul_rn(a.y, b.y)));
 }
+// The other choice of the two products: each term keeps the one its kernel has always had.
+__device__ __forceinline__ float dot3_yx(float3 a, float3 b) {
+    return __fmaf_rn(a.z, b.z, __fmaf_rn(a.y, b.y, __fmul_rn(a.x, b.x)));
+}
 __device__ __forceinline__ float3 fma3(float s, float3 a, float3 b) {  // s a + b
     return make_float3(__fmaf_rn(s, a.x, b.x), __fmaf_rn(s, a.y, b.y), __fmaf_rn(s, a.z, b.z));
+}
+__device__ __forceinline__ float3 mul3(float s, float3 a) {  // s a, rounded
+    return make_float3(__fmul_rn(s, a.x), __fmul_rn(s, a.y), __fmul_rn(s, a.z));
 }
 __device__ __forceinline__ float4 f4(float3 a, float w) { return make_float4(a.x, a.y, a.z, w); }
 __device__ __forceinline__ float3 cross3(float3 a, float3 b) {

@@ -488,7 +488,7 @@ struct HaloSetup : HaloMatvec<REL, -1> {
     __device__ static void finish(const Dev& d, uint32_t p, const SceneDev& S, const typename Base::Own& o, float3 acc,
                                   uint32_t ncnt, float* term) {
         const float3 b = f3(d.CB[p]);
-        const float3 r = b - visc_product(d, p, S, o.vi, acc, ncnt);
+        const float3 r = b - visc_product<false>(d, p, S, o.vi, acc, ncnt);
         d.CR[p] = f4(r, 0.0f);
         term[0] = dot_term(b, b);
         term[1] = dot_term(r, r);
@@ -504,7 +504,7 @@ struct HaloSpmv : HaloMatvec<REL, kLoopCG> {
     }
     __device__ static void finish(const Dev& d, uint32_t p, const SceneDev& S, const typename Base::Own& o, float3 acc,
                                   uint32_t ncnt, float* term) {
-        const float3 ap = visc_product(d, p, S, o.vi, acc, ncnt);
+        const float3 ap = visc_product<true>(d, p, S, o.vi, acc, ncnt);
         d.CAP[p] = f4(ap, 0.0f);
         term[0] = dot_term(o.vi, ap);
     }

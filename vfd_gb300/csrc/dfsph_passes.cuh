@@ -21,10 +21,9 @@ struct DensitySums {
     float3 gi = {0.0f, 0.0f, 0.0f};
     __device__ __forceinline__ void add(float V, float wj, float gs, float3 r, bool withDiv, float3 dv) {
         w += wj;
-        const float c = -V * gs;
-        const float3 gj = c * r;
+        const float3 gj = mul3(-V * gs, r);
         g2 += dot3(gj, gj);
-        gi = fma3(-c, r, gi);
+        gi -= gj;
         if (withDiv) div += dot3(dv, gs * r);
     }
 };
@@ -117,7 +116,7 @@ __device__ __forceinline__ void density_finish(const Dev& d, uint32_t p, const S
     }
     const float3 gi = s.gi + gb;
     d.RHO[p] = (__fmaf_rn(V, s.w, __fmul_rn(V, d.wZero)) + rhoB) * S.rho0;
-    const float g2 = s.g2 + dot3(gi, gi);
+    const float g2 = s.g2 + dot3_yx(gi, gi);
     const float alpha = g2 > kEps ? 1.0f / g2 : 0.0f;
     d.GB[p] = f4(gb, 0.0f);
     if (!div) {
@@ -126,7 +125,7 @@ __device__ __forceinline__ void density_finish(const Dev& d, uint32_t p, const S
     }
     // K4 (:498-528)
     float rhoAdv = s.div * V;
-    if (flags & kHasBoundary) rhoAdv += dot3(vi, gb);
+    if (flags & kHasBoundary) rhoAdv += dot3_yx(vi, gb);
     rhoAdv = (flags & kCountMask) < 20u ? 0.0f : fmaxf(rhoAdv, 0.0f);
     d.RHOADV[p] = rhoAdv;
     const float alphaDt = alpha * S.dtInv;
@@ -156,7 +155,7 @@ __device__ __forceinline__ void precond_finish(const Dev& d, uint32_t p, const S
             if (!(xb4.w > 0.0f)) continue;
             const float3 xb = f3(xb4);
             float3 normal = -(xi - xb);
-            const float nl = sqrtf(dot3(normal, normal));
+            const float nl = sqrtf(dot3_yx(normal, normal));
             if (!(nl > 0.0001f)) continue;
             normal = make_float3(normal.x / nl, normal.y / nl, normal.z / nl);
             float3 t1, t2;
@@ -203,7 +202,7 @@ __device__ __forceinline__ float jacobi_finish(const Dev& d, uint32_t p, const S
     if (flags & kHasBoundary) f += dot3(ai, f3(d.GB[p]));
     float r;
     if (DIV) {
-        r = (flags & kCountMask) < 20u ? 0.0f : fminf(__fmaf_rn(-f, S.dt, -d.RHOADV[p]), 0.0f);
+        r = (flags & kCountMask) < 20u ? 0.0f : fminf(-d.RHOADV[p] - __fmul_rn(f, S.dt), 0.0f);
         const float k = __fmaf_rn(-r, d.ALPHA[p], d.KAPPAV[p]);
         d.KAPPAV[p] = k;
         set_kappa(d, p, k);
@@ -217,11 +216,13 @@ __device__ __forceinline__ float jacobi_finish(const Dev& d, uint32_t p, const S
     return r;
 }
 
-// K14 after the pair sum: (A x)_p.
+// K14 after the pair sum: (A x)_p, of the first guess or (LOOP) of a direction of the loop.
+template <bool LOOP>
 __device__ __forceinline__ float3 visc_product(const Dev& d, uint32_t p, const SceneDev& S, float3 vi, float3 acc,
                                                uint32_t flags) {
     if (flags & kHasBoundaryVisc) acc += mul(load_mat(d.BVM, d.stride, p), vi);
-    return fma3(-(S.dt / d.RHO[p]), acc, vi);
+    const float c = S.dt / d.RHO[p];
+    return LOOP ? vi - mul3(c, acc) : fma3(-c, acc, vi);
 }
 
 // K17 after the pair sum: advected density, scaled factor, first kappa.
@@ -410,7 +411,7 @@ struct SpmvOp {
         acc += (__fdividef(o.cmu * vq.w * dot3(o.vi - f3(vq), r), r2 + o.eps2) * gs) * r;
     }
     __device__ static float finish(const Dev& d, uint32_t p, const SceneDev& S, const Own& o, Acc acc, uint32_t ncnt) {
-        const float3 ap = visc_product(d, p, S, o.vi, acc, ncnt);
+        const float3 ap = visc_product<true>(d, p, S, o.vi, acc, ncnt);
         d.CAP[p] = f4(ap, 0.0f);
         return dot_term(o.vi, ap);
     }

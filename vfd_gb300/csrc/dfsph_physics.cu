@@ -540,7 +540,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_visc_precond(Dev d) {
 
 // ComputeMatrixVecProdFunctionKernel (:758-842): (A x)_i with vec[q].w = m / rho_q; lane 0.
 // NS: gradW / r from the table, as in pressure_accel.
-template <uint32_t G, bool REL, bool NS = false>
+template <uint32_t G, bool REL, bool LOOP, bool NS = false>
 __device__ __forceinline__ float3 visc_matvec(const Dev& d, const Group<G>& grp, uint32_t p, const SceneDev& S,
                                               const float4* vec, float3 vi) {
     const Nbr nb = neighbors(d, p);
@@ -554,7 +554,7 @@ __device__ __forceinline__ float3 visc_matvec(const Dev& d, const Group<G>& grp,
         const float gs = NS ? grad_factor(d, r) : gsStream;
         add_viscous(acc, cmu * vq.w, vi - f3(vq), eps2, gs, r, ok);
     });
-    return visc_product(d, p, S, vi, grp.sum(acc), nb.flags);
+    return visc_product<LOOP>(d, p, S, vi, grp.sum(acc), nb.flags);
 }
 
 // Initial residual r = b - A g and the norms |b|^2, |r|^2 (:627-669).
@@ -570,7 +570,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_visc_setup(Dev d) {
     float bb = 0.0f, rr = 0.0f;
     if (valid) {
         const float4 g4 = d.CG[p];
-        const float3 ag = visc_matvec<G, REL>(d, grp, p, S, d.CG, f3(g4));
+        const float3 ag = visc_matvec<G, REL, false>(d, grp, p, S, d.CG, f3(g4));
         if (grp.lane == 0) {
             const float3 b = f3(d.CB[p]);
             const float3 r = b - ag;
@@ -694,7 +694,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_cg_spmv(Dev d) {
     float pap = 0.0f;
     if (valid) {
         const float3 pv = f3(d.CP[p]);
-        const float3 ap = visc_matvec<G, REL, NS>(d, grp, p, S, d.CP, pv);
+        const float3 ap = visc_matvec<G, REL, true, NS>(d, grp, p, S, d.CP, pv);
         if (grp.lane == 0) {
             d.CAP[p] = f4(ap, 0.0f);
             pap = dot_term(pv, ap);
@@ -719,7 +719,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_cg_spmv_b(Dev d) {
         if (in) {
             const Group<G> grp(p);
             const float3 pv = f3(d.CP[p]);
-            const float3 ap = visc_matvec<G, REL>(d, grp, p, d.scenes[sid], d.CP, pv);
+            const float3 ap = visc_matvec<G, REL, true>(d, grp, p, d.scenes[sid], d.CP, pv);
             if (grp.lane == 0) {
                 d.CAP[p] = f4(ap, 0.0f);
                 pap = dot_term(pv, ap);

@@ -1415,7 +1415,9 @@ int build_backward_graph(vfd_sim* s, AdjointState* A) {
         L.st = st;
         bwd_mid(L);
     });
-    if (e == cudaSuccess && visc) e = add_while(cap, g, hC, leaves, [&](cudaStream_t st) { launch_cg_iter(L.d, st); });
+    if (e == cudaSuccess && visc) e = add_while(cap, g, hC, leaves, [&](cudaStream_t st) {
+        for (uint32_t k = 0; k < iterations_per_turn(L.d, true); k++) launch_cg_iter(L.d, st);
+    });
     if (e == cudaSuccess) e = add_segment(cap, g, leaves, [&](cudaStream_t st) {
         L.st = st;
         if (visc) bwd_visc_tail(L);

@@ -628,8 +628,9 @@ int build_graph(vfd_sim* s, int parity, const void* rec, cudaGraph_t* gOut, cuda
         launch_density_div_init(d, st);
         T(kTapeDivInit, st);
     });
+    const uint32_t turns = rec ? 1u : iterations_per_turn(d, false);
     if (e == cudaSuccess && anyDiv) e = add_while(cap, g, h[0], leaves, [&](cudaStream_t st) {
-        launch_div_iter(d, st);
+        for (uint32_t k = 0; k < turns; k++) launch_div_iter(d, st);
         T(kTapeDivIter, st);
     });
     if (e == cudaSuccess)
@@ -639,7 +640,9 @@ int build_graph(vfd_sim* s, int parity, const void* rec, cudaGraph_t* gOut, cuda
             if (anyST) launch_surface_tension(d, passes, st);
             if (anyVisc) launch_visc_init(d, st);
         });
-    if (e == cudaSuccess && anyVisc) e = add_while(cap, g, h[1], leaves, [&](cudaStream_t st) { launch_cg_iter(d, st); });
+    if (e == cudaSuccess && anyVisc) e = add_while(cap, g, h[1], leaves, [&](cudaStream_t st) {
+        for (uint32_t k = 0; k < iterations_per_turn(d, true); k++) launch_cg_iter(d, st);
+    });
     if (e == cudaSuccess)
         e = add_segment(cap, g, leaves, [&](cudaStream_t st) {
             T(kTapeVisc, st);
@@ -649,7 +652,7 @@ int build_graph(vfd_sim* s, int parity, const void* rec, cudaGraph_t* gOut, cuda
             T(kTapePresInit, st);
         });
     if (e == cudaSuccess) e = add_while(cap, g, h[2], leaves, [&](cudaStream_t st) {
-        launch_pres_iter(d, st);
+        for (uint32_t k = 0; k < turns; k++) launch_pres_iter(d, st);
         T(kTapePresIter, st);
     });
     if (e == cudaSuccess) e = add_segment(cap, g, leaves, [&](cudaStream_t st) {

@@ -1286,6 +1286,7 @@ bool ensure_shadow(vfd_sim* s, AdjointState* A) {
     t->reserve = s->reserve;
     t->cellCap = s->cellCap;  // the search grid the simulation grew to, so replays do not abort on it
     std::memcpy(t->lanes, s->lanes, sizeof(t->lanes));
+    t->lanesChosen = true;
     std::memcpy(t->tiles, s->tiles, sizeof(t->tiles));
     t->halo = s->halo;
     std::memcpy(t->blocks, s->blocks, sizeof(t->blocks));
@@ -1416,7 +1417,7 @@ int build_backward_graph(vfd_sim* s, AdjointState* A) {
         bwd_mid(L);
     });
     if (e == cudaSuccess && visc) e = add_while(cap, g, hC, leaves, [&](cudaStream_t st) {
-        for (uint32_t k = 0; k < iterations_per_turn(L.d, true); k++) launch_cg_iter(L.d, st);
+        for (uint32_t k = 0; k < iterations_per_turn(L.d); k++) launch_cg_iter(L.d, st);
     });
     if (e == cudaSuccess) e = add_segment(cap, g, leaves, [&](cudaStream_t st) {
         L.st = st;

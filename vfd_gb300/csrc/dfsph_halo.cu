@@ -314,9 +314,7 @@ struct HaloDensity : HaloOp<kVectorField, kWriteGrad> {
         float V;
         bool div;
     };
-    struct Acc : DensitySums {
-        __device__ void operator+=(const Acc& b) { w += b.w, g2 += b.g2, div += b.div, gi += b.gi; }
-    };
+    using Acc = DensitySums;
     __device__ static const void* field(const Dev& d) { return d.V; }
     __device__ static void load(const Dev& d, uint32_t p, const SceneDev& S, Own& o) {
         o.xi = d.X[p];
@@ -441,9 +439,7 @@ struct HaloPrecond : HaloOp<kScalarField, kReadGrad, 2u> {
         float4 xi;
         float eps2, cmu, mass;
     };
-    struct Acc : Mat3 {
-        __device__ void operator+=(const Acc& b) { r0 += b.r0, r1 += b.r1, r2 += b.r2; }
-    };
+    using Acc = Mat3;
     __device__ static bool active(const SceneDev& S) { return S.enableVisc != 0; }
     __device__ static const void* field(const Dev& d) { return d.RHO; }
     __device__ static void load(const Dev& d, uint32_t p, const SceneDev& S, Own& o) {

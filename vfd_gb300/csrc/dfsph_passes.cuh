@@ -14,6 +14,19 @@ __device__ __forceinline__ void set_kappa(const Dev& d, uint32_t p, float k) {
     if (!d.cellRel) reinterpret_cast<float*>(d.X)[4 * (size_t)p + 3] = k;
 }
 
+// A lane's partial sums of a neighbour loop with G lanes a particle. Four lanes keep two, of
+// the even and of the odd rounds, which are those that eight lanes keep; total() adds them as
+// the eight lanes' shuffle tree does, so either lane count gives the same bits.
+template <uint32_t G, class T>
+struct LaneSums {
+    T s[2] = {};
+    __device__ __forceinline__ T& at(uint32_t round) { return s[G == 4u ? round & 1u : 0u]; }
+    __device__ __forceinline__ T total() {
+        if (G == 4u) s[0] += s[1];
+        return s[0];
+    }
+};
+
 // One pair's terms, shared by the row and the tile kernels so that their bits agree: the sums
 // of the density and factor (K2 - K4), ...
 struct DensitySums {
@@ -26,6 +39,7 @@ struct DensitySums {
         gi -= gj;
         if (withDiv) div += dot3(dv, gs * r);
     }
+    __device__ __forceinline__ void operator+=(const DensitySums& b) { w += b.w, g2 += b.g2, div += b.div, gi += b.gi; }
 };
 // ... the pressure acceleration (K5, K7, K18, K20) and the viscosity product (K14).
 __device__ __forceinline__ void add_pressure(float3& a, float sum, float V, float gs, float3 r, bool ok) {
@@ -62,6 +76,7 @@ __device__ __forceinline__ void kernel_wg(const Dev& d, float3 r, float& w, floa
 
 struct Mat3 {
     float3 r0, r1, r2;
+    __device__ __forceinline__ void operator+=(const Mat3& b) { r0 += b.r0, r1 += b.r1, r2 += b.r2; }
 };
 __device__ __forceinline__ float3 mul(const Mat3& m, float3 v) {
     return make_float3(dot3(m.r0, v), dot3(m.r1, v), dot3(m.r2, v));
@@ -268,11 +283,12 @@ __device__ __forceinline__ void st_classify_item(const Dev& d, const Group<G>& g
         if (grp.lane == 0) d.STN[p] = make_float4(0.f, 0.f, 0.f, 1.0f / S.h);
         return;
     }
-    float3 com = make_float3(0.f, 0.f, 0.f);
-    for (uint32_t j = grp.lane; j < cnt; j += G) com += at(j);
-    com = grp.sum(com);
+    LaneSums<G, float3> com3;
+    for (uint32_t j = grp.lane; j < cnt; j += G) com3.at(j / G) += at(j);
+    float3 com = grp.sum(com3.total());
     com = make_float3(com.x / S.h, com.y / S.h, com.z / S.h);
     const float input = sqrtf(dot3(com, com)) / (float)cnt;
+    LaneSums<G, float3> nsum3;
     float3 nsum = make_float3(0.f, 0.f, 0.f);
     float curv = 0.0f;
     if ((float)cnt <= S.slope * input + S.constant + 0.0f) {
@@ -291,9 +307,9 @@ __device__ __forceinline__ void st_classify_item(const Dev& d, const Group<G>& g
                 const float3 v = pt - at(j);
                 if (dot3(v, v) <= lim) { covered = true; break; }
             }
-            if (!covered) { nsum += pt; count++; }
+            if (!covered) { nsum3.at(k / G) += pt; count++; }
         }
-        nsum = grp.sum(nsum);
+        nsum = grp.sum(nsum3.total());
         count = grp.sum(count);
         if (count > 0) {
             if (dot3(nsum, nsum) > 0.0f) nsum = normalize3(nsum);

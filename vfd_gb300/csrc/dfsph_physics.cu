@@ -140,7 +140,7 @@ constexpr uint32_t kUnroll = 4u;
 // not wait for the count (rows have 72 slots, entries past the count are masked), so
 // the count, the indices and the particle's own fields are fetched together; within a
 // round the U gathers per lane are independent. Masked entries use the particle itself
-// as a stand-in index. The row and gradient streams are read once per pass, so they
+// as a stand-in index. f also gets the entry's place u among the round's (LaneSums). The row and gradient streams are read once per pass, so they
 // are loaded with the evict-first hint (ld.global.cs) to leave L2 to the gathered
 // fields.
 template <uint32_t G, bool WITH_GS, class F>
@@ -179,7 +179,7 @@ __device__ __forceinline__ void for_neighbors(const Group<G>& grp, const Nbr& nb
         for (uint32_t u = 0; u < U; u++) {
             const uint32_t j = base + grp.lane + u * G;
             const bool ok = j < nb.count;
-            f(ok ? nb.check(q[u]) : self, g[u], j, ok);
+            f(ok ? nb.check(q[u]) : self, g[u], j, ok, u);
         }
     }
 }
@@ -203,20 +203,21 @@ __global__ void __launch_bounds__(kMaxBlock) k_density_factor(Dev d) {
     const float4 xi4 = d.X[p];
     const float3 xi = f3(xi4);
     const Nbr nb = neighbors(d, p);
-    DensitySums s;
+    LaneSums<G, DensitySums> sums;
     const float V = S.volume;
     const bool div = DIV && S.enableDiv;
     const float3 vi = div ? f3(d.V[p]) : make_float3(0.f, 0.f, 0.f);
     uint2* ngRow = d.NG + (size_t)p * kRow;
-    for_neighbors<G, false>(grp, nb, p, [&](uint32_t q, float, uint32_t j, bool ok) {
+    for_neighbors<G, false>(grp, nb, p, [&](uint32_t q, float, uint32_t j, bool ok, uint32_t u) {
         const float3 r = pair_r<REL>(d, xi4, d.X[q]);
         float w, gs;
         kernel_wg(d, r, w, gs);
         const float3 vq = div ? f3(d.V[q]) : make_float3(0.f, 0.f, 0.f);
         if (!ok) return;
         __stcs(ngRow + j, make_uint2(q, __float_as_uint(gs)));
-        s.add(V, w, gs, r, div, vi - vq);
+        sums.at(u).add(V, w, gs, r, div, vi - vq);
     });
+    DensitySums s = sums.total();
     s.w = grp.sum(s.w);
     s.g2 = grp.sum(s.g2);
     s.gi = grp.sum(s.gi);
@@ -228,14 +229,14 @@ __global__ void __launch_bounds__(kMaxBlock) k_density_factor(Dev d) {
 template <uint32_t G, bool REL>
 __device__ __forceinline__ float velocity_divergence(const Dev& d, const Group<G>& grp, uint32_t p, const SceneDev& S,
                                                      const Nbr& nb, float4 xi, float3 vi) {
-    float s = 0.0f;
-    for_neighbors<G, true>(grp, nb, p, [&](uint32_t q, float gs, uint32_t, bool ok) {
+    LaneSums<G, float> sums;
+    for_neighbors<G, true>(grp, nb, p, [&](uint32_t q, float gs, uint32_t, bool ok, uint32_t u) {
         const float3 r = pair_r<REL>(d, xi, d.X[q]);
         const float3 vq = f3(d.V[q]);
         const float t = dot3(vi - vq, gs * r);
-        if (ok) s += t;
+        if (ok) sums.at(u) += t;
     });
-    s = grp.sum(s) * S.volume;
+    float s = grp.sum(sums.total()) * S.volume;
     if (nb.flags & kHasBoundary) s += dot3(vi, f3(d.GB[p]));
     return s;
 }
@@ -251,15 +252,15 @@ __device__ __forceinline__ float3 pressure_accel(const Dev& d, const Group<G>& g
     const float ki = kap[p];
     const float4 xi = d.X[p];
     const float V = S.volume;
-    float3 a = make_float3(0.f, 0.f, 0.f);
-    for_neighbors<G, !NS>(grp, nb, p, [&](uint32_t q, float gsStream, uint32_t, bool ok) {
+    LaneSums<G, float3> sums;
+    for_neighbors<G, !NS>(grp, nb, p, [&](uint32_t q, float gsStream, uint32_t, bool ok, uint32_t u) {
         const float4 xq = d.X[q];
         const float sum = ki + (REL ? kap[q] : xq.w);
         const float3 r = pair_r<REL>(d, xi, xq);
         const float gs = NS ? grad_factor(d, r) : gsStream;
-        add_pressure(a, sum, V, gs, r, ok);
+        add_pressure(sums.at(u), sum, V, gs, r, ok);
     });
-    a = grp.sum(a);
+    float3 a = grp.sum(sums.total());
     if (fabsf(ki) > kEps && (nb.flags & kHasBoundary)) a += ki * (-f3(d.GB[p]));
     return a;
 }
@@ -301,15 +302,15 @@ __device__ __forceinline__ float jacobi_item(const Dev& d, const Group<G>& grp, 
     const Nbr nb = neighbors(d, p);
     const float4 xi = d.X[p];
     const float3 ai = f3(d.AP[p]);
-    float f = 0.0f;
-    for_neighbors<G, !NS>(grp, nb, p, [&](uint32_t q, float gsStream, uint32_t, bool ok) {
+    LaneSums<G, float> sums;
+    for_neighbors<G, !NS>(grp, nb, p, [&](uint32_t q, float gsStream, uint32_t, bool ok, uint32_t u) {
         const float3 r = pair_r<REL>(d, xi, d.X[q]);
         const float gs = NS ? grad_factor(d, r) : gsStream;
         const float3 aq = f3(d.AP[q]);
         const float t = dot3(ai - aq, gs * r);
-        if (ok) f += t;
+        if (ok) sums.at(u) += t;
     });
-    f = grp.sum(f);
+    const float f = grp.sum(sums.total());
     return grp.lane == 0 ? jacobi_finish<DIV>(d, p, S, ai, f, nb.flags) : 0.0f;
 }
 
@@ -467,21 +468,20 @@ __global__ void __launch_bounds__(kMaxBlock) k_st_smooth(Dev d) {
     if (!nonzero3(ni)) return;
     const Nbr nb = neighbors(d, p);
     const float4 xi = d.X[p];
-    float3 nc = make_float3(0.f, 0.f, 0.f);
-    float cc = 0.0f, cf = 0.0f;
-    for_neighbors<G, false>(grp, nb, p, [&](uint32_t q, float, uint32_t, bool ok) {
+    LaneSums<G, float3> ncs;
+    LaneSums<G, float> ccs, cfs;
+    for_neighbors<G, false>(grp, nb, p, [&](uint32_t q, float, uint32_t, bool ok, uint32_t u) {
         const float4 nj = d.STN[q];
         const float3 dx = pair_r<REL>(d, d.X[q], xi);
         if (ok && nonzero3(nj)) {
             const float num = 1.0f - __fdividef(fast_sqrt(dot3(dx, dx)), S.h);
-            nc += f3(nj) * num;
-            cc += nj.w * num;
-            cf += num;
+            ncs.at(u) += f3(nj) * num;
+            ccs.at(u) += nj.w * num;
+            cfs.at(u) += num;
         }
     });
-    nc = grp.sum(nc);
-    cc = grp.sum(cc);
-    cf = grp.sum(cf);
+    const float3 nc = grp.sum(ncs.total());
+    const float cc = grp.sum(ccs.total()), cf = grp.sum(cfs.total());
     if (grp.lane != 0) return;
     st_smooth_finish(d, p, S, ni, nc, cc, cf);
 }
@@ -523,15 +523,16 @@ __global__ void __launch_bounds__(kMaxBlock) k_visc_precond(Dev d) {
     const float3 xi = f3(xi4);  // own frame of the boundary samples
     const float eps2 = 0.01f * S.h2;
     const float cmu = 10.0f * S.dynVisc;
-    Mat3 m = {make_float3(0.f, 0.f, 0.f), make_float3(0.f, 0.f, 0.f), make_float3(0.f, 0.f, 0.f)};
-    for_neighbors<G, true>(grp, nb, p, [&](uint32_t q, float gs, uint32_t, bool ok) {
+    LaneSums<G, Mat3> sums;
+    for_neighbors<G, true>(grp, nb, p, [&](uint32_t q, float gs, uint32_t, bool ok, uint32_t u) {
         const float3 r = pair_r<REL>(d, xi4, d.X[q]);
         const float rho = d.RHO[q];
         if (!ok) return;
         const float3 g = gs * r;
         const float c = __fdividef(cmu * __fdividef(S.mass, rho), dot3(r, r) + eps2);
-        add_outer(m, c, r, g);
+        add_outer(sums.at(u), c, r, g);
     });
+    Mat3 m = sums.total();
     m.r0 = grp.sum(m.r0);
     m.r1 = grp.sum(m.r1);
     m.r2 = grp.sum(m.r2);
@@ -547,14 +548,14 @@ __device__ __forceinline__ float3 visc_matvec(const Dev& d, const Group<G>& grp,
     const float4 xi = d.X[p];
     const float eps2 = 0.01f * S.h2;
     const float cmu = 10.0f * S.dynVisc;
-    float3 acc = make_float3(0.f, 0.f, 0.f);
-    for_neighbors<G, !NS>(grp, nb, p, [&](uint32_t q, float gsStream, uint32_t, bool ok) {
+    LaneSums<G, float3> sums;
+    for_neighbors<G, !NS>(grp, nb, p, [&](uint32_t q, float gsStream, uint32_t, bool ok, uint32_t u) {
         const float3 r = pair_r<REL>(d, xi, d.X[q]);
         const float4 vq = vec[q];
         const float gs = NS ? grad_factor(d, r) : gsStream;
-        add_viscous(acc, cmu * vq.w, vi - f3(vq), eps2, gs, r, ok);
+        add_viscous(sums.at(u), cmu * vq.w, vi - f3(vq), eps2, gs, r, ok);
     });
-    return visc_product<LOOP>(d, p, S, vi, grp.sum(acc), nb.flags);
+    return visc_product<LOOP>(d, p, S, vi, grp.sum(sums.total()), nb.flags);
 }
 
 // Initial residual r = b - A g and the norms |b|^2, |r|^2 (:627-669).

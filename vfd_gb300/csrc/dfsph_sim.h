@@ -29,15 +29,14 @@ void launch_visc_finish_dt(const Dev& d, cudaStream_t s);
 void launch_pres_init(const Dev& d, cudaStream_t s);
 void launch_pres_iter(const Dev& d, cudaStream_t s);
 void launch_pres_finish(const Dev& d, cudaStream_t s);
-// Iterations of a solver loop (the CG, or a Jacobi solve) per turn of its while node in a
+// Iterations of a solver loop per turn of its while node in a
 // step's graph. A turn's relaunch costs ~4 us; the kernels of an iteration past the last
-// return at once (~2 us each). Two for the Jacobi solves, whose usual minimum it is, and
-// four for the longer CG: a step of 26 Jacobi and 28 CG iterations at 33,000 particles took
-// 1481 us with one, 1396 with two and two, 1386 with two and four, 1382 with four and four;
-// one of 7 Jacobi iterations at 8,000 particles 374, 354, 356 and 364. An iteration of
-// 200,000 particles takes 60 us and more, and a batch's kernels walk lists of the scenes
-// still iterating: they keep one.
-inline uint32_t iterations_per_turn(const Dev& d, bool cg) { return d.nscenes > 1 || d.n >= 200000u ? 1u : cg ? 4u : 2u; }
+// return at once (~2 us each), and every node adds to the graph's construction. A step of 26
+// Jacobi and 28 CG iterations at 33,000 particles took 1481 us with one, 1396 with two and
+// 1382 with four; one of 7 Jacobi iterations at 8,000 particles 374, 354 and 364. An
+// iteration of 200,000 particles takes 60 us and more, and a batch's kernels walk lists of the
+// scenes still iterating: they keep one.
+inline uint32_t iterations_per_turn(const Dev& d) { return d.nscenes > 1 || d.n >= 200000u ? 1u : 2u; }
 // Occupancy and shared-memory limits of the cell-tile kernels (once, before any capture).
 cudaError_t prepare_tile_kernels();
 // Whether any solver-loop pass runs on cell tiles (then the search writes NBRC rows).
@@ -189,6 +188,7 @@ struct vfd_sim {
     vfd::Fp64State* fp64 = nullptr;
     bool graphFailed = false;
     uint8_t lanes[16] = {8, 8, 8, 8, 8, 8, 8, 8, 8, 8, 8, 8, 8, 8, 8, 8};
+    bool lanesChosen = false;  // by the caller or the autotuner; else by the number of particles
     // cell tiles of the solver-loop kernels per TunedKernel: 0 = neighbour rows, else log2
     // of the cells in a tile (vfd_set_tiles, vfd_autotune)
     uint8_t tiles[16] = {};

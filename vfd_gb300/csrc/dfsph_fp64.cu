@@ -8,10 +8,11 @@
 // doubles. It is the reference trajectory the FP32 paths are measured against on the
 // GPU (the FP64 CPU oracle is the same method, but too slow for millions of particles):
 // one scene, absolute positions, particles kept in their original order with neighbour
-// rows of original indices (as the reference keeps them), one thread per particle,
-// the solver loops driven from the host with one reduction read per iteration. Every
-// sum over particles is a per-block partial added on the host in block order, so runs
-// are reproducible. The SPH tables are built in double with the reference's formulas
+// rows of original indices (as the reference keeps them), one to eight lanes a particle in
+// the neighbour loops. The solver loops are launched a few iterations at a time: a one-block kernel
+// adds the blocks' partial sums in a fixed order (so runs are reproducible), takes the
+// loop's decision on the device, and the kernels of iterations past the last return at once;
+// the host looks once per group. The SPH tables are built in double with the reference's formulas
 // (Kernel/DFSPHKernels.h:13-131) and read with its midpoint lookup; the volume maps and
 // the surface-tension direction table are the FP32 path's (their values as doubles).
 #include <cuda_runtime.h>
@@ -30,7 +31,16 @@
 namespace vfd {
 namespace f64 {
 
-constexpr uint32_t kB = 256u;         // threads per block
+// What bounds the path is the FP64 pipe, 1/64 of the FP32 rate on this GPU (a dependent add
+// takes 64 cycles, a division or square root 650), and with few particles the chain of a
+// thread. So the density pass keeps each pair's gradient factor and the preconditioner each
+// pair's viscosity coefficient (16 bytes a pair together), and a pair of the loops costs 9 to 14
+// FP64 operations instead of ~40 to 70. Two steps of a viscous drop, before (a thread a particle
+// that formed them again, 256 threads a block, a wait of the host per reduction) and now: 7.3 and
+// 2.1 ms at 8,000 particles, 8.1 and 4.0 at 33,000, 35 and 16 at 300,000, 187 and 79 at 1M.
+constexpr uint32_t kB = 256u;         // threads per block, at most
+constexpr uint32_t kL = 8u;           // lanes per particle in the search, and at most in the neighbour loops
+constexpr uint32_t kLB = 128u;        // their threads per block
 constexpr uint32_t kCap = kMaxNeighbors;
 
 struct D3 {
@@ -49,6 +59,12 @@ __device__ __forceinline__ D3 cross(D3 a, D3 b) {
     return d3(a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x);
 }
 __device__ __forceinline__ D3 normalized(D3 a) { return a * (1.0 / sqrt(dot(a, a))); }
+// Sum over a particle's G lanes (all of the warp call it).
+__device__ __forceinline__ double lanes(uint32_t G, double v) {
+    for (uint32_t o = G / 2u; o > 0u; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+__device__ __forceinline__ D3 lanes(uint32_t G, D3 v) { return d3(lanes(G, v.x), lanes(G, v.y), lanes(G, v.z)); }
 __device__ __forceinline__ bool nonzero(D3 a) { return a.x != 0.0 || a.y != 0.0 || a.z != 0.0; }
 
 struct M3 {
@@ -87,11 +103,23 @@ __device__ __forceinline__ M3 inverse(const M3& a) {  // cofactors / determinant
 // Scene constants and the current time step (passed by value to every kernel).
 struct P {
     uint32_t n, bodies, bodyBegin, analytic, stSamples, temporal;
+    uint32_t lanes, lanesLog2;  // per particle in the neighbour loops
     double r, diam, h, h2, volume, rho0, mass, massInv, dynVisc, dynBVisc, tangDist, st;
     double slope, constant, smoothing, nbrRadius, mcFactor;
     double g[3];
     double dt, dt2, dtInv, dt2Inv;
     double K, L, invStep, wZero;  // spline constants and table step
+};
+
+// State of the solver loop in progress, on the device; the host reads it between groups of
+// iterations.
+struct Loop {
+    double err, rr, rhs, thr, absNew, alpha, beta;
+    uint32_t it, done, zeroG;
+};
+struct LoopBounds {
+    double eta;         // Jacobi: error bound; CG: MaxViscositySolverError
+    uint32_t mn, mx;    // iterations
 };
 
 // Device arrays of the FP64 state, original particle order.
@@ -102,7 +130,9 @@ struct A {
     M3* MINV;
     uint32_t *NCNT, *NBR, *KEY, *CNT, *START, *FILL, *TMP, *ORDER, *BSUM;
     int* MM;  // min cell xyz, max cell xyz
-    double* PART;
+    double *PART, *PART2;
+    double *GS, *VS;      // [particle][kCap]: gradW / r, and the viscosity's coefficient of (v . r) r
+    struct Loop* loop;
     const double *W, *G;  // midpoint tables
     const float* halton;
     const BodyDev* bodyTab;
@@ -145,8 +175,9 @@ __device__ __forceinline__ D3 kgrad(const P& p, const A& a, D3 r) {  // GetGradi
 
 // ---------------------------------------------------------------- reductions
 // Sum (or max) of one double per thread into PART[blockIdx.x].
-__device__ __forceinline__ void block_partial(const A& a, double v, bool isMax) {
+__device__ __forceinline__ void block_partial(double* part, double v, bool isMax) {
     __shared__ double s[kB / 32u];
+    __syncthreads();  // a second call reuses s
 #pragma unroll
     for (int o = 16; o >= 1; o >>= 1) {
         const double w = __shfl_xor_sync(0xffffffffu, v, o);
@@ -157,21 +188,37 @@ __device__ __forceinline__ void block_partial(const A& a, double v, bool isMax) 
     if (threadIdx.x == 0) {
         double t = s[0];
         for (uint32_t w = 1; w < blockDim.x / 32u; w++) t = isMax ? fmax(t, s[w]) : t + s[w];
-        a.PART[blockIdx.x] = t;
+        part[blockIdx.x] = t;
     }
+}
+// Sum (or max) of n values in every thread of a block of 256: a stride each, then a tree.
+__device__ double block_fold(const double* v, uint32_t n, bool isMax) {
+    __shared__ double s[256];
+    double t = 0.0;
+    for (uint32_t k = threadIdx.x; k < n; k += 256u) t = isMax ? fmax(t, v[k]) : t + v[k];
+    __syncthreads();
+    s[threadIdx.x] = t;
+    __syncthreads();
+    for (uint32_t o = 128u; o > 0u; o >>= 1) {
+        if (threadIdx.x < o) s[threadIdx.x] = isMax ? fmax(s[threadIdx.x], s[threadIdx.x + o]) : s[threadIdx.x] + s[threadIdx.x + o];
+        __syncthreads();
+    }
+    return s[0];
 }
 
 // ---------------------------------------------------------------- neighbour search
 __global__ void k_minmax(P p, A a) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= p.n) return;
-    const D3 x = a.X[i];
+    const D3 x = a.X[i < p.n ? i : p.n - 1u];  // the others repeat the last particle
     const double c[3] = {floor(x.x / p.h), floor(x.y / p.h), floor(x.z / p.h)};
 #pragma unroll
     for (int k = 0; k < 3; k++) {
         const int v = fabs(c[k]) < 1.0e9 ? (int)c[k] : 0;
-        atomicMin(a.MM + k, v);
-        atomicMax(a.MM + 3 + k, v);
+        const int lo = __reduce_min_sync(0xffffffffu, v), hi = __reduce_max_sync(0xffffffffu, v);
+        if ((threadIdx.x & 31u) == 0u) {
+            atomicMin(a.MM + k, lo);
+            atomicMax(a.MM + 3 + k, hi);
+        }
     }
 }
 __device__ __forceinline__ void cell_of(const P& p, const A& a, D3 x, int c[3]) {
@@ -216,13 +263,23 @@ __global__ void k_scan_blocks(A a) {
     if (c < a.cells) a.START[c] = excl;
     if (threadIdx.x == 1023u) a.BSUM[blockIdx.x] = ws[31];
 }
-__global__ void k_scan_carry(A a, uint32_t nblocks) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+__global__ void __launch_bounds__(1024) k_scan_carry(A a, uint32_t nblocks) {
+    __shared__ uint32_t ws[1024];
     uint32_t run = 0;
-    for (uint32_t b = 0; b < nblocks; b++) {
-        const uint32_t s = a.BSUM[b];
-        a.BSUM[b] = run;
-        run += s;
+    for (uint32_t base = 0; base < nblocks; base += 1024u) {
+        const uint32_t b = base + threadIdx.x;
+        const uint32_t v = b < nblocks ? a.BSUM[b] : 0u;
+        ws[threadIdx.x] = v;
+        __syncthreads();
+        for (uint32_t o = 1; o < 1024u; o <<= 1) {
+            const uint32_t t = threadIdx.x >= o ? ws[threadIdx.x - o] : 0u;
+            __syncthreads();
+            ws[threadIdx.x] += t;
+            __syncthreads();
+        }
+        if (b < nblocks) a.BSUM[b] = run + ws[threadIdx.x] - v;
+        run += ws[1023];
+        __syncthreads();
     }
 }
 __global__ void k_scan_add(A a) {
@@ -247,29 +304,48 @@ __global__ void k_order(P p, A a) {
 }
 // NeighborhoodQueryWithCountsKernel (ParticleSearchKernels.cu:146-193): z, y, x cells,
 // then cell order, 0 < d^2 < h^2, at most 70.
-__global__ void k_neighbors(P p, A a) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= p.n) return;
+__global__ void __launch_bounds__(kLB) k_neighbors(P p, A a) {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, l = t % kL, shift = threadIdx.x & 31u & ~(kL - 1u);
+    const bool live = t / kL < p.n;
+    const uint32_t i = live ? t / kL : p.n - 1u;
     const D3 xi = a.X[i];
     int c[3];
     cell_of(p, a, xi, c);
+    uint32_t cs[4], cc[4];  // the ranges of stencil cells l, l + 8, l + 16, l + 24
+#pragma unroll
+    for (uint32_t m = 0; m < 4u; m++) {
+        const uint32_t s = l + m * kL;
+        const int x = c[0] + (int)(s % 3u) - 1, y = c[1] + (int)(s / 3u % 3u) - 1, z = c[2] + (int)(s / 9u) - 1;
+        cs[m] = cc[m] = 0u;
+        if (s < 27u && x >= 0 && y >= 0 && z >= 0 && x < (int)a.dim[0] && y < (int)a.dim[1] && z < (int)a.dim[2]) {
+            const uint32_t k = ((uint32_t)z * a.dim[1] + (uint32_t)y) * a.dim[0] + (uint32_t)x;
+            cs[m] = a.START[k];
+            cc[m] = a.CNT[k];
+        }
+    }
     uint32_t cnt = 0;
     uint32_t* row = a.NBR + (size_t)i * kCap;
-    for (int dz = -1; dz <= 1 && cnt < kCap; dz++)
-        for (int dy = -1; dy <= 1 && cnt < kCap; dy++)
-            for (int dx = -1; dx <= 1 && cnt < kCap; dx++) {
-                const int x = c[0] + dx, y = c[1] + dy, z = c[2] + dz;
-                if (x < 0 || y < 0 || z < 0 || x >= (int)a.dim[0] || y >= (int)a.dim[1] || z >= (int)a.dim[2]) continue;
-                const uint32_t k = ((uint32_t)z * a.dim[1] + (uint32_t)y) * a.dim[0] + (uint32_t)x;
-                const uint32_t st = a.START[k], n = a.CNT[k];
-                for (uint32_t q = st; q < st + n && cnt < kCap; q++) {
-                    const uint32_t j = a.ORDER[q];
+#pragma unroll
+    for (uint32_t m = 0; m < 4u; m++)
+        for (uint32_t s = 0; s < kL; s++) {
+            const uint32_t st = __shfl_sync(0xffffffffu, cs[m], s, kL), n = __shfl_sync(0xffffffffu, cc[m], s, kL);
+            const uint32_t most = __reduce_max_sync(0xffffffffu, n);
+            for (uint32_t q = l; q - l < most; q += kL) {  // eight candidates at a time, kept in order
+                uint32_t j = 0u;
+                bool hit = false;
+                if (q < n) {
+                    j = a.ORDER[st + q];
                     const D3 e = a.X[j] - xi;
                     const double d2 = dot(e, e);
-                    if (d2 < p.h2 && d2 > 0.0) row[cnt++] = j;
+                    hit = d2 < p.h2 && d2 > 0.0;
                 }
+                const uint32_t bits = __ballot_sync(0xffffffffu, hit) >> shift & ((1u << kL) - 1u);
+                const uint32_t at = cnt + __popc(bits & ((1u << l) - 1u));
+                if (live && hit && at < kCap) row[at] = j;
+                cnt += __popc(bits);
             }
-    a.NCNT[i] = cnt;
+        }
+    if (live && l == 0u) a.NCNT[i] = min(cnt, kCap);
 }
 
 // ---------------------------------------------------------------- volume map
@@ -343,7 +419,23 @@ __device__ bool map_lookup(const BodyDev& m, D3 pt, double& phi0, D3& grad0, dou
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; \
     if (i >= p.n) return;
 
+// Lane l of the group of lanes of particle i; groups past the end repeat the last particle
+// and write nothing (`first`: the lane that writes).
+#define F64_LANES                                                                                   \
+    const uint32_t t_ = blockIdx.x * blockDim.x + threadIdx.x, l = t_ & (p.lanes - 1u);             \
+    const uint32_t i_ = t_ >> p.lanesLog2, i = i_ < p.n ? i_ : p.n - 1u;                            \
+    const bool first = l == 0u && i_ < p.n;
+
 __device__ __forceinline__ uint32_t nbr(const A& a, uint32_t i, uint32_t j) { return a.NBR[(size_t)i * kCap + j]; }
+// f(k, pair place, r) for the lane's share of the particle's neighbours k, r = x_i - x_k.
+template <class F>
+__device__ __forceinline__ void pairs(const P& p, const A& a, uint32_t i, uint32_t l, D3 xi, F&& f) {
+    const uint32_t cnt = a.NCNT[i];
+    for (uint32_t j = l; j < cnt; j += p.lanes) {
+        const uint32_t k = nbr(a, i, j);
+        f(k, (size_t)i * kCap + j, xi - a.X[k]);
+    }
+}
 
 // K1 ComputeVolumeAndBoundaryKernel (DFSPHKernels.cu:69-150)
 __global__ void k_boundary(P p, A a) {
@@ -379,19 +471,27 @@ __global__ void k_boundary(P p, A a) {
 }
 
 // K2 ComputeDensityKernel (:152-187) + K3 ComputeDFSPHFactorKernel (:189-231)
-__global__ void k_density_factor(P p, A a) {
-    F64_THREAD
+// (and each pair's gradient factor)
+__global__ void __launch_bounds__(kLB) k_density_factor(P p, A a) {
+    F64_LANES
     const D3 xi = a.X[i];
-    double rho = p.volume * p.wZero, sum = 0.0;
+    double w = 0.0, sum = 0.0;
     D3 gi = d3(0, 0, 0);
-    const uint32_t cnt = a.NCNT[i];
-    for (uint32_t j = 0; j < cnt; j++) {
-        const D3 r = xi - a.X[nbr(a, i, j)];
-        rho += p.volume * kw(p, a, r);
-        const D3 gj = -p.volume * kgrad(p, a, r);
+    pairs(p, a, i, l, xi, [&](uint32_t, size_t at, D3 r) {
+        const double r2 = dot(r, r), rl = sqrt(r2);
+        const uint32_t q = tpos(p, rl);
+        if (r2 <= p.h2) w += p.analytic ? spline_w(p, rl) : a.W[q];
+        const double gs = !(rl <= p.h) ? 0.0 : p.analytic ? spline_gs(p, rl) : a.G[q];
+        a.GS[at] = gs;
+        const D3 gj = (-p.volume * gs) * r;
         sum += dot(gj, gj);
         gi -= gj;
-    }
+    });
+    w = lanes(p.lanes, w);
+    sum = lanes(p.lanes, sum);
+    gi = lanes(p.lanes, gi);
+    if (!first) return;
+    double rho = p.volume * p.wZero + p.volume * w;
     for (uint32_t b = 0; b < p.bodies; b++) {
         const double vb = a.VB[(size_t)b * p.n + i];
         if (vb > 0.0) {
@@ -405,95 +505,114 @@ __global__ void k_density_factor(P p, A a) {
     a.ALPHA[i] = sum > (double)kEps ? 1.0 / sum : 0.0;
 }
 
-__device__ double velocity_divergence(const P& p, const A& a, uint32_t i) {  // K4 :498-522, K17 :253-271
+// The passes' sums over a particle, complete in every lane but for the bodies' share, which the
+// writing lane adds.
+__device__ double velocity_divergence(const P& p, const A& a, uint32_t i, uint32_t l, bool first) {  // K4 :498-522, K17 :253-271
     const D3 xi = a.X[i], vi = a.V[i];
     double d = 0.0;
-    const uint32_t cnt = a.NCNT[i];
-    for (uint32_t j = 0; j < cnt; j++) {
-        const uint32_t k = nbr(a, i, j);
-        d += dot(vi - a.V[k], kgrad(p, a, xi - a.X[k]));
-    }
-    d *= p.volume;
-    for (uint32_t b = 0; b < p.bodies; b++) {
-        const double vb = a.VB[(size_t)b * p.n + i];
-        if (vb > 0.0) d += vb * dot(vi, kgrad(p, a, xi - a.XB[(size_t)b * p.n + i]));
-    }
+    pairs(p, a, i, l, xi, [&](uint32_t k, size_t at, D3 r) { d += a.GS[at] * dot(vi - a.V[k], r); });
+    d = lanes(p.lanes, d) * p.volume;
+    if (first)
+        for (uint32_t b = 0; b < p.bodies; b++) {
+            const double vb = a.VB[(size_t)b * p.n + i];
+            if (vb > 0.0) d += vb * dot(vi, kgrad(p, a, xi - a.XB[(size_t)b * p.n + i]));
+        }
     return d;
 }
-__device__ D3 pressure_accel(const P& p, const A& a, uint32_t i, const double* kap) {  // K5/K7/K18/K20
+__device__ D3 pressure_accel(const P& p, const A& a, uint32_t i, uint32_t l, bool first, const double* kap) {  // K5/K7/K18/K20
     const D3 xi = a.X[i];
     const double ki = kap[i];
     D3 acc = d3(0, 0, 0);
-    const uint32_t cnt = a.NCNT[i];
-    for (uint32_t j = 0; j < cnt; j++) {
-        const uint32_t k = nbr(a, i, j);
+    pairs(p, a, i, l, xi, [&](uint32_t k, size_t at, D3 r) {
         const double s = ki + kap[k];
-        if (fabs(s) > (double)kEps) acc += s * (-p.volume * kgrad(p, a, xi - a.X[k]));
-    }
-    if (fabs(ki) > (double)kEps)
+        if (fabs(s) > (double)kEps) acc += (s * (-p.volume * a.GS[at])) * r;
+    });
+    acc = lanes(p.lanes, acc);
+    if (first && fabs(ki) > (double)kEps)
         for (uint32_t b = 0; b < p.bodies; b++) {
             const double vb = a.VB[(size_t)b * p.n + i];
             if (vb > 0.0) acc += ki * (-vb * kgrad(p, a, xi - a.XB[(size_t)b * p.n + i]));
         }
     return acc;
 }
-__device__ double pressure_force(const P& p, const A& a, uint32_t i) {  // :280-315
+__device__ double pressure_force(const P& p, const A& a, uint32_t i, uint32_t l, bool first) {  // :280-315
     const D3 xi = a.X[i], ai = a.AP[i];
     double f = 0.0;
-    const uint32_t cnt = a.NCNT[i];
-    for (uint32_t j = 0; j < cnt; j++) {
-        const uint32_t k = nbr(a, i, j);
-        f += dot(ai - a.AP[k], kgrad(p, a, xi - a.X[k]));
-    }
-    f *= p.volume;
-    for (uint32_t b = 0; b < p.bodies; b++) {
-        const double vb = a.VB[(size_t)b * p.n + i];
-        if (vb > 0.0) f += vb * dot(ai, kgrad(p, a, xi - a.XB[(size_t)b * p.n + i]));
-    }
+    pairs(p, a, i, l, xi, [&](uint32_t k, size_t at, D3 r) { f += a.GS[at] * dot(ai - a.AP[k], r); });
+    f = lanes(p.lanes, f) * p.volume;
+    if (first)
+        for (uint32_t b = 0; b < p.bodies; b++) {
+            const double vb = a.VB[(size_t)b * p.n + i];
+            if (vb > 0.0) f += vb * dot(ai, kgrad(p, a, xi - a.XB[(size_t)b * p.n + i]));
+        }
     return f;
 }
 
+// Starts a loop: the reference's while condition with error 0, iteration 0.
+__global__ void k_loop_start(A a, LoopBounds b) {
+    Loop& L = *a.loop;
+    L.err = 0.0;
+    L.it = 0u;
+    L.done = ((0.0 > b.eta || 0u < b.mn) && 0u < b.mx) ? 0u : 1u;
+}
+// Ends an iteration of a Jacobi solve (nb partial residual sums).
+__global__ void __launch_bounds__(256) k_jacobi_decide(P p, A a, LoopBounds b, uint32_t nb) {
+    Loop& L = *a.loop;
+    if (L.done) return;
+    const double sum = block_fold(a.PART, nb, false);
+    if (threadIdx.x != 0) return;
+    L.err = -p.rho0 * sum / (double)p.n;
+    L.it++;
+    L.done = ((L.err > b.eta || L.it < b.mn) && L.it < b.mx) ? 0u : 1u;
+}
+
 // K4 ComputeDensityChangeKernel (:483-529)
-__global__ void k_div_init(P p, A a) {
-    F64_THREAD
-    double d = velocity_divergence(p, a, i);
+__global__ void __launch_bounds__(kLB) k_div_init(P p, A a) {
+    F64_LANES
+    double d = velocity_divergence(p, a, i, l, first);
+    if (!first) return;
     d = a.NCNT[i] < 20u ? 0.0 : fmax(d, 0.0);
     a.RHOADV[i] = d;
     a.ALPHA[i] *= p.dtInv;
     a.KAPPAV[i] = d * a.ALPHA[i];
 }
-__global__ void k_paccel(P p, A a, int div) {  // K5 / K18
-    F64_THREAD
-    a.AP[i] = pressure_accel(p, a, i, div ? a.KAPPAV : a.KAPPA);
+__global__ void __launch_bounds__(kLB) k_paccel(P p, A a, int div) {  // K5 / K18
+    if (a.loop->done) return;
+    F64_LANES
+    const D3 ap = pressure_accel(p, a, i, l, first, div ? a.KAPPAV : a.KAPPA);
+    if (first) a.AP[i] = ap;
 }
 // K6 DivergenceSolveIterationKernel (:531-553) / K19 PressureSolveIterationKernel (:317-340)
-__global__ void k_jacobi(P p, A a, int div) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    double res = 0.0;
-    if (i < p.n) {
+__global__ void __launch_bounds__(kLB) k_jacobi(P p, A a, int div) {
+    if (a.loop->done) return;
+    F64_LANES
+    double s = pressure_force(p, a, i, l, first), res = 0.0;
+    if (first) {
         if (div) {
-            const double s = pressure_force(p, a, i) * p.dt;
+            s *= p.dt;
             res = a.NCNT[i] < 20u ? 0.0 : fmin(-a.RHOADV[i] - s, 0.0);
             a.KAPPAV[i] -= res * a.ALPHA[i];
         } else {
-            const double s = pressure_force(p, a, i) * p.dt2;
+            s *= p.dt2;
             res = fmin(1.0 - a.RHOADV[i] - s, 0.0);
             a.KAPPA[i] -= res * a.ALPHA[i];
         }
         a.RES[i] = res;
     }
-    block_partial(a, res, false);
+    block_partial(a.PART, res, false);
 }
 // K7 ComputePressureAccelerationAndFactorKernel (:555-602) + K8 ClearAccelerationKernel (:24-37)
-__global__ void k_div_finish(P p, A a, int div) {
-    F64_THREAD
+__global__ void __launch_bounds__(kLB) k_div_finish(P p, A a, int div) {
+    F64_LANES
     if (div) {
-        const D3 ap = pressure_accel(p, a, i, a.KAPPAV);
-        a.AP[i] = ap;
-        a.V[i] += p.dt * ap;
-        a.ALPHA[i] *= p.dt;
+        const D3 ap = pressure_accel(p, a, i, l, first, a.KAPPAV);
+        if (first) {
+            a.AP[i] = ap;
+            a.V[i] += p.dt * ap;
+            a.ALPHA[i] *= p.dt;
+        }
     }
-    a.Acc[i] = d3(p.g[0], p.g[1], p.g[2]);
+    if (first) a.Acc[i] = d3(p.g[0], p.g[1], p.g[2]);
 }
 
 // K9 ComputeSurfaceTensionClassificationKernel (:881-958)
@@ -540,23 +659,23 @@ __global__ void k_st_classify(P p, A a) {
     }
 }
 // K10 ComputeSurfaceTensionNormalsAndCurvatureKernel (:960-1006)
-__global__ void k_st_smooth(P p, A a) {
-    F64_THREAD
-    if (!nonzero(a.N[i])) return;
-    const D3 xi = a.X[i];
+__global__ void __launch_bounds__(kLB) k_st_smooth(P p, A a) {
+    F64_LANES
     D3 nc = d3(0, 0, 0);
     double cc = 0.0, cf = 0.0;
-    const uint32_t cnt = a.NCNT[i];
-    for (uint32_t j = 0; j < cnt; j++) {
-        const uint32_t k = nbr(a, i, j);
-        if (nonzero(a.N[k])) {
-            const D3 e = a.X[k] - xi;
-            const double num = 1.0 - sqrt(dot(e, e)) / p.h;
-            nc += a.N[k] * num;
-            cc += a.CURV[k] * num;
-            cf += num;
-        }
-    }
+    if (nonzero(a.N[i]))
+        pairs(p, a, i, l, a.X[i], [&](uint32_t k, size_t, D3 r) {
+            if (nonzero(a.N[k])) {
+                const double num = 1.0 - sqrt(dot(r, r)) / p.h;
+                nc += a.N[k] * num;
+                cc += a.CURV[k] * num;
+                cf += num;
+            }
+        });
+    nc = lanes(p.lanes, nc);
+    cc = lanes(p.lanes, cc);
+    cf = lanes(p.lanes, cf);
+    if (!first || !nonzero(a.N[i])) return;
     if (dot(nc, nc) > 0.0) nc = normalized(nc);
     D3 ns = (1.0 - p.smoothing) * a.N[i] + p.smoothing * nc;
     if (dot(ns, ns) > 0.0) ns = normalized(ns);
@@ -600,16 +719,18 @@ __device__ bool visc_samples(const P& p, const A& a, uint32_t i, uint32_t b, D3 
     return true;
 }
 // K12 ComputeViscosityPreconditionerKernel (:604-684) + K13's b = v and the warm start g
-__global__ void k_visc_precond(P p, A a) {
-    F64_THREAD
+// (and each pair's coefficient 10 mu (m / rho) gs / (r^2 + 0.01 h^2) of the product)
+__global__ void __launch_bounds__(kLB) k_visc_precond(P p, A a) {
+    F64_LANES
     M3 res = {};
-    const D3 xi = a.X[i];
-    const uint32_t cnt = a.NCNT[i];
-    for (uint32_t j = 0; j < cnt; j++) {
-        const uint32_t k = nbr(a, i, j);
-        const D3 d = xi - a.X[k];
-        add_outer(res, 10.0 * p.dynVisc * (p.mass / a.RHO[k]) / (dot(d, d) + 0.01 * p.h2), d, kgrad(p, a, d));
-    }
+    pairs(p, a, i, l, a.X[i], [&](uint32_t k, size_t at, D3 r) {
+        const double c = 10.0 * p.dynVisc * (p.mass / a.RHO[k]) / (dot(r, r) + 0.01 * p.h2) * a.GS[at];
+        a.VS[at] = c;
+        add_outer(res, c, r, r);
+    });
+    for (int r = 0; r < 3; r++)
+        for (int c = 0; c < 3; c++) res.m[r][c] = lanes(p.lanes, res.m[r][c]);
+    if (!first) return;
     if (p.dynBVisc != 0.0)
         for (uint32_t b = 0; b < p.bodies; b++) {
             D3 dir[4], grad[4];
@@ -627,19 +748,16 @@ __global__ void k_visc_precond(P p, A a) {
     a.CG[i] = a.V[i] + a.DV[i];
 }
 // ComputeMatrixVecProdFunctionKernel (:758-842): out = A vec; sum of vec . out per block
-__global__ void k_matvec(P p, A a, const D3* vec, D3* out, int dotWith) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    double t = 0.0;
-    if (i < p.n) {
-        const D3 xi = a.X[i], vi = vec[i];
-        D3 acc = d3(0, 0, 0);
-        const uint32_t cnt = a.NCNT[i];
-        for (uint32_t j = 0; j < cnt; j++) {
-            const uint32_t k = nbr(a, i, j);
-            const D3 d = xi - a.X[k];
-            acc += (10.0 * p.dynVisc * (p.mass / a.RHO[k]) * dot(vi - vec[k], d) / (dot(d, d) + 0.01 * p.h2)) *
-                   kgrad(p, a, d);
-        }
+// (in the loop; of the first guess: out = b - A vec, sum of its square and of b's)
+__global__ void __launch_bounds__(kLB) k_matvec(P p, A a, const D3* vec, D3* out, int loop) {
+    if (loop && a.loop->done) return;
+    F64_LANES
+    const D3 xi = a.X[i], vi = vec[i];
+    D3 acc = d3(0, 0, 0);
+    pairs(p, a, i, l, xi, [&](uint32_t k, size_t at, D3 r) { acc += (a.VS[at] * dot(vi - vec[k], r)) * r; });
+    acc = lanes(p.lanes, acc);
+    double t = 0.0, t2 = 0.0;
+    if (first) {
         if (p.dynBVisc != 0.0)
             for (uint32_t b = 0; b < p.bodies; b++) {
                 D3 dir[4], grad[4];
@@ -648,50 +766,90 @@ __global__ void k_matvec(P p, A a, const D3* vec, D3* out, int dotWith) {
                 for (int k = 0; k < 4; k++)
                     acc += (10.0 * p.dynBVisc * vol * dot(vi, dir[k]) / (dot(dir[k], dir[k]) + 0.01 * p.h2)) * grad[k];
             }
-        const D3 r = vi - (p.dt / a.RHO[i]) * acc;
+        D3 r = vi - (p.dt / a.RHO[i]) * acc;
+        if (loop) {
+            t = dot(vi, r);
+        } else {
+            const D3 b = a.CB[i];
+            r = b - r;
+            t = dot(r, r);
+            t2 = dot(b, b);
+        }
         out[i] = r;
-        if (dotWith) t = dot(vi, r);
     }
-    block_partial(a, t, false);
+    block_partial(a.PART, t, false);
+    if (!loop) block_partial(a.PART2, t2, false);
 }
-// the CG's vector steps (DFSPHImplementation.cu:627-805); each reduces one dot product
-__global__ void k_cg_residual(P p, A a) {  // r = b - A g, sum |r|^2
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    double t = 0.0;
-    if (i < p.n) {
-        const D3 r = a.CB[i] - a.CT[i];
-        a.CR[i] = r;
-        t = dot(r, r);
-    }
-    block_partial(a, t, false);
+// Early outs of SolveViscosity (DFSPHImplementation.cu:627-675) from the sums of |r|^2 and |b|^2.
+__global__ void __launch_bounds__(256) k_cg_start(A a, LoopBounds b, uint32_t nb) {
+    const double rr = block_fold(a.PART, nb, false), rhs = block_fold(a.PART2, nb, false);
+    if (threadIdx.x != 0) return;
+    Loop& L = *a.loop;
+    L.it = 0u;
+    L.rr = rr;
+    L.rhs = rhs;
+    L.zeroG = rhs == 0.0 ? 1u : 0u;
+    L.thr = fmax(b.eta * b.eta * 0.0001 * rhs, (double)FLT_MIN);
+    L.done = rhs == 0.0 || rr < L.thr || !(0u >= b.mn && 0u < b.mx) ? 1u : 0u;
 }
-__global__ void k_dot(P p, A a, const D3* u, const D3* w) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    block_partial(a, i < p.n ? dot(u[i], w[i]) : 0.0, false);
-}
-__global__ void k_precondition(P p, A a, D3* out) {  // out = M^-1 r, sum r . out
+// the CG's vector steps (:677-805)
+__global__ void k_precondition(P p, A a) {  // p = M^-1 r, sum r . p
+    if (a.loop->done) return;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     double t = 0.0;
     if (i < p.n) {
         const D3 z = mul(a.MINV[i], a.CR[i]);
-        out[i] = z;
+        a.CP[i] = z;
         t = dot(a.CR[i], z);
     }
-    block_partial(a, t, false);
+    block_partial(a.PART, t, false);
 }
-__global__ void k_cg_update(P p, A a, double alpha) {  // g += alpha p, r -= alpha Ap, sum |r|^2
+__global__ void __launch_bounds__(256) k_cg_first(A a, uint32_t nb) {
+    if (a.loop->done) return;
+    const double rz = block_fold(a.PART, nb, false);
+    if (threadIdx.x == 0) a.loop->absNew = fabs(rz);
+}
+__global__ void __launch_bounds__(256) k_cg_alpha(A a, uint32_t nb) {
+    if (a.loop->done) return;
+    const double pap = block_fold(a.PART, nb, false);
+    if (threadIdx.x == 0) a.loop->alpha = a.loop->absNew / pap;
+}
+__global__ void k_cg_update(P p, A a) {  // g += alpha p, r -= alpha Ap, z = M^-1 r, sums |r|^2 and r . z
+    if (a.loop->done) return;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    double t = 0.0;
+    double t = 0.0, t2 = 0.0;
     if (i < p.n) {
+        const double alpha = a.loop->alpha;
         a.CG[i] += a.CP[i] * alpha;
-        a.CR[i] -= a.CT[i] * alpha;
-        t = dot(a.CR[i], a.CR[i]);
+        const D3 r = a.CR[i] - a.CT[i] * alpha;
+        a.CR[i] = r;
+        const D3 z = mul(a.MINV[i], r);
+        a.CZ[i] = z;
+        t = dot(r, r);
+        t2 = dot(r, z);
     }
-    block_partial(a, t, false);
+    block_partial(a.PART, t, false);
+    block_partial(a.PART2, t2, false);
 }
-__global__ void k_cg_p(P p, A a, double beta) {
+__global__ void __launch_bounds__(256) k_cg_decide(A a, LoopBounds b, uint32_t nb) {
+    Loop& L = *a.loop;
+    if (L.done) return;
+    const double rr = block_fold(a.PART, nb, false), rz = block_fold(a.PART2, nb, false);
+    if (threadIdx.x != 0) return;
+    L.rr = rr;
+    if (rr < L.thr) {
+        L.done = 1u;
+        return;
+    }
+    L.beta = fabs(rz) / L.absNew;
+    L.absNew = fabs(rz);
+    L.it++;
+    L.done = L.it >= b.mn && L.it < b.mx ? 0u : 1u;
+}
+__global__ void k_cg_p(P p, A a) {
+    if (a.loop->done) return;
     F64_THREAD
-    a.CP[i] = a.CP[i] * beta + a.CZ[i];
+    a.CP[i] = a.CP[i] * a.loop->beta + a.CZ[i];
 }
 // K15 ApplyViscosityForceKernel (:844-862)
 __global__ void k_visc_apply(P p, A a, int zeroG) {
@@ -708,24 +866,30 @@ __global__ void k_cfl(P p, A a) {
         const D3 w = a.V[i] + a.Acc[i] * p.dt;
         m = dot(w, w);
     }
-    block_partial(a, m, true);
+    block_partial(a.PART, m, true);
+}
+__global__ void __launch_bounds__(256) k_cfl_fold(A a, uint32_t nb) {
+    const double m = block_fold(a.PART, nb, true);
+    if (threadIdx.x == 0) a.loop->err = m;
 }
 __global__ void k_velocity(P p, A a) {  // K16 ComputeVelocityKernel (:39-52)
     F64_THREAD
     a.V[i] += p.dt * a.Acc[i];
 }
-__global__ void k_pres_init(P p, A a) {  // K17 ComputeDensityAdvectionKernel (:233-278)
-    F64_THREAD
-    const double d = velocity_divergence(p, a, i);
+__global__ void __launch_bounds__(kLB) k_pres_init(P p, A a) {  // K17 ComputeDensityAdvectionKernel (:233-278)
+    F64_LANES
+    const double d = velocity_divergence(p, a, i, l, first);
+    if (!first) return;
     const double rhoAdv = a.RHO[i] / p.rho0 + p.dt * d;
     a.RHOADV[i] = rhoAdv;
     a.ALPHA[i] *= p.dt2Inv;
     a.KAPPA[i] = -fmin(1.0 - rhoAdv, 0.0) * a.ALPHA[i];
 }
 // K20 ComputePressureAccelerationAndVelocityKernel (:434-481); K21 positions after all
-__global__ void k_pres_finish(P p, A a) {
-    F64_THREAD
-    const D3 ap = pressure_accel(p, a, i, a.KAPPA);
+__global__ void __launch_bounds__(kLB) k_pres_finish(P p, A a) {
+    F64_LANES
+    const D3 ap = pressure_accel(p, a, i, l, first, a.KAPPA);
+    if (!first) return;
     a.AP[i] = ap;
     a.V[i] += p.dt * ap;
 }
@@ -752,12 +916,16 @@ struct Fp64State {
     f64::P p{};
     std::vector<void*> allocs;
     void* cellAllocs[5] = {};  // CNT, START, FILL, BSUM (grown with the grid)
-    uint32_t cellCap = 0, blockCap = 0;
+    uint32_t cellCap = 0;
+    uint32_t n = 0, bodies = 0;    // what the buffers were made for
+    double radius = 0.0;           // what the tables were made for
+    f64::Loop* hLoop = nullptr;    // pinned
     double frameTime = 0.0;
     vfd_step_stats stats{};
     ~Fp64State() {
         for (void* q : allocs) cudaFree(q);
         for (void* q : cellAllocs) cudaFree(q);
+        cudaFreeHost(hLoop);
     }
 };
 
@@ -779,14 +947,21 @@ int falloc(Fp64State* f, T** ptr, size_t count) {
         if (e_ != cudaSuccess) return fail(VFD_E_CUDA, "FP64 path: %s: %s", #call, cudaGetErrorString(e_)); \
     } while (0)
 
-// Sum (or max) of the per-block partials of the last reduction kernel, in block order.
-int partials(Fp64State* f, uint32_t nb, cudaStream_t st, bool isMax, double& out) {
-    std::vector<double> h(nb);
-    FCK(cudaMemcpyAsync(h.data(), f->a.PART, sizeof(double) * nb, cudaMemcpyDeviceToHost, st));
+// The loop's state as of now.
+int read_loop(Fp64State* f, cudaStream_t st) {
+    FCK(cudaMemcpyAsync(f->hLoop, f->a.loop, sizeof(f64::Loop), cudaMemcpyDeviceToHost, st));
     FCK(cudaStreamSynchronize(st));
-    double t = 0.0;
-    for (uint32_t b = 0; b < nb; b++) t = isMax ? std::max(t, h[b]) : t + h[b];
-    out = t;
+    return VFD_OK;
+}
+
+// Runs launch() (an iteration) until the loop is done, `group` iterations between looks.
+template <class F>
+int run_loop(Fp64State* f, cudaStream_t st, uint32_t group, F&& launch) {
+    do {
+        for (uint32_t k = 0; k < group; k++) launch();
+        TRY(read_loop(f, st));
+        group = 4u;
+    } while (!f->hLoop->done);
     return VFD_OK;
 }
 
@@ -806,14 +981,19 @@ uint32_t samples_for(const vfd_desc& d, double dt) {
 // Creates (or rebuilds) the FP64 state from the scene's initial particles.
 int fp64_upload(vfd_sim* s) {
     if (s->scenes.size() != 1) return fail(VFD_E_STATE, "the FP64 path runs single-scene simulations");
-    delete s->fp64;
-    s->fp64 = new Fp64State();
-    Fp64State* f = s->fp64;
     const host::SceneHost& sc = s->scenes[0];
     const uint32_t n = (uint32_t)(sc.x0.size() / 3);
     const uint32_t nb = (uint32_t)sc.bodies.size();
+    // the buffers and tables of an earlier upload serve again where they fit
+    const bool keep = s->fp64 && s->fp64->n == n && s->fp64->bodies == nb && s->fp64->radius == (double)sc.desc.ParticleRadius;
+    if (!keep) {
+        delete s->fp64;
+        s->fp64 = new Fp64State();
+    }
+    Fp64State* f = s->fp64;
     f64::A& a = f->a;
     f64::P& p = f->p;
+    if (!keep) {
     TRY(falloc(f, &a.X, n)); TRY(falloc(f, &a.V, n)); TRY(falloc(f, &a.Acc, n)); TRY(falloc(f, &a.AP, n));
     TRY(falloc(f, &a.DV, n)); TRY(falloc(f, &a.N, n)); TRY(falloc(f, &a.NS, n));
     TRY(falloc(f, &a.XB, (size_t)std::max(1u, nb) * n)); TRY(falloc(f, &a.VB, (size_t)std::max(1u, nb) * n));
@@ -824,7 +1004,11 @@ int fp64_upload(vfd_sim* s) {
     TRY(falloc(f, &a.CB, n)); TRY(falloc(f, &a.CG, n)); TRY(falloc(f, &a.MINV, n));
     TRY(falloc(f, &a.NCNT, n)); TRY(falloc(f, &a.NBR, (size_t)n * kCap)); TRY(falloc(f, &a.KEY, n));
     TRY(falloc(f, &a.TMP, n)); TRY(falloc(f, &a.ORDER, n)); TRY(falloc(f, &a.MM, 6));
-    TRY(falloc(f, &a.PART, (n + kB - 1) / kB + 1));
+    const size_t parts = std::max((n + 63u) / 64u, (uint32_t)(((uint64_t)n * kL + kLB - 1u) / kLB)) + 1u;
+    TRY(falloc(f, &a.PART, parts)); TRY(falloc(f, &a.PART2, parts)); TRY(falloc(f, &a.loop, 1));
+    TRY(falloc(f, &a.GS, (size_t)n * kCap)); TRY(falloc(f, &a.VS, (size_t)n * kCap));
+    FCK(cudaMallocHost(&f->hLoop, sizeof(f64::Loop)));
+    }
     // SPH tables in double (PrecomputedDFSPHCubicKernel::SetRadius, Kernel/DFSPHKernels.h:13-41)
     const double r = (double)sc.desc.ParticleRadius, h = 4.0 * r, pi = 3.14159265358979323846;
     p.h = h;
@@ -847,6 +1031,7 @@ int fp64_upload(vfd_sim* s) {
         const double v = q <= 0.5 ? ((p.L * q) * (3.0 * q - 2.0)) * gq : (p.L * (-(1.0 - q) * (1.0 - q))) * gq;
         return v / x;
     };
+    if (!keep) {
     std::vector<double> W(kTableRes), G(kTableRes + 1), WM(kTableRes), GM(kTableRes);
     for (uint32_t k = 0; k < kTableRes; k++) {
         const double x = step * (double)k;
@@ -866,12 +1051,22 @@ int fp64_upload(vfd_sim* s) {
     FCK(cudaMemcpy(dG, GM.data(), sizeof(double) * kTableRes, cudaMemcpyHostToDevice));
     a.W = dW;
     a.G = dG;
+    f->n = n;
+    f->bodies = nb;
+    f->radius = r;
+    }
     p.wZero = calcW(0.0);
     a.halton = s->dHalton;
     a.bodyTab = s->dBodies;
     // constants (DFSPHImplementation::SetDescription, :318-368) in double
     const vfd_desc& d = sc.desc;
     p.n = n;
+    // Few particles leave the chain of a thread (8 lanes), many the FP64 pipe, which the lanes'
+    // shuffled sums load too (1). Two steps of a viscous drop with 8, 4, 2, 1 lanes, ms: 1.8, 1.9,
+    // 2.3, 2.8 at 1,000 particles; 2.1, 2.1, 2.2, 2.8 at 8,000; 3.0, 2.8, 2.7, 3.1 at 16,000; 7.6,
+    // 6.7, 6.2, 6.5 at 66,000; 16.3, 13.8, 12.7, 12.3 at 150,000; 111, 92, 82, 79 at 1M.
+    p.lanesLog2 = n < 4000u ? 3u : n < 12000u ? 2u : n < 100000u ? 1u : 0u;
+    p.lanes = 1u << p.lanesLog2;
     p.bodies = nb;
     p.bodyBegin = 0;
     p.analytic = s->analyticKernel ? 1u : 0u;
@@ -922,11 +1117,14 @@ int fp64_step(vfd_sim* s, vfd_step_stats* out) {
     vfd_step_stats& S = f->stats;
     S.Flags = 0;
     if (n == 0) return VFD_OK;
-    const uint32_t g = (n + kB - 1) / kB;
+    // a thread per particle in blocks small enough to reach every SM; eight lanes per particle
+    const uint32_t tb = n < 300000u ? 64u : kB, g = (n + tb - 1u) / tb;
+    const uint32_t gs = (uint32_t)(((uint64_t)n * kL + kLB - 1u) / kLB);
+    const uint32_t gl = (uint32_t)(((uint64_t)n * p.lanes + kLB - 1u) / kLB);
     // ---- neighbour search (ParticleSearch::FindNeighbors)
     const int init[6] = {INT_MAX, INT_MAX, INT_MAX, INT_MIN, INT_MIN, INT_MIN};
     FCK(cudaMemcpyAsync(a.MM, init, sizeof(init), cudaMemcpyHostToDevice, st));
-    f64::k_minmax<<<g, kB, 0, st>>>(p, a);
+    f64::k_minmax<<<g, tb, 0, st>>>(p, a);
     int mm[6];
     FCK(cudaMemcpyAsync(mm, a.MM, sizeof(mm), cudaMemcpyDeviceToHost, st));
     FCK(cudaStreamSynchronize(st));
@@ -957,90 +1155,73 @@ int fp64_step(vfd_sim* s, vfd_step_stats* out) {
     a.BSUM = (uint32_t*)f->cellAllocs[3];
     FCK(cudaMemsetAsync(a.CNT, 0, sizeof(uint32_t) * a.cells, st));
     FCK(cudaMemsetAsync(a.FILL, 0, sizeof(uint32_t) * a.cells, st));
-    f64::k_keys<<<g, kB, 0, st>>>(p, a);
+    f64::k_keys<<<g, tb, 0, st>>>(p, a);
     f64::k_scan_blocks<<<sb, 1024, 0, st>>>(a);
-    f64::k_scan_carry<<<1, 32, 0, st>>>(a, sb);
+    f64::k_scan_carry<<<1, 1024, 0, st>>>(a, sb);
     f64::k_scan_add<<<sb, 1024, 0, st>>>(a);
-    f64::k_slots<<<g, kB, 0, st>>>(p, a);
-    f64::k_order<<<g, kB, 0, st>>>(p, a);
-    f64::k_neighbors<<<g, kB, 0, st>>>(p, a);
+    f64::k_slots<<<g, tb, 0, st>>>(p, a);
+    f64::k_order<<<g, tb, 0, st>>>(p, a);
+    f64::k_neighbors<<<gs, kLB, 0, st>>>(p, a);
     FCK(cudaGetLastError());
     // ---- boundary, density, factor
-    f64::k_boundary<<<g, kB, 0, st>>>(p, a);
-    f64::k_density_factor<<<g, kB, 0, st>>>(p, a);
+    f64::k_boundary<<<g, tb, 0, st>>>(p, a);
+    f64::k_density_factor<<<gl, kLB, 0, st>>>(p, a);
     // ---- divergence solve (ComputeDivergence, :506-575)
     const bool div = d.EnableDivergenceSolverError != 0;
     uint32_t itD = 0;
     double errD = 0.0;
     if (div) {
-        f64::k_div_init<<<g, kB, 0, st>>>(p, a);
+        f64::k_div_init<<<gl, kLB, 0, st>>>(p, a);
         const double eta = p.dtInv * (double)d.MaxDivergenceSolverError * 0.0001 * p.rho0;
-        while ((errD > eta || itD < d.MinDivergenceSolverIterations) && itD < d.MaxDivergenceSolverIterations) {
-            f64::k_paccel<<<g, kB, 0, st>>>(p, a, 1);
-            f64::k_jacobi<<<g, kB, 0, st>>>(p, a, 1);
-            double sum;
-            TRY(partials(f, g, st, false, sum));
-            errD = -p.rho0 * sum / (double)n;
-            itD++;
-        }
+        const LoopBounds lb{eta, d.MinDivergenceSolverIterations, d.MaxDivergenceSolverIterations};
+        f64::k_loop_start<<<1, 1, 0, st>>>(a, lb);
+        TRY(run_loop(f, st, 2u, [&]() {
+            f64::k_paccel<<<gl, kLB, 0, st>>>(p, a, 1);
+            f64::k_jacobi<<<gl, kLB, 0, st>>>(p, a, 1);
+            f64::k_jacobi_decide<<<1, 256, 0, st>>>(p, a, lb, gl);
+        }));
+        itD = f->hLoop->it;
+        errD = f->hLoop->err;
         if (itD >= d.MaxDivergenceSolverIterations && d.MaxDivergenceSolverIterations > 0 && errD > eta)
             S.Flags |= VFD_FLAG_DIVERGENCE_CAP;
     }
-    f64::k_div_finish<<<g, kB, 0, st>>>(p, a, div ? 1 : 0);
+    f64::k_div_finish<<<gl, kLB, 0, st>>>(p, a, div ? 1 : 0);
     // ---- surface tension (:810-839)
     const uint32_t samplesUsed = p.stSamples;
     if (d.EnableSurfaceTensionSolver) {
-        f64::k_st_classify<<<g, kB, 0, st>>>(p, a);
-        f64::k_st_smooth<<<g, kB, 0, st>>>(p, a);
-        for (uint32_t pass = 0; pass < d.SurfaceTensionSmoothPassCount; pass++) f64::k_st_blend<<<g, kB, 0, st>>>(p, a);
+        f64::k_st_classify<<<g, tb, 0, st>>>(p, a);
+        f64::k_st_smooth<<<gl, kLB, 0, st>>>(p, a);
+        for (uint32_t pass = 0; pass < d.SurfaceTensionSmoothPassCount; pass++) f64::k_st_blend<<<g, tb, 0, st>>>(p, a);
     }
     // ---- viscosity (ComputeViscosity + SolveViscosity, :577-808)
     uint32_t itV = 0;
     double errV = 0.0;
     if (d.EnableViscositySolver) {
-        f64::k_visc_precond<<<g, kB, 0, st>>>(p, a);
-        f64::k_matvec<<<g, kB, 0, st>>>(p, a, a.CG, a.CT, 0);
-        f64::k_cg_residual<<<g, kB, 0, st>>>(p, a);
-        double rr;
-        TRY(partials(f, g, st, false, rr));
-        f64::k_dot<<<g, kB, 0, st>>>(p, a, a.CB, a.CB);
-        double rhs;
-        TRY(partials(f, g, st, false, rhs));
-        int zeroG = 0;
-        if (rhs == 0.0) {
-            zeroG = 1;
-        } else {
-            const double e = (double)d.MaxViscositySolverError;
-            const double thr = std::max(e * e * 0.0001 * rhs, (double)FLT_MIN);
-            if (!(rr < thr)) {
-                f64::k_precondition<<<g, kB, 0, st>>>(p, a, a.CP);
-                double absNew;
-                TRY(partials(f, g, st, false, absNew));
-                absNew = std::fabs(absNew);
-                while (itV >= d.MinViscositySolverIterations && itV < d.MaxViscositySolverIterations) {
-                    f64::k_matvec<<<g, kB, 0, st>>>(p, a, a.CP, a.CT, 1);
-                    double pap;
-                    TRY(partials(f, g, st, false, pap));
-                    f64::k_cg_update<<<g, kB, 0, st>>>(p, a, absNew / pap);
-                    TRY(partials(f, g, st, false, rr));
-                    if (rr < thr) break;
-                    f64::k_precondition<<<g, kB, 0, st>>>(p, a, a.CZ);
-                    const double absOld = absNew;
-                    TRY(partials(f, g, st, false, absNew));
-                    absNew = std::fabs(absNew);
-                    f64::k_cg_p<<<g, kB, 0, st>>>(p, a, absNew / absOld);
-                    itV++;
-                }
-                if (itV >= d.MaxViscositySolverIterations && rr >= thr) S.Flags |= VFD_FLAG_VISCOSITY_CAP;
-            }
-            errV = std::sqrt(rr / rhs);
-        }
-        f64::k_visc_apply<<<g, kB, 0, st>>>(p, a, zeroG);
+        f64::k_visc_precond<<<gl, kLB, 0, st>>>(p, a);
+        const LoopBounds lb{(double)d.MaxViscositySolverError, d.MinViscositySolverIterations, d.MaxViscositySolverIterations};
+        f64::k_matvec<<<gl, kLB, 0, st>>>(p, a, a.CG, a.CR, 0);
+        f64::k_cg_start<<<1, 256, 0, st>>>(a, lb, gl);
+        f64::k_precondition<<<g, tb, 0, st>>>(p, a);
+        f64::k_cg_first<<<1, 256, 0, st>>>(a, g);
+        TRY(run_loop(f, st, 1u, [&]() {
+            f64::k_matvec<<<gl, kLB, 0, st>>>(p, a, a.CP, a.CT, 1);
+            f64::k_cg_alpha<<<1, 256, 0, st>>>(a, gl);
+            f64::k_cg_update<<<g, tb, 0, st>>>(p, a);
+            f64::k_cg_decide<<<1, 256, 0, st>>>(a, lb, g);
+            f64::k_cg_p<<<g, tb, 0, st>>>(p, a);
+        }));
+        const f64::Loop& L = *f->hLoop;
+        const int zeroG = (int)L.zeroG;
+        itV = L.it;
+        if (!zeroG && itV >= d.MaxViscositySolverIterations && L.rr >= L.thr) S.Flags |= VFD_FLAG_VISCOSITY_CAP;
+        if (!zeroG) errV = std::sqrt(L.rr / L.rhs);
+        f64::k_visc_apply<<<g, tb, 0, st>>>(p, a, zeroG);
     }
     // ---- CFL time step (ComputeTimeStepSize, :395-441)
-    f64::k_cfl<<<g, kB, 0, st>>>(p, a);
-    double mv;
-    TRY(partials(f, g, st, true, mv));
+    f64::k_cfl<<<g, tb, 0, st>>>(p, a);
+    f64::k_cfl_fold<<<1, 256, 0, st>>>(a, g);
+    TRY(read_loop(f, st));
+    double mv = f->hLoop->err;
     mv = std::max(0.1, mv);
     if (mv < 1.0e-9) mv = 1.0e-9;
     double dt = 0.4 * (p.diam / std::sqrt(mv));
@@ -1049,24 +1230,23 @@ int fp64_step(vfd_sim* s, vfd_step_stats* out) {
     set_dt(p, dt);
     p.stSamples = samples_for(d, dt);
     f->frameTime += dt;
-    f64::k_velocity<<<g, kB, 0, st>>>(p, a);
+    f64::k_velocity<<<g, tb, 0, st>>>(p, a);
     // ---- pressure solve (ComputePressure, :443-504)
-    f64::k_pres_init<<<g, kB, 0, st>>>(p, a);
+    f64::k_pres_init<<<gl, kLB, 0, st>>>(p, a);
     const double eta = (double)d.MaxPressureSolverError * 0.0001 * p.rho0;
-    uint32_t itP = 0;
-    double errP = 0.0;
-    while ((errP > eta || itP < d.MinPressureSolverIterations) && itP < d.MaxPressureSolverIterations) {
-        f64::k_paccel<<<g, kB, 0, st>>>(p, a, 0);
-        f64::k_jacobi<<<g, kB, 0, st>>>(p, a, 0);
-        double sum;
-        TRY(partials(f, g, st, false, sum));
-        errP = -p.rho0 * sum / (double)n;
-        itP++;
-    }
+    const LoopBounds lp{eta, d.MinPressureSolverIterations, d.MaxPressureSolverIterations};
+    f64::k_loop_start<<<1, 1, 0, st>>>(a, lp);
+    TRY(run_loop(f, st, 2u, [&]() {
+        f64::k_paccel<<<gl, kLB, 0, st>>>(p, a, 0);
+        f64::k_jacobi<<<gl, kLB, 0, st>>>(p, a, 0);
+        f64::k_jacobi_decide<<<1, 256, 0, st>>>(p, a, lp, gl);
+    }));
+    const uint32_t itP = f->hLoop->it;
+    const double errP = f->hLoop->err;
     if (itP >= d.MaxPressureSolverIterations && d.MaxPressureSolverIterations > 0 && errP > eta)
         S.Flags |= VFD_FLAG_PRESSURE_CAP;
-    f64::k_pres_finish<<<g, kB, 0, st>>>(p, a);
-    f64::k_position<<<g, kB, 0, st>>>(p, a);
+    f64::k_pres_finish<<<gl, kLB, 0, st>>>(p, a);
+    f64::k_position<<<g, tb, 0, st>>>(p, a);
     FCK(cudaGetLastError());
     FCK(cudaStreamSynchronize(st));
     if (S.FrameIndex < d.FrameCount && f->frameTime >= (double)d.FrameLength) {  // :148-167

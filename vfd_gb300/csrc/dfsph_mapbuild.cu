@@ -9,9 +9,7 @@
 #include <cfloat>
 #include <climits>
 #include <cmath>
-#include <map>
 #include <memory>
-#include <utility>
 #include <vector>
 
 #include "dfsph_common.cuh"
@@ -140,44 +138,128 @@ __device__ inline float closest_on_triangle(float3 p, float3 a, float3 b, float3
 }
 
 constexpr uint32_t kMeshBlock = 128;
-constexpr uint32_t kMeshTile = 256;  // faces staged in shared memory per pass
+constexpr uint32_t kMeshGroup = 32;  // consecutive faces that share a bounding sphere
+constexpr uint32_t kMeshLanes = 8;   // lanes per node
+
+// Bounding sphere (centre, radius) of each group of faces, a warp a group. The radius is
+// rounded up by far more than the rounding of the bounds that use it.
+__global__ void __launch_bounds__(kMeshBlock) k_mesh_groups(const float4* corners, uint32_t nf, float4* spheres) {
+    const uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
+    if (g * kMeshGroup >= nf) return;
+    const uint32_t f = min(g * kMeshGroup + lane, nf - 1u);
+    float3 c[3], lo, hi;
+    for (int k = 0; k < 3; k++) {
+        const float4 v = corners[3 * (size_t)f + k];
+        c[k] = make_float3(v.x, v.y, v.z);
+        lo = k ? make_float3(fminf(lo.x, v.x), fminf(lo.y, v.y), fminf(lo.z, v.z)) : c[k];
+        hi = k ? make_float3(fmaxf(hi.x, v.x), fmaxf(hi.y, v.y), fmaxf(hi.z, v.z)) : c[k];
+    }
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) {
+        lo = make_float3(fminf(lo.x, __shfl_xor_sync(0xffffffffu, lo.x, o)), fminf(lo.y, __shfl_xor_sync(0xffffffffu, lo.y, o)),
+                         fminf(lo.z, __shfl_xor_sync(0xffffffffu, lo.z, o)));
+        hi = make_float3(fmaxf(hi.x, __shfl_xor_sync(0xffffffffu, hi.x, o)), fmaxf(hi.y, __shfl_xor_sync(0xffffffffu, hi.y, o)),
+                         fmaxf(hi.z, __shfl_xor_sync(0xffffffffu, hi.z, o)));
+    }
+    const float3 m = 0.5f * (lo + hi);
+    float r2 = 0.0f;
+    for (int k = 0; k < 3; k++) r2 = fmaxf(r2, dot3(c[k] - m, c[k] - m));
+    const float top = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(r2)));
+    // (relative to the coordinates too: the node's distance to the centre rounds with them)
+    if (lane == 0) spheres[g] = make_float4(m.x, m.y, m.z, 1.0001f * sqrtf(top) + 1.0e-5f * (fabsf(m.x) + fabsf(m.y) + fabsf(m.z)));
+}
 
 // Field 0 of a mesh map: sign * (signed distance - tolerance) at every node
 // (RigidBody.cu:38-40; SDF.cu:16-36 for the sampler's map, tolerance 0). The distance is
 // the minimum over all faces (MeshDistance::Distance, MeshDistance.cpp:58-118, ties to the
 // lowest face index); it is negative when p - q points against the pseudo-normal of the
-// closest feature (MeshDistance::SignedDistance, MeshDistance.cpp:187-228). One thread per
-// node; the block walks the faces in tiles staged through shared memory.
+// closest feature (MeshDistance::SignedDistance, MeshDistance.cpp:187-228). Eight lanes take a
+// node: they find the group of faces with the nearest centre, measure it, and then only the
+// groups whose sphere comes nearer than the nearest face so far, four faces a lane. Meshes
+// whose consecutive faces lie together, as exported ones do, keep a few groups a node; any
+// order gives the same result. Measuring every face for every node (61,740 nodes, 5,120
+// faces) took 1718 us, this 331 us (20,480 faces, 262,548 nodes: 13.9 ms and 1.6).
 __global__ void __launch_bounds__(kMeshBlock) k_map_field0_mesh(const BoxMap* mp, const float4* corners,
-                                                                const float4* normals, uint32_t nf, float* nodes) {
-    __shared__ float4 tile[kMeshTile * 3];
+                                                                const float4* normals, const float4* spheres,
+                                                                uint32_t nf, float* nodes) {
     const BoxMap& m = *mp;
-    const uint32_t l = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool live = l < m.nodeCount;
-    float pv[3] = {0.0f, 0.0f, 0.0f};
-    if (live) node_position(m, l, pv);
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, lane = t % kMeshLanes;
+    const uint32_t shift = threadIdx.x & 31u & ~(kMeshLanes - 1u), mask = ((1u << kMeshLanes) - 1u) << shift;
+    const uint32_t l = t / kMeshLanes;
+    if (l >= m.nodeCount) return;  // whole groups of lanes
+    float pv[3];
+    node_position(m, l, pv);
     const float3 p = make_float3(pv[0], pv[1], pv[2]);
+    const uint32_t ng = (nf + kMeshGroup - 1u) / kMeshGroup;
     float best = FLT_MAX;
-    uint32_t bestFace = 0;
-    for (uint32_t base = 0; base < nf; base += kMeshTile) {
-        const uint32_t cnt = min(kMeshTile, nf - base);
-        __syncthreads();
-        for (uint32_t q = threadIdx.x; q < 3u * cnt; q += blockDim.x) tile[q] = corners[3 * (size_t)base + q];
-        __syncthreads();
-        if (!live) continue;
-        for (uint32_t f = 0; f < cnt; f++) {
-            const float4 a = tile[3 * f], b = tile[3 * f + 1], c = tile[3 * f + 2];
+    uint32_t bestFace = 0xFFFFFFFFu;
+    auto meet = [&]() {  // the nearest face of the lanes, ties to the lowest index
+#pragma unroll
+        for (uint32_t o = kMeshLanes / 2u; o > 0u; o >>= 1) {
+            const float d = __shfl_xor_sync(mask, best, o);
+            const uint32_t f = __shfl_xor_sync(mask, bestFace, o);
+            if (d < best || (d == best && f < bestFace)) {
+                best = d;
+                bestFace = f;
+            }
+        }
+    };
+    auto measure = [&](uint32_t g) {
+        for (uint32_t f = g * kMeshGroup + lane; f < min((g + 1u) * kMeshGroup, nf); f += kMeshLanes) {
+            const float4 a = __ldg(corners + 3 * (size_t)f), b = __ldg(corners + 3 * (size_t)f + 1),
+                         c = __ldg(corners + 3 * (size_t)f + 2);
             float3 q;
             int feature;
             const float d2 = closest_on_triangle(p, make_float3(a.x, a.y, a.z), make_float3(b.x, b.y, b.z),
                                                  make_float3(c.x, c.y, c.z), q, feature);
-            if (d2 < best) {
+            if (d2 < best || (d2 == best && f < bestFace)) {
                 best = d2;
-                bestFace = base + f;
+                bestFace = f;
             }
         }
+        meet();
+    };
+    float near = FLT_MAX;
+    uint32_t first = 0u;
+    for (uint32_t g = lane; g < ng; g += kMeshLanes) {
+        const float4 s = __ldg(spheres + g);
+        const float3 e = p - make_float3(s.x, s.y, s.z);
+        const float d2 = dot3(e, e);
+        if (d2 < near) {
+            near = d2;
+            first = g;
+        }
     }
-    if (!live) return;
+#pragma unroll
+    for (uint32_t o = kMeshLanes / 2u; o > 0u; o >>= 1) {
+        const float d = __shfl_xor_sync(mask, near, o);
+        const uint32_t g = __shfl_xor_sync(mask, first, o);
+        if (d < near || (d == near && g < first)) {
+            near = d;
+            first = g;
+        }
+    }
+    measure(first);
+    for (uint32_t base = 0; base < ng; base += kMeshLanes) {
+        const uint32_t g = base + lane;
+        const bool other = g < ng && g != first;
+        float bound = 0.0f;  // no face of the group is nearer
+        if (other) {
+            const float4 s = __ldg(spheres + g);
+            const float3 e = p - make_float3(s.x, s.y, s.z);
+            bound = sqrtf(dot3(e, e)) * 0.9999f - s.w;
+        }
+        uint32_t todo = __ballot_sync(mask, other && !(bound > 0.0f && bound * bound > best)) >> shift & 0xFFu;
+        while (todo) {
+            const uint32_t k = (uint32_t)__ffs((int)todo) - 1u;
+            todo &= todo - 1u;
+            const float b = __shfl_sync(mask, bound, k, kMeshLanes);
+            if (b > 0.0f && b * b > best) continue;  // nearer faces have been found since
+            measure(base + k);
+        }
+    }
+    if (lane != 0u) return;
+    if (bestFace == 0xFFFFFFFFu) bestFace = 0u;
     const float4 a = corners[3 * (size_t)bestFace], b = corners[3 * (size_t)bestFace + 1],
                  c = corners[3 * (size_t)bestFace + 2];
     float3 q;
@@ -243,17 +325,26 @@ int prepare_mesh(const float* vtx, uint32_t nv, const uint32_t* tri, uint32_t nf
     }
     // opposite face of each half-edge (face f, edge k = (tri[k], tri[(k+1)%3])); -1 on a border
     std::vector<int64_t> opp(3 * (size_t)nf, -1);
-    std::multimap<std::pair<uint32_t, uint32_t>, uint32_t> open;  // unpaired half-edges by (source, target)
+    // The unpaired half-edges of each source vertex, in face order, as a list threaded through
+    // `next`: a vertex has about six (an ordered map over all of them took most of the set-up).
+    constexpr uint32_t kNone = 0xFFFFFFFFu;
+    std::vector<uint32_t> head(nv, kNone), tail(nv, kNone), next(3 * (size_t)nf, kNone);
     for (uint32_t f = 0; f < nf; f++)
         for (uint32_t k = 0; k < 3; k++) {
-            const uint32_t u = tri[3 * f + k], v = tri[3 * f + (k + 1) % 3];
-            auto it = open.lower_bound({v, u});  // the earliest unpaired (v, u)
-            if (it != open.end() && it->first == std::make_pair(v, u)) {
-                opp[3 * (size_t)f + k] = it->second / 3;
-                opp[it->second] = f;
-                open.erase(it);
+            const uint32_t e = 3 * f + k, u = tri[e], v = tri[3 * f + (k + 1) % 3];
+            uint32_t before = kNone, o = head[v];  // the earliest unpaired (v, u)
+            while (o != kNone && tri[3 * (o / 3) + (o % 3 + 1) % 3] != u) {
+                before = o;
+                o = next[o];
+            }
+            if (o != kNone) {
+                opp[e] = o / 3;
+                opp[o] = f;
+                (before == kNone ? head[v] : next[before]) = next[o];
+                if (tail[v] == o) tail[v] = before;
             } else {
-                open.emplace(std::make_pair(u, v), 3 * f + k);
+                (tail[u] == kNone ? head[u] : next[tail[u]]) = e;
+                tail[u] = e;
             }
         }
     out.corners.resize(3 * (size_t)nf);
@@ -413,6 +504,7 @@ struct MapBuild {
     uint32_t* dc = nullptr;
     float4* dcorner = nullptr;
     float4* dnormal = nullptr;
+    float4* dsphere = nullptr;
     MapBuild() = default;
     MapBuild(const MapBuild&) = delete;
     MapBuild& operator=(const MapBuild&) = delete;
@@ -422,6 +514,7 @@ struct MapBuild {
         cudaFree(dc);
         cudaFree(dcorner);
         cudaFree(dnormal);
+        cudaFree(dsphere);
     }
 };
 
@@ -469,7 +562,12 @@ static cudaError_t map_build_fields(const BoxMap& hm, const std::vector<uint32_t
             e = cudaMemcpy(b.dnormal, mesh->normals.data(), sizeof(float4) * mesh->normals.size(),
                            cudaMemcpyHostToDevice);
         if (e != cudaSuccess) return e;
-        k_map_field0_mesh<<<(nn + kMeshBlock - 1) / kMeshBlock, kMeshBlock>>>(b.dm, b.dcorner, b.dnormal, nf, b.dn);
+        const uint32_t ng = (nf + kMeshGroup - 1u) / kMeshGroup;
+        e = cudaMalloc(&b.dsphere, sizeof(float4) * std::max(1u, ng));
+        if (e != cudaSuccess) return e;
+        if (ng) k_mesh_groups<<<(ng * 32u + kMeshBlock - 1u) / kMeshBlock, kMeshBlock>>>(b.dcorner, nf, b.dsphere);
+        k_map_field0_mesh<<<(uint32_t)(((uint64_t)nn * kMeshLanes + kMeshBlock - 1u) / kMeshBlock), kMeshBlock>>>(
+            b.dm, b.dcorner, b.dnormal, b.dsphere, nf, b.dn);
     } else {
         k_map_field0<<<(nn + 255) / 256, 256>>>(b.dm, b.dn);
     }

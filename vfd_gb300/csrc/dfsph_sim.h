@@ -154,6 +154,8 @@ struct SceneHost {
     std::vector<float> x0, v0;
     std::vector<BodyHost> bodies;
     uint32_t emitted = 0;  // particles appended by vfd_emit since the last upload
+    bool boundsKnown = false;  // lo, hi: bounds of x0
+    double lo[3], hi[3];
     uint32_t count() const { return (uint32_t)(x0.size() / 3) + emitted; }
 };
 
@@ -207,6 +209,8 @@ struct vfd_sim {
     vfd::Dev dev[2]{};
     int cs = 0;  // set holding the current carried state
     float4* XB = nullptr;
+    float* dInit = nullptr;      // initial positions, then velocities, 3 floats per slot each; null: no room
+    bool initValid = false;      // dInit holds the fluid objects
     float* dStage = nullptr;     // 3 floats per particle, original order
     float* dStage2 = nullptr;    // a second one (velocities beside positions in vfd_set_state)
     vfd::SceneDev* dScenes = nullptr;

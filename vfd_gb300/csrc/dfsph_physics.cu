@@ -36,11 +36,11 @@ __device__ __forceinline__ void set_condition(const Dev& d, int loop, uint32_t v
 
 // Batches: lists the scenes for which active(s) holds into loop `loop`'s work list
 // (prefix sums of their particle counts, and of their staged tiles, by a block-wide scan). One
-// block of 256 threads, called by all of them after the scenes' flags are final.
+// block of whole warps, called by all of its threads after the scenes' flags are final.
 template <class F>
 __device__ void build_work_list(const Dev& d, int loop, F active) {
-    __shared__ uint32_t scanP[256], scanA[256], scanT[256];
-    __shared__ uint32_t runP, runA, runT;
+    __shared__ uint3 part[32];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     const bool halo = halo_on(d);
     uint32_t* w = d.WORK + (size_t)loop * d.workStride;
     uint32_t* pre = w + 2;
@@ -48,42 +48,41 @@ __device__ void build_work_list(const Dev& d, int loop, F active) {
     uint32_t* tileN = beg + d.nscenes;
     uint32_t* tilePre = tileN + 1;
     uint32_t* tileBeg = tilePre + d.nscenes;
-    if (threadIdx.x == 0) runP = runA = runT = 0u;
-    __syncthreads();
+    uint32_t runP = 0u, runA = 0u, runT = 0u;  // of the scenes before this chunk, in every thread
     for (uint32_t c = 0; c < d.nscenes; c += blockDim.x) {
         const uint32_t sc = c + threadIdx.x;
         const bool a = sc < d.nscenes && active(sc);
         const uint32_t cnt = a ? d.scenes[sc].count : 0u;
         const uint2 tiles = a && halo ? d.haloScene[sc] : make_uint2(0u, 0u);
-        scanP[threadIdx.x] = cnt;
-        scanA[threadIdx.x] = a ? 1u : 0u;
-        scanT[threadIdx.x] = tiles.y;
-        __syncthreads();
-        for (uint32_t off = 1; off < blockDim.x; off <<= 1) {
-            const uint32_t tp = threadIdx.x >= off ? scanP[threadIdx.x - off] : 0u;
-            const uint32_t ta = threadIdx.x >= off ? scanA[threadIdx.x - off] : 0u;
-            const uint32_t tt = threadIdx.x >= off ? scanT[threadIdx.x - off] : 0u;
-            __syncthreads();
-            scanP[threadIdx.x] += tp;
-            scanA[threadIdx.x] += ta;
-            scanT[threadIdx.x] += tt;
-            __syncthreads();
+        uint32_t p = cnt, t = tiles.y;
+#pragma unroll
+        for (uint32_t o = 1; o < 32u; o <<= 1) {
+            const uint32_t tp = __shfl_up_sync(0xffffffffu, p, o), tt = __shfl_up_sync(0xffffffffu, t, o);
+            if (lane >= o) {
+                p += tp;
+                t += tt;
+            }
         }
+        const uint32_t on = __ballot_sync(0xffffffffu, a);
+        if (lane == 31u) part[warp] = make_uint3(p, __popc(on), t);
+        __syncthreads();
+        const uint3 q = lane < warps ? part[lane] : make_uint3(0u, 0u, 0u);
+        const bool earlier = lane < warp;
+        const uint32_t beforeP = __reduce_add_sync(0xffffffffu, earlier ? q.x : 0u),
+                       beforeA = __reduce_add_sync(0xffffffffu, earlier ? q.y : 0u),
+                       beforeT = __reduce_add_sync(0xffffffffu, earlier ? q.z : 0u);
         if (a) {
-            const uint32_t idx = runA + scanA[threadIdx.x] - 1u;
-            pre[idx] = runP + scanP[threadIdx.x] - cnt;
+            const uint32_t idx = runA + beforeA + __popc(on & ((1u << lane) - 1u));
+            pre[idx] = runP + beforeP + p - cnt;
             beg[idx] = d.scenes[sc].begin;
             if (halo) {
-                tilePre[idx] = runT + scanT[threadIdx.x] - tiles.y;
+                tilePre[idx] = runT + beforeT + t - tiles.y;
                 tileBeg[idx] = tiles.x;
             }
         }
-        __syncthreads();
-        if (threadIdx.x == blockDim.x - 1u) {
-            runP += scanP[threadIdx.x];
-            runA += scanA[threadIdx.x];
-            runT += scanT[threadIdx.x];
-        }
+        runP += __reduce_add_sync(0xffffffffu, q.x);
+        runA += __reduce_add_sync(0xffffffffu, q.y);
+        runT += __reduce_add_sync(0xffffffffu, q.z);
         __syncthreads();
     }
     if (threadIdx.x == 0) {
@@ -396,11 +395,16 @@ __device__ __forceinline__ bool jacobi_control(SceneDev& S, double sum) {
     return again;
 }
 
-// The loop controllers run as one block. With one scene its first warp folds the
-// buckets together (fold_acc_warp) and lane 0 takes the decisions; a batch gives each
-// scene a thread.
+// The loop controllers run as one block. With one scene its one warp folds the buckets
+// together (fold_acc_warp) and lane 0 takes the decisions. A batch gives each scene a warp to
+// fold its buckets as alone, then a thread for the decisions: bound by the latency of loads and
+// of dependent FP64 adds. For 48 scenes a launch takes 9.8 us, k_ctrl_cg_alpha 6.9 and k_ctrl_cg
+// 10.5; with a thread per scene to fold 32 buckets in a row they took 12.1, 8.1 and 15.7.
+constexpr uint32_t kCtrlThreads = 1024u;
+inline uint32_t ctrl_threads(const Dev& d) { return std::min(kCtrlThreads, 32u * d.nscenes); }
+
 template <bool DIV>
-__global__ void k_ctrl_jacobi(Dev d) {
+__global__ void __launch_bounds__(kCtrlThreads) k_ctrl_jacobi(Dev d) {
     VFD_COUNT_LAUNCH(d);
     if (d.nscenes == 1) {
         if (threadIdx.x >= 32u) return;
@@ -416,12 +420,20 @@ __global__ void k_ctrl_jacobi(Dev d) {
     __shared__ uint32_t any;
     if (threadIdx.x == 0) any = 0;
     __syncthreads();
-    for (uint32_t s = threadIdx.x; s < d.nscenes; s += blockDim.x) {
-        SceneDev& S = d.scenes[s];
-        if (!(DIV ? S.div.active : S.pres.active)) continue;
-        if (jacobi_control<DIV>(S, fold_acc(d, s, 0))) atomicOr(&any, 1u);
+    __shared__ double sums[kCtrlThreads];
+    auto active = [&](uint32_t s) { return (DIV ? d.scenes[s].div.active : d.scenes[s].pres.active) != 0u; };
+    for (uint32_t c = 0; c < d.nscenes; c += blockDim.x) {
+        const uint32_t end = min(c + blockDim.x, d.nscenes);
+        for (uint32_t s = c + (threadIdx.x >> 5); s < end; s += blockDim.x >> 5) {
+            if (!active(s)) continue;
+            const double sum = fold_acc_warp(d, s, 0, threadIdx.x & 31u);
+            if ((threadIdx.x & 31u) == 0u) sums[s - c] = sum;
+        }
+        __syncthreads();
+        const uint32_t s = c + threadIdx.x;
+        if (s < end && active(s) && jacobi_control<DIV>(d.scenes[s], sums[threadIdx.x])) atomicOr(&any, 1u);
+        __syncthreads();
     }
-    __syncthreads();
     if (d.nscenes > 1)
         build_work_list(d, DIV ? kLoopDiv : kLoopPres,
                         [&](uint32_t sc) { return (DIV ? d.scenes[sc].div.active : d.scenes[sc].pres.active) != 0u; });
@@ -734,7 +746,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_cg_spmv_b(Dev d) {
 }
 
 // alpha = |r . z| / (p . Ap) (:714-720).
-__global__ void k_ctrl_cg_alpha(Dev d) {
+__global__ void __launch_bounds__(kCtrlThreads) k_ctrl_cg_alpha(Dev d) {
     VFD_COUNT_LAUNCH(d);
     if (d.nscenes == 1) {
         if (threadIdx.x >= 32u) return;
@@ -744,10 +756,11 @@ __global__ void k_ctrl_cg_alpha(Dev d) {
         if (threadIdx.x == 0) S.cgAlpha = (float)(S.cgAbsNew / pap);
         return;
     }
-    for (uint32_t s = threadIdx.x; s < d.nscenes; s += blockDim.x) {
+    for (uint32_t s = threadIdx.x >> 5; s < d.nscenes; s += blockDim.x >> 5) {
         SceneDev& S = d.scenes[s];
         if (!S.cgActive) continue;
-        S.cgAlpha = (float)(S.cgAbsNew / fold_acc(d, s, 0));
+        const double pap = fold_acc_warp(d, s, 0, threadIdx.x & 31u);
+        if ((threadIdx.x & 31u) == 0u) S.cgAlpha = (float)(S.cgAbsNew / pap);
     }
 }
 
@@ -837,7 +850,7 @@ __device__ __forceinline__ bool cg_control(const Dev& d, SceneDev& S, double rr,
     return again;
 }
 
-__global__ void k_ctrl_cg(Dev d) {
+__global__ void __launch_bounds__(kCtrlThreads) k_ctrl_cg(Dev d) {
     VFD_COUNT_LAUNCH(d);
     if (d.nscenes == 1) {
         if (threadIdx.x >= 32u) return;
@@ -858,14 +871,23 @@ __global__ void k_ctrl_cg(Dev d) {
     __shared__ uint32_t any;
     if (threadIdx.x == 0) any = 0;
     __syncthreads();
-    for (uint32_t s = threadIdx.x; s < d.nscenes; s += blockDim.x) {
-        SceneDev& S = d.scenes[s];
-        S.cgUpdateP = 0;
-        if (!S.cgActive) continue;
-        const double rr = fold_acc(d, s, 1), rz = fold_acc(d, s, 2);
-        if (cg_control(d, S, rr, rz)) atomicOr(&any, 1u);
+    __shared__ double2 sums[kCtrlThreads];
+    for (uint32_t c = 0; c < d.nscenes; c += blockDim.x) {
+        const uint32_t end = min(c + blockDim.x, d.nscenes);
+        for (uint32_t s = c + (threadIdx.x >> 5); s < end; s += blockDim.x >> 5) {
+            if (!d.scenes[s].cgActive) continue;
+            const double rr = fold_acc_warp(d, s, 1, threadIdx.x & 31u), rz = fold_acc_warp(d, s, 2, threadIdx.x & 31u);
+            if ((threadIdx.x & 31u) == 0u) sums[s - c] = make_double2(rr, rz);
+        }
+        __syncthreads();
+        const uint32_t s = c + threadIdx.x;
+        if (s < end) {
+            SceneDev& S = d.scenes[s];
+            S.cgUpdateP = 0;
+            if (S.cgActive && cg_control(d, S, sums[threadIdx.x].x, sums[threadIdx.x].y)) atomicOr(&any, 1u);
+        }
+        __syncthreads();
     }
-    __syncthreads();
     if (d.nscenes > 1) build_work_list(d, kLoopCG, [&](uint32_t sc) { return d.scenes[sc].cgActive != 0u; });
     if (threadIdx.x == 0) set_condition(d, kLoopCG, any);
 }
@@ -1189,7 +1211,7 @@ void launch_div_iter(const Dev& d, cudaStream_t s) {
     if (halo_on(d)) {
         launch_halo_pass(d, kHaloPAccelD, s);
         launch_halo_pass(d, kHaloJacobiD, s);
-        VFD_LAUNCH("k_ctrl_jacobi", s, k_ctrl_jacobi<true><<<1, 256, 0, s>>>(d));
+        VFD_LAUNCH("k_ctrl_jacobi", s, k_ctrl_jacobi<true><<<1, ctrl_threads(d), 0, s>>>(d));
         return;
     }
     if (tiled(d, kTPAccel)) VFD_TILE_DISPATCH("k_pressure_accel", kTPAccel, FN_PACC_D, OP_PACC_D);
@@ -1200,7 +1222,7 @@ void launch_div_iter(const Dev& d, cudaStream_t s) {
     else if (d.nscenes > 1) VFD_LAUNCH_MODE(VFD_LAUNCH_LANES_BATCH, "k_jacobi_iter", kTJacobi, K_JACOBI_DB);
     else if (no_stream(d, kTJacobi)) VFD_LAUNCH_MODE(VFD_LAUNCH_LANES, "k_jacobi_iter", kTJacobi, K_JACOBI_D_NS);
     else VFD_LAUNCH_MODE(VFD_LAUNCH_LANES, "k_jacobi_iter", kTJacobi, K_JACOBI_D);
-    VFD_LAUNCH("k_ctrl_jacobi", s, k_ctrl_jacobi<true><<<1, 256, 0, s>>>(d));
+    VFD_LAUNCH("k_ctrl_jacobi", s, k_ctrl_jacobi<true><<<1, ctrl_threads(d), 0, s>>>(d));
 }
 void launch_div_finish(const Dev& d, cudaStream_t s) {
     if (halo_on(d)) launch_halo_pass(d, kHaloDivFinish, s);
@@ -1236,9 +1258,9 @@ void launch_cg_iter(const Dev& d, cudaStream_t s) {
     else if (no_stream(d, kTSpmv)) VFD_LAUNCH_MODE(VFD_LAUNCH_LANES, "k_cg_spmv", kTSpmv, K_SPMV_NS);
     else VFD_LAUNCH_MODE(VFD_LAUNCH_LANES, "k_cg_spmv", kTSpmv, K_SPMV);
     if (d.nscenes > 1) {
-        VFD_LAUNCH("k_ctrl_cg_alpha", s, k_ctrl_cg_alpha<<<1, 256, 0, s>>>(d));
+        VFD_LAUNCH("k_ctrl_cg_alpha", s, k_ctrl_cg_alpha<<<1, ctrl_threads(d), 0, s>>>(d));
         VFD_LAUNCH("k_cg_update", s, k_cg_update_b<<<d.batchBlocks, kBlock, 0, s>>>(d));
-        VFD_LAUNCH("k_ctrl_cg", s, k_ctrl_cg<<<1, 256, 0, s>>>(d));
+        VFD_LAUNCH("k_ctrl_cg", s, k_ctrl_cg<<<1, ctrl_threads(d), 0, s>>>(d));
         VFD_LAUNCH("k_cg_p", s, k_cg_p_b<<<d.batchBlocks, kBlock, 0, s>>>(d));
         return;
     }
@@ -1246,10 +1268,10 @@ void launch_cg_iter(const Dev& d, cudaStream_t s) {
     if (blocks_for(d.n) <= kFoldAlphaBlocks) {
         VFD_LAUNCH("k_cg_update", s, k_cg_update<true><<<blocks_for(d.n), kBlock, 0, s>>>(d));
     } else {
-        VFD_LAUNCH("k_ctrl_cg_alpha", s, k_ctrl_cg_alpha<<<1, 256, 0, s>>>(d));
+        VFD_LAUNCH("k_ctrl_cg_alpha", s, k_ctrl_cg_alpha<<<1, ctrl_threads(d), 0, s>>>(d));
         VFD_LAUNCH("k_cg_update", s, k_cg_update<false><<<blocks_for(d.n), kBlock, 0, s>>>(d));
     }
-    VFD_LAUNCH("k_ctrl_cg", s, k_ctrl_cg<<<1, 256, 0, s>>>(d));
+    VFD_LAUNCH("k_ctrl_cg", s, k_ctrl_cg<<<1, ctrl_threads(d), 0, s>>>(d));
     VFD_LAUNCH("k_cg_p", s, k_cg_p<<<blocks_for(d.n), kBlock, 0, s>>>(d));
 }
 void launch_visc_finish_dt(const Dev& d, cudaStream_t s) {
@@ -1266,7 +1288,7 @@ void launch_pres_iter(const Dev& d, cudaStream_t s) {
     if (halo_on(d)) {
         launch_halo_pass(d, kHaloPAccelP, s);
         launch_halo_pass(d, kHaloJacobiP, s);
-        VFD_LAUNCH("k_ctrl_jacobi", s, k_ctrl_jacobi<false><<<1, 256, 0, s>>>(d));
+        VFD_LAUNCH("k_ctrl_jacobi", s, k_ctrl_jacobi<false><<<1, ctrl_threads(d), 0, s>>>(d));
         return;
     }
     if (tiled(d, kTPAccel)) VFD_TILE_DISPATCH("k_pressure_accel", kTPAccel, FN_PACC_P, OP_PACC_P);
@@ -1277,7 +1299,7 @@ void launch_pres_iter(const Dev& d, cudaStream_t s) {
     else if (d.nscenes > 1) VFD_LAUNCH_MODE(VFD_LAUNCH_LANES_BATCH, "k_jacobi_iter", kTJacobi, K_JACOBI_PB);
     else if (no_stream(d, kTJacobi)) VFD_LAUNCH_MODE(VFD_LAUNCH_LANES, "k_jacobi_iter", kTJacobi, K_JACOBI_P_NS);
     else VFD_LAUNCH_MODE(VFD_LAUNCH_LANES, "k_jacobi_iter", kTJacobi, K_JACOBI_P);
-    VFD_LAUNCH("k_ctrl_jacobi", s, k_ctrl_jacobi<false><<<1, 256, 0, s>>>(d));
+    VFD_LAUNCH("k_ctrl_jacobi", s, k_ctrl_jacobi<false><<<1, ctrl_threads(d), 0, s>>>(d));
 }
 void launch_pres_finish(const Dev& d, cudaStream_t s) {
     if (halo_on(d)) launch_halo_pass(d, kHaloPresFinish, s);

@@ -177,8 +177,8 @@ __global__ void __launch_bounds__(kMeshBlock) k_mesh_groups(const float4* corner
 // node: they find the group of faces with the nearest centre, measure it, and then only the
 // groups whose sphere comes nearer than the nearest face so far, four faces a lane. Meshes
 // whose consecutive faces lie together, as exported ones do, keep a few groups a node; any
-// order gives the same result. Measuring every face for every node (61,740 nodes, 5,120
-// faces) took 1718 us, this 331 us (20,480 faces, 262,548 nodes: 13.9 ms and 1.6).
+// order gives the same result. Measuring every face for every node (62,181 nodes, 5,120
+// faces) took 1718 us, this 331 us (20,480 faces, 245,025 nodes: 13.9 ms and 1.6).
 __global__ void __launch_bounds__(kMeshBlock) k_map_field0_mesh(const BoxMap* mp, const float4* corners,
                                                                 const float4* normals, const float4* spheres,
                                                                 uint32_t nf, float* nodes) {

@@ -470,7 +470,7 @@ int vfd_get_launch_count(vfd_sim* sim, uint64_t* launches, int32_t reset);
  * runs. Inputs and outputs are the caller's device buffers: xyz (n*3 floats),
  * counts (n), neighbors (n * VFD_MAX_NEIGHBORS; row i holds particle i's neighbours in
  * the reference's order, original indices), sort_indices (n; sorted slot -> original
- * index). Intermediate data lives in a fixed ~10 MB __device__ array that every GPU
+ * index). Intermediate data lives in a fixed ~9 MB __device__ array that every GPU
  * loading the library keeps until exit; limits: n <= 16384 and a search grid of at most
  * 262144 cells, else VFD_E_CAPACITY. The first call on a device looks the array up
  * (cudaGetSymbolAddress, once per CUDA context) and should come before any stream

@@ -620,6 +620,15 @@ __device__ __forceinline__ uint32_t work_slot(const Dev& d, int loop, uint32_t v
 }
 
 // Host-side launch helpers.
+// Scenes that one cluster bins (k_search_small in dfsph_search.cu), against the nine kernels of
+// the general search: a step of 8,025 particles takes 790 us and 819, of 15,967 884 and 890, of
+// 23,871 1,048 and 1,047, of 32,423 1,055 and 1,072; beyond, its threads would need more
+// registers than they have. A larger cell table would keep eight SMs busy clearing it.
+constexpr uint32_t kSmallBlocks = 8u, kSearchSmallMax = 32768u, kSearchSmallCells = 262144u;
+inline bool search_small(const Dev& d) {
+    return d.nscenes == 1 && d.n <= kSearchSmallMax && d.cellCap <= kSearchSmallCells;
+}
+
 inline uint32_t blocks_for(uint32_t n, uint32_t block = kBlock) { return (n + block - 1) / block; }
 
 // Optional per-launch timing of eagerly launched kernels (CUDA events on the launch

@@ -13,11 +13,51 @@
 #include "dfsph_common.cuh"
 #include "dfsph_halo.cuh"
 
+#include <cooperative_groups.h>
+
+namespace cg = cooperative_groups;
+
 namespace vfd {
 
 constexpr uint32_t kScanItems = 1024u;  // cells per scan block (256 threads x 4)
 
 __device__ __forceinline__ bool aborted(const Dev& d) { return is_aborted(d); }
+
+// Cell of edge h around x; false (with the status set) when x is not finite.
+__device__ __forceinline__ bool position_cell(const Dev& d, SceneDev& S, float3 x, int* c) {
+    if (!(isfinite(x.x) && isfinite(x.y) && isfinite(x.z))) {
+        atomicOr(&S.flags, 0x10u);
+        atomicOr(d.status, 0x10u);
+        atomicExch(d.status + 1, 1u);
+        return false;
+    }
+    const float p[3] = {x.x, x.y, x.z};
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const float q = floorf(__fdiv_rn(p[k], S.h));
+        // positions beyond +-2^30 cells cannot be gridded; flag them.
+        const bool in = fabsf(q) < 1.0e9f;
+        if (!in) { atomicOr(d.status, 0x20u); atomicExch(d.status + 1, 1u); }
+        c[k] = in ? (int)q : 0;
+    }
+    return true;
+}
+
+// Search-grid key of a position (N2), or kNoKey with the status set.
+constexpr uint32_t kNoKey = 0xFFFFFFFFu;
+__device__ __forceinline__ uint32_t position_key(const Dev& d, const SceneDev& S, float3 x, uint32_t total) {
+    const float p[3] = {x.x, x.y, x.z};
+    int c[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) c[k] = (int)__fmul_rn(__fsub_rn(p[k], S.gridMin[k]), S.gridDelta[k]);
+    const uint32_t key = S.cellBase + cell_key(S, c[0], c[1], c[2]);
+    if (key >= total || c[0] < 0 || c[1] < 0 || c[2] < 0) {  // cannot happen for finite input
+        atomicOr(d.status, 0x20u);
+        atomicExch(d.status + 1, 1u);
+        return kNoKey;
+    }
+    return key;
+}
 
 // N1: ComputeMinMaxKernel (ParticleSearchKernels.cu:40-62) on the current positions.
 __global__ void __launch_bounds__(kBlock) k_minmax(Dev d) {
@@ -30,24 +70,8 @@ __global__ void __launch_bounds__(kBlock) k_minmax(Dev d) {
     if (valid) {
         const float4 x4 = d.XN[i];
         const float3 x = abs_pos(d, d.scenes[sid], x4);
-        const float h = d.scenes[sid].h;
-        const bool finite = isfinite(x.x) && isfinite(x.y) && isfinite(x.z);
-        if (!finite) {
-            atomicOr(&d.scenes[sid].flags, 0x10u);
-            atomicOr(d.status, 0x10u);
-            atomicExch(d.status + 1, 1u);
-        } else {
-            const float p[3] = {x.x, x.y, x.z};
-#pragma unroll
-            for (int k = 0; k < 3; k++) {
-                const float q = floorf(__fdiv_rn(p[k], h));
-                // positions beyond +-2^30 cells cannot be gridded; flag them.
-                const int v = (fabsf(q) < 1.0e9f) ? (int)q : 0;
-                if (!(fabsf(q) < 1.0e9f)) { atomicOr(d.status, 0x20u); atomicExch(d.status + 1, 1u); }
-                c[k] = v;
-                cmax[k] = v;
-            }
-        }
+        if (position_cell(d, d.scenes[sid], x, c))
+            for (int k = 0; k < 3; k++) cmax[k] = c[k];
     }
     const uint32_t s0 = __shfl_sync(0xffffffffu, sid, 0);
     const bool uniform = __all_sync(0xffffffffu, !valid || sid == s0);
@@ -69,6 +93,27 @@ __global__ void __launch_bounds__(kBlock) k_minmax(Dev d) {
             atomicMax(mm_bucket(d, sid, 3 + k, bucket), cmax[k]);
         }
     }
+}
+
+// ComputeCellInformation of a scene whose cell bounds are known.
+__device__ void scene_grid(SceneDev& S) {
+    const float R = S.h;
+    uint32_t cells = 1u;
+    bool ok = S.count > 0;
+    for (int k = 0; k < 3; k++) {
+        const float bmin = __fmul_rn((float)S.minCell[k], R);
+        const float bmax = __fmul_rn((float)(S.maxCell[k] + 1), R);
+        const float size = __fsub_rn(bmax, bmin);
+        const float q = ceilf(__fdiv_rn(size, R));
+        const uint32_t dim = (ok && q >= 0.0f && q < 1.0e7f) ? (uint32_t)q + 4u : 4u;
+        S.dim[k] = dim;
+        S.gridMin[k] = __fsub_rn(bmin, __fmul_rn(R, 2.0f));
+        S.meta[k] = (uint32_t)ceilf(__fdiv_rn((float)dim, 8.0f));
+        const float gs = __fmul_rn((float)dim, R);
+        S.gridDelta[k] = __fdiv_rn((float)dim, gs);
+        cells = (cells > 0xFFFFFFFFu / 8u) ? 0xFFFFFFFFu : cells * S.meta[k];
+    }
+    S.cellCount = (!ok) ? 0u : ((cells > 0xFFFFFFFFu / 512u) ? 0xFFFFFFFFu : cells * 512u);
 }
 
 // ParticleSearch::ComputeMinMax tail + ComputeCellInformation (ParticleSearch.cu:50-86),
@@ -125,23 +170,7 @@ __global__ void k_grid(Dev d) {
             }
             for (uint32_t b = 0; b < kBuckets; b++) *max_bucket(d, s, 1, b) = 0u;
         }
-        const float R = S.h;
-        uint32_t cells = 1u;
-        bool ok = S.count > 0;
-        for (int k = 0; k < 3; k++) {
-            const float bmin = __fmul_rn((float)S.minCell[k], R);
-            const float bmax = __fmul_rn((float)(S.maxCell[k] + 1), R);
-            const float size = __fsub_rn(bmax, bmin);
-            const float q = ceilf(__fdiv_rn(size, R));
-            const uint32_t dim = (ok && q >= 0.0f && q < 1.0e7f) ? (uint32_t)q + 4u : 4u;
-            S.dim[k] = dim;
-            S.gridMin[k] = __fsub_rn(bmin, __fmul_rn(R, 2.0f));
-            S.meta[k] = (uint32_t)ceilf(__fdiv_rn((float)dim, 8.0f));
-            const float gs = __fmul_rn((float)dim, R);
-            S.gridDelta[k] = __fdiv_rn((float)dim, gs);
-            cells = (cells > 0xFFFFFFFFu / 8u) ? 0xFFFFFFFFu : cells * S.meta[k];
-        }
-        S.cellCount = (!ok) ? 0u : ((cells > 0xFFFFFFFFu / 512u) ? 0xFFFFFFFFu : cells * 512u);
+        scene_grid(S);
         S.flags = 0u;
         if (halo_on(d)) d.haloScene[s] = make_uint2(0xFFFFFFFFu, 0u);
     }
@@ -179,17 +208,8 @@ __global__ void __launch_bounds__(kBlock) k_keys(Dev d) {
     if (i >= d.n || aborted(d)) return;
     const SceneDev& S = d.scenes[scene_of(d, i)];
     const float3 x = abs_pos(d, S, d.XN[i]);
-    const float p[3] = {x.x, x.y, x.z};
-    int c[3];
-#pragma unroll
-    for (int k = 0; k < 3; k++) c[k] = (int)__fmul_rn(__fsub_rn(p[k], S.gridMin[k]), S.gridDelta[k]);
-    uint32_t key = S.cellBase + cell_key(S, c[0], c[1], c[2]);
-    if (key >= d.status[2] || c[0] < 0 || c[1] < 0 || c[2] < 0) {  // cannot happen for finite input
-        atomicOr(d.status, 0x20u);
-        atomicExch(d.status + 1, 1u);
-        key = 0u;
-        return;
-    }
+    const uint32_t key = position_key(d, S, x, d.status[2]);
+    if (key == kNoKey) return;
     d.KEY[i] = key;
     atomicAdd(d.CELL_COUNT + key, 1u);
 }
@@ -380,6 +400,163 @@ __global__ void __launch_bounds__(kBlock) k_rank_gather(Dev d) {
     d.KEYS[dst] = key;
 }
 
+// N1 to N4 of one small scene in one launch: a cluster of kSmallBlocks blocks, with a barrier
+// of the cluster where the kernels above end. A thread keeps its particles' positions, keys and
+// places in registers. Bound by latency: a round trip to the L2 and a barrier that waits for the
+// stores before it take 1.3 to 2 us a phase, 15.8 us in all for 4,096 particles where the nine
+// kernels take 35.3 (each timed alone).
+constexpr uint32_t kSmallThreads = 1024u, kSmallPer = kSearchSmallMax / (kSmallBlocks * kSmallThreads);
+static_assert(kSmallPer * kSmallBlocks * kSmallThreads == kSearchSmallMax && kSmallBlocks <= 8u, "portable clusters");
+__global__ void __cluster_dims__(kSmallBlocks, 1, 1) __launch_bounds__(kSmallThreads) k_search_small(Dev d) {
+    VFD_COUNT_LAUNCH(d);
+    const cg::cluster_group cluster = cg::this_cluster();
+    constexpr uint32_t T = kSmallBlocks * kSmallThreads;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t rank = cluster.block_rank(), t = rank * kSmallThreads + threadIdx.x;
+    __shared__ int bounds[6];                                // of the block's particles
+    __shared__ int warpBounds[6][kSmallThreads / 32u];
+    __shared__ uint32_t blockCells;                          // particles in the block's cells
+    __shared__ uint32_t before, stop;
+    __shared__ __align__(16) unsigned char gridBytes[sizeof(SceneDev)];
+    SceneDev& G = *reinterpret_cast<SceneDev*>(gridBytes);   // the scene's grid, as d.scenes[0] gets it
+    SceneDev& S = d.scenes[0];
+
+    float3 x[kSmallPer];
+    int c[6] = {INT_MAX, INT_MAX, INT_MAX, INT_MIN, INT_MIN, INT_MIN};
+#pragma unroll
+    for (uint32_t u = 0; u < kSmallPer; u++) {
+        const uint32_t i = u * T + t;
+        if (i >= d.n) break;
+        x[u] = abs_pos(d, S, d.XN[i]);
+        int q[3];
+        if (!position_cell(d, S, x[u], q)) continue;
+        for (int k = 0; k < 3; k++) {
+            c[k] = min(c[k], q[k]);
+            c[3 + k] = max(c[3 + k], q[k]);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 6; k++) {
+        const int v = k < 3 ? __reduce_min_sync(0xffffffffu, c[k]) : __reduce_max_sync(0xffffffffu, c[k]);
+        if (lane == 0) warpBounds[k][warp] = v;
+    }
+    __syncthreads();
+    if (warp < 6u) {
+        const int v = warpBounds[warp][lane];
+        const int w = warp < 3u ? __reduce_min_sync(0xffffffffu, v) : __reduce_max_sync(0xffffffffu, v);
+        if (lane == 0) bounds[warp] = w;
+    }
+    cluster.sync();
+    if (warp == 0) {
+        int m[6];
+#pragma unroll
+        for (int k = 0; k < 6; k++) {
+            const int v = cluster.map_shared_rank(bounds, lane % kSmallBlocks)[k];
+            m[k] = k < 3 ? __reduce_min_sync(0xffffffffu, v) : __reduce_max_sync(0xffffffffu, v);
+        }
+        if (lane == 0) {
+            G.h = S.h;
+            G.count = S.count;
+            G.cellBase = 0u;
+            for (int k = 0; k < 3; k++) {
+                G.minCell[k] = m[k];
+                G.maxCell[k] = m[3 + k];
+            }
+            scene_grid(G);
+            // every block decides alike: the status changes again only behind the next barrier
+            stop = (__ldcg(d.status + 1) != 0u || G.cellCount > d.cellCap) ? 1u : 0u;
+        }
+        if (rank == 0u) *max_bucket(d, 0, 1, lane) = 0u;
+    }
+    __syncthreads();
+    const uint32_t total = G.cellCount;
+    if (!stop)
+        for (uint32_t i = t; i < total; i += T) d.CELL_COUNT[i] = 0u;
+    cluster.sync();
+    if (t == 0u) {
+        for (int k = 0; k < 3; k++) {
+            S.minCell[k] = G.minCell[k];
+            S.maxCell[k] = G.maxCell[k];
+            S.dim[k] = G.dim[k];
+            S.meta[k] = G.meta[k];
+            S.gridMin[k] = G.gridMin[k];
+            S.gridDelta[k] = G.gridDelta[k];
+        }
+        S.cellCount = total;
+        S.cellBase = 0u;
+        S.flags = 0u;
+        d.status[2] = total;
+        if (total > d.cellCap) {
+            atomicOr(d.status, 0x20u);
+            atomicExch(d.status + 1, 1u);
+        }
+    }
+    if (stop) return;
+
+    uint32_t key[kSmallPer], at[kSmallPer];
+#pragma unroll
+    for (uint32_t u = 0; u < kSmallPer; u++) {
+        key[u] = kNoKey;
+        if (u * T + t >= d.n) break;
+        key[u] = position_key(d, G, x[u], total);
+        if (key[u] != kNoKey) at[u] = atomicAdd(d.CELL_COUNT + key[u], 1u);
+    }
+    cluster.sync();
+    if (threadIdx.x == 0) stop = __ldcg(d.status + 1);
+
+    // a run of whole groups of four cells per thread
+    const uint32_t per = (total + 4u * T - 1u) / (4u * T), first = t * per, groups = total / 4u;
+    const uint4* counts = reinterpret_cast<const uint4*>(d.CELL_COUNT);
+    uint32_t sum = 0;
+    for (uint32_t g = first; g < min(first + per, groups); g++) {
+        const uint4 v = __ldcg(counts + g);
+        sum += v.x + v.y + v.z + v.w;
+    }
+    uint32_t inBlock;
+    uint32_t run = block_exclusive_scan_1024(sum, inBlock);
+    if (threadIdx.x == 0) blockCells = inBlock;
+    cluster.sync();
+    if (stop) return;
+    if (warp == 0) {
+        const uint32_t v = lane < rank ? *cluster.map_shared_rank(&blockCells, lane) : 0u;
+        const uint32_t w = __reduce_add_sync(0xffffffffu, v);
+        if (lane == 0) before = w;
+    }
+    __syncthreads();
+    run += before;
+    for (uint32_t g = first; g < min(first + per, groups); g++) {
+        const uint4 v = __ldcg(counts + g);
+        reinterpret_cast<uint4*>(d.CELL_START)[g] = make_uint4(run, run + v.x, run + v.x + v.y, run + v.x + v.y + v.z);
+        run += v.x + v.y + v.z + v.w;
+    }
+    cluster.sync();
+
+    uint32_t start[kSmallPer], pid[kSmallPer];
+#pragma unroll
+    for (uint32_t u = 0; u < kSmallPer; u++) {
+        const uint32_t i = u * T + t;
+        if (i >= d.n) break;
+        start[u] = __ldcg(d.CELL_START + key[u]);
+        pid[u] = d.PIDc[i];
+        d.TMP[start[u] + at[u]] = pid[u];
+    }
+    cluster.sync();
+#pragma unroll
+    for (uint32_t u = 0; u < kSmallPer; u++) {
+        const uint32_t i = u * T + t;
+        if (i >= d.n) break;
+        const uint32_t count = __ldcg(d.CELL_COUNT + key[u]);
+        uint32_t dst = start[u];
+        for (uint32_t q = start[u]; q < start[u] + count; q++) dst += __ldcg(d.TMP + q) < pid[u] ? 1u : 0u;
+        d.X[dst] = d.XN[i];
+        d.V[dst] = d.Vc[i];
+        d.DV[dst] = d.DVc[i];
+        d.DK[dst] = d.DKc[i];
+        d.PID[dst] = pid[u];
+        d.KEYS[dst] = key[u];
+    }
+}
+
 // N6-N8: ComputeCountsKernel + NeighborhoodQueryWithCountsKernel (ParticleSearchKernels.cu:93-193)
 // in one pass, one warp per cell. The particles of a cell share their 27 candidate cells,
 // so the warp walks that candidate set once, 32 candidates per round (lane j < 27 holds
@@ -503,8 +680,19 @@ __global__ void __launch_bounds__(kBlock) k_neighbors(Dev d) {
         if (profiled) VFD_LAUNCH(name, s, __VA_ARGS__); \
         else { __VA_ARGS__; }                    \
     } while (0)
+void launch_neighbors(const Dev& d, cudaStream_t s, bool profiled) {
+    // a warp per cell, a fixed grid striding over the cells the device counted
+    const uint32_t nbrBlocks = 4u * d.batchBlocks;
+    if (d.cellRel) SEARCH_LAUNCH("k_neighbors", k_neighbors<true><<<nbrBlocks, kBlock, 0, s>>>(d));
+    else SEARCH_LAUNCH("k_neighbors", k_neighbors<false><<<nbrBlocks, kBlock, 0, s>>>(d));
+}
 void launch_search(const Dev& d, cudaStream_t s, bool profiled) {
     const uint32_t nb = blocks_for(d.n);
+    if (search_small(d)) {
+        SEARCH_LAUNCH("k_search_small", k_search_small<<<kSmallBlocks, kSmallThreads, 0, s>>>(d));
+        launch_neighbors(d, s, profiled);
+        return;
+    }
     SEARCH_LAUNCH("k_minmax", k_minmax<<<nb, kBlock, 0, s>>>(d));
     SEARCH_LAUNCH("k_grid", k_grid<<<1, 256, 0, s>>>(d));
     SEARCH_LAUNCH("k_clear_cells", k_clear_cells<<<1216, 256, 0, s>>>(d));
@@ -515,10 +703,7 @@ void launch_search(const Dev& d, cudaStream_t s, bool profiled) {
     if (halo_on(d)) launch_halo_build(d, s);
     SEARCH_LAUNCH("k_slots", k_slots<<<nb, kBlock, 0, s>>>(d));
     SEARCH_LAUNCH("k_rank_gather", k_rank_gather<<<nb, kBlock, 0, s>>>(d));
-    // a warp per cell, a fixed grid striding over the cells the device counted
-    const uint32_t nbrBlocks = 4u * d.batchBlocks;
-    if (d.cellRel) SEARCH_LAUNCH("k_neighbors", k_neighbors<true><<<nbrBlocks, kBlock, 0, s>>>(d));
-    else SEARCH_LAUNCH("k_neighbors", k_neighbors<false><<<nbrBlocks, kBlock, 0, s>>>(d));
+    launch_neighbors(d, s, profiled);
 }
 #undef SEARCH_LAUNCH
 

@@ -218,6 +218,7 @@ struct vfd_sim {
     uint32_t* dStatus = nullptr;
     float *dWM = nullptr, *dGM = nullptr, *dHalton = nullptr;
     uint32_t* hStatus = nullptr;  // pinned
+    vfd::SceneDev* hStage = nullptr;  // pinned: the scenes after a step, on their way to hScenes
     std::vector<vfd::SceneDev> hScenes;
     uint32_t maxStPasses = 0;
     bool anyDiv = false, anyVisc = false, anyST = false;
@@ -269,6 +270,8 @@ struct vfd_sim {
         adjTapeSet = nullptr;
         if (hStatus) cudaFreeHost(hStatus);
         hStatus = nullptr;
+        if (hStage) cudaFreeHost(hStage);
+        hStage = nullptr;
         allocated = false;
         uploaded = false;
     }

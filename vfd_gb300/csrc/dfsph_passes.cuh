@@ -61,8 +61,7 @@ __device__ __forceinline__ float dot_term(float3 a, float3 b) {
 
 // W and gradW of one pair from one table position (GetW / GetGradientW keep their own
 // range tests: |r|^2 <= R^2 for W, |r| <= R for gradW).
-__device__ __forceinline__ void kernel_wg(const Dev& d, float3 r, float& w, float& gs) {
-    const float r2 = dot3(r, r);
+__device__ __forceinline__ void kernel_wg_r2(const Dev& d, float r2, float& w, float& gs) {
     const float rl = fast_sqrt(r2);
     if (d.analytic) {
         w = r2 <= d.radius2 ? spline_w(d, rl) : 0.0f;
@@ -72,6 +71,9 @@ __device__ __forceinline__ void kernel_wg(const Dev& d, float3 r, float& w, floa
     const uint32_t pos = table_pos(d, rl);
     w = r2 <= d.radius2 ? __ldg(d.WM + pos) : 0.0f;
     gs = rl <= d.radius ? __ldg(d.GM + pos) : 0.0f;
+}
+__device__ __forceinline__ void kernel_wg(const Dev& d, float3 r, float& w, float& gs) {
+    kernel_wg_r2(d, dot3(r, r), w, gs);
 }
 
 struct Mat3 {
@@ -123,7 +125,7 @@ __device__ __forceinline__ void density_finish(const Dev& d, uint32_t p, const S
             if (xb.w > 0.0f) {
                 const float3 r = xi - f3(xb);
                 float w, gs;
-                kernel_wg(d, r, w, gs);
+                kernel_wg_r2(d, dot3_yx(r, r), w, gs);
                 rhoB += xb.w * w;
                 gb += (xb.w * gs) * r;
             }

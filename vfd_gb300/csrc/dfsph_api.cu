@@ -54,12 +54,50 @@ __global__ void k_export1(const uint32_t* pid, const float* src, const float4* s
     out[o] = src4 ? (&src4[p].x)[comp] : src[p];
 }
 // Sets *bad, and the host's copy of it, when any of the n values of a or of b (either may be
-// null) is not finite (inputs checked on the device after their copy, before they are imported).
-__global__ void k_check_finite(const float* a, const float* b, size_t n, uint32_t* bad, uint32_t* hostBad) {
+// null) is not finite (inputs checked on the device before they are imported). With copies
+// wanted, a and b are pinned host memory and are copied on the way.
+__global__ void k_check_finite(const float* a, const float* b, float* copyA, float* copyB, size_t n, uint32_t* bad,
+                               uint32_t* hostBad) {
     bool finite = true;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        finite = finite && (!a || isfinite(a[i])) && (!b || isfinite(b[i]));
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        const float u = a ? a[i] : 0.0f, v = b ? b[i] : 0.0f;
+        finite = finite && isfinite(u) && isfinite(v);
+        if (copyA) copyA[i] = u;
+        if (copyB) copyB[i] = v;
+    }
     if (!finite) *bad = *hostBad = 1u;
+}
+// Device arrays to pinned host memory (null: not wanted).
+__global__ void k_copy_out(const float* x, const float* v, const float* a, float* hostX, float* hostV, float* hostA,
+                           size_t n) {
+    const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    if (hostX) hostX[i] = x[i];
+    if (hostV) hostV[i] = v[i];
+    if (hostA) hostA[i] = a[i];
+}
+// The status words and the scenes to pinned host memory.
+__global__ void k_report(const uint32_t* status, uint32_t* hostStatus, const uint32_t* scenes, uint32_t* hostScenes,
+                         uint32_t words) {
+    for (uint32_t i = threadIdx.x; i < 16u + words; i += blockDim.x) {
+        if (i < 16u) hostStatus[i] = status[i];
+        else hostScenes[i - 16u] = scenes[i - 16u];
+    }
+}
+// Whether a kernel can carry this host array in place of a copy: pinned (or not wanted). The
+// copy engine's start costs more than it saves at every size: with it 8,000 particles were set in
+// 27.5 us and read in 39.6 and 2.7 million in 411 and 639, by kernels in 24.7 and 26.8, 379 and 638.
+bool kernel_copy(const void* p, size_t bytes) {
+    if (!p) return true;
+    for (const char* q : {static_cast<const char*>(p), static_cast<const char*>(p) + bytes - 1}) {
+        cudaPointerAttributes a;
+        if (cudaPointerGetAttributes(&a, q) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        if (a.type != cudaMemoryTypeHost || a.devicePointer != q) return false;
+    }
+    return true;
 }
 // Positions out of the cell-relative form (Dev::cellRel): absolute FP32
 // coordinates of slots [begin, begin + count) in original order; `anchors` holds each
@@ -87,8 +125,8 @@ __device__ __forceinline__ float4 import_pos(const Dev& d, const SceneDev& S, co
 }
 // Positions and velocities of slots [begin, begin + count) in or out in one launch, in original
 // order (x, v, or both); an import leaves all of them when *bad is set. The state of 8,000
-// particles is set in 28 us and read in 38; with a launch for each array and each check, and a
-// wait before the import, 53 and 47.
+// particles was set in 53 us and read in 47 with a launch for each array and each check and a wait
+// before the import, in 28 and 38 so (and see kernel_copy).
 __global__ void k_import_state(Dev d, const float* x, const float* v, const uint32_t* bad, uint32_t begin,
                                uint32_t count) {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -105,23 +143,19 @@ __global__ void k_import_state(Dev d, const float* x, const float* v, const uint
         d.Vc[p] = make_float4(q[0], q[1], q[2], d.Vc[p].w);
     }
 }
-__global__ void k_export_state(Dev d, float* x, float* v, uint32_t begin, uint32_t count) {
+__global__ void k_export_state(Dev d, float* x, float* v, float* a, uint32_t begin, uint32_t count) {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= count) return;
     const uint32_t p = begin + k;
     const uint32_t o = d.PIDc[p];
     if (o >= count) return;
-    if (x) {
-        const float4 w = d.XN[p];
-        const float3 a = d.cellRel ? abs_pos(d, d.scenes[scene_of(d, p)], w) : f3(w);
-        float* q = x + 3 * (size_t)o;
-        q[0] = a.x, q[1] = a.y, q[2] = a.z;
-    }
-    if (v) {
-        const float4 w = d.Vc[p];
-        float* q = v + 3 * (size_t)o;
-        q[0] = w.x, q[1] = w.y, q[2] = w.z;
-    }
+    auto put = [&](float* out, float3 w) {
+        out += 3 * (size_t)o;
+        out[0] = w.x, out[1] = w.y, out[2] = w.z;
+    };
+    if (x) put(x, d.cellRel ? abs_pos(d, d.scenes[scene_of(d, p)], d.XN[p]) : f3(d.XN[p]));
+    if (v) put(v, f3(d.Vc[p]));
+    if (a) put(a, f3(d.A[p]));
 }
 
 // Frame output of vfd_simulate. When a step completes a frame (k_ctrl_end sets frameDue;
@@ -439,7 +473,7 @@ int allocate(vfd_sim* s) {
     for (const auto& sc : s->scenes) bodyTotal += (uint32_t)sc.bodies.size();
     TRY(dalloc(s, &s->dBodies, std::max<uint32_t>(1u, bodyTotal)));
     TRY(dalloc(s, &s->dStatus, 16));
-    TRY(dalloc(s, &s->dStage, 3 * st));
+    TRY(dalloc(s, &s->dStage, 6 * st));
     TRY(dalloc(s, &s->dStage2, 3 * st));
     TRY(dalloc(s, &base.ACCB, (size_t)base.nscenes * kAccSlots * kBuckets * 16u));
     TRY(dalloc(s, &base.MAXB, (size_t)base.nscenes * 2u * kBuckets * 32u));
@@ -863,8 +897,10 @@ int launch_one(vfd_sim* s) {
 // carried state, so the table is grown and the same step launched again.
 int finish_steps(vfd_sim* s, vfd_step_stats* stats, uint32_t& flags) {
     const size_t bytes = sizeof(SceneDev) * s->hScenes.size();
-    CK(cudaMemcpyAsync(s->hStatus, s->dStatus, 16 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s->stream));
-    if (stats) CK(cudaMemcpyAsync(s->hStage, s->dScenes, bytes, cudaMemcpyDeviceToHost, s->stream));
+    static_assert(sizeof(SceneDev) % sizeof(uint32_t) == 0, "k_report copies words");
+    k_report<<<1, 1024, 0, s->stream>>>(s->dStatus, s->hStatus, reinterpret_cast<const uint32_t*>(s->dScenes),
+                                       reinterpret_cast<uint32_t*>(s->hStage),
+                                       stats ? (uint32_t)(bytes / sizeof(uint32_t)) : 0u);
     CK(cudaStreamSynchronize(s->stream));
     CK(cudaGetLastError());
     flags = s->hStatus[0];
@@ -961,16 +997,15 @@ int check_sim(const vfd_sim* s) { return s ? VFD_OK : fail(VFD_E_ARG, "null hand
 
 // The scatters export through one staging buffer in stream order; wait = false leaves the
 // copy to a later synchronisation of the stream (the caller's).
-int scatter_vec(vfd_sim* s, uint32_t scene, const float4* dsrc, float* out, bool wait) {
+int scatter_vec(vfd_sim* s, uint32_t scene, const float4* dsrc, float* out) {
     const uint32_t b = s->sceneBegin[scene], cnt = s->scenes[scene].count();
     if (cnt == 0) return VFD_OK;
     k_export3<<<blocks_for(cnt, 256), 256, 0, s->stream>>>(s->dev[s->cs].PIDc, dsrc, s->dStage, b, cnt);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(out, s->dStage, sizeof(float) * 3 * (size_t)cnt, cudaMemcpyDeviceToHost, s->stream));
-    if (wait) CK(cudaStreamSynchronize(s->stream));
+    CK(cudaStreamSynchronize(s->stream));
     return VFD_OK;
 }
-int scatter_vec(vfd_sim* s, uint32_t scene, const float4* dsrc, float* out) { return scatter_vec(s, scene, dsrc, out, true); }
 
 int scatter_scalar(vfd_sim* s, uint32_t scene, const float* dsrc, float* out, int comp = -1, const float4* d4 = nullptr) {
     const uint32_t b = s->sceneBegin[scene], cnt = s->scenes[scene].count();
@@ -1538,17 +1573,21 @@ int vfd_scene_get_state(vfd_sim* s, uint32_t scene, float* x, float* v, float* a
     TRY(ensure_ready(s));
     if (s->fp64Mode) return fp64_get_state(s, nullptr, nullptr, x, v, a);
     const Dev& d = s->dev[s->cs];
-    // the accelerations reuse the positions' staging buffer in stream order; one wait for all
     const uint32_t b = s->sceneBegin[scene], cnt = s->scenes[scene].count();
-    if (cnt && (x || v)) {
-        k_export_state<<<blocks_for(cnt, 256), 256, 0, s->stream>>>(d, x ? s->dStage : nullptr,
-                                                                    v ? s->dStage2 : nullptr, b, cnt);
-        CK(cudaGetLastError());
+    if (cnt && (x || v || a)) {
+        float *const sx = s->dStage, *const sv = s->dStage2, *const sa = s->dStage + 3 * (size_t)s->stride;
+        k_export_state<<<blocks_for(cnt, 256), 256, 0, s->stream>>>(d, x ? sx : nullptr, v ? sv : nullptr,
+                                                                    a ? sa : nullptr, b, cnt);
         const size_t bytes = sizeof(float) * 3 * (size_t)cnt;
-        if (x) CK(cudaMemcpyAsync(x, s->dStage, bytes, cudaMemcpyDeviceToHost, s->stream));
-        if (v) CK(cudaMemcpyAsync(v, s->dStage2, bytes, cudaMemcpyDeviceToHost, s->stream));
+        if (kernel_copy(x, bytes) && kernel_copy(v, bytes) && kernel_copy(a, bytes)) {
+            k_copy_out<<<blocks_for(3 * cnt, 256), 256, 0, s->stream>>>(sx, sv, sa, x, v, a, 3 * (size_t)cnt);
+        } else {
+            if (x) CK(cudaMemcpyAsync(x, sx, bytes, cudaMemcpyDeviceToHost, s->stream));
+            if (v) CK(cudaMemcpyAsync(v, sv, bytes, cudaMemcpyDeviceToHost, s->stream));
+            if (a) CK(cudaMemcpyAsync(a, sa, bytes, cudaMemcpyDeviceToHost, s->stream));
+        }
+        CK(cudaGetLastError());
     }
-    if (a) TRY(scatter_vec(s, scene, d.A, a, false));
     CK(cudaStreamSynchronize(s->stream));
     return VFD_OK;
 }
@@ -1564,10 +1603,15 @@ int vfd_set_state(vfd_sim* s, const float* x, const float* v) {
     // both arrays are copied and checked on the device before either is imported
     uint32_t* bad = s->dStatus + 10;  // zero between calls
     s->hStatus[10] = 0u;
-    if (x) CK(cudaMemcpyAsync(s->dStage, x, bytes, cudaMemcpyHostToDevice, s->stream));
-    if (v) CK(cudaMemcpyAsync(s->dStage2, v, bytes, cudaMemcpyHostToDevice, s->stream));
-    const float *const dx = x ? s->dStage : nullptr, *const dv = v ? s->dStage2 : nullptr;
-    k_check_finite<<<blocks_for(3 * cnt, 256), 256, 0, s->stream>>>(dx, dv, 3 * (size_t)cnt, bad, s->hStatus + 10);
+    float *const dx = x ? s->dStage : nullptr, *const dv = v ? s->dStage2 : nullptr;
+    const uint32_t blocks = blocks_for(3 * cnt, 256);
+    if (kernel_copy(x, bytes) && kernel_copy(v, bytes)) {
+        k_check_finite<<<blocks, 256, 0, s->stream>>>(x, v, dx, dv, 3 * (size_t)cnt, bad, s->hStatus + 10);
+    } else {
+        if (x) CK(cudaMemcpyAsync(dx, x, bytes, cudaMemcpyHostToDevice, s->stream));
+        if (v) CK(cudaMemcpyAsync(dv, v, bytes, cudaMemcpyHostToDevice, s->stream));
+        k_check_finite<<<blocks, 256, 0, s->stream>>>(dx, dv, nullptr, nullptr, 3 * (size_t)cnt, bad, s->hStatus + 10);
+    }
     k_import_state<<<blocks_for(cnt, 256), 256, 0, s->stream>>>(s->dev[s->cs], dx, dv, bad, s->sceneBegin[0], cnt);
     CK(cudaGetLastError());
     // calls that write the state with default-stream copies (restore, upload) must find it settled

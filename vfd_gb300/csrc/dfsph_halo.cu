@@ -204,6 +204,7 @@ __device__ __forceinline__ void halo_pass(const Dev& d) {
     float4* const sx = haloSmem;
     float4* const sv = haloSmem + kHaloCap;                            // kVectorField
     float* const ss = reinterpret_cast<float*>(haloSmem + kHaloCap);   // kScalarField
+    Op::start(d);
     if (is_aborted(d)) return;
     HaloSum<Op::kTerms> sum;
     const uint32_t nt = halo_tile_total(d, Op::kLoop);
@@ -302,6 +303,7 @@ struct HaloOp {
     __device__ static bool active(const SceneDev&) { return true; }
     __device__ static const void* field(const Dev&) { return nullptr; }
     __device__ static const int* slots() { return nullptr; }
+    __device__ static void start(const Dev&) {}  // by every block, before all else
 };
 __device__ constexpr int kSlots01[2] = {0, 1};
 
@@ -314,6 +316,7 @@ struct HaloDensity : HaloOp<kVectorField, kWriteGrad> {
         float V;
         bool div;
     };
+    __device__ static void start(const Dev& d) { jacobi_start<true>(d); }
     using Acc = DensitySums;
     __device__ static const void* field(const Dev& d) { return d.V; }
     __device__ static void load(const Dev& d, uint32_t p, const SceneDev& S, Own& o) {
@@ -414,6 +417,7 @@ struct HaloPresInit : HaloOp<kVectorField> {
         float4 xi;
         float3 vi;
     };
+    __device__ static void start(const Dev& d) { jacobi_start<false>(d); }
     using Acc = float;
     __device__ static const void* field(const Dev& d) { return d.V; }
     __device__ static void load(const Dev& d, uint32_t p, const SceneDev&, Own& o) {

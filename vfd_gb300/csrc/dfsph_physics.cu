@@ -29,11 +29,6 @@ namespace vfd {
 
 __device__ __forceinline__ bool aborted_p(const Dev& d) { return is_aborted(d); }
 
-__device__ __forceinline__ void set_condition(const Dev& d, int loop, uint32_t value) {
-    if (d.condHandle[loop]) cudaGraphSetConditional((cudaGraphConditionalHandle)d.condHandle[loop], value);
-    d.status[4 + loop] = value;
-}
-
 // Batches: lists the scenes for which active(s) holds into loop `loop`'s work list
 // (prefix sums of their particle counts, and of their staged tiles, by a block-wide scan). One
 // block of whole warps, called by all of its threads after the scenes' flags are final.
@@ -197,6 +192,7 @@ __device__ __forceinline__ void for_neighbors(const Group<G>& grp, const Nbr& nb
 template <uint32_t G, bool REL, bool DIV = false>
 __global__ void __launch_bounds__(kMaxBlock) k_density_factor(Dev d) {
     VFD_COUNT_LAUNCH(d);
+    if (DIV) jacobi_start<true>(d);
     GROUP_PROLOGUE(G)
     const SceneDev& S = d.scenes[scene_of(d, p)];
     const float4 xi4 = d.X[p];
@@ -351,30 +347,18 @@ __global__ void __launch_bounds__(kMaxBlock) k_jacobi_iter_b(Dev d) {
     }
 }
 
-// Loop start: the reference's while condition evaluated with error 0, iteration 0
-// (DFSPHImplementation.cu:461, :532).
+// Loop start of a batch (a single scene's first pass does it, jacobi_start).
 template <bool DIV>
 __global__ void k_ctrl_jacobi_init(Dev d) {
     VFD_COUNT_LAUNCH(d);
     __shared__ uint32_t any;
     if (threadIdx.x == 0) any = 0;
     __syncthreads();
-    const bool ab = aborted_p(d);
-    for (uint32_t s = threadIdx.x; s < d.nscenes; s += blockDim.x) {
-        SceneDev& S = d.scenes[s];
-        LoopState& L = DIV ? S.div : S.pres;
-        L.it = 0;
-        L.err = 0.0f;
-        const uint32_t mn = DIV ? S.minIterD : S.minIterP, mx = DIV ? S.maxIterD : S.maxIterP;
-        const bool enabled = (DIV ? S.enableDiv != 0 : true) && S.count > 0 && !ab;
-        const float eta = DIV ? S.dtInv * S.maxErrD * 0.0001f * S.rho0 : S.maxErrP * 0.0001f * S.rho0;
-        L.active = (enabled && ((0.0f > eta) || 0u < mn) && 0u < mx) ? 1u : 0u;
-        if (L.active) atomicOr(&any, 1u);
-    }
+    for (uint32_t s = threadIdx.x; s < d.nscenes; s += blockDim.x)
+        if (jacobi_begin<DIV>(d, d.scenes[s])) atomicOr(&any, 1u);
     __syncthreads();
-    if (d.nscenes > 1)
-        build_work_list(d, DIV ? kLoopDiv : kLoopPres,
-                        [&](uint32_t sc) { return (DIV ? d.scenes[sc].div.active : d.scenes[sc].pres.active) != 0u; });
+    build_work_list(d, DIV ? kLoopDiv : kLoopPres,
+                    [&](uint32_t sc) { return (DIV ? d.scenes[sc].div.active : d.scenes[sc].pres.active) != 0u; });
     if (threadIdx.x == 0) set_condition(d, DIV ? kLoopDiv : kLoopPres, any);
 }
 
@@ -977,6 +961,7 @@ __global__ void __launch_bounds__(kBlock) k_velocity(Dev d) {
 template <uint32_t G, bool REL>
 __global__ void __launch_bounds__(kMaxBlock) k_pres_init(Dev d) {
     VFD_COUNT_LAUNCH(d);
+    jacobi_start<false>(d);
     GROUP_PROLOGUE(G)
     const SceneDev& S = d.scenes[scene_of(d, p)];
     const Nbr nb = neighbors(d, p);
@@ -1183,7 +1168,7 @@ void launch_density(const Dev& d, cudaStream_t s) { VFD_LAUNCH_MODE(VFD_LAUNCH_L
 void launch_density_div_init(const Dev& d, cudaStream_t s) {
     if (halo_on(d)) launch_halo_pass(d, kHaloDensity, s);
     else VFD_LAUNCH_MODE(VFD_LAUNCH_LANES, "k_density_factor", kTDensity, K_DENSITY_DIV);
-    VFD_LAUNCH("k_ctrl_jacobi_init", s, k_ctrl_jacobi_init<true><<<1, 256, 0, s>>>(d));
+    if (d.nscenes > 1) VFD_LAUNCH("k_ctrl_jacobi_init", s, k_ctrl_jacobi_init<true><<<1, 256, 0, s>>>(d));
 }
 #define K_PACCEL_DB(G) k_pressure_accel_b<true, G, false>
 #define K_PACCEL_DB_R(G) k_pressure_accel_b<true, G, true>
@@ -1282,7 +1267,7 @@ void launch_visc_finish_dt(const Dev& d, cudaStream_t s) {
 void launch_pres_init(const Dev& d, cudaStream_t s) {
     if (halo_on(d)) launch_halo_pass(d, kHaloPresInit, s);
     else VFD_LAUNCH_MODE(VFD_LAUNCH_LANES, "k_pres_init", kTPresInit, K_PRES_INIT);
-    VFD_LAUNCH("k_ctrl_jacobi_init", s, k_ctrl_jacobi_init<false><<<1, 256, 0, s>>>(d));
+    if (d.nscenes > 1) VFD_LAUNCH("k_ctrl_jacobi_init", s, k_ctrl_jacobi_init<false><<<1, 256, 0, s>>>(d));
 }
 void launch_pres_iter(const Dev& d, cudaStream_t s) {
     if (halo_on(d)) {

@@ -23,7 +23,8 @@
 // viscosity product 179 / 146 / 110. Tried and left out: four lanes a particle (124 us for
 // the Jacobi update; the same gathers, more instructions), 4x4x4 tiles (102), two halo buffers
 // (164: half the resident warps), and bulk copies of the halo's runs of 8 to 16 particles by
-// the TMA unit (213: about 80 cycles a copy and SM).
+// the TMA unit (213: about 80 cycles a copy and SM), and tiles drawn by an atomic ticket instead of
+// strided (103, and 2 % at 8M; 1 % less for 48 scenes).
 #include "dfsph_common.cuh"
 #include "dfsph_passes.cuh"
 #include "dfsph_halo.cuh"
@@ -204,7 +205,6 @@ __device__ __forceinline__ void halo_pass(const Dev& d) {
     float4* const sx = haloSmem;
     float4* const sv = haloSmem + kHaloCap;                            // kVectorField
     float* const ss = reinterpret_cast<float*>(haloSmem + kHaloCap);   // kScalarField
-    Op::start(d);
     if (is_aborted(d)) return;
     HaloSum<Op::kTerms> sum;
     const uint32_t nt = halo_tile_total(d, Op::kLoop);
@@ -303,7 +303,6 @@ struct HaloOp {
     __device__ static bool active(const SceneDev&) { return true; }
     __device__ static const void* field(const Dev&) { return nullptr; }
     __device__ static const int* slots() { return nullptr; }
-    __device__ static void start(const Dev&) {}  // by every block, before all else
 };
 __device__ constexpr int kSlots01[2] = {0, 1};
 
@@ -316,7 +315,6 @@ struct HaloDensity : HaloOp<kVectorField, kWriteGrad> {
         float V;
         bool div;
     };
-    __device__ static void start(const Dev& d) { jacobi_start<true>(d); }
     using Acc = DensitySums;
     __device__ static const void* field(const Dev& d) { return d.V; }
     __device__ static void load(const Dev& d, uint32_t p, const SceneDev& S, Own& o) {
@@ -417,7 +415,6 @@ struct HaloPresInit : HaloOp<kVectorField> {
         float4 xi;
         float3 vi;
     };
-    __device__ static void start(const Dev& d) { jacobi_start<false>(d); }
     using Acc = float;
     __device__ static const void* field(const Dev& d) { return d.V; }
     __device__ static void load(const Dev& d, uint32_t p, const SceneDev&, Own& o) {

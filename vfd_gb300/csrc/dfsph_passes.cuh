@@ -454,10 +454,12 @@ __device__ __forceinline__ bool jacobi_begin(const Dev& d, SceneDev& S) {
     L.active = (enabled && ((0.0f > eta) || 0u < mn) && 0u < mx) ? 1u : 0u;
     return L.active != 0u;
 }
-// A single scene's loop is started by the pass before it, which reads nothing of LoopState: a
-// launch less for each of the two loops. (A loop's later decisions stay launches: taken by the
+// A single scene's loop is started by the row pass before it, which reads nothing of LoopState: a
+// launch less for each of the two loops. Not by the tile passes: the same lines take the density
+// pass from 203 to 231 us at 1M particles. (A loop's later decisions stay launches: taken by the
 // last block of a pass, with a fence and an arrival per block, a step of 64,000 particles went
 // from 1,419 to 1,509 us and one of 33,401 from 1,170 to 1,221.)
+inline bool start_apart(const Dev& d) { return d.nscenes > 1 || halo_on(d); }
 template <bool DIV>
 __device__ __forceinline__ void jacobi_start(const Dev& d) {
     if (d.nscenes == 1 && blockIdx.x == 0 && threadIdx.x == 0)

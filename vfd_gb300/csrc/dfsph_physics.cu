@@ -347,7 +347,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_jacobi_iter_b(Dev d) {
     }
 }
 
-// Loop start of a batch (a single scene's first pass does it, jacobi_start).
+// Loop start of batches and of staged tiles (else the pass before it does it, jacobi_start).
 template <bool DIV>
 __global__ void k_ctrl_jacobi_init(Dev d) {
     VFD_COUNT_LAUNCH(d);
@@ -357,8 +357,9 @@ __global__ void k_ctrl_jacobi_init(Dev d) {
     for (uint32_t s = threadIdx.x; s < d.nscenes; s += blockDim.x)
         if (jacobi_begin<DIV>(d, d.scenes[s])) atomicOr(&any, 1u);
     __syncthreads();
-    build_work_list(d, DIV ? kLoopDiv : kLoopPres,
-                    [&](uint32_t sc) { return (DIV ? d.scenes[sc].div.active : d.scenes[sc].pres.active) != 0u; });
+    if (d.nscenes > 1)
+        build_work_list(d, DIV ? kLoopDiv : kLoopPres,
+                        [&](uint32_t sc) { return (DIV ? d.scenes[sc].div.active : d.scenes[sc].pres.active) != 0u; });
     if (threadIdx.x == 0) set_condition(d, DIV ? kLoopDiv : kLoopPres, any);
 }
 
@@ -1168,7 +1169,7 @@ void launch_density(const Dev& d, cudaStream_t s) { VFD_LAUNCH_MODE(VFD_LAUNCH_L
 void launch_density_div_init(const Dev& d, cudaStream_t s) {
     if (halo_on(d)) launch_halo_pass(d, kHaloDensity, s);
     else VFD_LAUNCH_MODE(VFD_LAUNCH_LANES, "k_density_factor", kTDensity, K_DENSITY_DIV);
-    if (d.nscenes > 1) VFD_LAUNCH("k_ctrl_jacobi_init", s, k_ctrl_jacobi_init<true><<<1, 256, 0, s>>>(d));
+    if (start_apart(d)) VFD_LAUNCH("k_ctrl_jacobi_init", s, k_ctrl_jacobi_init<true><<<1, 256, 0, s>>>(d));
 }
 #define K_PACCEL_DB(G) k_pressure_accel_b<true, G, false>
 #define K_PACCEL_DB_R(G) k_pressure_accel_b<true, G, true>
@@ -1267,7 +1268,7 @@ void launch_visc_finish_dt(const Dev& d, cudaStream_t s) {
 void launch_pres_init(const Dev& d, cudaStream_t s) {
     if (halo_on(d)) launch_halo_pass(d, kHaloPresInit, s);
     else VFD_LAUNCH_MODE(VFD_LAUNCH_LANES, "k_pres_init", kTPresInit, K_PRES_INIT);
-    if (d.nscenes > 1) VFD_LAUNCH("k_ctrl_jacobi_init", s, k_ctrl_jacobi_init<false><<<1, 256, 0, s>>>(d));
+    if (start_apart(d)) VFD_LAUNCH("k_ctrl_jacobi_init", s, k_ctrl_jacobi_init<false><<<1, 256, 0, s>>>(d));
 }
 void launch_pres_iter(const Dev& d, cudaStream_t s) {
     if (halo_on(d)) {

@@ -392,7 +392,7 @@ int allocate_halo(vfd_sim* s, Dev& base) {
     base.haloGrad = reinterpret_cast<float*>(base.NG);
     base.haloRow = reinterpret_cast<uint16_t*>(base.haloGrad + st * kHaloRow);
     CK(prepare_halo_kernels());
-    base.haloOn = s->halo != 0 ? 1u : 0u;
+    base.haloOn = s->halo != 0 ? kHaloWide : 0u;
     return VFD_OK;
 }
 
@@ -686,18 +686,21 @@ int upload(vfd_sim* s) {
     TRY(reset_buckets(s, d));
     CK(cudaDeviceSynchronize());
     s->uploaded = true;
+    s->tilesNarrow = true;
+    s->stepsSince = 0;
     s->generation++;
     if (s->fp64Mode) TRY(fp64_upload(s));
     return VFD_OK;
 }
 
 // ---------------------------------------------------------------- step recording
-int build_graph(vfd_sim* s, int parity, const void* rec, cudaGraph_t* gOut, cudaGraphExec_t* execOut) {
+int build_graph(vfd_sim* s, int parity, const void* rec, cudaGraph_t* gOut, cudaGraphExec_t* execOut, bool narrow) {
     cudaGraph_t g;
     CK(cudaGraphCreate(&g, 0));
     // One conditional handle per while node the graph has (divergence, CG, pressure): a
     // handle that no node uses makes cudaGraphInstantiate fail with "invalid argument".
     Dev d = s->dev[parity];
+    if (narrow) d.haloOn = kHaloNarrow;
     const bool used[3] = {s->anyDiv, s->anyVisc, true};
     cudaGraphConditionalHandle h[3] = {};
     for (int k = 0; k < 3; k++) {
@@ -770,7 +773,16 @@ int build_graph(vfd_sim* s, int parity, const void* rec, cudaGraph_t* gOut, cuda
     return VFD_OK;
 }
 
-int build_graph(vfd_sim* s, int parity) { return build_graph(s, parity, nullptr, &s->graph[parity], &s->exec[parity]); }
+// The narrow tile form serves where the last step that was waited for, at most kNarrowSteps
+// launches ago, found few tiles beyond it (or the run starts): its state is near enough.
+constexpr uint32_t kNarrowSteps = 8u;
+int step_graph(vfd_sim* s, int* slot) {
+    const bool narrow = s->dev[s->cs].haloOn == kHaloWide && s->tilesNarrow && s->stepsSince < kNarrowSteps;
+    s->stepsSince++;
+    *slot = s->cs + (narrow ? 2 : 0);
+    if (s->exec[*slot]) return VFD_OK;
+    return build_graph(s, s->cs, nullptr, &s->graph[*slot], &s->exec[*slot], narrow);
+}
 
 int read_flag(vfd_sim* s, int idx, uint32_t& v) {
     CK(cudaMemcpyAsync(s->hStatus + idx, s->dStatus + idx, sizeof(uint32_t), cudaMemcpyDeviceToHost, s->stream));
@@ -873,17 +885,15 @@ int ensure_ready(vfd_sim* s) {
 
 int launch_one(vfd_sim* s) {
     if (s->graphMode && !s->graphFailed) {
-        if (!s->exec[s->cs]) {
-            const int rc = build_graph(s, s->cs);
-            if (rc != VFD_OK) {
-                // keep the kernels, drop the graph: eager launches of the same kernels
-                s->graphFailed = true;
-                s->releaseGraphs();
-            }
+        int slot = 0;
+        if (step_graph(s, &slot) != VFD_OK) {
+            // keep the kernels, drop the graph: eager launches of the same kernels
+            s->graphFailed = true;
+            s->releaseGraphs();
         }
         if (!s->graphFailed) {
             PhaseRange r("vfd_step (graph)");
-            CK(cudaGraphLaunch(s->exec[s->cs], s->stream));
+            CK(cudaGraphLaunch(s->exec[slot], s->stream));
             s->cs = 1 - s->cs;
             return VFD_OK;
         }
@@ -904,6 +914,8 @@ int finish_steps(vfd_sim* s, vfd_step_stats* stats, uint32_t& flags) {
     CK(cudaStreamSynchronize(s->stream));
     CK(cudaGetLastError());
     flags = s->hStatus[0];
+    s->tilesNarrow = s->hStatus[12] * 4u <= s->hStatus[13];
+    s->stepsSince = 0;
     if (stats) std::memcpy(s->hScenes.data(), s->hStage, bytes);
     return VFD_OK;
 }
@@ -2144,7 +2156,7 @@ int vfd_profile_kernels(vfd_sim* s, uint32_t steps, vfd_kernel_time* out, uint32
 // Whether the layout's steps run on staged tiles (where it has the buffers for them).
 static void set_halo(vfd_sim* s, int8_t on) {
     s->halo = on;
-    for (int k = 0; k < 2; k++) s->dev[k].haloOn = on && s->dev[k].haloTiles ? 1u : 0u;
+    for (int k = 0; k < 2; k++) s->dev[k].haloOn = on && s->dev[k].haloTiles ? kHaloWide : 0u;
 }
 
 int vfd_set_lanes(vfd_sim* s, const uint8_t* lanes, uint32_t count) {
@@ -2276,7 +2288,7 @@ int vfd_autotune(vfd_sim* s, uint32_t steps, uint8_t* lanes_out, uint32_t count)
         const bool halo = ct == 3 * kForms * 3;
         const int c = ct % 3, tl = (ct / 3) % kForms, bs = ct / (3 * kForms) % 3;
         for (int k = 0; k < 2; k++) {
-            s->dev[k].haloOn = halo ? 1u : 0u;
+            s->dev[k].haloOn = halo ? kHaloWide : 0u;
             for (int t = 0; t < kTunedCount; t++) {
                 s->dev[k].lanes[t] = cand[c];
                 s->dev[k].tiles[t] = tileCand[tl];

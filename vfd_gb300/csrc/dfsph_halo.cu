@@ -41,6 +41,7 @@ __global__ void __launch_bounds__(256) k_halo_build(Dev d) {
     __shared__ uint32_t warpSum[8], base[kHaloCells], start[kHaloCells], offset;
     const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
     const uint32_t nt = d.haloInfo[0];
+    if (blockIdx.x == 0 && threadIdx.x == 0) d.status[13] = nt;
     for (uint32_t t = blockIdx.x; t < nt; t += gridDim.x) {
         HaloTile& T = d.haloTiles[t];
         const SceneDev& S = d.scenes[T.scene];
@@ -78,11 +79,12 @@ __global__ void __launch_bounds__(256) k_halo_build(Dev d) {
             d.haloBase[(size_t)(T.cell0 / kHaloTileCells) * kHaloCells + threadIdx.x] = (uint16_t)(pre + x - cc);
         }
         if (threadIdx.x == 0) {
-            const bool fits = total <= kHaloCap;
+            const bool fits = total <= halo_cap(d);
             const uint32_t at = fits ? atomicAdd(d.haloInfo + 1, total) : 0u;
             offset = fits ? at : 0xFFFFFFFFu;
             T.list = at;
             T.staged = total;
+            if (T.last - T.first > kHaloThreads || total > kHaloCap) atomicAdd(d.status + 12, 1u);
         }
         __syncthreads();
         if (offset != 0xFFFFFFFFu)
@@ -109,14 +111,20 @@ __device__ __forceinline__ void copy_async4(void* smem, const void* g) {
 __device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 enum HaloField { kNoField = 0, kScalarField = 1, kVectorField = 4 };  // floats staged beside the position
-enum HaloGrad { kReadGrad = 0, kWriteGrad = 1, kNoGrad = 2 };
+enum HaloGrad { kReadGrad = 0, kWriteGrad = 1 };
 
-template <class Op>
-constexpr size_t halo_smem() { return (size_t)kHaloCap * (16u + 4u * (size_t)Op::kField); }
+// Threads and resident blocks of a pass, and the particles it can stage, in the narrow and the wide form.
+template <class Op, bool WIDE>
+struct HaloShape {
+    static constexpr uint32_t kThreads = WIDE ? Op::kWideThreads : kHaloThreads, kCap = WIDE ? kHaloWideCap : kHaloCap;
+    static constexpr uint32_t kBlocks = kThreads == kHaloThreads ? Op::kBlocks : Op::kBlocks >= 4u ? 3u : 2u;
+    static constexpr bool kAhead = Op::kAhead && kThreads == kHaloThreads;
+    static constexpr size_t kSmem = (size_t)kCap * (16u + 4u * (size_t)Op::kField);
+};
 
 // FP32-pair sums of a pass's K reduction terms over a block's tiles, added to the scene's
 // FP64 buckets when the scene changes and at the end.
-template <int K>
+template <int K, uint32_t THREADS>
 struct HaloSum {
     float hi[K], lo[K];
     int scene = -1;
@@ -126,7 +134,7 @@ struct HaloSum {
     }
     // all threads of the block, with the same scene
     __device__ void flush(const Dev& d, const int* slot) {
-        __shared__ float2 part[kHaloThreads / 32u][K];
+        __shared__ float2 part[THREADS / 32u][K];
 #pragma unroll
         for (int k = 0; k < K; k++) {
             float h = hi[k], l = lo[k];
@@ -141,7 +149,7 @@ struct HaloSum {
         __syncthreads();
         if (threadIdx.x < (uint32_t)K && scene >= 0) {
             float a = 0.0f, b = 0.0f;
-            for (uint32_t w = 0; w < kHaloThreads / 32u; w++) pair_add(a, b, part[w][threadIdx.x].x, part[w][threadIdx.x].y);
+            for (uint32_t w = 0; w < THREADS / 32u; w++) pair_add(a, b, part[w][threadIdx.x].x, part[w][threadIdx.x].y);
             const double t = pair_value(make_float2(a, b));
             if (t != 0.0) atomicAdd(acc_bucket(d, (uint32_t)scene, slot[threadIdx.x], blockIdx.x % kBuckets), t);
         }
@@ -151,25 +159,25 @@ struct HaloSum {
     }
 };
 
-template <>
-struct HaloSum<0> {
+template <uint32_t THREADS>
+struct HaloSum<0, THREADS> {
     int scene = -1;
     float hi[1], lo[1];
     __device__ __forceinline__ void flush(const Dev&, const int*) {}
 };
 
 // Starts the copies of a tile's halo into shared memory.
-template <int FIELD>
+template <int FIELD, uint32_t THREADS, uint32_t CAP>
 __device__ __forceinline__ void halo_fetch(const Dev& d, const HaloTile& T, const void* field, float4* sx) {
-    if (T.staged <= kHaloCap) {
+    if (T.staged <= CAP) {
         const uint32_t* list = d.haloList + T.list;
 #pragma unroll 2
-        for (uint32_t i = threadIdx.x; i < T.staged; i += kHaloThreads) {
+        for (uint32_t i = threadIdx.x; i < T.staged; i += THREADS) {
             const uint32_t q = checked_index(d.status, __ldg(list + i), d.n);
             copy_async16(sx + i, d.X + q);
-            if (FIELD == kVectorField) copy_async16(sx + kHaloCap + i, reinterpret_cast<const float4*>(field) + q);
+            if (FIELD == kVectorField) copy_async16(sx + CAP + i, reinterpret_cast<const float4*>(field) + q);
             if (FIELD == kScalarField)
-                copy_async4(reinterpret_cast<float*>(sx + kHaloCap) + i, reinterpret_cast<const float*>(field) + q);
+                copy_async4(reinterpret_cast<float*>(sx + CAP) + i, reinterpret_cast<const float*>(field) + q);
         }
     }
 }
@@ -199,14 +207,17 @@ __device__ __forceinline__ void halo_entries(const Dev& d, uint32_t p, uint32_t 
     }
 }
 
-template <class Op>
+template <class Op, bool WIDE>
 __device__ __forceinline__ void halo_pass(const Dev& d) {
+    using Shape = HaloShape<Op, WIDE>;
+    constexpr uint32_t kThreads = Shape::kThreads, kCap = Shape::kCap;
+    constexpr bool kAhead = Shape::kAhead;
     extern __shared__ float4 haloSmem[];
     float4* const sx = haloSmem;
-    float4* const sv = haloSmem + kHaloCap;                            // kVectorField
-    float* const ss = reinterpret_cast<float*>(haloSmem + kHaloCap);   // kScalarField
+    float4* const sv = haloSmem + kCap;                            // kVectorField
+    float* const ss = reinterpret_cast<float*>(haloSmem + kCap);   // kScalarField
     if (is_aborted(d)) return;
-    HaloSum<Op::kTerms> sum;
+    HaloSum<Op::kTerms, kThreads> sum;
     const uint32_t nt = halo_tile_total(d, Op::kLoop);
     for (uint32_t v = blockIdx.x; v < nt; v += gridDim.x) {
         const HaloTile T = d.haloTiles[halo_tile_at(d, Op::kLoop, v)];
@@ -216,10 +227,10 @@ __device__ __forceinline__ void halo_pass(const Dev& d) {
             if (sum.scene >= 0) sum.flush(d, Op::slots());
             sum.scene = (int)T.scene;
         }
-        const bool fits = T.staged <= kHaloCap;
-        halo_fetch<Op::kField>(d, T, Op::field(d), sx);
+        const bool fits = T.staged <= kCap;
+        halo_fetch<Op::kField, kThreads, kCap>(d, T, Op::field(d), sx);
         bool waiting = true;
-        for (uint32_t pb = T.first; pb < T.last; pb += kHaloThreads) {
+        for (uint32_t pb = T.first; pb < T.last; pb += kThreads) {
             const bool live = pb + threadIdx.x < T.last;
             const uint32_t p = live ? pb + threadIdx.x : T.first;
             const uint32_t ncnt = d.NCNT[p];
@@ -238,8 +249,8 @@ __device__ __forceinline__ void halo_pass(const Dev& d) {
             if (fits) {
                 for (uint32_t k = 0; k < cnt; k += 8u) {
                     HaloEntries y;
-                    if (Op::kAhead && k + 8u < cnt) halo_entries<Op::kGrad>(d, p, k + 8u, y);
-                    if (!Op::kAhead && k > 0u) halo_entries<Op::kGrad>(d, p, k, x);
+                    if (kAhead && k + 8u < cnt) halo_entries<Op::kGrad>(d, p, k + 8u, y);
+                    if (!kAhead && k > 0u) halo_entries<Op::kGrad>(d, p, k, x);
                     const uint32_t ee[4] = {x.e.x, x.e.y, x.e.z, x.e.w};
                     float gg[8] = {x.g0.x, x.g0.y, x.g0.z, x.g0.w, x.g1.x, x.g1.y, x.g1.z, x.g1.w};
 #pragma unroll
@@ -255,7 +266,7 @@ __device__ __forceinline__ void halo_pass(const Dev& d) {
                         __stcs(reinterpret_cast<float4*>(d.haloGrad + halo_grad_at(p, k)), make_float4(gg[0], gg[1], gg[2], gg[3]));
                         __stcs(reinterpret_cast<float4*>(d.haloGrad + halo_grad_at(p, k + 4u)), make_float4(gg[4], gg[5], gg[6], gg[7]));
                     }
-                    if (Op::kAhead) x = y;
+                    if (kAhead) x = y;
                 }
             } else {
                 for (uint32_t k = 0; k < cnt; k += 8u)
@@ -299,6 +310,7 @@ struct HaloOp {
     // product, against 75, 107 and 118 with three and 73, 106 and 125 with three and entries
     // ahead); the others, with more sums a particle, with three and entries ahead.
     static constexpr uint32_t kBlocks = BLOCKS;
+    static constexpr uint32_t kWideThreads = kHaloWideThreads;
     static constexpr bool kAhead = BLOCKS < 4u;
     __device__ static bool active(const SceneDev&) { return true; }
     __device__ static const void* field(const Dev&) { return nullptr; }
@@ -411,6 +423,7 @@ struct HaloJacobi : HaloOp<kVectorField, kReadGrad, 4u, 1, DIV ? kLoopDiv : kLoo
 // K17.
 template <bool REL>
 struct HaloPresInit : HaloOp<kVectorField> {
+    static constexpr uint32_t kWideThreads = kHaloThreads;  // the registers of more threads would spill
     struct Own {
         float4 xi;
         float3 vi;
@@ -436,6 +449,7 @@ struct HaloPresInit : HaloOp<kVectorField> {
 // K12 + K13.
 template <bool REL>
 struct HaloPrecond : HaloOp<kScalarField, kReadGrad, 2u> {
+    static constexpr uint32_t kWideThreads = kHaloThreads;  // the registers of more threads would spill
     struct Own {
         float4 xi;
         float eps2, cmu, mass;
@@ -507,84 +521,13 @@ struct HaloSpmv : HaloMatvec<REL, kLoopCG> {
     }
 };
 
-// K10.
-template <bool REL>
-struct HaloSmooth : HaloOp<kVectorField, kNoGrad> {
-    struct Own {
-        float4 xi, ni;
-        float h;
-    };
-    struct Acc {
-        float3 nc = {0.0f, 0.0f, 0.0f};
-        float cc = 0.0f, cf = 0.0f;
-        __device__ void operator+=(const Acc& b) { nc += b.nc, cc += b.cc, cf += b.cf; }
-    };
-    __device__ static bool active(const SceneDev& S) { return S.enableST != 0; }
-    __device__ static const void* field(const Dev& d) { return d.STN; }
-    __device__ static void load(const Dev& d, uint32_t p, const SceneDev& S, Own& o) {
-        o.xi = d.X[p];
-        o.ni = d.STN[p];
-        o.h = S.h;
-    }
-    __device__ static void pair(const Dev& d, const Own& o, float4 xq, float4 nj, float&, bool ok, Acc& a) {
-        if (!nonzero3(o.ni)) return;
-        const float3 dx = pair_r<REL>(d, xq, o.xi);
-        if (ok && nonzero3(nj)) {
-            const float num = 1.0f - __fdividef(fast_sqrt(dot3(dx, dx)), o.h);
-            a.nc += f3(nj) * num;
-            a.cc += nj.w * num;
-            a.cf += num;
-        }
-    }
-    __device__ static void finish(const Dev& d, uint32_t p, const SceneDev& S, const Own& o, const Acc& a, uint32_t, float*) {
-        if (nonzero3(o.ni)) st_smooth_finish(d, p, S, o.ni, a.nc, a.cc, a.cf);
-    }
-};
-
-constexpr uint32_t kClassifyLanes = 8u;
-
-// K9: the samples walk the staged neighbours of their particle.
-template <bool REL>
-struct HaloClassify : HaloOp<kNoField, kNoGrad> {};
-template <bool REL>
-__global__ void __launch_bounds__(kHaloThreads) k_st_classify_halo(Dev d) {
-    VFD_COUNT_LAUNCH(d);
-    extern __shared__ float4 haloSmem[];
-    if (is_aborted(d)) return;
-    const uint32_t nt = halo_tile_total(d, -1), pp = threadIdx.x / kClassifyLanes;
-    for (uint32_t t = blockIdx.x; t < nt; t += gridDim.x) {
-        const HaloTile T = d.haloTiles[t];
-        const SceneDev& S = d.scenes[T.scene];
-        halo_fetch<kNoField>(d, T, nullptr, haloSmem);
-        const bool fits = T.staged <= kHaloCap;
-        copy_async_wait();
-        __syncthreads();
-        for (uint32_t p = T.first + pp; S.enableST && p < T.last; p += kHaloThreads / kClassifyLanes) {  // whole groups together
-            const float4 xi = d.X[p];
-            const uint32_t cnt = d.NCNT[p] & kCountMask;
-            const Group<kClassifyLanes> grp(p);
-            if (fits) {
-                const uint16_t* row = d.haloRow;
-                st_classify_item<kClassifyLanes>(d, grp, p, S, cnt, [&](uint32_t j) {
-                    return pair_r<REL>(d, haloSmem[checked_index(d.status, row[halo_row_at(p, j)], T.staged)], xi);
-                });
-            } else {
-                const uint32_t* row = d.NBR + (size_t)p * kRow;
-                st_classify_item<kClassifyLanes>(d, grp, p, S, cnt, [&](uint32_t j) {
-                    return pair_r<REL>(d, d.X[checked_index(d.status, row[j], d.n)], xi);
-                });
-            }
-        }
-        __syncthreads();  // the next tile overwrites the halo
-    }
-}
-
 // One kernel name per pass, for profilers.
 #define HALO_KERNEL(NAME, OP)                                                          \
-    template <bool REL>                                                                \
-    __global__ void __launch_bounds__(kHaloThreads, OP::kBlocks) NAME(Dev d) {         \
+    template <bool REL, bool WIDE>                                                     \
+    __global__ void __launch_bounds__(HaloShape<OP HALO_COMMA WIDE>::kThreads, HaloShape<OP HALO_COMMA WIDE>::kBlocks) \
+        NAME(Dev d) {                                                                  \
         VFD_COUNT_LAUNCH(d);                                                           \
-        halo_pass<OP>(d);                                                              \
+        halo_pass<OP HALO_COMMA WIDE>(d);                                              \
     }
 #define HALO_COMMA ,
 HALO_KERNEL(k_density_factor_halo, HaloDensity<REL>)
@@ -598,7 +541,6 @@ HALO_KERNEL(k_pres_finish_halo, HaloPresFinish<REL>)
 HALO_KERNEL(k_visc_precond_halo, HaloPrecond<REL>)
 HALO_KERNEL(k_visc_setup_halo, HaloSetup<REL>)
 HALO_KERNEL(k_cg_spmv_halo, HaloSpmv<REL>)
-HALO_KERNEL(k_st_smooth_halo, HaloSmooth<REL>)
 
 // ---------------------------------------------------------------- launches
 // Grid of a pass: the blocks that are resident at once (found by prepare_halo_kernels, which
@@ -609,17 +551,17 @@ int& halo_resident() {
     return resident;
 }
 template <void (*K)(Dev)>
-cudaError_t prepare_halo(size_t smem) {
+cudaError_t prepare_halo(uint32_t threads, size_t smem) {
     cudaError_t e = cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     int n = 0;
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, K, kHaloThreads, smem);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, K, (int)threads, smem);
     halo_resident<K>() = n > 0 ? n : 1;
     return e;
 }
 template <void (*K)(Dev)>
-void launch_halo(const Dev& d, size_t smem, const char* name, cudaStream_t s) {
+void launch_halo(const Dev& d, uint32_t threads, size_t smem, const char* name, cudaStream_t s) {
     const uint32_t sms = d.batchBlocks / (2048u / kBlock);
-    VFD_LAUNCH(name, s, K<<<sms * (uint32_t)halo_resident<K>(), kHaloThreads, smem, s>>>(d));
+    VFD_LAUNCH(name, s, K<<<sms * (uint32_t)halo_resident<K>(), threads, smem, s>>>(d));
 }
 
 #define HALO_PASSES(ACT)                                                     \
@@ -633,34 +575,42 @@ void launch_halo(const Dev& d, size_t smem, const char* name, cudaStream_t s) {
     ACT(kHaloPresFinish, "k_pres_finish", k_pres_finish_halo, HaloPresFinish<REL>)                                  \
     ACT(kHaloPrecond, "k_visc_precond", k_visc_precond_halo, HaloPrecond<REL>)                                      \
     ACT(kHaloSetup, "k_visc_setup", k_visc_setup_halo, HaloSetup<REL>)                                              \
-    ACT(kHaloSpmv, "k_cg_spmv", k_cg_spmv_halo, HaloSpmv<REL>)                                                      \
-    ACT(kHaloClassify, "k_st_classify", k_st_classify_halo, HaloClassify<REL>)                                      \
-    ACT(kHaloSmooth, "k_st_smooth", k_st_smooth_halo, HaloSmooth<REL>)
+    ACT(kHaloSpmv, "k_cg_spmv", k_cg_spmv_halo, HaloSpmv<REL>)
 
-template <bool REL>
+template <bool REL, bool WIDE>
 cudaError_t prepare_halo_kernels() {
     cudaError_t e = cudaSuccess;
-#define HALO_PREPARE(ID, NAME, K, ...) \
-    if (e == cudaSuccess) e = prepare_halo<K<REL>>(halo_smem<__VA_ARGS__>());
+#define HALO_PREPARE(ID, NAME, K, ...)                                  \
+    if (e == cudaSuccess) {                                             \
+        using Shape = HaloShape<__VA_ARGS__, WIDE>;                     \
+        e = prepare_halo<K<REL, WIDE>>(Shape::kThreads, Shape::kSmem);  \
+    }
     HALO_PASSES(HALO_PREPARE)
     return e;
 }
 cudaError_t prepare_halo_kernels() {
-    const cudaError_t e = prepare_halo_kernels<false>();
-    return e == cudaSuccess ? prepare_halo_kernels<true>() : e;
+    cudaError_t e = prepare_halo_kernels<false, false>();
+    if (e == cudaSuccess) e = prepare_halo_kernels<true, false>();
+    if (e == cudaSuccess) e = prepare_halo_kernels<false, true>();
+    return e == cudaSuccess ? prepare_halo_kernels<true, true>() : e;
 }
 
-template <bool REL>
+template <bool REL, bool WIDE>
 void launch_halo_pass(const Dev& d, HaloPass pass, cudaStream_t s) {
     switch (pass) {
-#define HALO_LAUNCH(ID, NAME, K, ...) \
-    case ID: launch_halo<K<REL>>(d, halo_smem<__VA_ARGS__>(), NAME, s); break;
+#define HALO_LAUNCH(ID, NAME, K, ...)                                                   \
+    case ID: {                                                                          \
+        using Shape = HaloShape<__VA_ARGS__, WIDE>;                                     \
+        launch_halo<K<REL, WIDE>>(d, Shape::kThreads, Shape::kSmem, NAME, s);           \
+        break;                                                                          \
+    }
         HALO_PASSES(HALO_LAUNCH)
     }
 }
 void launch_halo_pass(const Dev& d, HaloPass pass, cudaStream_t s) {
-    if (d.cellRel) launch_halo_pass<true>(d, pass, s);
-    else launch_halo_pass<false>(d, pass, s);
+    const bool wide = d.haloOn == kHaloWide;
+    if (d.cellRel) wide ? launch_halo_pass<true, true>(d, pass, s) : launch_halo_pass<true, false>(d, pass, s);
+    else wide ? launch_halo_pass<false, true>(d, pass, s) : launch_halo_pass<false, false>(d, pass, s);
 }
 
 void launch_halo_build(const Dev& d, cudaStream_t s) {

@@ -10,10 +10,16 @@ constexpr uint32_t kHaloLog2 = 5u;                        // 2^5 Morton cells a 
 constexpr uint32_t kHaloTileCells = 1u << kHaloLog2;
 constexpr uint32_t kHaloX = (1u << ((kHaloLog2 + 2u) / 3u)) + 2u, kHaloY = (1u << ((kHaloLog2 + 1u) / 3u)) + 2u,
                    kHaloZ = (1u << (kHaloLog2 / 3u)) + 2u, kHaloCells = kHaloX * kHaloY * kHaloZ;
-constexpr uint32_t kHaloThreads = 256u;
-// Staged particles at most: cells hold eight particles at rest spacing, 1152 a halo; a fifth
-// more than that lets five blocks of a two-array pass share an SM.
-constexpr uint32_t kHaloCap = 1408u;
+// Two forms (Dev::haloOn). A lattice at the particles' diameter holds eight particles a cell, 256
+// a tile and 1,152 a halo; a fluid at rest density ten, 320 and 1,440. The narrow form takes the
+// first in one round of its threads with four blocks an SM, and spills over into a second,
+// nearly empty one in the other; the wide form takes both, with three. Mean step of the viscous
+// dam at 1M particles: 6.9 ms narrow and 7.7 wide from the lattice, 8.2 and 7.7 after 300 steps
+// (row kernels 8.2 and 8.2), where halos above the cap walk their rows: 12.3 with the narrow one.
+constexpr uint32_t kHaloNarrow = 1u, kHaloWide = 2u;
+constexpr uint32_t kHaloThreads = 256u, kHaloWideThreads = 384u;
+constexpr uint32_t kHaloCap = 1408u, kHaloWideCap = 1760u;
+__host__ __device__ inline uint32_t halo_cap(const Dev& d) { return d.haloOn == kHaloWide ? kHaloWideCap : kHaloCap; }
 constexpr uint32_t kHaloRow = 96u;                        // row length: kMaxNeighbors rounded up to 32
 
 // Layouts that run on staged tiles. Against the row kernels with four lanes a particle, a step
@@ -58,7 +64,7 @@ __device__ __forceinline__ uint32_t halo_tile_at(const Dev& d, int loop, uint32_
 
 enum HaloPass {
     kHaloDensity, kHaloPAccelD, kHaloPAccelP, kHaloJacobiD, kHaloJacobiP, kHaloDivFinish, kHaloPresInit, kHaloPresFinish,
-    kHaloPrecond, kHaloSetup, kHaloSpmv, kHaloClassify, kHaloSmooth
+    kHaloPrecond, kHaloSetup, kHaloSpmv
 };
 void launch_halo_pass(const Dev& d, HaloPass pass, cudaStream_t s);
 void launch_halo_build(const Dev& d, cudaStream_t s);

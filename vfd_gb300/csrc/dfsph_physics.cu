@@ -1215,13 +1215,10 @@ void launch_div_finish(const Dev& d, cudaStream_t s) {
     else VFD_LAUNCH_MODE(VFD_LAUNCH_LANES, "k_div_finish", kTDivFinish, K_DIV_FINISH);
 }
 void launch_surface_tension(const Dev& d, uint32_t maxPasses, cudaStream_t s) {
-    if (halo_on(d)) {
-        launch_halo_pass(d, kHaloClassify, s);
-        launch_halo_pass(d, kHaloSmooth, s);
-    } else {
-        VFD_LAUNCH_MODE(VFD_LAUNCH_LANES, "k_st_classify", kTStClassify, K_ST_CLASSIFY);
-        VFD_LAUNCH_MODE(VFD_LAUNCH_LANES, "k_st_smooth", kTStSmooth, K_ST_SMOOTH);
-    }
+    // by rows whatever the other passes run on: most particles of a step end early (36 us for
+    // k_st_smooth at 1M particles where a tile pass takes 73 to 105, k_st_classify 143 to 163 and 136 to 201)
+    VFD_LAUNCH_MODE(VFD_LAUNCH_LANES, "k_st_classify", kTStClassify, K_ST_CLASSIFY);
+    VFD_LAUNCH_MODE(VFD_LAUNCH_LANES, "k_st_smooth", kTStSmooth, K_ST_SMOOTH);
     for (uint32_t pass = 0; pass < maxPasses; pass++)
         VFD_LAUNCH("k_st_blend", s, k_st_blend<<<blocks_for(d.n), kBlock, 0, s>>>(d, pass));
 }

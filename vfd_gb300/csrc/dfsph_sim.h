@@ -224,8 +224,11 @@ struct vfd_sim {
     bool anyDiv = false, anyVisc = false, anyST = false;
 
     // graphs (one per parity)
-    cudaGraphExec_t exec[2] = {nullptr, nullptr};
-    cudaGraph_t graph[2] = {nullptr, nullptr};
+    // step graphs per parity of the state sets, then those with the narrow tile form
+    cudaGraphExec_t exec[4] = {nullptr, nullptr, nullptr, nullptr};
+    cudaGraph_t graph[4] = {nullptr, nullptr, nullptr, nullptr};
+    bool tilesNarrow = true;    // what the last look at the tiles says (a fresh start is a lattice)
+    uint32_t stepsSince = 0;    // steps launched since
     bool searchOnlyPending = false;
 
     // adjoint: checkpoints and tapes of the last vfd_adjoint_forward; `generation`
@@ -245,11 +248,13 @@ struct vfd_sim {
     ~vfd_sim() { release(); }
 
     void releaseGraphs() {
-        for (int k = 0; k < 2; k++) {
+        for (int k = 0; k < 4; k++) {
             if (exec[k]) cudaGraphExecDestroy(exec[k]);
             if (graph[k]) cudaGraphDestroy(graph[k]);
             exec[k] = nullptr;
             graph[k] = nullptr;
+        }
+        for (int k = 0; k < 2; k++) {
             if (adjRecExec[k]) cudaGraphExecDestroy(adjRecExec[k]);
             if (adjRecGraph[k]) cudaGraphDestroy(adjRecGraph[k]);
             adjRecExec[k] = nullptr;
@@ -351,7 +356,8 @@ enum TapePoint {
 void tape_point(const Dev& d, const void* rec, int point, cudaStream_t st);
 
 // One step as a graph (rec: the adjoint's device tape set, or null) into *gOut / *execOut.
-int build_graph(vfd_sim* s, int parity, const void* rec, cudaGraph_t* gOut, cudaGraphExec_t* execOut);
+int build_graph(vfd_sim* s, int parity, const void* rec, cudaGraph_t* gOut, cudaGraphExec_t* execOut,
+                bool narrow = false);
 // One eagerly launched step (one flag read per solver iteration), optionally recording.
 int launch_eager(vfd_sim* s, const void* rec);
 

@@ -18,13 +18,15 @@
 //     a particle's sums have the same bits on either path.
 // What bounds it: shared-memory gathers (ncu, 512k particles: the data pipe 78 % busy while an
 // SM is active, 2.4 wavefronts of bank conflict each; DRAM 260 bytes a particle, a third of
-// its bandwidth). Per launch at 1M particles, row kernels with their default eight lanes,
-// with four, and tiles: Jacobi update 147 / 128 / 100 us, pressure acceleration 83 / 75 / 67,
-// viscosity product 179 / 146 / 110. Tried and left out: four lanes a particle (124 us for
+// its bandwidth). Per launch at 1M particles on a lattice, row kernels with eight lanes, with
+// four, and tiles (narrow form): Jacobi update 147 / 131 / 101 us, pressure acceleration 83 / 89 /
+// 68, viscosity product 179 / 148 / 110; after 300 steps rows with four lanes and the wide form:
+// 160 / 139, 106 / 100, 178 / 162 (and the density pass 285 / 316). Tried and left out: four lanes a particle (124 us for
 // the Jacobi update; the same gathers, more instructions), 4x4x4 tiles (102), two halo buffers
 // (164: half the resident warps), and bulk copies of the halo's runs of 8 to 16 particles by
 // the TMA unit (213: about 80 cycles a copy and SM), and tiles drawn by an atomic ticket instead of
-// strided (103, and 2 % at 8M; 1 % less for 48 scenes).
+// strided (103, and 2 % at 8M; 1 % less for 48 scenes), and part-filled rounds with two or four
+// threads a particle (after 300 steps 184 us for the Jacobi update, 155 with idle threads).
 #include "dfsph_common.cuh"
 #include "dfsph_passes.cuh"
 #include "dfsph_halo.cuh"

@@ -420,7 +420,8 @@ int vfd_profile_kernels(vfd_sim* sim, uint32_t steps, vfd_kernel_time* out, uint
  * pressure finish (no counterpart in the reference, which launches every kernel
  * with 256 threads, one per particle). The neighbour search runs a warp per cell.
  * Untuned, 8 lanes run below 24,000 particles and 4 from there on, and from 100,000
- * on the loops run on cell tiles staged in shared memory, a thread per particle; setting
+ * on (700,000 for fluid denser than a lattice at the particles' diameter) the loops run on
+ * cell tiles staged in shared memory, a thread per particle; setting
  * lanes, tiles or blocks selects the row (or cell-tile) kernels. 4 lanes, 8 lanes and
  * staged tiles give the same bits per particle.
  */

@@ -392,7 +392,7 @@ int allocate_halo(vfd_sim* s, Dev& base) {
     base.haloGrad = reinterpret_cast<float*>(base.NG);
     base.haloRow = reinterpret_cast<uint16_t*>(base.haloGrad + st * kHaloRow);
     CK(prepare_halo_kernels());
-    base.haloOn = s->halo != 0 ? kHaloWide : 0u;
+    base.haloOn = s->halo != 0 && s->n >= kHaloWideMinParticles ? kHaloWide : 0u;
     return VFD_OK;
 }
 
@@ -774,10 +774,11 @@ int build_graph(vfd_sim* s, int parity, const void* rec, cudaGraph_t* gOut, cuda
 }
 
 // The narrow tile form serves where the last step that was waited for, at most kNarrowSteps
-// launches ago, found few tiles beyond it (or the run starts): its state is near enough.
+// launches ago, found few tiles beyond it (or the run starts): its state is near enough. Else the
+// wide form or, in smaller scenes, the row kernels run (Dev::haloOn). The same bits by all.
 constexpr uint32_t kNarrowSteps = 8u;
 int step_graph(vfd_sim* s, int* slot) {
-    const bool narrow = s->dev[s->cs].haloOn == kHaloWide && s->tilesNarrow && s->stepsSince < kNarrowSteps;
+    const bool narrow = s->halo != 0 && s->dev[s->cs].haloTiles && s->tilesNarrow && s->stepsSince < kNarrowSteps;
     s->stepsSince++;
     *slot = s->cs + (narrow ? 2 : 0);
     if (s->exec[*slot]) return VFD_OK;
@@ -2156,7 +2157,7 @@ int vfd_profile_kernels(vfd_sim* s, uint32_t steps, vfd_kernel_time* out, uint32
 // Whether the layout's steps run on staged tiles (where it has the buffers for them).
 static void set_halo(vfd_sim* s, int8_t on) {
     s->halo = on;
-    for (int k = 0; k < 2; k++) s->dev[k].haloOn = on && s->dev[k].haloTiles ? kHaloWide : 0u;
+    for (int k = 0; k < 2; k++) s->dev[k].haloOn = on && s->dev[k].haloTiles && s->n >= kHaloWideMinParticles ? kHaloWide : 0u;
 }
 
 int vfd_set_lanes(vfd_sim* s, const uint8_t* lanes, uint32_t count) {
@@ -2283,7 +2284,7 @@ int vfd_autotune(vfd_sim* s, uint32_t steps, uint8_t* lanes_out, uint32_t count)
     double times[kTunedCount][3][kForms][3] = {};  // [kernel][lanes][form][block]
     double haloTime = 0.0;  // the same kernels on staged tiles, with the pass that lists them
     int rc = VFD_OK;
-    const bool canHalo = s->dev[0].haloTiles != nullptr;
+    const bool canHalo = s->dev[0].haloTiles != nullptr && s->n >= kHaloWideMinParticles;
     for (int ct = 0; ct < 3 * kForms * 3 + (canHalo ? 1 : 0) && rc == VFD_OK; ct++) {
         const bool halo = ct == 3 * kForms * 3;
         const int c = ct % 3, tl = (ct / 3) % kForms, bs = ct / (3 * kForms) % 3;

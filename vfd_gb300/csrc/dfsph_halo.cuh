@@ -25,8 +25,11 @@ constexpr uint32_t kHaloRow = 96u;                        // row length: kMaxNei
 // Layouts that run on staged tiles. Against the row kernels with four lanes a particle, a step
 // of a viscous drop (graph) took 1374 us against 1184 at 33,000 particles, 1795 against 1732 at
 // 66,000, 2180 against 2199 at 100,000 and 2705 against 3027 at 260,000; below the line there
-// are too few tiles for the SMs. List places fit 32 bits up to the other.
-constexpr uint32_t kHaloMinParticles = 100000u, kHaloMaxParticles = 1u << 28;
+// are too few tiles for the SMs. List places fit 32 bits up to the other. Where the narrow form
+// does not fit, the wide one runs from a line further up: 50 steps to 350 of a viscous dam took
+// 1.7 to 2.2 ms a step against 1.7 to 2.0 by rows at 157,000 particles, 2.5 to 2.8 against 2.5 to 2.6
+// at 262,000, 4.0 to 4.7 against 3.7 to 4.8 at 512,000 and 7.4 to 7.7 against 8.0 to 8.3 at 1M.
+constexpr uint32_t kHaloMinParticles = 100000u, kHaloMaxParticles = 1u << 28, kHaloWideMinParticles = 700000u;
 // Where row entry j of slot p lies: the rows of 32 consecutive slots are interleaved, eight
 // places (four gradient factors) of a slot at a time, so that a warp with a particle a lane
 // loads 16 bytes a lane from consecutive addresses.

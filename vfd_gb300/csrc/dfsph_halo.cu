@@ -547,17 +547,24 @@ HALO_KERNEL(k_cg_spmv_halo, HaloSpmv<REL>)
 // ---------------------------------------------------------------- launches
 // Grid of a pass: the blocks that are resident at once (found by prepare_halo_kernels, which
 // also raises the shared-memory limit, before any capture).
+constexpr int kMaxDevices = 64;
+inline int current_device() {
+    int device = 0;
+    cudaGetDevice(&device);
+    return device < kMaxDevices ? device : 0;
+}
 template <void (*K)(Dev)>
 int& halo_resident() {
-    static int resident = 0;
-    return resident;
+    static int resident[kMaxDevices] = {};
+    return resident[current_device()];
 }
 template <void (*K)(Dev)>
 cudaError_t prepare_halo(uint32_t threads, size_t smem) {
+    if (halo_resident<K>() > 0) return cudaSuccess;
     cudaError_t e = cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     int n = 0;
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, K, (int)threads, smem);
-    halo_resident<K>() = n > 0 ? n : 1;
+    if (e == cudaSuccess) halo_resident<K>() = n > 0 ? n : 1;
     return e;
 }
 template <void (*K)(Dev)>

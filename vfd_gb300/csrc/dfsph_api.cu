@@ -5,6 +5,7 @@
 // viscosity and pressure loops) or as eagerly launched kernels with one flag
 // read per solver iteration, and converts results back to the caller's
 // particle order.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -27,6 +28,7 @@
 
 #include "dfsph_halo.cuh"
 #include "dfsph_sim.h"
+#include "host_array.h"
 
 namespace vfd {
 LaunchProfiler* g_profiler = nullptr;
@@ -84,20 +86,35 @@ __global__ void k_report(const uint32_t* status, uint32_t* hostStatus, const uin
         else hostScenes[i - 16u] = scenes[i - 16u];
     }
 }
-// Whether a kernel can carry this host array in place of a copy: pinned (or not wanted). The
+// The allocation or registration that an address lies in (cuPointerGetAttributes, through the
+// entry point that the runtime hands out).
+bool address_range(const void* p, HostRange& r) {
+    typedef CUresult (*GetFn)(unsigned int, CUpointer_attribute*, void**, CUdeviceptr);
+    static const GetFn get = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        const cudaError_t e = cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 12000, cudaEnableDefault, &q);
+        return (GetFn)(e == cudaSuccess && q == cudaDriverEntryPointSuccess ? f : nullptr);
+    }();
+    CUpointer_attribute what[2] = {CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    CUdeviceptr start = 0;
+    void* out[2] = {&start, &r.size};
+    if (!get || get(2, what, out, (CUdeviceptr)p) != CUDA_SUCCESS) return false;
+    r.start = (const void*)start;
+    return true;
+}
+// Whether a kernel can carry this host array in place of a copy (or it is not wanted). The
 // copy engine's start costs more than it saves at every size: with it 8,000 particles were set in
 // 27.5 us and read in 39.6 and 2.7 million in 411 and 639, by kernels in 24.7 and 26.8, 379 and 638.
 bool kernel_copy(const void* p, size_t bytes) {
     if (!p) return true;
-    for (const char* q : {static_cast<const char*>(p), static_cast<const char*>(p) + bytes - 1}) {
-        cudaPointerAttributes a;
-        if (cudaPointerGetAttributes(&a, q) != cudaSuccess) {
-            cudaGetLastError();
-            return false;
-        }
-        if (a.type != cudaMemoryTypeHost || a.devicePointer != q) return false;
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
     }
-    return true;
+    HostRange r{a.type == cudaMemoryTypeHost, a.devicePointer, nullptr, 0};
+    return r.pinned && address_range(p, r) && kernel_reaches(p, bytes, r);
 }
 // Positions out of the cell-relative form (Dev::cellRel): absolute FP32
 // coordinates of slots [begin, begin + count) in original order; `anchors` holds each

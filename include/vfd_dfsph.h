@@ -423,10 +423,19 @@ int vfd_profile_kernels(vfd_sim* sim, uint32_t steps, vfd_kernel_time* out, uint
  * on (700,000 for fluid denser than a lattice at the particles' diameter) the loops run on
  * cell tiles staged in shared memory, a thread per particle; setting
  * lanes, tiles or blocks selects the row (or cell-tile) kernels. 4 lanes, 8 lanes and
- * staged tiles give the same bits per particle.
+ * staged tiles give the same bits for each particle's sums; the sums over all particles are
+ * grouped differently (a relative 1e-13, vfd_get_tile_form).
  */
 int vfd_set_lanes(vfd_sim* sim, const uint8_t* lanes, uint32_t count);
 int vfd_get_lanes(const vfd_sim* sim, uint8_t* lanes, uint32_t count);
+
+/*
+ * Form of the staged tiles that the last step that was waited for ran on: 0 = none (rows), 1 =
+ * narrow (for a lattice at the particles' diameter), 2 = wide (for denser fluid). Each step
+ * takes the form that the cells of its own state ask for, so the same state steps alike
+ * whatever was run before it.
+ */
+int vfd_get_tile_form(const vfd_sim* sim, uint32_t* form);
 
 /*
  * Form of the solver-loop kernels (pressure acceleration, Jacobi update, CG

@@ -37,6 +37,7 @@ EXPORTS = [
     "vfd_set_position_mode", "vfd_build_mesh_map", "vfd_sample_mesh_volume", "vfd_set_kernel_mode",
     "vfd_emit", "vfd_get_graph_mode", "vfd_checkpoint_size", "vfd_checkpoint", "vfd_restore",
     "vfd_set_tiles", "vfd_get_tiles", "vfd_set_precision", "vfd_get_state_f64", "vfd_set_blocks", "vfd_get_blocks",
+    "vfd_get_tile_form",
     "vfd_adjoint_set_warm_start", "vfd_adjoint_get_stats", "vfd_adjoint_set_tolerance",
     # include/vfd_sph.h: the legacy SPH pipeline (vfd_gb300.sph)
     "vfd_sph_create", "vfd_sph_destroy", "vfd_sph_on_update", "vfd_sph_steps", "vfd_sph_reset",
@@ -124,6 +125,7 @@ def lib() -> C.CDLL:
                 "vfd_set_precision": [P, C.c_int32],
                 "vfd_set_blocks": [P, C.POINTER(C.c_uint16), C.c_uint32],
                 "vfd_get_blocks": [P, C.POINTER(C.c_uint16), C.c_uint32],
+                "vfd_get_tile_form": [P, C.POINTER(C.c_uint32)],
                 "vfd_get_state_f64": [P, C.POINTER(C.c_double), C.POINTER(C.c_double)],
                 "vfd_get_tiles": [P, C.POINTER(C.c_uint8), C.c_uint32],
                 "vfd_autotune": [P, C.c_uint32, C.POINTER(C.c_uint8), C.c_uint32],
@@ -578,6 +580,12 @@ class DFSPHSimulation:
         dp = lambda a: a.ctypes.data_as(C.POINTER(C.c_double))  # noqa: E731
         _check(lib().vfd_get_state_f64(self._h, dp(x), dp(v)), "vfd_get_state_f64")
         return x, v
+
+    def TileForm(self) -> int:
+        """Form of the staged tiles of the last step that was waited for: 0 rows, 1 narrow, 2 wide."""
+        form = C.c_uint32()
+        _check(lib().vfd_get_tile_form(self._h, C.byref(form)), "vfd_get_tile_form")
+        return form.value
 
     def SetTiles(self, tiles):
         """Per solver-loop pass, in TUNED_KERNELS order: 0 = walk neighbour rows (gradW / r

@@ -1044,13 +1044,13 @@ struct TapeBank {
 struct ShadowKey {
     vfd_desc desc{};
     uint8_t lanes[16] = {}, tiles[16] = {};
-    int8_t halo = -1;
+    uint8_t forms = 0;
     uint16_t blocks[16] = {};
     uint32_t n = 0, graphs = 0, analytic = 0, cellCap = 0;
     bool operator==(const ShadowKey& o) const {
         return std::memcmp(&desc, &o.desc, sizeof(desc)) == 0 && std::memcmp(lanes, o.lanes, sizeof(lanes)) == 0 &&
                std::memcmp(tiles, o.tiles, sizeof(tiles)) == 0 && std::memcmp(blocks, o.blocks, sizeof(blocks)) == 0 &&
-               n == o.n && halo == o.halo && graphs == o.graphs && analytic == o.analytic && cellCap == o.cellCap;
+               n == o.n && forms == o.forms && graphs == o.graphs && analytic == o.analytic && cellCap == o.cellCap;
     }
 };
 
@@ -1245,7 +1245,7 @@ ShadowKey shadow_key(const vfd_sim* s) {
     k.desc = s->scenes[0].desc;
     std::memcpy(k.lanes, s->lanes, sizeof(k.lanes));
     std::memcpy(k.tiles, s->tiles, sizeof(k.tiles));
-    k.halo = s->halo;
+    k.forms = s->forms;
     std::memcpy(k.blocks, s->blocks, sizeof(k.blocks));
     k.n = s->n;
     k.graphs = s->graphMode && !s->graphFailed ? 1u : 0u;
@@ -1288,9 +1288,10 @@ bool ensure_shadow(vfd_sim* s, AdjointState* A) {
     std::memcpy(t->lanes, s->lanes, sizeof(t->lanes));
     t->lanesChosen = true;
     std::memcpy(t->tiles, s->tiles, sizeof(t->tiles));
-    t->halo = s->halo;
+    t->forms = s->forms;
     std::memcpy(t->blocks, s->blocks, sizeof(t->blocks));
-    if (ensure_ready(t) != VFD_OK || t->n != s->n || t->stride != s->stride || t->dev[0].haloOn != s->dev[0].haloOn) {
+    if (ensure_ready(t) != VFD_OK || t->n != s->n || t->stride != s->stride || wide_form(t) != wide_form(s) ||
+        chooses_form(t) != chooses_form(s)) {
         delete t;
         cudaGetLastError();
         return false;

@@ -409,7 +409,6 @@ int allocate_halo(vfd_sim* s, Dev& base) {
     base.haloGrad = reinterpret_cast<float*>(base.NG);
     base.haloRow = reinterpret_cast<uint16_t*>(base.haloGrad + st * kHaloRow);
     CK(prepare_halo_kernels());
-    base.haloOn = s->halo != 0 && s->n >= kHaloWideMinParticles ? kHaloWide : 0u;
     return VFD_OK;
 }
 
@@ -520,6 +519,7 @@ int allocate(vfd_sim* s) {
     TRY(dalloc(s, &s->dGM, kTableRes));
     TRY(dalloc(s, &s->dHalton, kHaltonCount));
     CK(cudaMallocHost(&s->hStatus, 16 * sizeof(uint32_t)));
+    std::memset(s->hStatus, 0, 16 * sizeof(uint32_t));
     CK(cudaMallocHost(&s->hStage, sizeof(SceneDev) * s->scenes.size()));
     base.scenes = s->dScenes;
     base.bodies = s->dBodies;
@@ -537,6 +537,7 @@ int allocate(vfd_sim* s) {
         d.X = X[1 - k]; d.V = V[1 - k]; d.DV = DV[1 - k]; d.DK = DK[1 - k]; d.PID = PID[1 - k];
         s->dev[k] = d;
     }
+    for (int k = 0; k < 2; k++) s->dev[k].haloOn = wide_form(s);
     // static uploads: tables, scene ids, bodies
     std::vector<float> wm(kTableRes), gm(kTableRes);
     for (uint32_t i = 0; i + 1 < kTableRes; i++) {
@@ -703,44 +704,47 @@ int upload(vfd_sim* s) {
     TRY(reset_buckets(s, d));
     CK(cudaDeviceSynchronize());
     s->uploaded = true;
-    s->tilesNarrow = true;
-    s->stepsSince = 0;
     s->generation++;
     if (s->fp64Mode) TRY(fp64_upload(s));
     return VFD_OK;
 }
 
 // ---------------------------------------------------------------- step recording
-int build_graph(vfd_sim* s, int parity, const void* rec, cudaGraph_t* gOut, cudaGraphExec_t* execOut, bool narrow) {
-    cudaGraph_t g;
-    CK(cudaGraphCreate(&g, 0));
+uint32_t wide_form(const vfd_sim* s) {
+    const bool can = s->dev[0].haloTiles && (s->forms >> kHaloWide & 1u) && s->n >= kHaloWideMinParticles;
+    return can ? kHaloWide : 0u;
+}
+bool chooses_form(const vfd_sim* s) { return s->dev[0].haloTiles && (s->forms >> kHaloNarrow & 1u); }
+
+// The step's launches from its search on (from the search's rows on when its cells are done),
+// appended to g behind `leaves`: segments, and a while node per solver loop.
+static cudaError_t add_step(vfd_sim* s, Dev d, const void* rec, bool cellsDone, cudaGraph_t g,
+                            std::vector<cudaGraphNode_t>& leaves) {
     // One conditional handle per while node the graph has (divergence, CG, pressure): a
     // handle that no node uses makes cudaGraphInstantiate fail with "invalid argument".
-    Dev d = s->dev[parity];
-    if (narrow) d.haloOn = kHaloNarrow;
     const bool used[3] = {s->anyDiv, s->anyVisc, true};
     cudaGraphConditionalHandle h[3] = {};
+    cudaError_t e = cudaSuccess;
     for (int k = 0; k < 3; k++) {
         d.condHandle[k] = 0ull;
-        if (!used[k]) continue;
-        cudaError_t e = cudaGraphConditionalHandleCreate(&h[k], g, 0, 0);
-        if (e != cudaSuccess) {
-            cudaGraphDestroy(g);
-            return fail(VFD_E_CUDA, "cudaGraphConditionalHandleCreate: %s", cudaGetErrorString(e));
-        }
+        if (!used[k] || e != cudaSuccess) continue;
+        e = cudaGraphConditionalHandleCreate(&h[k], g, 0, 0);
         d.condHandle[k] = (unsigned long long)h[k];
     }
     cudaStream_t cap = s->stream;
-    std::vector<cudaGraphNode_t> leaves;
     const uint32_t passes = s->maxStPasses;
     const bool anyDiv = s->anyDiv, anyVisc = s->anyVisc, anyST = s->anyST;
     // with a recorder, tape_point() adds the adjoint's tape writes between the stages
     auto T = [&](int point, cudaStream_t st) {
         if (rec) tape_point(d, rec, point, st);
     };
-    cudaError_t e = add_segment(cap, g, leaves, [&](cudaStream_t st) {
-        T(kTapeBegin, st);
-        launch_search(d, st);
+    if (e == cudaSuccess) e = add_segment(cap, g, leaves, [&](cudaStream_t st) {
+        if (cellsDone) {
+            launch_search_rows(d, st);
+        } else {
+            T(kTapeBegin, st);
+            launch_search(d, st);
+        }
         T(kTapeSearch, st);
         launch_boundary(d, st);
         T(kTapeBoundary, st);
@@ -778,6 +782,48 @@ int build_graph(vfd_sim* s, int parity, const void* rec, cudaGraph_t* gOut, cuda
         launch_pres_finish(d, st);
         T(kTapeEnd, st);
     });
+    return e;
+}
+
+// The step of a layout with staged tiles: the search's cells and tile lists, the choice of the
+// form that fits them, and an if / else node with the rest of the step in either form. So each
+// step runs on the form that its own state needs, whatever set that state (a start, a restore,
+// a run of queued steps).
+static cudaError_t add_step_by_form(vfd_sim* s, Dev d, const void* rec, cudaGraph_t g) {
+    cudaGraphConditionalHandle h;
+    cudaError_t e = cudaGraphConditionalHandleCreate(&h, g, 0, 0);
+    if (e != cudaSuccess) return e;
+    const uint32_t other = d.haloOn;
+    std::vector<cudaGraphNode_t> leaves;
+    e = add_segment(s->stream, g, leaves, [&](cudaStream_t st) {
+        Dev c = d;
+        c.haloOn = kHaloNarrow;
+        c.formHandle = (unsigned long long)h;
+        if (rec) tape_point(d, rec, kTapeBegin, st);
+        launch_search_cells(c, st);
+        launch_tile_form(c, other, st);
+    });
+    if (e != cudaSuccess) return e;
+    cudaGraphNodeParams np = {cudaGraphNodeTypeConditional};
+    np.conditional.handle = h;
+    np.conditional.type = cudaGraphCondTypeIf;
+    np.conditional.size = 2;
+    cudaGraphNode_t node;
+    e = cudaGraphAddNode(&node, g, leaves.data(), nullptr, leaves.size(), &np);
+    for (int k = 0; k < 2 && e == cudaSuccess; k++) {
+        std::vector<cudaGraphNode_t> none;
+        d.haloOn = k == 0 ? kHaloNarrow : other;
+        e = add_step(s, d, rec, true, np.conditional.phGraph_out[k], none);
+    }
+    return e;
+}
+
+int build_graph(vfd_sim* s, int parity, const void* rec, cudaGraph_t* gOut, cudaGraphExec_t* execOut) {
+    cudaGraph_t g;
+    CK(cudaGraphCreate(&g, 0));
+    std::vector<cudaGraphNode_t> leaves;
+    cudaError_t e = chooses_form(s) ? add_step_by_form(s, s->dev[parity], rec, g)
+                                    : add_step(s, s->dev[parity], rec, false, g, leaves);
     cudaGraphExec_t exec = nullptr;
     if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, g, 0);
     if (e != cudaSuccess) {
@@ -788,18 +834,6 @@ int build_graph(vfd_sim* s, int parity, const void* rec, cudaGraph_t* gOut, cuda
     *gOut = g;
     *execOut = exec;
     return VFD_OK;
-}
-
-// The narrow tile form serves where the last step that was waited for, at most kNarrowSteps
-// launches ago, found few tiles beyond it (or the run starts): its state is near enough. Else the
-// wide form or, in smaller scenes, the row kernels run (Dev::haloOn). The same bits by all.
-constexpr uint32_t kNarrowSteps = 8u;
-int step_graph(vfd_sim* s, int* slot) {
-    const bool narrow = s->halo != 0 && s->dev[s->cs].haloTiles && s->tilesNarrow && s->stepsSince < kNarrowSteps;
-    s->stepsSince++;
-    *slot = s->cs + (narrow ? 2 : 0);
-    if (s->exec[*slot]) return VFD_OK;
-    return build_graph(s, s->cs, nullptr, &s->graph[*slot], &s->exec[*slot], narrow);
 }
 
 int read_flag(vfd_sim* s, int idx, uint32_t& v) {
@@ -820,7 +854,7 @@ struct PhaseRange {
 
 // The reference's host-driven control flow: one flag read per solver iteration.
 int launch_eager(vfd_sim* s, const void* rec) {
-    const Dev& d = s->dev[s->cs];
+    Dev d = s->dev[s->cs];
     cudaStream_t st = s->stream;
     auto T = [&](int point) {
         if (rec) tape_point(d, rec, point, st);
@@ -830,7 +864,16 @@ int launch_eager(vfd_sim* s, const void* rec) {
     T(kTapeBegin);
     {
         PhaseRange r("neighbour search");
-        launch_search(d, st);
+        if (chooses_form(s)) {  // as in the step's graph
+            Dev c = d;
+            c.haloOn = kHaloNarrow;
+            launch_search_cells(c, st);
+            launch_tile_form(c, d.haloOn, st);
+            TRY(read_flag(s, 14, d.haloOn));
+            launch_search_rows(d, st);
+        } else {
+            launch_search(d, st);
+        }
     }
     T(kTapeSearch);
     {
@@ -903,15 +946,14 @@ int ensure_ready(vfd_sim* s) {
 
 int launch_one(vfd_sim* s) {
     if (s->graphMode && !s->graphFailed) {
-        int slot = 0;
-        if (step_graph(s, &slot) != VFD_OK) {
+        if (!s->exec[s->cs] && build_graph(s, s->cs, nullptr, &s->graph[s->cs], &s->exec[s->cs]) != VFD_OK) {
             // keep the kernels, drop the graph: eager launches of the same kernels
             s->graphFailed = true;
             s->releaseGraphs();
         }
         if (!s->graphFailed) {
             PhaseRange r("vfd_step (graph)");
-            CK(cudaGraphLaunch(s->exec[slot], s->stream));
+            CK(cudaGraphLaunch(s->exec[s->cs], s->stream));
             s->cs = 1 - s->cs;
             return VFD_OK;
         }
@@ -932,8 +974,6 @@ int finish_steps(vfd_sim* s, vfd_step_stats* stats, uint32_t& flags) {
     CK(cudaStreamSynchronize(s->stream));
     CK(cudaGetLastError());
     flags = s->hStatus[0];
-    s->tilesNarrow = s->hStatus[12] * 4u <= s->hStatus[13];
-    s->stepsSince = 0;
     if (stats) std::memcpy(s->hScenes.data(), s->hStage, bytes);
     return VFD_OK;
 }
@@ -2171,10 +2211,10 @@ int vfd_profile_kernels(vfd_sim* s, uint32_t steps, vfd_kernel_time* out, uint32
     return VFD_OK;
 }
 
-// Whether the layout's steps run on staged tiles (where it has the buffers for them).
-static void set_halo(vfd_sim* s, int8_t on) {
-    s->halo = on;
-    for (int k = 0; k < 2; k++) s->dev[k].haloOn = on && s->dev[k].haloTiles && s->n >= kHaloWideMinParticles ? kHaloWide : 0u;
+// The forms of the staged tiles that steps may run on from here (where the layout has buffers for them).
+static void set_forms(vfd_sim* s, uint8_t forms) {
+    s->forms = forms;
+    for (int k = 0; k < 2; k++) s->dev[k].haloOn = wide_form(s);
 }
 
 int vfd_set_lanes(vfd_sim* s, const uint8_t* lanes, uint32_t count) {
@@ -2184,7 +2224,7 @@ int vfd_set_lanes(vfd_sim* s, const uint8_t* lanes, uint32_t count) {
         if (lanes[k] != 4 && lanes[k] != 8 && lanes[k] != 16) return fail(VFD_E_ARG, "lanes must be 4, 8 or 16");
     std::memcpy(s->lanes, lanes, count);
     s->lanesChosen = true;
-    set_halo(s, 0);
+    set_forms(s, 0);
     for (int k = 0; k < 2; k++) std::memcpy(s->dev[k].lanes, s->lanes, sizeof(s->lanes));
     s->releaseGraphs();
     return VFD_OK;
@@ -2205,7 +2245,7 @@ int vfd_set_tiles(vfd_sim* s, const uint8_t* tiles, uint32_t count) {
             return fail(VFD_E_ARG, "pass form must be 0 (neighbour rows), 1 (rows, gradW recomputed), 3 (2x2x2 tiles) "
                                    "or 4 (4x2x2 tiles)");
     std::memcpy(s->tiles, tiles, count);
-    set_halo(s, 0);
+    set_forms(s, 0);
     for (int k = 0; k < 2; k++) {
         std::memcpy(s->dev[k].tiles, s->tiles, sizeof(s->tiles));
         s->dev[k].compactRows = uses_tiles(s->tiles) ? 1u : 0u;
@@ -2221,7 +2261,7 @@ int vfd_set_blocks(vfd_sim* s, const uint16_t* blocks, uint32_t count) {
         if (blocks[k] != 64 && blocks[k] != 128 && blocks[k] != 256)
             return fail(VFD_E_ARG, "threads per block must be 64, 128 or 256");
     std::memcpy(s->blocks, blocks, count * sizeof(uint16_t));
-    set_halo(s, 0);
+    set_forms(s, 0);
     for (int k = 0; k < 2; k++) std::memcpy(s->dev[k].blocks, s->blocks, sizeof(s->blocks));
     s->releaseGraphs();
     return VFD_OK;
@@ -2238,6 +2278,13 @@ int vfd_get_tiles(const vfd_sim* s, uint8_t* tiles, uint32_t count) {
     TRY(check_sim(s));
     if (!tiles) return fail(VFD_E_ARG, "null output");
     std::memcpy(tiles, s->tiles, std::min<uint32_t>(count, 16));
+    return VFD_OK;
+}
+
+int vfd_get_tile_form(const vfd_sim* s, uint32_t* form) {
+    TRY(check_sim(s));
+    if (!form) return fail(VFD_E_ARG, "null output");
+    *form = !s->uploaded || s->fp64Mode ? 0u : chooses_form(s) ? s->hStatus[14] : s->dev[0].haloOn;
     return VFD_OK;
 }
 
@@ -2302,6 +2349,8 @@ int vfd_autotune(vfd_sim* s, uint32_t steps, uint8_t* lanes_out, uint32_t count)
     double haloTime = 0.0;  // the same kernels on staged tiles, with the pass that lists them
     int rc = VFD_OK;
     const bool canHalo = s->dev[0].haloTiles != nullptr && s->n >= kHaloWideMinParticles;
+    const uint8_t forms0 = s->forms, allForms = 1u << kHaloNarrow | 1u << kHaloWide;
+    s->forms = 0;  // each run on what it times
     for (int ct = 0; ct < 3 * kForms * 3 + (canHalo ? 1 : 0) && rc == VFD_OK; ct++) {
         const bool halo = ct == 3 * kForms * 3;
         const int c = ct % 3, tl = (ct / 3) % kForms, bs = ct / (3 * kForms) % 3;
@@ -2348,7 +2397,7 @@ int vfd_autotune(vfd_sim* s, uint32_t steps, uint8_t* lanes_out, uint32_t count)
             std::memcpy(s->dev[k].blocks, s->blocks, sizeof(s->blocks));
             s->dev[k].compactRows = uses_tiles(s->tiles) ? 1u : 0u;
         }
-        set_halo(s, s->halo);
+        set_forms(s, forms0);
         return rc;
     }
     double rowTime = 0.0;
@@ -2388,7 +2437,7 @@ int vfd_autotune(vfd_sim* s, uint32_t steps, uint8_t* lanes_out, uint32_t count)
         s->dev[k].compactRows = uses_tiles(s->tiles) ? 1u : 0u;
     }
     s->lanesChosen = true;
-    set_halo(s, canHalo && haloTime < rowTime ? 1 : 0);
+    set_forms(s, canHalo && haloTime < rowTime ? allForms : 0);
     s->releaseGraphs();
     if (lanes_out) std::memcpy(lanes_out, s->lanes, std::min<uint32_t>(count, 16));
     return VFD_OK;

@@ -168,6 +168,7 @@ struct Dev {
     uint32_t* MAXB;            // [scene][2][kBuckets] x32: max |v + a dt|^2 bits, max neighbours
     int32_t* MMB;              // [scene][6][kBuckets] x32: min cell xyz, max cell xyz
     unsigned long long condHandle[3];  // while-node handles (div, cg, pres); 0 = eager
+    unsigned long long formHandle;     // handle of the choice of the tile form (k_tile_form); 0 = eager
     uint8_t lanes[16];                 // lanes per particle of each TunedKernel
     uint16_t blocks[16];               // threads per block of each TunedKernel's row kernels (0 = kBlock)
     // Batches: per solver loop (div, cg, pres) the controllers list the scenes still
@@ -185,7 +186,8 @@ struct Dev {
     // 1: the passes walk the neighbour rows instead of cell tiles (the adjoint's passes run
     // on recorded rows of a past step, whose cell tables are no longer current)
     uint32_t rowLoops;
-    // Staged-tile passes (dfsph_halo.cu); haloOn: the step's neighbour loops run on them.
+    // Staged-tile passes (dfsph_halo.cu); haloOn: the form of them that the step's neighbour
+    // loops run on, 0 the row kernels.
     // The rows and gradient factors take the place of NG, whose bytes they share.
     uint32_t haloOn;
     HaloTile* haloTiles;

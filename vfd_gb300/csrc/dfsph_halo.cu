@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(256) k_halo_build(Dev d) {
             d.haloBase[(size_t)(T.cell0 / kHaloTileCells) * kHaloCells + threadIdx.x] = (uint16_t)(pre + x - cc);
         }
         if (threadIdx.x == 0) {
-            const bool fits = total <= halo_cap(d);
+            const bool fits = total <= kHaloWideCap;
             const uint32_t at = fits ? atomicAdd(d.haloInfo + 1, total) : 0u;
             offset = fits ? at : 0xFFFFFFFFu;
             T.list = at;
@@ -99,6 +99,15 @@ __global__ void __launch_bounds__(256) k_halo_build(Dev d) {
             }
         __syncthreads();
     }
+}
+
+// The form of this step's tiles, from its own lists: narrow where at most a quarter of the tiles
+// outgrow it, else `otherwise` (wide tiles, or rows in smaller scenes).
+__global__ void k_tile_form(Dev d, uint32_t otherwise) {
+    VFD_COUNT_LAUNCH(d);
+    const bool narrow = !is_aborted(d) && d.status[12] * 4u <= d.status[13];
+    d.status[14] = narrow ? kHaloNarrow : otherwise;
+    if (d.formHandle) cudaGraphSetConditional((cudaGraphConditionalHandle)d.formHandle, narrow ? 1u : 0u);
 }
 
 // ---------------------------------------------------------------- the tile loop
@@ -624,6 +633,9 @@ void launch_halo_pass(const Dev& d, HaloPass pass, cudaStream_t s) {
 
 void launch_halo_build(const Dev& d, cudaStream_t s) {
     VFD_LAUNCH("k_halo_build", s, k_halo_build<<<d.batchBlocks / 2u, 256, 0, s>>>(d));
+}
+void launch_tile_form(const Dev& d, uint32_t otherwise, cudaStream_t s) {
+    VFD_LAUNCH("k_tile_form", s, k_tile_form<<<1, 1, 0, s>>>(d, otherwise));
 }
 
 }  // namespace vfd

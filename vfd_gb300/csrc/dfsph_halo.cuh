@@ -19,7 +19,6 @@ constexpr uint32_t kHaloX = (1u << ((kHaloLog2 + 2u) / 3u)) + 2u, kHaloY = (1u <
 constexpr uint32_t kHaloNarrow = 1u, kHaloWide = 2u;
 constexpr uint32_t kHaloThreads = 256u, kHaloWideThreads = 384u;
 constexpr uint32_t kHaloCap = 1408u, kHaloWideCap = 1760u;
-__host__ __device__ inline uint32_t halo_cap(const Dev& d) { return d.haloOn == kHaloWide ? kHaloWideCap : kHaloCap; }
 constexpr uint32_t kHaloRow = 96u;                        // row length: kMaxNeighbors rounded up to 32
 
 // Layouts that run on staged tiles. Against the row kernels with four lanes a particle, a step
@@ -71,6 +70,7 @@ enum HaloPass {
 };
 void launch_halo_pass(const Dev& d, HaloPass pass, cudaStream_t s);
 void launch_halo_build(const Dev& d, cudaStream_t s);
+void launch_tile_form(const Dev& d, uint32_t otherwise, cudaStream_t s);
 cudaError_t prepare_halo_kernels();
 
 }  // namespace vfd

@@ -711,13 +711,9 @@ void launch_neighbors(const Dev& d, cudaStream_t s, bool profiled) {
     if (d.cellRel) SEARCH_LAUNCH("k_neighbors", k_neighbors<true><<<nbrBlocks, kBlock, 0, s>>>(d));
     else SEARCH_LAUNCH("k_neighbors", k_neighbors<false><<<nbrBlocks, kBlock, 0, s>>>(d));
 }
-void launch_search(const Dev& d, cudaStream_t s, bool profiled) {
+// Cells and (with staged tiles) tiles of the current positions; then the order and the rows.
+void launch_search_cells(const Dev& d, cudaStream_t s, bool profiled) {
     const uint32_t nb = blocks_for(d.n);
-    if (search_small(d)) {
-        SEARCH_LAUNCH("k_search_small", k_search_small<<<kSmallBlocks, kSmallThreads, 0, s>>>(d));
-        launch_neighbors(d, s, profiled);
-        return;
-    }
     SEARCH_LAUNCH("k_minmax", k_minmax<<<nb, kBlock, 0, s>>>(d));
     SEARCH_LAUNCH("k_grid", k_grid<<<1, 256, 0, s>>>(d));
     SEARCH_LAUNCH("k_clear_cells", k_clear_cells<<<1216, 256, 0, s>>>(d));
@@ -726,9 +722,21 @@ void launch_search(const Dev& d, cudaStream_t s, bool profiled) {
     SEARCH_LAUNCH("k_scan_top", k_scan_top<<<1, 1024, 0, s>>>(d));
     SEARCH_LAUNCH("k_scan_down", k_scan_down<<<d.scanBlocks, 256, 0, s>>>(d));
     if (halo_on(d)) launch_halo_build(d, s);
+}
+void launch_search_rows(const Dev& d, cudaStream_t s, bool profiled) {
+    const uint32_t nb = blocks_for(d.n);
     SEARCH_LAUNCH("k_slots", k_slots<<<nb, kBlock, 0, s>>>(d));
     SEARCH_LAUNCH("k_rank_gather", k_rank_gather<<<nb, kBlock, 0, s>>>(d));
     launch_neighbors(d, s, profiled);
+}
+void launch_search(const Dev& d, cudaStream_t s, bool profiled) {
+    if (search_small(d)) {
+        SEARCH_LAUNCH("k_search_small", k_search_small<<<kSmallBlocks, kSmallThreads, 0, s>>>(d));
+        launch_neighbors(d, s, profiled);
+        return;
+    }
+    launch_search_cells(d, s, profiled);
+    launch_search_rows(d, s, profiled);
 }
 #undef SEARCH_LAUNCH
 

@@ -13,9 +13,12 @@
 
 #include "../../include/vfd_dfsph.h"
 #include "dfsph_common.cuh"
+#include "dfsph_halo.cuh"
 
 namespace vfd {
 void launch_search(const Dev& d, cudaStream_t s, bool profiled = true);
+void launch_search_cells(const Dev& d, cudaStream_t s, bool profiled = true);
+void launch_search_rows(const Dev& d, cudaStream_t s, bool profiled = true);
 uint32_t scan_block_count(uint32_t cellCap);
 void launch_boundary(const Dev& d, cudaStream_t s);
 void launch_density(const Dev& d, cudaStream_t s);
@@ -196,9 +199,10 @@ struct vfd_sim {
     uint8_t tiles[16] = {};
     // threads per block of each TunedKernel's neighbour-row kernels (vfd_autotune; 0 = 128)
     uint16_t blocks[16] = {};
-    // staged-tile passes (dfsph_halo.cu): -1 = by the number of particles, 0 = not (the caller
-    // chose lanes, tiles or blocks of the row kernels), 1 = the autotuner measured them faster
-    int8_t halo = -1;
+    // forms of the staged tiles (dfsph_halo.cu) that steps may run on, 1 << form: none where the
+    // caller chose lanes, tiles or blocks of the row kernels, else all but those that the
+    // autotuner found slower
+    uint8_t forms = 1u << vfd::kHaloNarrow | 1u << vfd::kHaloWide;
 
     // layout
     bool allocated = false, uploaded = false;
@@ -224,11 +228,8 @@ struct vfd_sim {
     bool anyDiv = false, anyVisc = false, anyST = false;
 
     // graphs (one per parity)
-    // step graphs per parity of the state sets, then those with the narrow tile form
-    cudaGraphExec_t exec[4] = {nullptr, nullptr, nullptr, nullptr};
-    cudaGraph_t graph[4] = {nullptr, nullptr, nullptr, nullptr};
-    bool tilesNarrow = true;    // what the last look at the tiles says (a fresh start is a lattice)
-    uint32_t stepsSince = 0;    // steps launched since
+    cudaGraphExec_t exec[2] = {nullptr, nullptr};
+    cudaGraph_t graph[2] = {nullptr, nullptr};
     bool searchOnlyPending = false;
 
     // adjoint: checkpoints and tapes of the last vfd_adjoint_forward; `generation`
@@ -248,13 +249,11 @@ struct vfd_sim {
     ~vfd_sim() { release(); }
 
     void releaseGraphs() {
-        for (int k = 0; k < 4; k++) {
+        for (int k = 0; k < 2; k++) {
             if (exec[k]) cudaGraphExecDestroy(exec[k]);
             if (graph[k]) cudaGraphDestroy(graph[k]);
             exec[k] = nullptr;
             graph[k] = nullptr;
-        }
-        for (int k = 0; k < 2; k++) {
             if (adjRecExec[k]) cudaGraphExecDestroy(adjRecExec[k]);
             if (adjRecGraph[k]) cudaGraphDestroy(adjRecGraph[k]);
             adjRecExec[k] = nullptr;
@@ -355,9 +354,12 @@ enum TapePoint {
 };
 void tape_point(const Dev& d, const void* rec, int point, cudaStream_t st);
 
+// The form of the staged tiles for fluid denser than the narrow one holds (0: rows), and whether
+// each step chooses between that and the narrow form from its own search (k_tile_form).
+uint32_t wide_form(const vfd_sim* s);
+bool chooses_form(const vfd_sim* s);
 // One step as a graph (rec: the adjoint's device tape set, or null) into *gOut / *execOut.
-int build_graph(vfd_sim* s, int parity, const void* rec, cudaGraph_t* gOut, cudaGraphExec_t* execOut,
-                bool narrow = false);
+int build_graph(vfd_sim* s, int parity, const void* rec, cudaGraph_t* gOut, cudaGraphExec_t* execOut);
 // One eagerly launched step (one flag read per solver iteration), optionally recording.
 int launch_eager(vfd_sim* s, const void* rec);
 

@@ -464,8 +464,9 @@ int vfd_get_blocks(const vfd_sim* sim, uint16_t* blocks, uint32_t count);
  * Autotuner: runs `steps` steps from a snapshot of the current state once per
  * lane count, tile size and block size, times every neighbour-loop kernel with CUDA events,
  * keeps the fastest lane count (and tile size, vfd_set_tiles, and block size,
- * vfd_set_blocks) per kernel, or the staged tiles where they are faster, and restores the state exactly (positions,
- * velocities, accelerations and all carried solver state; the simulation does not
+ * vfd_set_blocks) per kernel and the forms of the staged tiles (vfd_get_tile_form) that are
+ * faster or that no step here asked for, and restores the state exactly (positions, velocities,
+ * accelerations and all carried solver state; the simulation does not
  * advance). Per-step diagnostics (vfd_get_field, vfd_get_neighbors) reflect the
  * last tuning step until the next step. lanes_out (may be NULL) receives the choice.
  */

@@ -62,3 +62,26 @@ def test_launched_by_the_host(squeeze, form):
     assert graph.GetGraphMode() == (True, True)
     for a, b in zip(graph.GetState(), host.GetState()):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("counts,other", [((64, 64, 64), ROWS), (LARGE, WIDE)])
+@pytest.mark.parametrize("tuned_on_lattice", [True, False])
+def test_tuning_keeps_the_forms_it_does_not_find_slower(counts, other, tuned_on_lattice):
+    # the narrow form takes 2,705 us a step of 260,000 particles on a lattice, rows 3,027; at
+    # 729,000 the lines lie further apart
+    s, dense = scene(counts), scene(counts, 0.88)
+    sim = V.scene_simulation(s if tuned_on_lattice else dense)
+    before = sim.GetState()
+    sim.Autotune(2)
+    for a, b in zip(before, sim.GetState()):
+        np.testing.assert_array_equal(a, b)
+    sim.SetState(s["x"], s["v"])
+    sim.Steps(1)
+    assert sim.TileForm() == NARROW
+    sim.SetState(dense["x"], dense["v"])
+    sim.Steps(1)
+    assert sim.TileForm() in (other, ROWS)  # wide tiles against tuned rows on dense fluid: either
+    sim.SetLanes([8] * len(V.TUNED_KERNELS))
+    sim.SetState(s["x"], s["v"])
+    sim.Steps(1)
+    assert sim.TileForm() == ROWS

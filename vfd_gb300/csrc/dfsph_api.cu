@@ -2346,16 +2346,25 @@ int vfd_autotune(vfd_sim* s, uint32_t steps, uint8_t* lanes_out, uint32_t count)
                                                                 // stream, 2x2x2 and 4x2x2 tiles
     const uint16_t blockCand[3] = {128, 64, 256};  // threads per block of the row kernels
     double times[kTunedCount][3][kForms][3] = {};  // [kernel][lanes][form][block]
-    double haloTime = 0.0;  // the same kernels on staged tiles, with the pass that lists them
+    // the same kernels on each form of the staged tiles, with the pass that lists them: the wide one
+    // from its line up, the narrow one in the steps whose state asks for it
+    struct {
+        double ms = 0.0;
+        uint32_t steps = 0;
+        double step() const { return ms / steps; }
+    } tileTime[kHaloWide + 1u];
     int rc = VFD_OK;
-    const bool canHalo = s->dev[0].haloTiles != nullptr && s->n >= kHaloWideMinParticles;
-    const uint8_t forms0 = s->forms, allForms = 1u << kHaloNarrow | 1u << kHaloWide;
-    s->forms = 0;  // each run on what it times
-    for (int ct = 0; ct < 3 * kForms * 3 + (canHalo ? 1 : 0) && rc == VFD_OK; ct++) {
-        const bool halo = ct == 3 * kForms * 3;
+    const bool canWide = s->dev[0].haloTiles && s->n >= kHaloWideMinParticles;
+    std::vector<uint32_t> runs(3 * kForms * 3, 0u);  // the form each run times (0: the rows' configurations)
+    if (canWide) runs.push_back(kHaloWide);
+    if (s->dev[0].haloTiles) runs.push_back(kHaloNarrow);
+    const uint8_t forms0 = s->forms;
+    for (int ct = 0; ct < (int)runs.size() && rc == VFD_OK; ct++) {
+        const uint32_t form = runs[ct];
         const int c = ct % 3, tl = (ct / 3) % kForms, bs = ct / (3 * kForms) % 3;
+        s->forms = form == kHaloNarrow ? 1u << kHaloNarrow : 0u;
         for (int k = 0; k < 2; k++) {
-            s->dev[k].haloOn = halo ? kHaloWide : 0u;
+            s->dev[k].haloOn = form == kHaloWide ? kHaloWide : 0u;
             for (int t = 0; t < kTunedCount; t++) {
                 s->dev[k].lanes[t] = cand[c];
                 s->dev[k].tiles[t] = tileCand[tl];
@@ -2363,24 +2372,24 @@ int vfd_autotune(vfd_sim* s, uint32_t steps, uint8_t* lanes_out, uint32_t count)
             }
             s->dev[k].compactRows = tileCand[tl] >= kTileMinLog2 ? 1u : 0u;
         }
-        EventProfiler prof;
-        g_profiler = &prof;
         for (uint32_t k = 0; k < steps && rc == VFD_OK; k++) {
+            EventProfiler prof;
+            g_profiler = &prof;
             rc = launch_eager(s);
-            if (rc == VFD_OK) s->cs = 1 - s->cs;
-        }
-        g_profiler = nullptr;
-        if (rc == VFD_OK) {
+            g_profiler = nullptr;
+            if (rc != VFD_OK) break;
+            s->cs = 1 - s->cs;
             cudaError_t r = cudaStreamSynchronize(s->stream);
             if (r != cudaSuccess) rc = fail(VFD_E_CUDA, "autotune: %s", cudaGetErrorString(r));
-        }
-        for (const auto& rec : prof.recs) {
-            float ms = 0.0f;
-            if (rc == VFD_OK && cudaEventElapsedTime(&ms, rec.a, rec.b) == cudaSuccess) {
-                if (halo && rec.name == "k_halo_build") haloTime += ms;
+            if (form == kHaloNarrow && s->hStatus[14] != kHaloNarrow) continue;
+            if (form) tileTime[form].steps++;
+            for (const auto& rec : prof.recs) {
+                float ms = 0.0f;
+                if (rc != VFD_OK || cudaEventElapsedTime(&ms, rec.a, rec.b) != cudaSuccess) continue;
+                if (form && rec.name == "k_halo_build") tileTime[form].ms += ms;
                 for (int t = 0; t < kTunedCount; t++) {
                     if (rec.name != names[t]) continue;
-                    if (halo) haloTime += ms;
+                    if (form) tileTime[form].ms += ms;
                     else times[t][c][tl][bs] += ms;
                 }
             }
@@ -2437,7 +2446,15 @@ int vfd_autotune(vfd_sim* s, uint32_t steps, uint8_t* lanes_out, uint32_t count)
         s->dev[k].compactRows = uses_tiles(s->tiles) ? 1u : 0u;
     }
     s->lanesChosen = true;
-    set_forms(s, canHalo && haloTime < rowTime ? allForms : 0);
+    // a form that lost goes; one that was not timed (no step here asks for it) stays to be chosen
+    uint8_t forms = 1u << kHaloNarrow | 1u << kHaloWide;
+    double other = rowTime / steps;
+    if (canWide) {
+        if (tileTime[kHaloWide].step() < other) other = tileTime[kHaloWide].step();
+        else forms &= ~(1u << kHaloWide);
+    }
+    if (tileTime[kHaloNarrow].steps && !(tileTime[kHaloNarrow].step() < other)) forms &= ~(1u << kHaloNarrow);
+    set_forms(s, forms);
     s->releaseGraphs();
     if (lanes_out) std::memcpy(lanes_out, s->lanes, std::min<uint32_t>(count, 16));
     return VFD_OK;

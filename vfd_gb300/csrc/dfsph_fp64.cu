@@ -35,7 +35,8 @@ namespace f64 {
 // takes 64 cycles, a division or square root 650), and with few particles the chain of a
 // thread. So the density pass keeps each pair's gradient factor and the preconditioner each
 // pair's viscosity coefficient (16 bytes a pair together), and a pair of the loops costs 9 to 14
-// FP64 operations instead of ~40 to 70. Two steps of a viscous drop, before (a thread a particle
+// FP64 operations instead of ~40 to 70; where there is no room for them the loops form both
+// again (KEPT false). Two steps of a viscous drop, before (a thread a particle
 // that formed them again, 256 threads a block, a wait of the host per reduction) and now: 7.3 and
 // 2.1 ms at 8,000 particles, 8.1 and 4.0 at 33,000, 35 and 16 at 300,000, 187 and 79 at 1M.
 constexpr uint32_t kB = 256u;         // threads per block, at most
@@ -131,7 +132,7 @@ struct A {
     uint32_t *NCNT, *NBR, *KEY, *CNT, *START, *FILL, *TMP, *ORDER, *BSUM;
     int* MM;  // min cell xyz, max cell xyz
     double *PART, *PART2;
-    double *GS, *VS;      // [particle][kCap]: gradW / r, and the viscosity's coefficient of (v . r) r
+    double *GS, *VS;      // [particle][kCap]: gradW / r, and the viscosity's coefficient of (v . r) r; null: no room
     struct Loop* loop;
     const double *W, *G;  // midpoint tables
     const float* halton;
@@ -167,7 +168,11 @@ __device__ __forceinline__ double kw(const P& p, const A& a, D3 r) {  // GetW
     const double rl = sqrt(r2);
     return p.analytic ? spline_w(p, rl) : a.W[tpos(p, rl)];
 }
-__device__ __forceinline__ D3 kgrad(const P& p, const A& a, D3 r) {  // GetGradientW
+__device__ __forceinline__ double kgs(const P& p, const A& a, D3 r) {  // GetGradientW = kgs r
+    const double rl = sqrt(dot(r, r));
+    return !(rl <= p.h) ? 0.0 : p.analytic ? spline_gs(p, rl) : a.G[tpos(p, rl)];
+}
+__device__ __forceinline__ D3 kgrad(const P& p, const A& a, D3 r) {
     const double rl = sqrt(dot(r, r));
     if (!(rl <= p.h)) return d3(0, 0, 0);
     return (p.analytic ? spline_gs(p, rl) : a.G[tpos(p, rl)]) * r;
@@ -437,6 +442,16 @@ __device__ __forceinline__ void pairs(const P& p, const A& a, uint32_t i, uint32
     }
 }
 
+// A pair's gradient factor, and its coefficient 10 mu (m / rho) gs / (r^2 + 0.01 h^2) in the viscosity
+// product: as the density and the preconditioner pass left them, or formed again.
+template <bool KEPT>
+__device__ __forceinline__ double pair_gs(const P& p, const A& a, size_t at, D3 r) {
+    return KEPT ? a.GS[at] : kgs(p, a, r);
+}
+__device__ __forceinline__ double visc_coefficient(const P& p, const A& a, uint32_t k, D3 r, double gs) {
+    return 10.0 * p.dynVisc * (p.mass / a.RHO[k]) / (dot(r, r) + 0.01 * p.h2) * gs;
+}
+
 // K1 ComputeVolumeAndBoundaryKernel (DFSPHKernels.cu:69-150)
 __global__ void k_boundary(P p, A a) {
     F64_THREAD
@@ -472,6 +487,7 @@ __global__ void k_boundary(P p, A a) {
 
 // K2 ComputeDensityKernel (:152-187) + K3 ComputeDFSPHFactorKernel (:189-231)
 // (and each pair's gradient factor)
+template <bool KEPT>
 __global__ void __launch_bounds__(kLB) k_density_factor(P p, A a) {
     F64_LANES
     const D3 xi = a.X[i];
@@ -482,7 +498,7 @@ __global__ void __launch_bounds__(kLB) k_density_factor(P p, A a) {
         const uint32_t q = tpos(p, rl);
         if (r2 <= p.h2) w += p.analytic ? spline_w(p, rl) : a.W[q];
         const double gs = !(rl <= p.h) ? 0.0 : p.analytic ? spline_gs(p, rl) : a.G[q];
-        a.GS[at] = gs;
+        if (KEPT) a.GS[at] = gs;
         const D3 gj = (-p.volume * gs) * r;
         sum += dot(gj, gj);
         gi -= gj;
@@ -507,10 +523,11 @@ __global__ void __launch_bounds__(kLB) k_density_factor(P p, A a) {
 
 // The passes' sums over a particle, complete in every lane but for the bodies' share, which the
 // writing lane adds.
+template <bool KEPT>
 __device__ double velocity_divergence(const P& p, const A& a, uint32_t i, uint32_t l, bool first) {  // K4 :498-522, K17 :253-271
     const D3 xi = a.X[i], vi = a.V[i];
     double d = 0.0;
-    pairs(p, a, i, l, xi, [&](uint32_t k, size_t at, D3 r) { d += a.GS[at] * dot(vi - a.V[k], r); });
+    pairs(p, a, i, l, xi, [&](uint32_t k, size_t at, D3 r) { d += pair_gs<KEPT>(p, a, at, r) * dot(vi - a.V[k], r); });
     d = lanes(p.lanes, d) * p.volume;
     if (first)
         for (uint32_t b = 0; b < p.bodies; b++) {
@@ -519,13 +536,14 @@ __device__ double velocity_divergence(const P& p, const A& a, uint32_t i, uint32
         }
     return d;
 }
+template <bool KEPT>
 __device__ D3 pressure_accel(const P& p, const A& a, uint32_t i, uint32_t l, bool first, const double* kap) {  // K5/K7/K18/K20
     const D3 xi = a.X[i];
     const double ki = kap[i];
     D3 acc = d3(0, 0, 0);
     pairs(p, a, i, l, xi, [&](uint32_t k, size_t at, D3 r) {
         const double s = ki + kap[k];
-        if (fabs(s) > (double)kEps) acc += (s * (-p.volume * a.GS[at])) * r;
+        if (fabs(s) > (double)kEps) acc += (s * (-p.volume * pair_gs<KEPT>(p, a, at, r))) * r;
     });
     acc = lanes(p.lanes, acc);
     if (first && fabs(ki) > (double)kEps)
@@ -535,10 +553,11 @@ __device__ D3 pressure_accel(const P& p, const A& a, uint32_t i, uint32_t l, boo
         }
     return acc;
 }
+template <bool KEPT>
 __device__ double pressure_force(const P& p, const A& a, uint32_t i, uint32_t l, bool first) {  // :280-315
     const D3 xi = a.X[i], ai = a.AP[i];
     double f = 0.0;
-    pairs(p, a, i, l, xi, [&](uint32_t k, size_t at, D3 r) { f += a.GS[at] * dot(ai - a.AP[k], r); });
+    pairs(p, a, i, l, xi, [&](uint32_t k, size_t at, D3 r) { f += pair_gs<KEPT>(p, a, at, r) * dot(ai - a.AP[k], r); });
     f = lanes(p.lanes, f) * p.volume;
     if (first)
         for (uint32_t b = 0; b < p.bodies; b++) {
@@ -567,26 +586,29 @@ __global__ void __launch_bounds__(256) k_jacobi_decide(P p, A a, LoopBounds b, u
 }
 
 // K4 ComputeDensityChangeKernel (:483-529)
+template <bool KEPT>
 __global__ void __launch_bounds__(kLB) k_div_init(P p, A a) {
     F64_LANES
-    double d = velocity_divergence(p, a, i, l, first);
+    double d = velocity_divergence<KEPT>(p, a, i, l, first);
     if (!first) return;
     d = a.NCNT[i] < 20u ? 0.0 : fmax(d, 0.0);
     a.RHOADV[i] = d;
     a.ALPHA[i] *= p.dtInv;
     a.KAPPAV[i] = d * a.ALPHA[i];
 }
+template <bool KEPT>
 __global__ void __launch_bounds__(kLB) k_paccel(P p, A a, int div) {  // K5 / K18
     if (a.loop->done) return;
     F64_LANES
-    const D3 ap = pressure_accel(p, a, i, l, first, div ? a.KAPPAV : a.KAPPA);
+    const D3 ap = pressure_accel<KEPT>(p, a, i, l, first, div ? a.KAPPAV : a.KAPPA);
     if (first) a.AP[i] = ap;
 }
 // K6 DivergenceSolveIterationKernel (:531-553) / K19 PressureSolveIterationKernel (:317-340)
+template <bool KEPT>
 __global__ void __launch_bounds__(kLB) k_jacobi(P p, A a, int div) {
     if (a.loop->done) return;
     F64_LANES
-    double s = pressure_force(p, a, i, l, first), res = 0.0;
+    double s = pressure_force<KEPT>(p, a, i, l, first), res = 0.0;
     if (first) {
         if (div) {
             s *= p.dt;
@@ -602,10 +624,11 @@ __global__ void __launch_bounds__(kLB) k_jacobi(P p, A a, int div) {
     block_partial(a.PART, res, false);
 }
 // K7 ComputePressureAccelerationAndFactorKernel (:555-602) + K8 ClearAccelerationKernel (:24-37)
+template <bool KEPT>
 __global__ void __launch_bounds__(kLB) k_div_finish(P p, A a, int div) {
     F64_LANES
     if (div) {
-        const D3 ap = pressure_accel(p, a, i, l, first, a.KAPPAV);
+        const D3 ap = pressure_accel<KEPT>(p, a, i, l, first, a.KAPPAV);
         if (first) {
             a.AP[i] = ap;
             a.V[i] += p.dt * ap;
@@ -719,13 +742,14 @@ __device__ bool visc_samples(const P& p, const A& a, uint32_t i, uint32_t b, D3 
     return true;
 }
 // K12 ComputeViscosityPreconditionerKernel (:604-684) + K13's b = v and the warm start g
-// (and each pair's coefficient 10 mu (m / rho) gs / (r^2 + 0.01 h^2) of the product)
+// (and each pair's coefficient of the product)
+template <bool KEPT>
 __global__ void __launch_bounds__(kLB) k_visc_precond(P p, A a) {
     F64_LANES
     M3 res = {};
     pairs(p, a, i, l, a.X[i], [&](uint32_t k, size_t at, D3 r) {
-        const double c = 10.0 * p.dynVisc * (p.mass / a.RHO[k]) / (dot(r, r) + 0.01 * p.h2) * a.GS[at];
-        a.VS[at] = c;
+        const double c = visc_coefficient(p, a, k, r, pair_gs<KEPT>(p, a, at, r));
+        if (KEPT) a.VS[at] = c;
         add_outer(res, c, r, r);
     });
     for (int r = 0; r < 3; r++)
@@ -749,12 +773,16 @@ __global__ void __launch_bounds__(kLB) k_visc_precond(P p, A a) {
 }
 // ComputeMatrixVecProdFunctionKernel (:758-842): out = A vec; sum of vec . out per block
 // (in the loop; of the first guess: out = b - A vec, sum of its square and of b's)
+template <bool KEPT>
 __global__ void __launch_bounds__(kLB) k_matvec(P p, A a, const D3* vec, D3* out, int loop) {
     if (loop && a.loop->done) return;
     F64_LANES
     const D3 xi = a.X[i], vi = vec[i];
     D3 acc = d3(0, 0, 0);
-    pairs(p, a, i, l, xi, [&](uint32_t k, size_t at, D3 r) { acc += (a.VS[at] * dot(vi - vec[k], r)) * r; });
+    pairs(p, a, i, l, xi, [&](uint32_t k, size_t at, D3 r) {
+        const double c = KEPT ? a.VS[at] : visc_coefficient(p, a, k, r, kgs(p, a, r));
+        acc += (c * dot(vi - vec[k], r)) * r;
+    });
     acc = lanes(p.lanes, acc);
     double t = 0.0, t2 = 0.0;
     if (first) {
@@ -876,9 +904,10 @@ __global__ void k_velocity(P p, A a) {  // K16 ComputeVelocityKernel (:39-52)
     F64_THREAD
     a.V[i] += p.dt * a.Acc[i];
 }
+template <bool KEPT>
 __global__ void __launch_bounds__(kLB) k_pres_init(P p, A a) {  // K17 ComputeDensityAdvectionKernel (:233-278)
     F64_LANES
-    const double d = velocity_divergence(p, a, i, l, first);
+    const double d = velocity_divergence<KEPT>(p, a, i, l, first);
     if (!first) return;
     const double rhoAdv = a.RHO[i] / p.rho0 + p.dt * d;
     a.RHOADV[i] = rhoAdv;
@@ -886,9 +915,10 @@ __global__ void __launch_bounds__(kLB) k_pres_init(P p, A a) {  // K17 ComputeDe
     a.KAPPA[i] = -fmin(1.0 - rhoAdv, 0.0) * a.ALPHA[i];
 }
 // K20 ComputePressureAccelerationAndVelocityKernel (:434-481); K21 positions after all
+template <bool KEPT>
 __global__ void __launch_bounds__(kLB) k_pres_finish(P p, A a) {
     F64_LANES
-    const D3 ap = pressure_accel(p, a, i, l, first, a.KAPPA);
+    const D3 ap = pressure_accel<KEPT>(p, a, i, l, first, a.KAPPA);
     if (!first) return;
     a.AP[i] = ap;
     a.V[i] += p.dt * ap;
@@ -926,6 +956,22 @@ struct Fp64State {
         for (void* q : allocs) cudaFree(q);
         for (void* q : cellAllocs) cudaFree(q);
         cudaFreeHost(hLoop);
+        drop_pairs();
+    }
+    // The pairs' factors, two thirds of the state: kept where there is room (1M particles 79 ms a
+    // pair of steps with them, see the top of the file).
+    void keep_pairs() {
+        const size_t bytes = std::max<size_t>(1, n) * kCap * sizeof(double);
+        if (a.GS || (cudaMalloc(&a.GS, bytes) == cudaSuccess && cudaMalloc(&a.VS, bytes) == cudaSuccess)) return;
+        drop_pairs();
+    }
+    bool drop_pairs() {
+        const bool had = a.GS != nullptr;
+        cudaFree(a.GS);
+        cudaFree(a.VS);
+        a.GS = a.VS = nullptr;
+        cudaGetLastError();
+        return had;
     }
 };
 
@@ -1006,7 +1052,6 @@ int fp64_upload(vfd_sim* s) {
     TRY(falloc(f, &a.TMP, n)); TRY(falloc(f, &a.ORDER, n)); TRY(falloc(f, &a.MM, 6));
     const size_t parts = std::max((n + 63u) / 64u, (uint32_t)(((uint64_t)n * kL + kLB - 1u) / kLB)) + 1u;
     TRY(falloc(f, &a.PART, parts)); TRY(falloc(f, &a.PART2, parts)); TRY(falloc(f, &a.loop, 1));
-    TRY(falloc(f, &a.GS, (size_t)n * kCap)); TRY(falloc(f, &a.VS, (size_t)n * kCap));
     FCK(cudaMallocHost(&f->hLoop, sizeof(f64::Loop)));
     }
     // SPH tables in double (PrecomputedDFSPHCubicKernel::SetRadius, Kernel/DFSPHKernels.h:13-41)
@@ -1055,6 +1100,7 @@ int fp64_upload(vfd_sim* s) {
     f->bodies = nb;
     f->radius = r;
     }
+    f->keep_pairs();
     p.wZero = calcW(0.0);
     a.halton = s->dHalton;
     a.bodyTab = s->dBodies;
@@ -1105,6 +1151,9 @@ int fp64_upload(vfd_sim* s) {
     return VFD_OK;
 }
 
+// The form of a kernel that reads the pairs' factors or forms them again.
+#define F64_KEPT(K) (a.GS ? f64::K<true> : f64::K<false>)
+
 // One OnUpdate step (DFSPHImplementation.cu:63-170) in FP64.
 int fp64_step(vfd_sim* s, vfd_step_stats* out) {
     Fp64State* f = s->fp64;
@@ -1143,10 +1192,13 @@ int fp64_step(vfd_sim* s, vfd_step_stats* out) {
             q = nullptr;
         }
         const size_t cap = (size_t)a.cells + a.cells / 4u;
-        FCK(cudaMalloc(&f->cellAllocs[0], cap * sizeof(uint32_t)));
-        FCK(cudaMalloc(&f->cellAllocs[1], cap * sizeof(uint32_t)));
-        FCK(cudaMalloc(&f->cellAllocs[2], cap * sizeof(uint32_t)));
-        FCK(cudaMalloc(&f->cellAllocs[3], (cap / 1024u + 2u) * sizeof(uint32_t)));
+        const size_t bytes[4] = {cap * sizeof(uint32_t), cap * sizeof(uint32_t), cap * sizeof(uint32_t),
+                                 (cap / 1024u + 2u) * sizeof(uint32_t)};
+        for (int k = 0; k < 4; k++) {
+            cudaError_t e = cudaMalloc(&f->cellAllocs[k], bytes[k]);
+            if (e != cudaSuccess && f->drop_pairs()) e = cudaMalloc(&f->cellAllocs[k], bytes[k]);  // the cells come first
+            FCK(e);
+        }
         f->cellCap = (uint32_t)cap;
     }
     a.CNT = (uint32_t*)f->cellAllocs[0];
@@ -1165,19 +1217,19 @@ int fp64_step(vfd_sim* s, vfd_step_stats* out) {
     FCK(cudaGetLastError());
     // ---- boundary, density, factor
     f64::k_boundary<<<g, tb, 0, st>>>(p, a);
-    f64::k_density_factor<<<gl, kLB, 0, st>>>(p, a);
+    F64_KEPT(k_density_factor)<<<gl, kLB, 0, st>>>(p, a);
     // ---- divergence solve (ComputeDivergence, :506-575)
     const bool div = d.EnableDivergenceSolverError != 0;
     uint32_t itD = 0;
     double errD = 0.0;
     if (div) {
-        f64::k_div_init<<<gl, kLB, 0, st>>>(p, a);
+        F64_KEPT(k_div_init)<<<gl, kLB, 0, st>>>(p, a);
         const double eta = p.dtInv * (double)d.MaxDivergenceSolverError * 0.0001 * p.rho0;
         const LoopBounds lb{eta, d.MinDivergenceSolverIterations, d.MaxDivergenceSolverIterations};
         f64::k_loop_start<<<1, 1, 0, st>>>(a, lb);
         TRY(run_loop(f, st, 2u, [&]() {
-            f64::k_paccel<<<gl, kLB, 0, st>>>(p, a, 1);
-            f64::k_jacobi<<<gl, kLB, 0, st>>>(p, a, 1);
+            F64_KEPT(k_paccel)<<<gl, kLB, 0, st>>>(p, a, 1);
+            F64_KEPT(k_jacobi)<<<gl, kLB, 0, st>>>(p, a, 1);
             f64::k_jacobi_decide<<<1, 256, 0, st>>>(p, a, lb, gl);
         }));
         itD = f->hLoop->it;
@@ -1185,7 +1237,7 @@ int fp64_step(vfd_sim* s, vfd_step_stats* out) {
         if (itD >= d.MaxDivergenceSolverIterations && d.MaxDivergenceSolverIterations > 0 && errD > eta)
             S.Flags |= VFD_FLAG_DIVERGENCE_CAP;
     }
-    f64::k_div_finish<<<gl, kLB, 0, st>>>(p, a, div ? 1 : 0);
+    F64_KEPT(k_div_finish)<<<gl, kLB, 0, st>>>(p, a, div ? 1 : 0);
     // ---- surface tension (:810-839)
     const uint32_t samplesUsed = p.stSamples;
     if (d.EnableSurfaceTensionSolver) {
@@ -1197,14 +1249,14 @@ int fp64_step(vfd_sim* s, vfd_step_stats* out) {
     uint32_t itV = 0;
     double errV = 0.0;
     if (d.EnableViscositySolver) {
-        f64::k_visc_precond<<<gl, kLB, 0, st>>>(p, a);
+        F64_KEPT(k_visc_precond)<<<gl, kLB, 0, st>>>(p, a);
         const LoopBounds lb{(double)d.MaxViscositySolverError, d.MinViscositySolverIterations, d.MaxViscositySolverIterations};
-        f64::k_matvec<<<gl, kLB, 0, st>>>(p, a, a.CG, a.CR, 0);
+        F64_KEPT(k_matvec)<<<gl, kLB, 0, st>>>(p, a, a.CG, a.CR, 0);
         f64::k_cg_start<<<1, 256, 0, st>>>(a, lb, gl);
         f64::k_precondition<<<g, tb, 0, st>>>(p, a);
         f64::k_cg_first<<<1, 256, 0, st>>>(a, g);
         TRY(run_loop(f, st, 1u, [&]() {
-            f64::k_matvec<<<gl, kLB, 0, st>>>(p, a, a.CP, a.CT, 1);
+            F64_KEPT(k_matvec)<<<gl, kLB, 0, st>>>(p, a, a.CP, a.CT, 1);
             f64::k_cg_alpha<<<1, 256, 0, st>>>(a, gl);
             f64::k_cg_update<<<g, tb, 0, st>>>(p, a);
             f64::k_cg_decide<<<1, 256, 0, st>>>(a, lb, g);
@@ -1232,20 +1284,20 @@ int fp64_step(vfd_sim* s, vfd_step_stats* out) {
     f->frameTime += dt;
     f64::k_velocity<<<g, tb, 0, st>>>(p, a);
     // ---- pressure solve (ComputePressure, :443-504)
-    f64::k_pres_init<<<gl, kLB, 0, st>>>(p, a);
+    F64_KEPT(k_pres_init)<<<gl, kLB, 0, st>>>(p, a);
     const double eta = (double)d.MaxPressureSolverError * 0.0001 * p.rho0;
     const LoopBounds lp{eta, d.MinPressureSolverIterations, d.MaxPressureSolverIterations};
     f64::k_loop_start<<<1, 1, 0, st>>>(a, lp);
     TRY(run_loop(f, st, 2u, [&]() {
-        f64::k_paccel<<<gl, kLB, 0, st>>>(p, a, 0);
-        f64::k_jacobi<<<gl, kLB, 0, st>>>(p, a, 0);
+        F64_KEPT(k_paccel)<<<gl, kLB, 0, st>>>(p, a, 0);
+        F64_KEPT(k_jacobi)<<<gl, kLB, 0, st>>>(p, a, 0);
         f64::k_jacobi_decide<<<1, 256, 0, st>>>(p, a, lp, gl);
     }));
     const uint32_t itP = f->hLoop->it;
     const double errP = f->hLoop->err;
     if (itP >= d.MaxPressureSolverIterations && d.MaxPressureSolverIterations > 0 && errP > eta)
         S.Flags |= VFD_FLAG_PRESSURE_CAP;
-    f64::k_pres_finish<<<gl, kLB, 0, st>>>(p, a);
+    F64_KEPT(k_pres_finish)<<<gl, kLB, 0, st>>>(p, a);
     f64::k_position<<<g, tb, 0, st>>>(p, a);
     FCK(cudaGetLastError());
     FCK(cudaStreamSynchronize(st));

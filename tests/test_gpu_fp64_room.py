@@ -72,3 +72,24 @@ def test_without_room_for_the_pairs(analytic):
     sim.Steps(2)
     for a, b in zip(want, sim.GetStateF64()):
         np.testing.assert_array_equal(a, b)
+
+
+def test_a_refused_search_grid_leaves_no_cells_behind():
+    # two particles 900 cells apart on each axis: 730 million cells, 8.7 GB
+    s = scenes.small_dam_break(n_side=4, r=0.01)
+    far = dict(s, x=s["x"].copy())
+    far["x"][0] += np.float32(900 * 0.04)
+    sim = V.scene_simulation(dict(s, boxes=[]))
+    sim.SetPrecision(True)
+    sim.Steps(1)
+    want = sim.GetStateF64()
+    sim.SetFluidObjects(far["x"], s["v"])
+    sim.Reset()
+    with Filled(1024 * MB):
+        with pytest.raises(V.VFDError):
+            sim.Steps(1)
+    sim.SetFluidObjects(s["x"], s["v"])
+    sim.Reset()  # the same particle count: the FP64 state serves again, with cells of its own
+    sim.Steps(1)
+    for a, b in zip(want, sim.GetStateF64()):
+        np.testing.assert_array_equal(a, b)

@@ -1191,12 +1191,14 @@ int fp64_step(vfd_sim* s, vfd_step_stats* out) {
             cudaFree(q);
             q = nullptr;
         }
+        f->cellCap = 0;  // a state that outlives a refusal below has no cells
         const size_t cap = (size_t)a.cells + a.cells / 4u;
         const size_t bytes[4] = {cap * sizeof(uint32_t), cap * sizeof(uint32_t), cap * sizeof(uint32_t),
                                  (cap / 1024u + 2u) * sizeof(uint32_t)};
         for (int k = 0; k < 4; k++) {
             cudaError_t e = cudaMalloc(&f->cellAllocs[k], bytes[k]);
             if (e != cudaSuccess && f->drop_pairs()) e = cudaMalloc(&f->cellAllocs[k], bytes[k]);  // the cells come first
+            if (e != cudaSuccess) cudaGetLastError();
             FCK(e);
         }
         f->cellCap = (uint32_t)cap;

@@ -15,6 +15,7 @@
 #include "dfsph_common.cuh"
 #include "dfsph_map.cuh"
 #include "dfsph_sim.h"
+#include "mesh_edges.h"
 
 namespace vfd {
 
@@ -323,30 +324,7 @@ int prepare_mesh(const float* vtx, uint32_t nv, const uint32_t* tri, uint32_t nf
         for (int k = 0; k < 3; k++) vertN[tri[3 * f + k]] = add(vertN[tri[3 * f + k]], scale(alpha[k], n));
         faceN[f] = n;
     }
-    // opposite face of each half-edge (face f, edge k = (tri[k], tri[(k+1)%3])); -1 on a border
-    std::vector<int64_t> opp(3 * (size_t)nf, -1);
-    // The unpaired half-edges of each source vertex, in face order, as a list threaded through
-    // `next`: a vertex has about six (an ordered map over all of them took most of the set-up).
-    constexpr uint32_t kNone = 0xFFFFFFFFu;
-    std::vector<uint32_t> head(nv, kNone), tail(nv, kNone), next(3 * (size_t)nf, kNone);
-    for (uint32_t f = 0; f < nf; f++)
-        for (uint32_t k = 0; k < 3; k++) {
-            const uint32_t e = 3 * f + k, u = tri[e], v = tri[3 * f + (k + 1) % 3];
-            uint32_t before = kNone, o = head[v];  // the earliest unpaired (v, u)
-            while (o != kNone && tri[3 * (o / 3) + (o % 3 + 1) % 3] != u) {
-                before = o;
-                o = next[o];
-            }
-            if (o != kNone) {
-                opp[e] = o / 3;
-                opp[o] = f;
-                (before == kNone ? head[v] : next[before]) = next[o];
-                if (tail[v] == o) tail[v] = before;
-            } else {
-                (tail[u] == kNone ? head[u] : next[tail[u]]) = e;
-                tail[u] = e;
-            }
-        }
+    const std::vector<int64_t> opp = opposite_faces(tri, nv, nf);
     out.corners.resize(3 * (size_t)nf);
     out.normals.resize(7 * (size_t)nf);
     auto f4 = [](F3 a) { return make_float4(a.x, a.y, a.z, 0.0f); };

@@ -382,11 +382,53 @@ __device__ __forceinline__ bool jacobi_control(SceneDev& S, double sum) {
 
 // The loop controllers run as one block. With one scene its one warp folds the buckets
 // together (fold_acc_warp) and lane 0 takes the decisions. A batch gives each scene a warp to
-// fold its buckets as alone, then a thread for the decisions: bound by the latency of loads and
+// fold its buckets as alone, or, with more scenes than kWarpScenes, four lanes that add theirs as the
+// warp's tree does, then a thread for the decisions: bound by the latency of loads and
 // of dependent FP64 adds. For 48 scenes a launch takes 9.8 us, k_ctrl_cg_alpha 6.9 and k_ctrl_cg
-// 10.5; with a thread per scene to fold 32 buckets in a row they took 12.1, 8.1 and 15.7.
-constexpr uint32_t kCtrlThreads = 1024u;
+// 10.5; with a thread per scene to fold 32 buckets in a row they took 12.1, 8.1 and 15.7. A step of
+// 96 viscous scenes of 27 particles takes 620 us, of 4,096 11.2 ms; 734 and 14.2 with a warp for each.
+constexpr uint32_t kCtrlThreads = 1024u, kWarpScenes = 64u;
 inline uint32_t ctrl_threads(const Dev& d) { return std::min(kCtrlThreads, 32u * d.nscenes); }
+
+// put(s, sums) for the scenes s of [begin, end) with active(s), by one thread each: the sums of
+// their buckets in the accumulators `slot`, which are reset. All threads of a block of whole warps.
+template <int SLOTS, class ACTIVE, class PUT>
+__device__ __forceinline__ void fold_scenes(const Dev& d, uint32_t begin, uint32_t end, const int (&slot)[SLOTS],
+                                            ACTIVE active, PUT put) {
+    double sum[SLOTS];
+    if (d.nscenes <= kWarpScenes) {
+        for (uint32_t s = begin + (threadIdx.x >> 5); s < end; s += blockDim.x >> 5) {
+            if (!active(s)) continue;
+#pragma unroll
+            for (int i = 0; i < SLOTS; i++) sum[i] = fold_acc_warp(d, s, slot[i], threadIdx.x & 31u);
+            if ((threadIdx.x & 31u) == 0u) put(s, sum);
+        }
+        return;
+    }
+    constexpr uint32_t G = 4u, PER = kBuckets / G;  // lanes a scene, buckets a lane
+    const uint32_t lane = threadIdx.x % G;
+    for (uint32_t base = begin + threadIdx.x / 32u * PER; base < end; base += blockDim.x / G) {
+        const uint32_t s = base + (threadIdx.x & 31u) / G;
+        const bool on = s < end && active(s);
+#pragma unroll
+        for (int i = 0; i < SLOTS; i++) {
+            double v[PER];
+#pragma unroll
+            for (uint32_t k = 0; k < PER; k++) v[k] = on ? __ldcg(acc_bucket(d, s, slot[i], lane + k * G)) : 0.0;
+#pragma unroll
+            for (uint32_t k = 0; k < PER; k++)
+                if (on) *acc_bucket(d, s, slot[i], lane + k * G) = 0.0;
+#pragma unroll
+            for (uint32_t o = PER / 2u; o > 0u; o >>= 1)
+#pragma unroll
+                for (uint32_t k = 0; k < o; k++) v[k] += v[k + o];
+#pragma unroll
+            for (uint32_t o = G / 2u; o > 0u; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+            sum[i] = v[0];
+        }
+        if (on && lane == 0u) put(s, sum);
+    }
+}
 
 template <bool DIV>
 __global__ void __launch_bounds__(kCtrlThreads) k_ctrl_jacobi(Dev d) {
@@ -409,11 +451,7 @@ __global__ void __launch_bounds__(kCtrlThreads) k_ctrl_jacobi(Dev d) {
     auto active = [&](uint32_t s) { return (DIV ? d.scenes[s].div.active : d.scenes[s].pres.active) != 0u; };
     for (uint32_t c = 0; c < d.nscenes; c += blockDim.x) {
         const uint32_t end = min(c + blockDim.x, d.nscenes);
-        for (uint32_t s = c + (threadIdx.x >> 5); s < end; s += blockDim.x >> 5) {
-            if (!active(s)) continue;
-            const double sum = fold_acc_warp(d, s, 0, threadIdx.x & 31u);
-            if ((threadIdx.x & 31u) == 0u) sums[s - c] = sum;
-        }
+        fold_scenes(d, c, end, {0}, active, [&](uint32_t s, const double* sum) { sums[s - c] = sum[0]; });
         __syncthreads();
         const uint32_t s = c + threadIdx.x;
         if (s < end && active(s) && jacobi_control<DIV>(d.scenes[s], sums[threadIdx.x])) atomicOr(&any, 1u);
@@ -741,12 +779,8 @@ __global__ void __launch_bounds__(kCtrlThreads) k_ctrl_cg_alpha(Dev d) {
         if (threadIdx.x == 0) S.cgAlpha = (float)(S.cgAbsNew / pap);
         return;
     }
-    for (uint32_t s = threadIdx.x >> 5; s < d.nscenes; s += blockDim.x >> 5) {
-        SceneDev& S = d.scenes[s];
-        if (!S.cgActive) continue;
-        const double pap = fold_acc_warp(d, s, 0, threadIdx.x & 31u);
-        if ((threadIdx.x & 31u) == 0u) S.cgAlpha = (float)(S.cgAbsNew / pap);
-    }
+    fold_scenes(d, 0u, d.nscenes, {0}, [&](uint32_t s) { return d.scenes[s].cgActive != 0u; },
+                [&](uint32_t s, const double* pap) { d.scenes[s].cgAlpha = (float)(d.scenes[s].cgAbsNew / pap[0]); });
 }
 
 // Loop body 2: g += alpha p, r -= alpha Ap, |r|^2, z = M^-1 r, r . z (:722-784).
@@ -859,11 +893,8 @@ __global__ void __launch_bounds__(kCtrlThreads) k_ctrl_cg(Dev d) {
     __shared__ double2 sums[kCtrlThreads];
     for (uint32_t c = 0; c < d.nscenes; c += blockDim.x) {
         const uint32_t end = min(c + blockDim.x, d.nscenes);
-        for (uint32_t s = c + (threadIdx.x >> 5); s < end; s += blockDim.x >> 5) {
-            if (!d.scenes[s].cgActive) continue;
-            const double rr = fold_acc_warp(d, s, 1, threadIdx.x & 31u), rz = fold_acc_warp(d, s, 2, threadIdx.x & 31u);
-            if ((threadIdx.x & 31u) == 0u) sums[s - c] = make_double2(rr, rz);
-        }
+        fold_scenes(d, c, end, {1, 2}, [&](uint32_t s) { return d.scenes[s].cgActive != 0u; },
+                    [&](uint32_t s, const double* sum) { sums[s - c] = make_double2(sum[0], sum[1]); });
         __syncthreads();
         const uint32_t s = c + threadIdx.x;
         if (s < end) {

@@ -421,7 +421,7 @@ int vfd_profile_kernels(vfd_sim* sim, uint32_t steps, vfd_kernel_time* out, uint
  * with 256 threads, one per particle). The neighbour search runs a warp per cell.
  * Untuned, 8 lanes run below 24,000 particles and 4 from there on, and from 100,000
  * on (700,000 for fluid denser than a lattice at the particles' diameter) the loops run on
- * cell tiles staged in shared memory, a thread per particle; setting
+ * cell tiles staged in shared memory, a thread per particle, where these are cheaper; setting
  * lanes, tiles or blocks selects the row (or cell-tile) kernels. 4 lanes, 8 lanes and
  * staged tiles give the same bits for each particle's sums; the sums over all particles are
  * grouped differently (a relative 1e-13, vfd_get_tile_form).
@@ -432,10 +432,16 @@ int vfd_get_lanes(const vfd_sim* sim, uint8_t* lanes, uint32_t count);
 /*
  * Form of the staged tiles that the last step that was waited for ran on: 0 = none (rows), 1 =
  * narrow (for a lattice at the particles' diameter), 2 = wide (for denser fluid). Each step
- * takes the form that the cells of its own state ask for, so the same state steps alike
- * whatever was run before it.
+ * takes the cheapest for the cells of its own state, so the same state steps alike
+ * whatever was run before it: rows where the tiles hold few particles or are few.
  */
 int vfd_get_tile_form(const vfd_sim* sim, uint32_t* form);
+/*
+ * Fixes the form for the steps to come, for measurements (-1, the default: each step
+ * chooses). Layouts below 100,000 particles run rows whatever is fixed. Undone by setting
+ * lanes, tiles or blocks and by vfd_autotune.
+ */
+int vfd_set_tile_form(vfd_sim* sim, int32_t form);
 
 /*
  * Form of the solver-loop kernels (pressure acceleration, Jacobi update, CG

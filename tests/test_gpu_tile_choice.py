@@ -1,6 +1,8 @@
-"""Each step takes the form of the staged tiles that its own state asks for: narrow on a lattice,
-rows (below 700,000 particles) or wide tiles on denser fluid, however the state came about (set,
-restored, queued, launched by the host) and whatever ran before it."""
+"""Each step takes the form of the staged tiles that is cheapest for its own state, however the state
+came about (set, restored, queued, launched by the host) and whatever ran before it: narrow tiles on a
+lattice, rows on sparse fluid and where halos outgrow the shared memory, wide tiles on denser fluid from
+700,000 particles on. The states here lie well inside the range of each form (by the steps that the
+rule is fitted to, its choice is 10 % faster than the next, or 3 % where the note says so)."""
 import numpy as np
 import pytest
 
@@ -9,21 +11,24 @@ import vfd_gb300 as V
 
 pytestmark = pytest.mark.gpu
 
-SMALL, LARGE = (47, 48, 49), (89, 90, 91)
+SMALL, LARGE = (69, 69, 69), (89, 90, 91)  # 328,509 and 728,910 particles
 ROWS, NARROW, WIDE = 0, 1, 2
 
 
-def scene(counts, squeeze=1.0):
-    # squeezed to 0.88 of the spacing, a cell holds 11.7 particles: tiles of 376, beyond the narrow form
+def scene(counts, squeeze=1.0, keep=1.0):
+    """A lattice at rest; squeezed to 0.95 of the spacing its tiles outgrow the narrow form, at 0.88 the wide one."""
     s = block_scene(counts, 0.05)
-    return dict(s, x=s["x"] * np.float32(squeeze), v=0 * s["v"],
+    x = s["x"] * np.float32(squeeze)
+    if keep < 1:
+        x = x[np.random.default_rng(2).random(len(x)) < keep]
+    return dict(s, x=x, v=0 * x,
                 desc=dict(s["desc"], MaxPressureSolverIterations=3, MaxDivergenceSolverIterations=3,
                           MaxViscositySolverIterations=3))
 
 
 @pytest.mark.parametrize("counts,other", [(SMALL, ROWS), (LARGE, WIDE)])
 def test_set_states(counts, other):
-    s, dense = scene(counts), scene(counts, 0.88)
+    s, dense = scene(counts), scene(counts, 0.95)
     sim = V.scene_simulation(s)
     for state, form in ((s, NARROW), (dense, other), (dense, other), (s, NARROW)):
         sim.SetState(state["x"], state["v"])
@@ -64,12 +69,29 @@ def test_launched_by_the_host(squeeze, form):
         np.testing.assert_array_equal(a, b)
 
 
-@pytest.mark.parametrize("counts,other", [((64, 64, 64), ROWS), (LARGE, WIDE)])
+@pytest.mark.parametrize("counts,squeeze,keep", [
+    ((47, 48, 49), 1.0, 1.0),   # 110,544 particles: few more tiles than blocks run at once
+    (LARGE, 1.0, 0.3),          # 70 particles a tile
+    (LARGE, 0.88, 1.0)])        # halos beyond the shared memory of either form
+def test_states_that_rows_suit(counts, squeeze, keep):
+    sim = V.scene_simulation(scene(counts, squeeze, keep))
+    sim.Steps(1)
+    assert sim.TileForm() == ROWS
+
+
+def test_batch_of_small_scenes():
+    s = block_scene((8, 8, 8), 0.0)  # 200 scenes of 512 particles: 64 a tile
+    sim = V.DFSPHSimulation(scenes=[V._abi.make_desc(**s["desc"])] * 200)
+    for k in range(200):
+        sim.SetFluidObjects(s["x"], 0 * s["v"], scene=k)
+    sim.Steps(1)
+    assert sim.TileForm() == ROWS
+
+
+@pytest.mark.parametrize("counts,other", [(SMALL, ROWS), (LARGE, WIDE)])
 @pytest.mark.parametrize("tuned_on_lattice", [True, False])
 def test_tuning_keeps_the_forms_it_does_not_find_slower(counts, other, tuned_on_lattice):
-    # the narrow form takes 2,705 us a step of 260,000 particles on a lattice, rows 3,027; at
-    # 729,000 the lines lie further apart
-    s, dense = scene(counts), scene(counts, 0.88)
+    s, dense = scene(counts), scene(counts, 0.95)
     sim = V.scene_simulation(s if tuned_on_lattice else dense)
     before = sim.GetState()
     sim.Autotune(2)
@@ -80,8 +102,15 @@ def test_tuning_keeps_the_forms_it_does_not_find_slower(counts, other, tuned_on_
     assert sim.TileForm() == NARROW
     sim.SetState(dense["x"], dense["v"])
     sim.Steps(1)
-    assert sim.TileForm() in (other, ROWS)  # wide tiles against tuned rows on dense fluid: either
+    assert sim.TileForm() in (other, ROWS)  # (wide tiles against tuned rows: either)
     sim.SetLanes([8] * len(V.TUNED_KERNELS))
     sim.SetState(s["x"], s["v"])
     sim.Steps(1)
     assert sim.TileForm() == ROWS
+    sim.SetTileForm(WIDE)
+    sim.Steps(1)
+    assert sim.TileForm() == WIDE
+    sim.SetTileForm()
+    sim.SetState(s["x"], s["v"])
+    sim.Steps(1)
+    assert sim.TileForm() == NARROW

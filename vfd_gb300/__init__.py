@@ -37,7 +37,7 @@ EXPORTS = [
     "vfd_set_position_mode", "vfd_build_mesh_map", "vfd_sample_mesh_volume", "vfd_set_kernel_mode",
     "vfd_emit", "vfd_get_graph_mode", "vfd_checkpoint_size", "vfd_checkpoint", "vfd_restore",
     "vfd_set_tiles", "vfd_get_tiles", "vfd_set_precision", "vfd_get_state_f64", "vfd_set_blocks", "vfd_get_blocks",
-    "vfd_get_tile_form",
+    "vfd_get_tile_form", "vfd_set_tile_form",
     "vfd_adjoint_set_warm_start", "vfd_adjoint_get_stats", "vfd_adjoint_set_tolerance",
     # include/vfd_sph.h: the legacy SPH pipeline (vfd_gb300.sph)
     "vfd_sph_create", "vfd_sph_destroy", "vfd_sph_on_update", "vfd_sph_steps", "vfd_sph_reset",
@@ -126,6 +126,7 @@ def lib() -> C.CDLL:
                 "vfd_set_blocks": [P, C.POINTER(C.c_uint16), C.c_uint32],
                 "vfd_get_blocks": [P, C.POINTER(C.c_uint16), C.c_uint32],
                 "vfd_get_tile_form": [P, C.POINTER(C.c_uint32)],
+                "vfd_set_tile_form": [P, C.c_int32],
                 "vfd_get_state_f64": [P, C.POINTER(C.c_double), C.POINTER(C.c_double)],
                 "vfd_get_tiles": [P, C.POINTER(C.c_uint8), C.c_uint32],
                 "vfd_autotune": [P, C.c_uint32, C.POINTER(C.c_uint8), C.c_uint32],
@@ -586,6 +587,10 @@ class DFSPHSimulation:
         form = C.c_uint32()
         _check(lib().vfd_get_tile_form(self._h, C.byref(form)), "vfd_get_tile_form")
         return form.value
+
+    def SetTileForm(self, form: int = -1):
+        """The form of all steps to come (0 rows, 1 narrow, 2 wide); -1: each step chooses."""
+        _check(lib().vfd_set_tile_form(self._h, form), "vfd_set_tile_form")
 
     def SetTiles(self, tiles):
         """Per solver-loop pass, in TUNED_KERNELS order: 0 = walk neighbour rows (gradW / r

@@ -1045,12 +1045,13 @@ struct ShadowKey {
     vfd_desc desc{};
     uint8_t lanes[16] = {}, tiles[16] = {};
     uint8_t forms = 0;
+    int8_t fixedForm = -1;
     uint16_t blocks[16] = {};
     uint32_t n = 0, graphs = 0, analytic = 0, cellCap = 0;
     bool operator==(const ShadowKey& o) const {
         return std::memcmp(&desc, &o.desc, sizeof(desc)) == 0 && std::memcmp(lanes, o.lanes, sizeof(lanes)) == 0 &&
                std::memcmp(tiles, o.tiles, sizeof(tiles)) == 0 && std::memcmp(blocks, o.blocks, sizeof(blocks)) == 0 &&
-               n == o.n && forms == o.forms && graphs == o.graphs && analytic == o.analytic && cellCap == o.cellCap;
+               n == o.n && forms == o.forms && fixedForm == o.fixedForm && graphs == o.graphs && analytic == o.analytic && cellCap == o.cellCap;
     }
 };
 
@@ -1246,6 +1247,7 @@ ShadowKey shadow_key(const vfd_sim* s) {
     std::memcpy(k.lanes, s->lanes, sizeof(k.lanes));
     std::memcpy(k.tiles, s->tiles, sizeof(k.tiles));
     k.forms = s->forms;
+    k.fixedForm = s->fixedForm;
     std::memcpy(k.blocks, s->blocks, sizeof(k.blocks));
     k.n = s->n;
     k.graphs = s->graphMode && !s->graphFailed ? 1u : 0u;
@@ -1289,9 +1291,10 @@ bool ensure_shadow(vfd_sim* s, AdjointState* A) {
     t->lanesChosen = true;
     std::memcpy(t->tiles, s->tiles, sizeof(t->tiles));
     t->forms = s->forms;
+    t->fixedForm = s->fixedForm;
     std::memcpy(t->blocks, s->blocks, sizeof(t->blocks));
-    if (ensure_ready(t) != VFD_OK || t->n != s->n || t->stride != s->stride || wide_form(t) != wide_form(s) ||
-        chooses_form(t) != chooses_form(s)) {
+    if (ensure_ready(t) != VFD_OK || t->n != s->n || t->stride != s->stride || tile_forms(t) != tile_forms(s) ||
+        t->dev[0].haloOn != s->dev[0].haloOn) {
         delete t;
         cudaGetLastError();
         return false;

@@ -394,7 +394,7 @@ int allocate_halo(vfd_sim* s, Dev& base) {
     const size_t st = s->stride, cellTiles = s->cellCap / kHaloTileCells + 1u, kept = s->allocs.size();
     const size_t tiles = std::min(st, cellTiles);
     int rc = dalloc(s, &base.haloTiles, tiles);
-    if (rc == VFD_OK) rc = dalloc(s, &base.haloInfo, 2);
+    if (rc == VFD_OK) rc = dalloc(s, &base.haloInfo, 2 + sizeof(HaloCounts) / sizeof(uint32_t));
     if (rc == VFD_OK) rc = dalloc(s, &base.haloScan, base.scanBlocks + 1);
     if (rc == VFD_OK) rc = dalloc(s, &base.haloScene, base.nscenes);
     if (rc == VFD_OK) rc = dalloc(s, &base.haloList, 8 * st);
@@ -537,7 +537,7 @@ int allocate(vfd_sim* s) {
         d.X = X[1 - k]; d.V = V[1 - k]; d.DV = DV[1 - k]; d.DK = DK[1 - k]; d.PID = PID[1 - k];
         s->dev[k] = d;
     }
-    for (int k = 0; k < 2; k++) s->dev[k].haloOn = wide_form(s);
+    fix_form(s, s->fixedForm);
     // static uploads: tables, scene ids, bodies
     std::vector<float> wm(kTableRes), gm(kTableRes);
     for (uint32_t i = 0; i + 1 < kTableRes; i++) {
@@ -710,11 +710,16 @@ int upload(vfd_sim* s) {
 }
 
 // ---------------------------------------------------------------- step recording
-uint32_t wide_form(const vfd_sim* s) {
-    const bool can = s->dev[0].haloTiles && (s->forms >> kHaloWide & 1u) && s->n >= kHaloWideMinParticles;
-    return can ? kHaloWide : 0u;
+uint32_t tile_forms(const vfd_sim* s) {
+    if (!s->dev[0].haloTiles || s->fixedForm >= 0) return 0u;
+    return s->forms & (s->n >= kHaloWideMinParticles ? ~0u : ~(1u << kHaloWide));
 }
-bool chooses_form(const vfd_sim* s) { return s->dev[0].haloTiles && (s->forms >> kHaloNarrow & 1u); }
+
+// Dev::haloOn outside of a choice: the form that the caller fixed.
+void fix_form(vfd_sim* s, int8_t form) {
+    s->fixedForm = form;
+    for (int k = 0; k < 2; k++) s->dev[k].haloOn = form > 0 && s->dev[k].haloTiles ? (uint32_t)form : 0u;
+}
 
 // The step's launches from its search on (from the search's rows on when its cells are done),
 // appended to g behind `leaves`: segments, and a while node per solver loop.
@@ -786,33 +791,37 @@ static cudaError_t add_step(vfd_sim* s, Dev d, const void* rec, bool cellsDone, 
 }
 
 // The step of a layout with staged tiles: the search's cells and tile lists, the choice of the
-// form that fits them, and an if / else node with the rest of the step in either form. So each
-// step runs on the form that its own state needs, whatever set that state (a start, a restore,
-// a run of queued steps).
+// form that fits them, and a switch node with the rest of the step on rows and in each form. So
+// each step runs on the form that its own state needs, whatever set that state (a start, a
+// restore, a run of queued steps).
 static cudaError_t add_step_by_form(vfd_sim* s, Dev d, const void* rec, cudaGraph_t g) {
     cudaGraphConditionalHandle h;
     cudaError_t e = cudaGraphConditionalHandleCreate(&h, g, 0, 0);
     if (e != cudaSuccess) return e;
-    const uint32_t other = d.haloOn;
+    const uint32_t forms = tile_forms(s);
+    std::vector<uint32_t> branch = {0u};
+    for (uint32_t f : {kHaloNarrow, kHaloWide})
+        if (forms >> f & 1u) branch.push_back(f);
     std::vector<cudaGraphNode_t> leaves;
     e = add_segment(s->stream, g, leaves, [&](cudaStream_t st) {
         Dev c = d;
         c.haloOn = kHaloNarrow;
+        c.formChoice = 1u;
         c.formHandle = (unsigned long long)h;
         if (rec) tape_point(d, rec, kTapeBegin, st);
         launch_search_cells(c, st);
-        launch_tile_form(c, other, st);
+        launch_tile_form(c, forms, st);
     });
     if (e != cudaSuccess) return e;
     cudaGraphNodeParams np = {cudaGraphNodeTypeConditional};
     np.conditional.handle = h;
-    np.conditional.type = cudaGraphCondTypeIf;
-    np.conditional.size = 2;
+    np.conditional.type = cudaGraphCondTypeSwitch;
+    np.conditional.size = (unsigned int)branch.size();
     cudaGraphNode_t node;
     e = cudaGraphAddNode(&node, g, leaves.data(), nullptr, leaves.size(), &np);
-    for (int k = 0; k < 2 && e == cudaSuccess; k++) {
+    for (size_t k = 0; k < branch.size() && e == cudaSuccess; k++) {
         std::vector<cudaGraphNode_t> none;
-        d.haloOn = k == 0 ? kHaloNarrow : other;
+        d.haloOn = branch[k];
         e = add_step(s, d, rec, true, np.conditional.phGraph_out[k], none);
     }
     return e;
@@ -822,7 +831,7 @@ int build_graph(vfd_sim* s, int parity, const void* rec, cudaGraph_t* gOut, cuda
     cudaGraph_t g;
     CK(cudaGraphCreate(&g, 0));
     std::vector<cudaGraphNode_t> leaves;
-    cudaError_t e = chooses_form(s) ? add_step_by_form(s, s->dev[parity], rec, g)
+    cudaError_t e = tile_forms(s) ? add_step_by_form(s, s->dev[parity], rec, g)
                                     : add_step(s, s->dev[parity], rec, false, g, leaves);
     cudaGraphExec_t exec = nullptr;
     if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, g, 0);
@@ -864,11 +873,12 @@ int launch_eager(vfd_sim* s, const void* rec) {
     T(kTapeBegin);
     {
         PhaseRange r("neighbour search");
-        if (chooses_form(s)) {  // as in the step's graph
+        if (tile_forms(s)) {  // as in the step's graph
             Dev c = d;
             c.haloOn = kHaloNarrow;
+            c.formChoice = 1u;
             launch_search_cells(c, st);
-            launch_tile_form(c, d.haloOn, st);
+            launch_tile_form(c, tile_forms(s), st);
             TRY(read_flag(s, 14, d.haloOn));
             launch_search_rows(d, st);
         } else {
@@ -2211,10 +2221,10 @@ int vfd_profile_kernels(vfd_sim* s, uint32_t steps, vfd_kernel_time* out, uint32
     return VFD_OK;
 }
 
-// The forms of the staged tiles that steps may run on from here (where the layout has buffers for them).
-static void set_forms(vfd_sim* s, uint8_t forms) {
-    s->forms = forms;
-    for (int k = 0; k < 2; k++) s->dev[k].haloOn = wide_form(s);
+// The row (or cell-tile) kernels, in the form that the caller sets.
+static void rows_only(vfd_sim* s) {
+    fix_form(s, -1);
+    s->forms = 0;
 }
 
 int vfd_set_lanes(vfd_sim* s, const uint8_t* lanes, uint32_t count) {
@@ -2224,7 +2234,7 @@ int vfd_set_lanes(vfd_sim* s, const uint8_t* lanes, uint32_t count) {
         if (lanes[k] != 4 && lanes[k] != 8 && lanes[k] != 16) return fail(VFD_E_ARG, "lanes must be 4, 8 or 16");
     std::memcpy(s->lanes, lanes, count);
     s->lanesChosen = true;
-    set_forms(s, 0);
+    rows_only(s);
     for (int k = 0; k < 2; k++) std::memcpy(s->dev[k].lanes, s->lanes, sizeof(s->lanes));
     s->releaseGraphs();
     return VFD_OK;
@@ -2245,7 +2255,7 @@ int vfd_set_tiles(vfd_sim* s, const uint8_t* tiles, uint32_t count) {
             return fail(VFD_E_ARG, "pass form must be 0 (neighbour rows), 1 (rows, gradW recomputed), 3 (2x2x2 tiles) "
                                    "or 4 (4x2x2 tiles)");
     std::memcpy(s->tiles, tiles, count);
-    set_forms(s, 0);
+    rows_only(s);
     for (int k = 0; k < 2; k++) {
         std::memcpy(s->dev[k].tiles, s->tiles, sizeof(s->tiles));
         s->dev[k].compactRows = uses_tiles(s->tiles) ? 1u : 0u;
@@ -2261,7 +2271,7 @@ int vfd_set_blocks(vfd_sim* s, const uint16_t* blocks, uint32_t count) {
         if (blocks[k] != 64 && blocks[k] != 128 && blocks[k] != 256)
             return fail(VFD_E_ARG, "threads per block must be 64, 128 or 256");
     std::memcpy(s->blocks, blocks, count * sizeof(uint16_t));
-    set_forms(s, 0);
+    rows_only(s);
     for (int k = 0; k < 2; k++) std::memcpy(s->dev[k].blocks, s->blocks, sizeof(s->blocks));
     s->releaseGraphs();
     return VFD_OK;
@@ -2284,7 +2294,17 @@ int vfd_get_tiles(const vfd_sim* s, uint8_t* tiles, uint32_t count) {
 int vfd_get_tile_form(const vfd_sim* s, uint32_t* form) {
     TRY(check_sim(s));
     if (!form) return fail(VFD_E_ARG, "null output");
-    *form = !s->uploaded || s->fp64Mode ? 0u : chooses_form(s) ? s->hStatus[14] : s->dev[0].haloOn;
+    *form = !s->uploaded || s->fp64Mode ? 0u : tile_forms(s) ? s->hStatus[14] : s->dev[0].haloOn;
+    return VFD_OK;
+}
+
+int vfd_set_tile_form(vfd_sim* s, int32_t form) {
+    TRY(check_sim(s));
+    if (form < -1 || form > (int32_t)kHaloWide)
+        return fail(VFD_E_ARG, "tile form must be -1 (chosen by each step), 0 (rows), 1 (narrow) or 2 (wide)");
+    fix_form(s, (int8_t)form);
+    s->forms = 1u << kHaloNarrow | 1u << kHaloWide;
+    s->releaseGraphs();
     return VFD_OK;
 }
 
@@ -2346,32 +2366,17 @@ int vfd_autotune(vfd_sim* s, uint32_t steps, uint8_t* lanes_out, uint32_t count)
                                                                 // stream, 2x2x2 and 4x2x2 tiles
     const uint16_t blockCand[3] = {128, 64, 256};  // threads per block of the row kernels
     double times[kTunedCount][3][kForms][3] = {};  // [kernel][lanes][form][block]
-    // the same kernels on each form of the staged tiles, with the pass that lists them: the wide one
-    // from its line up, the narrow one in the steps whose state asks for it
-    struct {
-        double ms = 0.0;
-        uint32_t steps = 0;
-        double step() const { return ms / steps; }
-    } tileTime[kHaloWide + 1u];
-    int rc = VFD_OK;
-    const bool canWide = s->dev[0].haloTiles && s->n >= kHaloWideMinParticles;
-    std::vector<uint32_t> runs(3 * kForms * 3, 0u);  // the form each run times (0: the rows' configurations)
-    if (canWide) runs.push_back(kHaloWide);
-    if (s->dev[0].haloTiles) runs.push_back(kHaloNarrow);
+    uint8_t lanes0[16], tiles0[16];
+    uint16_t blocks0[16];
+    std::memcpy(lanes0, s->lanes, sizeof(lanes0));
+    std::memcpy(tiles0, s->tiles, sizeof(tiles0));
+    std::memcpy(blocks0, s->blocks, sizeof(blocks0));
+    const bool chosen0 = s->lanesChosen;
     const uint8_t forms0 = s->forms;
-    for (int ct = 0; ct < (int)runs.size() && rc == VFD_OK; ct++) {
-        const uint32_t form = runs[ct];
-        const int c = ct % 3, tl = (ct / 3) % kForms, bs = ct / (3 * kForms) % 3;
-        s->forms = form == kHaloNarrow ? 1u << kHaloNarrow : 0u;
-        for (int k = 0; k < 2; k++) {
-            s->dev[k].haloOn = form == kHaloWide ? kHaloWide : 0u;
-            for (int t = 0; t < kTunedCount; t++) {
-                s->dev[k].lanes[t] = cand[c];
-                s->dev[k].tiles[t] = tileCand[tl];
-                s->dev[k].blocks[t] = blockCand[bs];
-            }
-            s->dev[k].compactRows = tileCand[tl] >= kTileMinLog2 ? 1u : 0u;
-        }
+    const int8_t fixed0 = s->fixedForm;
+    int rc = VFD_OK;
+    // `steps` steps from the snapshot: sink(kernel, ms) for each launch, `each` after each step
+    auto run = [&](auto sink, auto each) {
         for (uint32_t k = 0; k < steps && rc == VFD_OK; k++) {
             EventProfiler prof;
             g_profiler = &prof;
@@ -2381,32 +2386,52 @@ int vfd_autotune(vfd_sim* s, uint32_t steps, uint8_t* lanes_out, uint32_t count)
             s->cs = 1 - s->cs;
             cudaError_t r = cudaStreamSynchronize(s->stream);
             if (r != cudaSuccess) rc = fail(VFD_E_CUDA, "autotune: %s", cudaGetErrorString(r));
-            if (form == kHaloNarrow && s->hStatus[14] != kHaloNarrow) continue;
-            if (form) tileTime[form].steps++;
             for (const auto& rec : prof.recs) {
                 float ms = 0.0f;
-                if (rc != VFD_OK || cudaEventElapsedTime(&ms, rec.a, rec.b) != cudaSuccess) continue;
-                if (form && rec.name == "k_halo_build") tileTime[form].ms += ms;
-                for (int t = 0; t < kTunedCount; t++) {
-                    if (rec.name != names[t]) continue;
-                    if (form) tileTime[form].ms += ms;
-                    else times[t][c][tl][bs] += ms;
-                }
+                if (rc == VFD_OK && cudaEventElapsedTime(&ms, rec.a, rec.b) == cudaSuccess) sink(rec.name, (double)ms);
             }
+            each();
         }
         s->cs = cs0;
         e = copy_all(false);
         if (e != cudaSuccess && rc == VFD_OK) rc = fail(VFD_E_CUDA, "autotune restore: %s", cudaGetErrorString(e));
+    };
+    rows_only(s);
+    for (int ct = 0; ct < 3 * kForms * 3 && rc == VFD_OK; ct++) {
+        const int c = ct % 3, tl = (ct / 3) % kForms, bs = ct / (3 * kForms);
+        for (int k = 0; k < 2; k++) {
+            for (int t = 0; t < kTunedCount; t++) {
+                s->dev[k].lanes[t] = cand[c];
+                s->dev[k].tiles[t] = tileCand[tl];
+                s->dev[k].blocks[t] = blockCand[bs];
+            }
+            s->dev[k].compactRows = tileCand[tl] >= kTileMinLog2 ? 1u : 0u;
+        }
+        run([&](const std::string& name, double ms) {
+            for (int t = 0; t < kTunedCount; t++)
+                if (name == names[t]) times[t][c][tl][bs] += ms;
+        }, [] {});
     }
-    release();
-    if (rc != VFD_OK) {
+    auto settle = [&]() {  // the choice of lanes, tiles and blocks into the kernels' arguments
         for (int k = 0; k < 2; k++) {
             std::memcpy(s->dev[k].lanes, s->lanes, sizeof(s->lanes));
             std::memcpy(s->dev[k].tiles, s->tiles, sizeof(s->tiles));
             std::memcpy(s->dev[k].blocks, s->blocks, sizeof(s->blocks));
             s->dev[k].compactRows = uses_tiles(s->tiles) ? 1u : 0u;
         }
-        set_forms(s, forms0);
+    };
+    auto restore = [&]() {  // after a failure: what was set before the call
+        std::memcpy(s->lanes, lanes0, sizeof(lanes0));
+        std::memcpy(s->tiles, tiles0, sizeof(tiles0));
+        std::memcpy(s->blocks, blocks0, sizeof(blocks0));
+        s->lanesChosen = chosen0;
+        s->forms = forms0;
+        fix_form(s, fixed0);
+        settle();
+    };
+    if (rc != VFD_OK) {
+        release();
+        restore();
         return rc;
     }
     double rowTime = 0.0;
@@ -2439,22 +2464,34 @@ int vfd_autotune(vfd_sim* s, uint32_t steps, uint8_t* lanes_out, uint32_t count)
         s->tiles[t] = tileable ? tileCand[bestTile] : 0;
         s->blocks[t] = tileCand[bestTile] < kTileMinLog2 ? blockCand[bestBlock] : 0;
     }
-    for (int k = 0; k < 2; k++) {
-        std::memcpy(s->dev[k].lanes, s->lanes, sizeof(s->lanes));
-        std::memcpy(s->dev[k].tiles, s->tiles, sizeof(s->tiles));
-        std::memcpy(s->dev[k].blocks, s->blocks, sizeof(s->blocks));
-        s->dev[k].compactRows = uses_tiles(s->tiles) ? 1u : 0u;
-    }
+    settle();
     s->lanesChosen = true;
-    // a form that lost goes; one that was not timed (no step here asks for it) stays to be chosen
-    uint8_t forms = 1u << kHaloNarrow | 1u << kHaloWide;
-    double other = rowTime / steps;
-    if (canWide) {
-        if (tileTime[kHaloWide].step() < other) other = tileTime[kHaloWide].step();
-        else forms &= ~(1u << kHaloWide);
+    // The same kernels on the forms of the staged tiles that these steps choose, with the pass that
+    // lists the tiles: a form that is slower than the tuned rows goes, the others stay to be chosen.
+    s->forms = 1u << kHaloNarrow | 1u << kHaloWide;
+    for (bool again = tile_forms(s) != 0u; again && rc == VFD_OK;) {
+        double total[kHaloWide + 1u] = {}, part = 0.0;
+        uint32_t ran[kHaloWide + 1u] = {};
+        run([&](const std::string& name, double ms) {
+            if (name == "k_halo_build" || std::find(names, names + kTunedCount, name) != names + kTunedCount) part += ms;
+        }, [&] {
+            const uint32_t form = std::min(s->hStatus[14], kHaloWide);
+            total[form] += part;
+            ran[form]++;
+            part = 0.0;
+        });
+        again = false;
+        for (uint32_t f : {kHaloNarrow, kHaloWide})
+            if (rc == VFD_OK && ran[f] && total[f] * steps > rowTime * ran[f]) {
+                s->forms &= ~(1u << f);
+                again = tile_forms(s) != 0u;
+            }
     }
-    if (tileTime[kHaloNarrow].steps && !(tileTime[kHaloNarrow].step() < other)) forms &= ~(1u << kHaloNarrow);
-    set_forms(s, forms);
+    release();
+    if (rc != VFD_OK) {
+        restore();
+        return rc;
+    }
     s->releaseGraphs();
     if (lanes_out) std::memcpy(lanes_out, s->lanes, std::min<uint32_t>(count, 16));
     return VFD_OK;

@@ -127,6 +127,12 @@ struct __align__(16) HaloTile {
     uint32_t cell0, first, last, scene, staged, list, pad[2];
 };
 
+// What the staged-tile forms would have to do this step: rounds of a block's threads over the
+// tiles, and those of them whose halo outgrows the shared memory.
+struct HaloCounts {
+    uint32_t narrow, narrowRows, wide, wideRows;
+};
+
 // Device pointers and sizes of one simulation; one instance per sort parity
 // (cur = state sorted by the previous step, srt = state sorted by this step).
 struct Dev {
@@ -190,8 +196,9 @@ struct Dev {
     // loops run on, 0 the row kernels.
     // The rows and gradient factors take the place of NG, whose bytes they share.
     uint32_t haloOn;
+    uint32_t formChoice;       // 1: the step's form is yet to be chosen (the search's cells and tile lists)
     HaloTile* haloTiles;
-    uint32_t* haloInfo;        // [0] tiles, [1] list slots handed out
+    uint32_t* haloInfo;        // [0] tiles, [1] list slots handed out, then a HaloCounts
     uint32_t* haloScan;        // tiles before each scan block
     uint2* haloScene;          // per scene: first tile, tiles
     uint32_t* haloList;        // slots of the tiles' halos (at most 8 a particle)

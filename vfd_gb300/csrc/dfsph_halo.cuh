@@ -21,11 +21,11 @@ constexpr uint32_t kHaloThreads = 256u, kHaloWideThreads = 384u;
 constexpr uint32_t kHaloCap = 1408u, kHaloWideCap = 1760u;
 constexpr uint32_t kHaloRow = 96u;                        // row length: kMaxNeighbors rounded up to 32
 
-// Layouts that run on staged tiles. Against the row kernels with four lanes a particle, a step
-// of a viscous drop (graph) took 1374 us against 1184 at 33,000 particles, 1795 against 1732 at
+// Layouts that have staged tiles; each step chooses whether it runs on them (k_tile_form). Against
+// the row kernels with four lanes a particle, a step of a viscous drop (graph) took 1374 us against 1184 at 33,000 particles, 1795 against 1732 at
 // 66,000, 2180 against 2199 at 100,000 and 2705 against 3027 at 260,000; below the line there
-// are too few tiles for the SMs. List places fit 32 bits up to the other. Where the narrow form
-// does not fit, the wide one runs from a line further up: 50 steps to 350 of a viscous dam took
+// are too few tiles for the SMs. List places fit 32 bits up to the other. The wide form is
+// chosen from a line further up: 50 steps to 350 of a viscous dam took
 // 1.7 to 2.2 ms a step against 1.7 to 2.0 by rows at 157,000 particles, 2.5 to 2.8 against 2.5 to 2.6
 // at 262,000, 4.0 to 4.7 against 3.7 to 4.8 at 512,000 and 7.4 to 7.7 against 8.0 to 8.3 at 1M.
 constexpr uint32_t kHaloMinParticles = 100000u, kHaloMaxParticles = 1u << 28, kHaloWideMinParticles = 700000u;
@@ -70,7 +70,7 @@ enum HaloPass {
 };
 void launch_halo_pass(const Dev& d, HaloPass pass, cudaStream_t s);
 void launch_halo_build(const Dev& d, cudaStream_t s);
-void launch_tile_form(const Dev& d, uint32_t otherwise, cudaStream_t s);
+void launch_tile_form(const Dev& d, uint32_t forms, cudaStream_t s);
 cudaError_t prepare_halo_kernels();
 
 }  // namespace vfd

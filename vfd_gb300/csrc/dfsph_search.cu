@@ -183,7 +183,8 @@ __global__ void k_grid(Dev d) {
         }
         total = (uint32_t)min(acc, (uint64_t)0xFFFFFFFFu);
         d.status[2] = total;
-        if (halo_on(d)) d.haloInfo[0] = d.haloInfo[1] = d.status[12] = 0u;
+        if (halo_on(d))
+            for (int k = 0; k < 6; k++) d.haloInfo[k] = 0u;
         if (acc > d.cellCap) {
             atomicOr(d.status, 0x20u);
             atomicExch(d.status + 1, 1u);

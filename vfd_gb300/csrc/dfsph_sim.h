@@ -203,6 +203,7 @@ struct vfd_sim {
     // caller chose lanes, tiles or blocks of the row kernels, else all but those that the
     // autotuner found slower
     uint8_t forms = 1u << vfd::kHaloNarrow | 1u << vfd::kHaloWide;
+    int8_t fixedForm = -1;  // the form that all steps run on (vfd_set_tile_form), or -1
 
     // layout
     bool allocated = false, uploaded = false;
@@ -354,10 +355,10 @@ enum TapePoint {
 };
 void tape_point(const Dev& d, const void* rec, int point, cudaStream_t st);
 
-// The form of the staged tiles for fluid denser than the narrow one holds (0: rows), and whether
-// each step chooses between that and the narrow form from its own search (k_tile_form).
-uint32_t wide_form(const vfd_sim* s);
-bool chooses_form(const vfd_sim* s);
+// The forms of the staged tiles that each step chooses from, beside rows, by its own search
+// (k_tile_form): 1 << form; 0 where the layout has none.
+uint32_t tile_forms(const vfd_sim* s);
+void fix_form(vfd_sim* s, int8_t form);
 // One step as a graph (rec: the adjoint's device tape set, or null) into *gOut / *execOut.
 int build_graph(vfd_sim* s, int parity, const void* rec, cudaGraph_t* gOut, cudaGraphExec_t* execOut);
 // One eagerly launched step (one flag read per solver iteration), optionally recording.

@@ -44,3 +44,25 @@ def test_scenes_step_as_alone(count):
             assert got[key] == info[key], (k, key)
         for a, b in zip(batch.GetState(k)[:2], state):
             assert np.linalg.norm(a - b) <= 1e-6 * max(np.linalg.norm(b), 1e-6), k
+
+
+def test_a_report_does_not_grow_with_the_scenes():
+    """What a step brings back is the status and the first scene: a wait with nothing to do takes as long for
+    4,096 scenes as for 16 (16 us; 210 where all scenes came back, so twice the smaller one leaves room)."""
+    import time
+    s = kinds()[1]
+
+    def wait(count):
+        sim = V.DFSPHSimulation(scenes=[V._abi.make_desc(**s["desc"])] * count)
+        for k in range(count):
+            sim.SetFluidObjects(s["x"], s["v"], scene=k)
+        first = sim.OnUpdate()
+        assert first["IterationCount"] == 1 and sim.GetDebugInfo(count - 1)["IterationCount"] == 1
+        took = []
+        for _ in range(30):
+            t = time.perf_counter()
+            sim.Synchronize()
+            took.append(time.perf_counter() - t)
+        return np.median(took)
+    few, many = wait(16), wait(4096)
+    assert many < 2.0 * few, (few, many)

@@ -223,8 +223,8 @@ struct vfd_sim {
     uint32_t* dStatus = nullptr;
     float *dWM = nullptr, *dGM = nullptr, *dHalton = nullptr;
     uint32_t* hStatus = nullptr;  // pinned
-    vfd::SceneDev* hStage = nullptr;  // pinned: the scenes after a step, on their way to hScenes
-    std::vector<vfd::SceneDev> hScenes;
+    vfd::SceneDev* hStage = nullptr;  // pinned: the first scene after a step, on its way to hScenes
+    std::vector<vfd::SceneDev> hScenes;  // the first as of the last step waited for, the others as last written
     uint32_t maxStPasses = 0;
     bool anyDiv = false, anyVisc = false, anyST = false;
 

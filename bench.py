@@ -660,6 +660,8 @@ def profile_case(args):
         log("lanes", sim.Autotune(1))
     if args.tiles >= 0:
         sim.SetTiles([args.tiles] * len(V.TUNED_KERNELS))
+    if args.tile_form is not None:
+        sim.SetTileForm(args.tile_form)
     sim.Steps(args.graph_steps)
     sim.SetGraphMode(False)
     import torch
@@ -668,7 +670,7 @@ def profile_case(args):
     st = sim.Steps(args.eager_steps)
     torch.cuda.synchronize()
     torch.cuda.profiler.stop()
-    log("particles", len(s["x"]), "stats", st, "tiles", sim.GetTiles())
+    log("particles", len(s["x"]), "stats", st, "tiles", sim.GetTiles(), "tile form", sim.TileForm())
 
 
 def adjoint_profile_case(args):
@@ -795,6 +797,8 @@ def main():
     ap.add_argument("--tiles", type=int, default=-1, help="form of the three solver-loop passes instead of the "
                     "autotuner's choice: 0 = neighbour rows, 1 = rows with gradW recomputed, 3 = 2x2x2 cell tiles, "
                     "4 = 4x2x2 cell tiles")
+    ap.add_argument("--tile-form", type=int, help="form of the staged tiles instead of each step's choice: 0 = rows, "
+                    "1 = narrow, 2 = wide")
     ap.add_argument("--adjoint-profile-case", action="store_true",
                     help="profiling run instead of the benchmark: the adjoint form's run with every kernel launched "
                          "from the host")
@@ -856,6 +860,8 @@ def main():
         lanes = sim.Autotune(2)  # per-kernel lanes per particle and tile sizes, state restored
     if args.tiles >= 0:
         sim.SetTiles([args.tiles] * len(V.TUNED_KERNELS))
+    if args.tile_form is not None:
+        sim.SetTileForm(args.tile_form)
     sim.SetGraphMode(not args.eager)
     sim.Steps(args.warmup)
     stream = torch.cuda.ExternalStream(sim.GetStream())
@@ -962,7 +968,7 @@ def main():
         "config": dict(dam_break_config(args.n_side), launch="eager" if args.eager else "cuda graph per step"),
         "clocks": clocks, "e2e": e2e, "gpu_launches": launches,
         "roofline": roof, "step_roofline": step_roof, "kernel_shares": shares, "lanes_per_particle": lanes,
-        "tile_log2_cells": sim.GetTiles(), "threads_per_block": sim.GetBlocks(),
+        "tile_log2_cells": sim.GetTiles(), "threads_per_block": sim.GetBlocks(), "tile_form": sim.TileForm(),
         "solver": {k: st[k] for k in ("DivergenceSolverIterationCount", "PressureSolverIterationCount",
                                       "ViscositySolverIterationCount", "PressureSolverError", "TimeStepSize",
                                       "MaxNeighborCount", "Flags")},

@@ -388,11 +388,11 @@ int reset_buckets(vfd_sim* s, const Dev& d) {
     return VFD_OK;
 }
 
-// Buffers of the staged-tile passes, for layouts that run on them. Without room for them the
-// row kernels run, as for smaller scenes.
-int allocate_halo(vfd_sim* s, Dev& base) {
+// Buffers of the staged-tile passes, for layouts that run on them. Without room for them, or where
+// their kernels cannot be set up, the row kernels run, as for smaller scenes.
+void allocate_halo(vfd_sim* s, Dev& base) {
     base.haloOn = 0u;
-    if (s->n < kHaloMinParticles || s->n > kHaloMaxParticles) return VFD_OK;
+    if (s->n < kHaloMinParticles || s->n > kHaloMaxParticles) return;
     const size_t st = s->stride, cellTiles = s->cellCap / kHaloTileCells + 1u, kept = s->allocs.size();
     const size_t tiles = std::min(st, cellTiles);
     int rc = dalloc(s, &base.haloTiles, tiles);
@@ -401,17 +401,15 @@ int allocate_halo(vfd_sim* s, Dev& base) {
     if (rc == VFD_OK) rc = dalloc(s, &base.haloScene, base.nscenes);
     if (rc == VFD_OK) rc = dalloc(s, &base.haloList, 8 * st);
     if (rc == VFD_OK) rc = dalloc(s, &base.haloBase, cellTiles * kHaloCells);
-    if (rc != VFD_OK) {
+    if (rc != VFD_OK || prepare_halo_kernels() != cudaSuccess) {
         cudaGetLastError();
         for (; s->allocs.size() > kept; s->allocs.pop_back()) cudaFree(s->allocs.back());
         base.haloTiles = nullptr;
-        return VFD_OK;
+        return;
     }
     static_assert(kHaloRow * (sizeof(float) + sizeof(uint16_t)) == kRow * sizeof(uint2), "the rows share NG's bytes");
     base.haloGrad = reinterpret_cast<float*>(base.NG);
     base.haloRow = reinterpret_cast<uint16_t*>(base.haloGrad + st * kHaloRow);
-    CK(prepare_halo_kernels());
-    return VFD_OK;
 }
 
 int allocate(vfd_sim* s) {
@@ -491,7 +489,7 @@ int allocate(vfd_sim* s) {
     for (const auto& sc : s->scenes) bodyTotal += (uint32_t)sc.bodies.size();
     TRY(dalloc(s, &s->dBodies, std::max<uint32_t>(1u, bodyTotal)));
     TRY(dalloc(s, &s->dStatus, 16));
-    TRY(dalloc(s, &s->dStage, 6 * st));
+    TRY(dalloc(s, &s->dStage, 3 * st));
     TRY(dalloc(s, &s->dStage2, 3 * st));
     TRY(dalloc(s, &base.ACCB, (size_t)base.nscenes * kAccSlots * kBuckets * 16u));
     TRY(dalloc(s, &base.MAXB, (size_t)base.nscenes * 2u * kBuckets * 32u));
@@ -511,18 +509,19 @@ int allocate(vfd_sim* s) {
     std::memcpy(base.blocks, s->blocks, sizeof(base.blocks));
     base.compactRows = uses_tiles(s->tiles) ? 1u : 0u;
     CK(prepare_tile_kernels());
-    TRY(allocate_halo(s, base));
-    s->initValid = false;
-    if (dalloc(s, &s->dInit, 6 * st) != VFD_OK) {  // each reset then copies the start again
-        cudaGetLastError();
-        s->dInit = nullptr;
-    }
     TRY(dalloc(s, &s->dWM, kTableRes));
     TRY(dalloc(s, &s->dGM, kTableRes));
     TRY(dalloc(s, &s->dHalton, kHaltonCount));
     CK(cudaMallocHost(&s->hStatus, 16 * sizeof(uint32_t)));
     std::memset(s->hStatus, 0, 16 * sizeof(uint32_t));
     CK(cudaMallocHost(&s->hStage, sizeof(SceneDev)));
+    // what a layout can do without comes last
+    allocate_halo(s, base);
+    s->initValid = false;
+    if (dalloc(s, &s->dInit, 6 * st) != VFD_OK) {  // each reset then copies the start again
+        cudaGetLastError();
+        s->dInit = nullptr;
+    }
     base.scenes = s->dScenes;
     base.bodies = s->dBodies;
     base.status = s->dStatus;
@@ -1667,7 +1666,8 @@ int vfd_scene_get_state(vfd_sim* s, uint32_t scene, float* x, float* v, float* a
     const Dev& d = s->dev[s->cs];
     const uint32_t b = s->sceneBegin[scene], cnt = s->scenes[scene].count();
     if (cnt && (x || v || a)) {
-        float *const sx = s->dStage, *const sv = s->dStage2, *const sa = s->dStage + 3 * (size_t)s->stride;
+        // (the CG's A p is scratch of a step's loop; it stages the third array)
+        float *const sx = s->dStage, *const sv = s->dStage2, *const sa = reinterpret_cast<float*>(d.CAP);
         k_export_state<<<blocks_for(cnt, 256), 256, 0, s->stream>>>(d, x ? sx : nullptr, v ? sv : nullptr,
                                                                     a ? sa : nullptr, b, cnt);
         const size_t bytes = sizeof(float) * 3 * (size_t)cnt;

@@ -216,7 +216,7 @@ struct vfd_sim {
     float4* XB = nullptr;
     float* dInit = nullptr;      // initial positions, then velocities, 3 floats per slot each; null: no room
     bool initValid = false;      // dInit holds the fluid objects
-    float* dStage = nullptr;     // 6 floats per slot: an array in original order, and another behind it
+    float* dStage = nullptr;     // 3 floats per slot, original order
     float* dStage2 = nullptr;    // a second one (velocities beside positions in vfd_set_state)
     vfd::SceneDev* dScenes = nullptr;
     vfd::BodyDev* dBodies = nullptr;

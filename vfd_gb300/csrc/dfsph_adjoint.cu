@@ -1051,7 +1051,8 @@ struct ShadowKey {
     bool operator==(const ShadowKey& o) const {
         return std::memcmp(&desc, &o.desc, sizeof(desc)) == 0 && std::memcmp(lanes, o.lanes, sizeof(lanes)) == 0 &&
                std::memcmp(tiles, o.tiles, sizeof(tiles)) == 0 && std::memcmp(blocks, o.blocks, sizeof(blocks)) == 0 &&
-               n == o.n && forms == o.forms && fixedForm == o.fixedForm && graphs == o.graphs && analytic == o.analytic && cellCap == o.cellCap;
+               n == o.n && forms == o.forms && fixedForm == o.fixedForm && graphs == o.graphs && analytic == o.analytic &&
+               cellCap == o.cellCap;
     }
 };
 

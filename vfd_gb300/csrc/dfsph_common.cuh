@@ -203,8 +203,8 @@ struct Dev {
     uint2* haloScene;          // per scene: first tile, tiles
     uint32_t* haloList;        // slots of the tiles' halos (at most 8 a particle)
     uint16_t* haloBase;        // [tile of cells][kHaloCells] staged place of each halo cell's first particle
-    uint16_t* haloRow;         // [slot][kHaloRow] staged places of the neighbours (halo_place order)
-    float* haloGrad;           // [slot][kHaloRow] their gradient factors, gradW = haloGrad * r
+    uint16_t* haloRow;         // [slot][kHaloRow] staged places of the neighbours, at halo_row_at
+    float* haloGrad;           // [slot][kHaloRow] their gradient factors, at halo_grad_at: gradW = haloGrad * r
 };
 
 // ---------------------------------------------------------------- float3 math

@@ -1040,19 +1040,19 @@ int fp64_upload(vfd_sim* s) {
     f64::A& a = f->a;
     f64::P& p = f->p;
     if (!keep) {
-    TRY(falloc(f, &a.X, n)); TRY(falloc(f, &a.V, n)); TRY(falloc(f, &a.Acc, n)); TRY(falloc(f, &a.AP, n));
-    TRY(falloc(f, &a.DV, n)); TRY(falloc(f, &a.N, n)); TRY(falloc(f, &a.NS, n));
-    TRY(falloc(f, &a.XB, (size_t)std::max(1u, nb) * n)); TRY(falloc(f, &a.VB, (size_t)std::max(1u, nb) * n));
-    TRY(falloc(f, &a.RHO, n)); TRY(falloc(f, &a.ALPHA, n)); TRY(falloc(f, &a.RHOADV, n)); TRY(falloc(f, &a.KAPPA, n));
-    TRY(falloc(f, &a.KAPPAV, n)); TRY(falloc(f, &a.RES, n)); TRY(falloc(f, &a.CURV, n)); TRY(falloc(f, &a.CURVS, n));
-    TRY(falloc(f, &a.DK, n));
-    TRY(falloc(f, &a.CR, n)); TRY(falloc(f, &a.CP, n)); TRY(falloc(f, &a.CZ, n)); TRY(falloc(f, &a.CT, n));
-    TRY(falloc(f, &a.CB, n)); TRY(falloc(f, &a.CG, n)); TRY(falloc(f, &a.MINV, n));
-    TRY(falloc(f, &a.NCNT, n)); TRY(falloc(f, &a.NBR, (size_t)n * kCap)); TRY(falloc(f, &a.KEY, n));
-    TRY(falloc(f, &a.TMP, n)); TRY(falloc(f, &a.ORDER, n)); TRY(falloc(f, &a.MM, 6));
-    const size_t parts = std::max((n + 63u) / 64u, (uint32_t)(((uint64_t)n * kL + kLB - 1u) / kLB)) + 1u;
-    TRY(falloc(f, &a.PART, parts)); TRY(falloc(f, &a.PART2, parts)); TRY(falloc(f, &a.loop, 1));
-    FCK(cudaMallocHost(&f->hLoop, sizeof(f64::Loop)));
+        TRY(falloc(f, &a.X, n)); TRY(falloc(f, &a.V, n)); TRY(falloc(f, &a.Acc, n)); TRY(falloc(f, &a.AP, n));
+        TRY(falloc(f, &a.DV, n)); TRY(falloc(f, &a.N, n)); TRY(falloc(f, &a.NS, n));
+        TRY(falloc(f, &a.XB, (size_t)std::max(1u, nb) * n)); TRY(falloc(f, &a.VB, (size_t)std::max(1u, nb) * n));
+        TRY(falloc(f, &a.RHO, n)); TRY(falloc(f, &a.ALPHA, n)); TRY(falloc(f, &a.RHOADV, n)); TRY(falloc(f, &a.KAPPA, n));
+        TRY(falloc(f, &a.KAPPAV, n)); TRY(falloc(f, &a.RES, n)); TRY(falloc(f, &a.CURV, n)); TRY(falloc(f, &a.CURVS, n));
+        TRY(falloc(f, &a.DK, n));
+        TRY(falloc(f, &a.CR, n)); TRY(falloc(f, &a.CP, n)); TRY(falloc(f, &a.CZ, n)); TRY(falloc(f, &a.CT, n));
+        TRY(falloc(f, &a.CB, n)); TRY(falloc(f, &a.CG, n)); TRY(falloc(f, &a.MINV, n));
+        TRY(falloc(f, &a.NCNT, n)); TRY(falloc(f, &a.NBR, (size_t)n * kCap)); TRY(falloc(f, &a.KEY, n));
+        TRY(falloc(f, &a.TMP, n)); TRY(falloc(f, &a.ORDER, n)); TRY(falloc(f, &a.MM, 6));
+        const size_t parts = std::max((n + 63u) / 64u, (uint32_t)(((uint64_t)n * kL + kLB - 1u) / kLB)) + 1u;
+        TRY(falloc(f, &a.PART, parts)); TRY(falloc(f, &a.PART2, parts)); TRY(falloc(f, &a.loop, 1));
+        FCK(cudaMallocHost(&f->hLoop, sizeof(f64::Loop)));
     }
     // SPH tables in double (PrecomputedDFSPHCubicKernel::SetRadius, Kernel/DFSPHKernels.h:13-41)
     const double r = (double)sc.desc.ParticleRadius, h = 4.0 * r, pi = 3.14159265358979323846;
@@ -1077,28 +1077,28 @@ int fp64_upload(vfd_sim* s) {
         return v / x;
     };
     if (!keep) {
-    std::vector<double> W(kTableRes), G(kTableRes + 1), WM(kTableRes), GM(kTableRes);
-    for (uint32_t k = 0; k < kTableRes; k++) {
-        const double x = step * (double)k;
-        W[k] = calcW(x);
-        G[k] = x > 1.0e-9 ? calcG(x) : 0.0;
-    }
-    G[kTableRes] = 0.0;
-    for (uint32_t k = 0; k + 1 < kTableRes; k++) {
-        WM[k] = 0.5 * (W[k] + W[k + 1]);
-        GM[k] = 0.5 * (G[k] + G[k + 1]);
-    }
-    WM[kTableRes - 1] = GM[kTableRes - 1] = 0.0;
-    double *dW = nullptr, *dG = nullptr;
-    TRY(falloc(f, &dW, kTableRes));
-    TRY(falloc(f, &dG, kTableRes));
-    FCK(cudaMemcpy(dW, WM.data(), sizeof(double) * kTableRes, cudaMemcpyHostToDevice));
-    FCK(cudaMemcpy(dG, GM.data(), sizeof(double) * kTableRes, cudaMemcpyHostToDevice));
-    a.W = dW;
-    a.G = dG;
-    f->n = n;
-    f->bodies = nb;
-    f->radius = r;
+        std::vector<double> W(kTableRes), G(kTableRes + 1), WM(kTableRes), GM(kTableRes);
+        for (uint32_t k = 0; k < kTableRes; k++) {
+            const double x = step * (double)k;
+            W[k] = calcW(x);
+            G[k] = x > 1.0e-9 ? calcG(x) : 0.0;
+        }
+        G[kTableRes] = 0.0;
+        for (uint32_t k = 0; k + 1 < kTableRes; k++) {
+            WM[k] = 0.5 * (W[k] + W[k + 1]);
+            GM[k] = 0.5 * (G[k] + G[k + 1]);
+        }
+        WM[kTableRes - 1] = GM[kTableRes - 1] = 0.0;
+        double *dW = nullptr, *dG = nullptr;
+        TRY(falloc(f, &dW, kTableRes));
+        TRY(falloc(f, &dG, kTableRes));
+        FCK(cudaMemcpy(dW, WM.data(), sizeof(double) * kTableRes, cudaMemcpyHostToDevice));
+        FCK(cudaMemcpy(dG, GM.data(), sizeof(double) * kTableRes, cudaMemcpyHostToDevice));
+        a.W = dW;
+        a.G = dG;
+        f->n = n;
+        f->bodies = nb;
+        f->radius = r;
     }
     f->keep_pairs();
     p.wZero = calcW(0.0);

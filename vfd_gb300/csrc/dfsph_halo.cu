@@ -240,17 +240,6 @@ __device__ __forceinline__ void halo_fetch(const Dev& d, const HaloTile& T, cons
     }
 }
 
-// What a pass supplies (static members of Op):
-//   kField, kGrad          staged field; whether the pass reads or writes the gradient factors
-//   kTerms, slots()        reduction terms of finish() and their accumulators
-//   kLoop                  solver loop whose active scenes it walks, or -1
-//   active(S)              whether scene S runs the pass
-//   field(d)               the staged array (float4 or float)
-//   Own, load()            the particle's own data
-//   pair(d, o, xq, fq, gs, ok, acc)  one neighbour's term, added when ok (gs written by a
-//                          kWriteGrad pass)
-//   Acc, sum()             the pair sums and their fold over the particle's lanes
-//   finish(d, p, S, o, acc, ncnt, term)  lane 0: writes the outputs, sets the terms
 // Eight row entries: staged places and gradient factors.
 struct HaloEntries {
     uint4 e;
@@ -265,6 +254,17 @@ __device__ __forceinline__ void halo_entries(const Dev& d, uint32_t p, uint32_t 
     }
 }
 
+// A pass over the tiles, a thread a particle. What it supplies (static members of Op):
+//   kField, kGrad          staged field; whether the pass reads or writes the gradient factors
+//   kTerms, slots()        reduction terms of finish() and their accumulators
+//   kLoop                  solver loop whose active scenes it walks, or -1
+//   active(S)              whether scene S runs the pass
+//   field(d)               the staged array (float4 or float)
+//   Own, load()            the particle's own data
+//   pair(d, o, xq, fq, gs, ok, acc)  one neighbour's term, added when ok (gs written by a
+//                          kWriteGrad pass)
+//   Acc                    the pair sums: eight a thread, added with += as the rows' lanes meet
+//   finish(d, p, S, o, acc, ncnt, term)  writes the outputs, sets the terms
 template <class Op, bool WIDE>
 __device__ __forceinline__ void halo_pass(const Dev& d) {
     using Shape = HaloShape<Op, WIDE>;

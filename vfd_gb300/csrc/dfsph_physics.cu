@@ -134,9 +134,9 @@ constexpr uint32_t kUnroll = 4u;
 // not wait for the count (rows have 72 slots, entries past the count are masked), so
 // the count, the indices and the particle's own fields are fetched together; within a
 // round the U gathers per lane are independent. Masked entries use the particle itself
-// as a stand-in index. f also gets the entry's place u among the round's (LaneSums). The row and gradient streams are read once per pass, so they
-// are loaded with the evict-first hint (ld.global.cs) to leave L2 to the gathered
-// fields.
+// as a stand-in index. f also gets the entry's place u among the round's (LaneSums). The row
+// and gradient streams are read once per pass, so they are loaded with the evict-first hint
+// (ld.global.cs) to leave L2 to the gathered fields.
 template <uint32_t G, bool WITH_GS, class F>
 __device__ __forceinline__ void for_neighbors(const Group<G>& grp, const Nbr& nb, uint32_t self, F&& f) {
     constexpr uint32_t U = kUnroll;

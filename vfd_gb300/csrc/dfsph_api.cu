@@ -818,11 +818,11 @@ static cudaError_t add_step_by_form(vfd_sim* s, Dev d, const void* rec, cudaGrap
     e = add_segment(s->stream, g, leaves, [&](cudaStream_t st) {
         Dev c = d;
         c.haloOn = kHaloNarrow;
-        c.formChoice = 1u;
+        c.formChoice = forms;
         c.formHandle = (unsigned long long)h;
         if (rec) tape_point(d, rec, kTapeBegin, st);
         launch_search_cells(c, st);
-        launch_tile_form(c, forms, st);
+        launch_tile_form(c, st);
     });
     if (e != cudaSuccess) return e;
     cudaGraphNodeParams np = {cudaGraphNodeTypeConditional};
@@ -888,9 +888,9 @@ int launch_eager(vfd_sim* s, const void* rec) {
         if (tile_forms(s)) {  // as in the step's graph
             Dev c = d;
             c.haloOn = kHaloNarrow;
-            c.formChoice = 1u;
+            c.formChoice = tile_forms(s);
             launch_search_cells(c, st);
-            launch_tile_form(c, tile_forms(s), st);
+            launch_tile_form(c, st);
             TRY(read_flag(s, 14, d.haloOn));
             launch_search_rows(d, st);
         } else {

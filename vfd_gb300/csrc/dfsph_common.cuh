@@ -196,7 +196,7 @@ struct Dev {
     // loops run on, 0 the row kernels.
     // The rows and gradient factors take the place of NG, whose bytes they share.
     uint32_t haloOn;
-    uint32_t formChoice;       // 1: the step's form is yet to be chosen (the search's cells and tile lists)
+    uint32_t formChoice;       // forms that the step is yet to choose from (1 << form), in its search's cells and tile lists
     HaloTile* haloTiles;
     uint32_t* haloInfo;        // [0] tiles, [1] list slots handed out, then a HaloCounts
     uint32_t* haloScan;        // tiles before each scan block

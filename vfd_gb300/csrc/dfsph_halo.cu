@@ -56,6 +56,17 @@ __device__ __forceinline__ float narrow_cost(const Dev& d, uint32_t tiles, uint3
 __device__ __forceinline__ float wide_cost(const Dev& d, uint32_t tiles, uint32_t rounds, uint32_t rows) {
     return rounds_cost(d, tiles, rounds, 3u, 170.0f, rows, 250000.0f, 900.0f);
 }
+// Of the allowed forms (bit 1 << form; rows always).
+__device__ __forceinline__ uint32_t cheapest_form(const Dev& d, uint32_t tiles, uint32_t narrow, uint32_t narrowRows,
+                                                  uint32_t wide, uint32_t wideRows, uint32_t forms) {
+    if (tiles == 0u) return 0u;
+    const float n = narrow_cost(d, tiles, narrow, narrowRows), w = wide_cost(d, tiles, wide, wideRows);
+    uint32_t form = 0u;
+    float best = (float)d.n;
+    if ((forms >> kHaloNarrow & 1u) && n < best) form = kHaloNarrow, best = n;
+    if ((forms >> kHaloWide & 1u) && w < best) form = kHaloWide;
+    return form;
+}
 
 // One block per tile: its halo's slots into haloList and the staged place of each halo
 // cell's first particle into haloBase. The list space is handed out in any order (the lists'
@@ -66,9 +77,10 @@ __global__ void __launch_bounds__(256) k_halo_build(Dev d) {
     __shared__ uint32_t warpSum[8], base[kHaloCells], start[kHaloCells], offset;
     const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
     const uint32_t nt = d.haloInfo[0];
-    // a round for every tile, the least: where rows are cheaper than that, nothing is listed
-    if (d.formChoice && fminf(narrow_cost(d, nt, nt, 0u), wide_cost(d, nt, nt, 0u)) >= (float)d.n) return;
-    HaloCounts mine = {};  // in thread 0
+    // where rows are cheaper than either form with all halos staged, nothing is listed
+    HaloCounts* all = halo_counts(d);
+    if (d.formChoice && cheapest_form(d, nt, all->narrow, 0u, all->wide, 0u, d.formChoice) == 0u) return;
+    uint32_t narrowRows = 0u, wideRows = 0u;  // in thread 0: rounds over tiles that outgrow the shared memory
     for (uint32_t t = blockIdx.x; t < nt; t += gridDim.x) {
         HaloTile& T = d.haloTiles[t];
         const SceneDev& S = d.scenes[T.scene];
@@ -111,13 +123,8 @@ __global__ void __launch_bounds__(256) k_halo_build(Dev d) {
             offset = fits ? at : 0xFFFFFFFFu;
             T.list = at;
             T.staged = total;
-            const uint32_t count = T.last - T.first;
-            const uint32_t narrow = (count + kHaloThreads - 1u) / kHaloThreads;
-            const uint32_t wide = (count + kHaloWideThreads - 1u) / kHaloWideThreads;
-            mine.narrow += narrow;
-            mine.wide += wide;
-            if (total > kHaloCap) mine.narrowRows += narrow;
-            if (total > kHaloWideCap) mine.wideRows += wide;
+            if (total > kHaloCap) narrowRows += halo_rounds(T.last - T.first, kHaloThreads);
+            if (total > kHaloWideCap) wideRows += halo_rounds(T.last - T.first, kHaloWideThreads);
         }
         __syncthreads();
         if (offset != 0xFFFFFFFFu)
@@ -130,31 +137,22 @@ __global__ void __launch_bounds__(256) k_halo_build(Dev d) {
             }
         __syncthreads();
     }
-    if (threadIdx.x == 0 && mine.narrow > 0u) {
-        HaloCounts* all = reinterpret_cast<HaloCounts*>(d.haloInfo + 2);
-        atomicAdd(&all->narrow, mine.narrow);
-        atomicAdd(&all->wide, mine.wide);
-        if (mine.narrowRows) atomicAdd(&all->narrowRows, mine.narrowRows);
-        if (mine.wideRows) atomicAdd(&all->wideRows, mine.wideRows);
+    if (threadIdx.x == 0) {
+        if (narrowRows) atomicAdd(&all->narrowRows, narrowRows);
+        if (wideRows) atomicAdd(&all->wideRows, wideRows);
     }
 }
 
-// The form that this step runs on, of those allowed (bit 1 << form; rows always).
-__global__ void k_tile_form(Dev d, uint32_t forms) {
+// The form that this step runs on, of Dev::formChoice and rows.
+__global__ void k_tile_form(Dev d) {
     VFD_COUNT_LAUNCH(d);
-    const HaloCounts c = *reinterpret_cast<const HaloCounts*>(d.haloInfo + 2);
-    uint32_t form = 0u;
-    if (c.narrow > 0u && !is_aborted(d)) {
-        const uint32_t tiles = d.haloInfo[0];
-        const float narrow = narrow_cost(d, tiles, c.narrow, c.narrowRows), wide = wide_cost(d, tiles, c.wide, c.wideRows);
-        float best = (float)d.n;
-        if ((forms >> kHaloNarrow & 1u) && narrow < best) form = kHaloNarrow, best = narrow;
-        if ((forms >> kHaloWide & 1u) && wide < best) form = kHaloWide;
-    }
+    const HaloCounts c = *halo_counts(d);
+    const uint32_t form =
+        is_aborted(d) ? 0u : cheapest_form(d, d.haloInfo[0], c.narrow, c.narrowRows, c.wide, c.wideRows, d.formChoice);
     d.status[14] = form;
     // the graph's branches: rows, then the allowed forms
     if (d.formHandle)
-        cudaGraphSetConditional((cudaGraphConditionalHandle)d.formHandle, form ? __popc(forms & ((2u << form) - 1u)) : 0u);
+        cudaGraphSetConditional((cudaGraphConditionalHandle)d.formHandle, form ? __popc(d.formChoice & ((2u << form) - 1u)) : 0u);
 }
 
 // ---------------------------------------------------------------- the tile loop
@@ -681,8 +679,8 @@ void launch_halo_pass(const Dev& d, HaloPass pass, cudaStream_t s) {
 void launch_halo_build(const Dev& d, cudaStream_t s) {
     VFD_LAUNCH("k_halo_build", s, k_halo_build<<<d.batchBlocks / 2u, 256, 0, s>>>(d));
 }
-void launch_tile_form(const Dev& d, uint32_t forms, cudaStream_t s) {
-    VFD_LAUNCH("k_tile_form", s, k_tile_form<<<1, 1, 0, s>>>(d, forms));
+void launch_tile_form(const Dev& d, cudaStream_t s) {
+    VFD_LAUNCH("k_tile_form", s, k_tile_form<<<1, 1, 0, s>>>(d));
 }
 
 }  // namespace vfd

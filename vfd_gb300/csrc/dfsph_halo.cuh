@@ -19,6 +19,11 @@ constexpr uint32_t kHaloX = (1u << ((kHaloLog2 + 2u) / 3u)) + 2u, kHaloY = (1u <
 constexpr uint32_t kHaloNarrow = 1u, kHaloWide = 2u;
 constexpr uint32_t kHaloThreads = 256u, kHaloWideThreads = 384u;
 constexpr uint32_t kHaloCap = 1408u, kHaloWideCap = 1760u;
+// Rounds of a block's threads over a tile's particles.
+__device__ __forceinline__ uint32_t halo_rounds(uint32_t particles, uint32_t threads) {
+    return (particles + threads - 1u) / threads;
+}
+__device__ __forceinline__ HaloCounts* halo_counts(const Dev& d) { return reinterpret_cast<HaloCounts*>(d.haloInfo + 2); }
 constexpr uint32_t kHaloRow = 96u;                        // row length: kMaxNeighbors rounded up to 32
 
 // Layouts that have staged tiles; each step chooses whether it runs on them (k_tile_form). Against
@@ -70,7 +75,7 @@ enum HaloPass {
 };
 void launch_halo_pass(const Dev& d, HaloPass pass, cudaStream_t s);
 void launch_halo_build(const Dev& d, cudaStream_t s);
-void launch_tile_form(const Dev& d, uint32_t forms, cudaStream_t s);
+void launch_tile_form(const Dev& d, cudaStream_t s);
 cudaError_t prepare_halo_kernels();
 
 }  // namespace vfd

@@ -353,8 +353,9 @@ __global__ void __launch_bounds__(256) k_scan_down(Dev d) {
         mine += full;
         if (k < (lane & ~(kTileLanes - 1u))) before += full;
     }
-    __shared__ uint32_t wt[8];
+    __shared__ uint32_t wt[8], rounds[2];  // of a block's threads over the tiles, narrow and wide
     if (lane == 0) wt[warp] = mine;
+    if (threadIdx.x < 2u) rounds[threadIdx.x] = 0u;
     __syncthreads();
     for (uint32_t w = 0; w < warp; w++) before += wt[w];
     if (lane % kTileLanes == 0u && (filled & mask)) {
@@ -367,6 +368,14 @@ __global__ void __launch_bounds__(256) k_scan_down(Dev d) {
         d.haloTiles[at] = T;
         atomicMin(&d.haloScene[T.scene].x, at);
         atomicAdd(&d.haloScene[T.scene].y, 1u);
+        atomicAdd(&rounds[0], halo_rounds(inTile, kHaloThreads));
+        atomicAdd(&rounds[1], halo_rounds(inTile, kHaloWideThreads));
+    }
+    __syncthreads();
+    if (threadIdx.x == 0 && rounds[0] > 0u) {
+        HaloCounts* all = halo_counts(d);
+        atomicAdd(&all->narrow, rounds[0]);
+        atomicAdd(&all->wide, rounds[1]);
     }
 }
 

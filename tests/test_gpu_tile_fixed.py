@@ -59,23 +59,29 @@ def test_analytic_kernel(form, squeeze):
     H.assert_like_rows(make)
 
 
-@FORMS
-def test_recorded_steps(form):
-    """Gradients of two recorded steps and their replay, on the analytic kernel with a fixed step length: the
-    recorded states agree with the rows' to 1e-6 (test_gpu_halo.py), and a gradient is a smooth function
-    of them here, so a bound of 1e-4 of its norm leaves a factor of a hundred."""
-    s = H.block_scene((47, 47, 47), 0.0)
-    s = dict(s, desc=dict(s["desc"], MaxTimeStepSize=1e-4, TimeStepSize=1e-4, MaxPressureSolverIterations=5,
-                          MaxDivergenceSolverIterations=5, MaxViscositySolverIterations=5))
+@pytest.mark.parametrize("counts,form,squeeze", [
+    ((47, 47, 47), 1, 1.0), ((47, 47, 47), 2, 1.0), ((64, 64, 64), -1, 1.0), ((47, 47, 47), -1, 0.9)])
+@pytest.mark.parametrize("graphs", [True, False])
+def test_recorded_steps(counts, form, squeeze, graphs):
+    """Gradients of two recorded steps and their replay, on the analytic kernel with a fixed step length, on a fixed
+    form and on the one that the steps choose (narrow tiles; rows): the recorded states agree with the
+    rows' to 1e-6 (test_gpu_halo.py), and a gradient is a smooth function of them here, so a bound of
+    1e-4 of its norm leaves a factor of a hundred."""
+    s = H.block_scene(counts, 0.0)
+    s = dict(s, x=s["x"] * np.float32(squeeze),
+             desc=dict(s["desc"], MaxTimeStepSize=1e-4, TimeStepSize=1e-4, MaxPressureSolverIterations=5,
+                       MaxDivergenceSolverIterations=5, MaxViscositySolverIterations=5))
     rng = np.random.default_rng(4)
     bars = [rng.normal(0, 1, s["x"].shape).astype(np.float32) / len(s["x"]) for _ in range(2)]
     got = []
     for f in (form, 0):
         sim = V.scene_simulation(s)
         sim.SetKernelMode(True)
+        sim.SetGraphMode(graphs)
         sim.SetTileForm(f)
         sim.AdjointForward(2, 1)
         got.append(sim.GetState()[:2] + tuple(sim.AdjointBackward(*bars)[:2]))
+        assert sim.GetGraphMode() == (graphs, graphs)
     for a, b in zip(*got):
         assert np.isfinite(a).all()
         assert np.linalg.norm(a - b) <= 1e-4 * np.linalg.norm(b)

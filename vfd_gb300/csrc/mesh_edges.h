@@ -24,30 +24,27 @@ inline std::vector<int64_t> opposite_faces(const uint32_t* tri, uint32_t nv, uin
     auto target = [&](uint32_t e) { return tri[3 * (e / 3) + (e % 3 + 1) % 3]; };
     std::vector<int64_t> opp(ne, -1);
     std::vector<uint32_t> head(nv, kNone), tail(nv, kNone), next(ne, kNone);
-    auto pair = [&](uint32_t e, uint32_t o) {
-        opp[e] = o / 3;
-        opp[o] = e / 3;
-    };
     uint64_t left = kWalk * ne;
-    uint32_t e = 0;
-    for (; e < ne; e++) {
-        const uint32_t u = tri[e], v = target(e);
-        uint32_t before = kNone, o = head[v];
-        for (; o != kNone && target(o) != u && left > 0; left--) {
-            before = o;
-            o = next[o];
+    for (uint32_t f = 0; f < nf && left > 0; f++)
+        for (uint32_t k = 0; k < 3; k++) {
+            const uint32_t e = 3 * f + k, u = tri[e], v = tri[3 * f + (k + 1) % 3];
+            uint32_t before = kNone, o = head[v];
+            for (; o != kNone && target(o) != u && left > 0; left--) {
+                before = o;
+                o = next[o];
+            }
+            if (left == 0) break;
+            if (o != kNone) {
+                opp[e] = o / 3;
+                opp[o] = f;
+                (before == kNone ? head[v] : next[before]) = next[o];
+                if (tail[v] == o) tail[v] = before;
+            } else {
+                (tail[u] == kNone ? head[u] : next[tail[u]]) = e;
+                tail[u] = e;
+            }
         }
-        if (left == 0) break;
-        if (o != kNone) {
-            pair(e, o);
-            (before == kNone ? head[v] : next[before]) = next[o];
-            if (tail[v] == o) tail[v] = before;
-        } else {
-            (tail[u] == kNone ? head[u] : next[tail[u]]) = e;
-            tail[u] = e;
-        }
-    }
-    if (e == ne) return opp;
+    if (left > 0) return opp;
 
     // an edge's slot: its first half-edge names it, then its unpaired ones in order
     struct Slot {
@@ -65,12 +62,13 @@ inline std::vector<int64_t> opposite_faces(const uint32_t* tri, uint32_t nv, uin
         }
     };
     std::fill(opp.begin(), opp.end(), -1);
-    for (e = 0; e < ne; e++) {
+    for (uint32_t e = 0; e < ne; e++) {
         const uint32_t u = tri[e], v = target(e);
         Slot& other = find(v, u);
         if (other.name != kNone && other.head != kNone) {
             const uint32_t o = other.head;
-            pair(e, o);
+            opp[e] = o / 3;
+            opp[o] = e / 3;
             other.head = next[o];
             if (other.head == kNone) other.tail = kNone;
         } else {

@@ -690,7 +690,8 @@ int upload(vfd_sim* s) {
         s->anyST |= sc.desc.EnableSurfaceTensionSolver != 0;
     }
     if (fresh && s->n) {
-        // one copy for all scenes, packed in slot order (with copies for each, a reset of 4,096 scenes took 60 ms, so 1.3)
+        // one copy for all scenes, packed in slot order (a reset of 4,096 scenes 1.3 ms, with copies for
+        // each 60)
         const bool one = s->scenes.size() == 1;
         std::vector<float> packed(one ? 0 : 3 * (size_t)s->n);
         auto put = [&](float* dst, std::vector<float> SceneHost::*field) -> cudaError_t {
